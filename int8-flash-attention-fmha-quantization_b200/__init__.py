@@ -5,14 +5,18 @@ This module is the Python mirror of the reference's C++ host interface (inc/fmha
 inc/fmha_param_i8.h:3-17): the same names (`FMHAInferI8`, `FMHAParamI8`, `AttnDataDescriptor`), the
 same argument order and meaning.  It binds the C ABI of libfmha_i8_sm100.so (include/fmha_i8_c.h)
 with ctypes; there is no other implementation behind it: if the library is missing the import
-fails, and every call needs a B200.
+fails, and every call needs a B200.  The calls of a serving loop go through a small native module
+(csrc/py_binding.cpp) that reads the arguments and calls the same C ABI.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 from dataclasses import dataclass
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libfmha_i8_sm100.so")
+BINDING_PATH = os.path.join(HERE, "_fmha_i8_py.so")
 
 OK = 0
 ERR_NULL_POINTER = -1
@@ -119,6 +123,35 @@ def lib():
     return _lib
 
 
+_binding = None
+
+
+def _native():
+    """The native binding of the calls below (it is linked against the library that lib() opens)."""
+    global _binding
+    if _binding is None:
+        lib()
+        if not os.path.exists(BINDING_PATH):
+            raise ImportError(f"{BINDING_PATH} is missing: build it with `python {os.path.join(HERE, 'build.py')}`")
+        loader = importlib.machinery.ExtensionFileLoader("_fmha_i8_py", BINDING_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fmha_i8_py", loader))
+        loader.exec_module(mod)
+        mod.set_stream_source(_current_stream)
+        _binding = mod
+    return _binding
+
+
+def _current_stream():
+    """Handle of torch's current stream.  The first call initialises torch's CUDA state; from then on the binding asks
+    torch's raw getters itself (0.2 us a call instead of 3.6)."""
+    import torch
+    handle = torch.cuda.current_stream().cuda_stream
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is not None and device is not None:
+        _binding.set_raw_stream(raw, device)
+    return handle
+
+
 def status_string(status):
     return lib().fmha_i8_sm100_status_string(int(status)).decode()
 
@@ -156,8 +189,7 @@ def FMHAInferI8(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, use_tcu
     Enqueues on `stream` (None = torch's current stream) and returns the status without
     synchronising.  With check=True a non-zero status raises FmhaError (the reference returns void
     and silently does nothing on unsupported input)."""
-    st = lib().fmha_i8_sm100_infer(_stream_handle(stream), fmha_param.as_c(), attn_desc.as_c(), _ptr(q), _ptr(k),
-                                   _ptr(v), _ptr(padding_mask), _ptr(o), _flags(use_tcu, uint8_p))
+    st = (_binding or _native()).infer(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, _flags(use_tcu, uint8_p))
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8")
     return st
@@ -167,11 +199,8 @@ def FMHAInferI8Cross(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, 
                      use_tcu=True, check=True, uint8_p=False):
     """Query rows and keys differ in number: q, o int8 [B,H,Sq,D]; k, v int8 [B,H,Sk,D]; padding_mask int8
     [B,Sk].  attn_desc_x is an AttnDataDescriptorX.  bh_begin/bh_count select heads as in FMHAInferI8Slice."""
-    if bh_count is None:
-        bh_count = attn_desc_x.batch_num * attn_desc_x.head_num - bh_begin
-    st = lib().fmha_i8_sm100_infer_cross(_stream_handle(stream), fmha_param.as_c(), attn_desc_x.as_c(), _ptr(q), _ptr(k),
-                                         _ptr(v), _ptr(padding_mask), _ptr(o), int(bh_begin), int(bh_count),
-                                         _flags(use_tcu, uint8_p))
+    st = (_binding or _native()).infer_cross(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, bh_begin, bh_count,
+                                             _flags(use_tcu, uint8_p))
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8Cross")
     return st
@@ -185,11 +214,8 @@ def FMHAInferI8Policy(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o,
     """Whole-row scaling policies for the 8-bit P (reference fmha_i8_quant_deviation.py:57-121): POLICY_ROW = per-row
     ("dynamic") scale, POLICY_STATIC = one calibrated scale fmha_param.s_max for all rows, POLICY_TILE = the reference
     kernel's tile-local scale.  row_scratch: float32 device tensor with 2 elements per query row of the slice."""
-    if bh_count is None:
-        bh_count = attn_desc_x.batch_num * attn_desc_x.head_num - bh_begin
-    st = lib().fmha_i8_sm100_infer_policy(_stream_handle(stream), fmha_param.as_c(), attn_desc_x.as_c(), _ptr(q), _ptr(k), _ptr(v),
-                                          _ptr(padding_mask), _ptr(o), int(bh_begin), int(bh_count), _flags(True, False),
-                                          int(policy), _ptr(row_scratch))
+    st = (_binding or _native()).infer_policy(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, bh_begin, bh_count,
+                                              FLAG_USE_TCU, policy, row_scratch)
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8Policy")
     return st
@@ -207,8 +233,8 @@ def calibrate_o_amax(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o_a
 
 def FMHAInferI8Slice(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, bh_begin, bh_count, check=True, uint8_p=False):
     """Heads [bh_begin, bh_begin+bh_count) of the flattened batch*head axis; q,k,v,o hold only the slice."""
-    st = lib().fmha_i8_sm100_infer_slice(_stream_handle(stream), fmha_param.as_c(), attn_desc.as_c(), _ptr(q), _ptr(k),
-                                         _ptr(v), _ptr(padding_mask), _ptr(o), int(bh_begin), int(bh_count), _flags(True, uint8_p))
+    st = (_binding or _native()).infer_slice(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, bh_begin, bh_count,
+                                             _flags(True, uint8_p))
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8Slice")
     return st
@@ -216,8 +242,8 @@ def FMHAInferI8Slice(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, bh
 
 def FMHAInferI8Host(fmha_param, attn_desc, host_q, host_k, host_v, host_mask, host_o, check=True, uint8_p=False):
     """Host buffers in, host buffer out (copies inside); synchronous."""
-    st = lib().fmha_i8_sm100_infer_host(fmha_param.as_c(), attn_desc.as_c(), _ptr(host_q), _ptr(host_k), _ptr(host_v),
-                                        _ptr(host_mask), _ptr(host_o), _flags(True, uint8_p))
+    st = (_binding or _native()).infer_host(fmha_param, attn_desc, host_q, host_k, host_v, host_mask, host_o, None, None,
+                                            _flags(True, uint8_p))
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8Host")
     return st
@@ -226,8 +252,8 @@ def FMHAInferI8Host(fmha_param, attn_desc, host_q, host_k, host_v, host_mask, ho
 def FMHAInferI8HostSlice(fmha_param, attn_desc, host_q, host_k, host_v, host_mask, host_o, bh_begin, bh_count,
                          check=True, uint8_p=False):
     """Host buffers of heads [bh_begin, bh_begin+bh_count) in, host buffer of those heads out; the mask is whole."""
-    st = lib().fmha_i8_sm100_infer_host_slice(fmha_param.as_c(), attn_desc.as_c(), _ptr(host_q), _ptr(host_k), _ptr(host_v),
-                                              _ptr(host_mask), _ptr(host_o), int(bh_begin), int(bh_count), _flags(True, uint8_p))
+    st = (_binding or _native()).infer_host(fmha_param, attn_desc, host_q, host_k, host_v, host_mask, host_o, bh_begin, bh_count,
+                                            _flags(True, uint8_p))
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8HostSlice")
     return st
@@ -271,8 +297,10 @@ def quantize_f32(stream, x, out, amax_out=None, n=None, entry="fmha_i8_sm100_qua
     amax written to the one-element device tensor `amax_out`.  Enqueues on `stream`, no synchronisation.
     entry="fmha_i8_sm100_quantize_f32_noalloc" selects the variant that never allocates device memory
     (built-in scratch, at most 268,435,456 elements, calls on one device must not overlap)."""
-    count = int(n if n is not None else x.numel())
-    st = getattr(lib(), entry)(_stream_handle(stream), _ptr(x), count, _ptr(out), _ptr(amax_out))
+    if entry not in ("fmha_i8_sm100_quantize_f32", "fmha_i8_sm100_quantize_f32_noalloc"):
+        raise AttributeError(entry)
+    st = (_binding or _native()).quantize(stream, x, int(n if n is not None else x.numel()), out, amax_out,
+                                          entry == "fmha_i8_sm100_quantize_f32_noalloc")
     if st != OK:
         raise FmhaError(st, entry)
 
