@@ -935,6 +935,9 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const uint32_t k_smem = q_smem + NQ * Cfg::kTileBytes;
   const uint32_t v_smem = k_smem + NK * Cfg::kTileBytes;
 
+  // The next launch of the stream may set itself up (barriers, tensor memory, constant operands: about 1.5 us with the
+  // launch latency) on SMs this one leaves free, and waits below for this one to finish before it reads anything.
+  grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_tiles = (p.S + kTile - 1) / kTile;
   const int first_unit = blockIdx.x, unit_step = gridDim.x;
@@ -981,6 +984,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&ctl->tmem_base);
   volatile int* abort_flag = &ctl->abort;
+  grid_dependency_wait();      // nothing above touches global memory
 
   // Every role walks the same unit sequence: `it` counts this CTA's units, info buffer = it % kInfoBufs,
   // phase of an info barrier = (it / kInfoBufs) & 1; `g` counts its steps (live key tiles) across units.

@@ -122,6 +122,14 @@ __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&r)[8]) 
                : "memory");
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// Blocks until every kernel before this one in the stream has finished and its writes are visible.  With the launch
+// attribute that allows it, a kernel starts before that: what precedes this instruction must not touch global memory
+// that an earlier kernel may write or still read.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream start (up to its own grid_dependency_wait) once all CTAs have executed this.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
