@@ -246,7 +246,7 @@ def run_quantize_bench(args, pkg, w, dev, rank, world):
                           "data": "synthetic", "config": {"workload": f"quantize one {w.name} tensor: {n} elements", "l2": "input larger than L2"},
                           "gpu_launches": pkg.launch_count() - l0,
                           "roofline": {"bound": "hbm", "achieved": gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"],
-                                       "traffic": None, "kernel": "quant_absmax_kernel + quant_apply_kernel"}}), flush=True)
+                                       "traffic": None, "kernel": "quant_grid_kernel"}}), flush=True)
 
 
 # ------------------------------------------------------------------------------------------------ timing helpers

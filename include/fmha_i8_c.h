@@ -58,7 +58,8 @@ enum {
   FMHA_I8_DEV_WAIT_O_READY = 8,    /* softmax waiting for P.V */
   FMHA_I8_DEV_WAIT_O_FREE = 9,     /* MMA issuer waiting for the previous P.V to be drained */
   FMHA_I8_DEV_WAIT_DEBUG = 10,     /* a wait inside a debug kernel */
-  FMHA_I8_DEV_WAIT_INFO = 11       /* a role waiting for (or the scanner waiting to reuse) a unit's mask information */
+  FMHA_I8_DEV_WAIT_INFO = 11,      /* a role waiting for (or the scanner waiting to reuse) a unit's mask information */
+  FMHA_I8_DEV_WAIT_QUANT = 12      /* quantiser: a tile of the tensor, or the other CTAs' maxima */
 };
 
 #define FMHA_I8_FLAG_USE_TCU 1u    /* mirrors the reference's use_tcu argument; must be set */
@@ -177,25 +178,16 @@ int fmha_i8_sm100_debug_wait_probe(void* stream, long long limit_cycles);
  * amax = max|x| (abs_max, inc/utils.hpp:31-39) and q[i] = clamp(floor(x[i]*127/amax + 0.5), -127, 127)
  * (float_quant2_int8, inc/utils.hpp:23-29; the reference does both on the host, test_fmha_i8.cpp:95-110).
  * x: n floats (device, 16-byte aligned), out: n int8 (device, 16-byte aligned), amax_out: one float on
- * the device (may be NULL).  Two kernels on `stream`, no synchronisation.  Uses a scratch buffer of
- * partial maxima that the library allocates per device and keeps (calls on different streams of one
- * device that overlap in time would share it: serialise them). */
+ * the device (may be NULL).  One kernel on `stream`, no synchronisation, nothing allocated.  Calls on different
+ * streams may overlap (up to 64 in flight on one device). */
 int fmha_i8_sm100_quantize_f32(void* stream, const float* x, long long n, int8_t* out, float* amax_out);
 
-/* The same quantisation for callers that must not allocate device memory.  (No counterpart in the
- * reference project.)  Some hosts of this library hand every byte of the GPU to their own memory pool
- * when they start, so a cudaMalloc made later by a library either fails or escapes the pool's
- * accounting; others run a latency-critical loop and cannot afford the device-wide synchronisation that
- * cudaMalloc and cudaFree imply.  For them the partial maxima are kept in a 16 KB array that is part of
- * the library's device image: this entry point calls no cudaMalloc, no cudaFree and nothing else that
- * allocates.
- *   - Limit: n <= 268,435,456 elements (4096 chunks of 65536); larger tensors are refused with
- *     FMHA_I8_ERR_TOO_LARGE and one line on stderr.
- *   - The first call on each device looks up the device address of that array (with that device
- *     current); make that first call before any stream capture begins.
- *   - All calls on one device share the one array.  Nothing in it has to be cleared between calls (each
- *     call overwrites every slot it later reads), but two calls whose kernels overlap on the GPU --
- *     different streams without an ordering between them -- race on it: keep them ordered.
+/* The same quantisation under a name that promises what some callers need: it never allocates device memory.  (No
+ * counterpart in the reference project.)  Some hosts of this library hand every byte of the GPU to their own memory
+ * pool when they start, so a cudaMalloc made later by a library either fails or escapes the pool's accounting; others
+ * run a latency-critical loop and cannot afford the device-wide synchronisation that cudaMalloc and cudaFree imply.
+ * Limit: n <= 268,435,456 elements; larger tensors are refused with FMHA_I8_ERR_TOO_LARGE and one line on stderr.
+ * Make the first call on each device before any stream capture begins (one-time kernel attributes).
  * Arguments and results are those of fmha_i8_sm100_quantize_f32. */
 int fmha_i8_sm100_quantize_f32_noalloc(void* stream, const float* x, long long n, int8_t* out, float* amax_out);
 

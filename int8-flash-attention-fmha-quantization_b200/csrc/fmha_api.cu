@@ -101,6 +101,8 @@ int set_kernel_attributes(DeviceInfo* d) {
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, false>), fwd_smem_bytes<128>());
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>), fwd_smem_bytes<64>());
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>), fwd_smem_bytes<128>());
+  set(reinterpret_cast<const void*>(&quant_grid_kernel), kQuantGridSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&quant_cluster_kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   set(reinterpret_cast<const void*>(&debug_qk_kernel<64>), qk_smem_bytes<64>());
   set(reinterpret_cast<const void*>(&debug_qk_kernel<128>), qk_smem_bytes<128>());
   set(reinterpret_cast<const void*>(&debug_pv_kernel<64, true>), pv_smem_bytes<64>());
@@ -207,21 +209,37 @@ int fill_params(FwdParams* p, const float amax[5], int D, unsigned flags = 0u) {
   return FMHA_I8_OK;
 }
 
-// Launches `fn`; with `overlap` it may start while the kernel before it in the stream drains (the kernel waits for that one
-// itself, grid_dependency_wait): the set-up of a call and most of its launch latency leave the critical path.  Measured:
-// the smallest call 8.4 -> 6.2 us a pass, a one-request encoder call 10.4 -> 8.2 us.
+// How a kernel is launched.  `overlap`: it may start while the kernel before it in the stream drains (the kernel waits for
+// that one itself, grid_dependency_wait): the set-up of a call and most of its launch latency leave the critical path.
+// Measured: the smallest call 8.4 -> 6.2 us a pass, a one-request encoder call 10.4 -> 8.2 us.
+struct LaunchHow {
+  bool overlap = false;
+  bool cooperative = false;    // the CTAs wait for one another: all of them have to be resident
+  unsigned cluster = 0;        // CTAs per cluster, 0 = no clusters
+};
 template <typename... Params, typename... Args>
-int launch_kernel(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool overlap, Args&&... args) {
+int launch_kernel(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const LaunchHow& how, Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[3];
   cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1 : 0;
+  if (how.overlap) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (how.cooperative) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
+    attr[cfg.numAttrs++].val.cooperative = 1;
+  }
+  if (how.cluster != 0) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = how.cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   g_launch_count.fetch_add(1, std::memory_order_relaxed);
   if (cudaLaunchKernelEx(&cfg, fn, std::forward<Args>(args)...) == cudaSuccess) return FMHA_I8_OK;
   cudaGetLastError();
@@ -241,8 +259,9 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q,
   // whole-row policy 65.0 -> 62.5 us).  Beyond that it gives nothing (B8 H32 S2048: 461 us either way) and where whole
   // K/V tiles stream through every few hundred ns it costs: CTAs then land on SMs in the order the launch before frees
   // them, neighbours that share a head are no longer neighbours on the chip (B256 H16 S256 D64: 132 -> 141 us).
-  const bool overlap = p.n_units <= 4 * dev->sm_count;
-  return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, overlap, mq, mk, mv, p);
+  LaunchHow how;
+  how.overlap = p.n_units <= 4 * dev->sm_count;
+  return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
 
 // calib == nullptr: the forward pass into o.  calib != nullptr: calibration, o is not touched (may be null).
@@ -340,14 +359,6 @@ struct HostStaging {
 HostStaging g_staging[kMaxDevices];
 std::mutex g_staging_mutex[kMaxDevices];     // one lock per device: host threads that drive different GPUs do not wait for each other
 
-// Scratch of fmha_i8_sm100_quantize_f32 (partial maxima), one buffer per device, grown on demand.
-struct QuantScratch {
-  float* partial = nullptr;
-  long long capacity_chunks = 0;
-};
-QuantScratch g_quant_scratch[kMaxDevices];
-std::mutex g_quant_mutex;
-
 int check_quant_args(const float* x, long long n, const int8_t* out) {
   if (!x || !out) return FMHA_I8_ERR_NULL_POINTER;
   if (n < 1) return FMHA_I8_ERR_BAD_SHAPE;
@@ -355,20 +366,32 @@ int check_quant_args(const float* x, long long n, const int8_t* out) {
   return FMHA_I8_OK;
 }
 
-// Scratch of fmha_i8_sm100_quantize_f32_noalloc: the partial maxima live in the library's own device
-// image instead of the heap.  Every GPU that loads the library carries these 16 KB until the process
-// exits.  4096 chunks x 65536 elements = 268,435,456 elements (1 GiB of fp32) is the largest tensor
-// the entry point accepts.
-constexpr long long kNoAllocMaxChunks = 4096;
-static __device__ __align__(256) float g_quant_partial_static[kNoAllocMaxChunks];
-float* g_quant_static_ptr[kMaxDevices];      // device address of the array above, per device (0 = not looked up yet)
-std::mutex g_quant_static_mutex;
+// The largest tensor of fmha_i8_sm100_quantize_f32_noalloc (1 GiB of fp32), part of its contract.
+constexpr long long kNoAllocMaxElements = 268435456LL;
+std::atomic<unsigned> g_quant_calls{0};
 
-int launch_quantize(cudaStream_t stream, const float* x, long long n, int8_t* out, float* amax_out, float* partial, long long n_chunks) {
-  quant_absmax_kernel<<<static_cast<unsigned>(n_chunks), kQuantThreads, 0, stream>>>(x, n, partial);
-  quant_apply_kernel<<<static_cast<unsigned>(n_chunks), kQuantThreads, 0, stream>>>(x, n, partial, static_cast<int>(n_chunks), out, amax_out);
-  g_launch_count.fetch_add(2, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? FMHA_I8_OK : FMHA_I8_ERR_LAUNCH;
+// Up to what the registers of one cluster hold: one cluster.  Beyond: the whole chip, every CTA with work for all its warps.
+int launch_quantize(cudaStream_t stream, DeviceInfo* dev, const float* x, long long n, int8_t* out, float* amax_out) {
+  LaunchHow how;
+  if (n <= kQuantClusterMax * kQuantPerCta) {
+    how.cluster = static_cast<unsigned>(quant_cluster_size(n));
+    how.overlap = true;
+    return launch_kernel(quant_cluster_kernel, dim3(how.cluster), dim3(kQuantClusterThreads), 0, stream, how, x, static_cast<int>(n), out, amax_out);
+  }
+  if (n / kQuantTile > 0x7FFFFFFFLL) return FMHA_I8_ERR_TOO_LARGE;
+  how.cooperative = true;
+  const long long ctas = (n / kQuantTile + kQuantWarps - 1) / kQuantWarps;
+  const int slot = static_cast<int>(g_quant_calls.fetch_add(1, std::memory_order_relaxed) % kQuantSlots);
+  return launch_kernel(quant_grid_kernel, dim3(static_cast<unsigned>(ctas < dev->sm_count ? ctas : dev->sm_count)), dim3(kQuantThreads), kQuantGridSmem,
+                       stream, how, x, n, out, amax_out, slot, dev->status);
+}
+
+int quantize_impl(void* stream, const float* x, long long n, int8_t* out, float* amax_out) {
+  int err = FMHA_I8_OK;
+  DeviceInfo* dev = current_device(&err);
+  if (!dev) return err;
+  const int st = set_kernel_attributes(dev);
+  return st != FMHA_I8_OK ? st : launch_quantize(static_cast<cudaStream_t>(stream), dev, x, n, out, amax_out);
 }
 
 }  // namespace
@@ -633,59 +656,19 @@ int fmha_i8_sm100_debug_wait_probe(void* stream, long long limit_cycles) {
 }
 
 int fmha_i8_sm100_quantize_f32(void* stream, const float* x, long long n, int8_t* out, float* amax_out) {
-  int st = check_quant_args(x, n, out);
-  if (st != FMHA_I8_OK) return finish(st);
-  int err = FMHA_I8_OK;
-  if (!current_device(&err)) return finish(err);
-  int dev_id = 0;
-  cudaGetDevice(&dev_id);
-  const long long n_chunks = (n + kQuantChunk - 1) / kQuantChunk;
-  if (n_chunks > 0x7FFFFFFFLL) return finish(FMHA_I8_ERR_TOO_LARGE);
-  // The lock is held until the kernels are enqueued: another host thread that has to grow the scratch
-  // synchronises the device before it frees the old buffer, and that only covers work already enqueued.
-  std::lock_guard<std::mutex> lock(g_quant_mutex);
-  QuantScratch& q = g_quant_scratch[dev_id];
-  if (q.capacity_chunks < n_chunks) {
-    // growing frees the old buffer: wait for work that may still read it
-    if (q.partial) { cudaDeviceSynchronize(); cudaFree(q.partial); q.partial = nullptr; q.capacity_chunks = 0; }
-    const long long cap = n_chunks < 4096 ? 4096 : n_chunks;
-    if (cudaMalloc(&q.partial, sizeof(float) * cap) != cudaSuccess) { cudaGetLastError(); return finish(FMHA_I8_ERR_LAUNCH); }
-    q.capacity_chunks = cap;
-  }
-  return finish(launch_quantize(static_cast<cudaStream_t>(stream), x, n, out, amax_out, q.partial, n_chunks));
+  const int st = check_quant_args(x, n, out);
+  return finish(st != FMHA_I8_OK ? st : quantize_impl(stream, x, n, out, amax_out));
 }
 
 int fmha_i8_sm100_quantize_f32_noalloc(void* stream, const float* x, long long n, int8_t* out, float* amax_out) {
-  int st = check_quant_args(x, n, out);
+  const int st = check_quant_args(x, n, out);
   if (st != FMHA_I8_OK) return finish(st);
-  const long long n_chunks = (n + kQuantChunk - 1) / kQuantChunk;
-  if (n_chunks > kNoAllocMaxChunks) {
-    std::fprintf(stderr, "fmha_i8_sm100_quantize_f32_noalloc: %lld elements exceed the built-in scratch (at most %lld)\n", n,
-                 kNoAllocMaxChunks * kQuantChunk);
+  if (n > kNoAllocMaxElements) {
+    std::fprintf(stderr, "fmha_i8_sm100_quantize_f32_noalloc: %lld elements exceed the limit of this entry point (at most %lld)\n", n,
+                 kNoAllocMaxElements);
     return finish(FMHA_I8_ERR_TOO_LARGE);
   }
-  int err = FMHA_I8_OK;
-  if (!current_device(&err)) return finish(err);
-  int dev_id = 0;
-  if (cudaGetDevice(&dev_id) != cudaSuccess || dev_id < 0 || dev_id >= kMaxDevices) return finish(FMHA_I8_ERR_LAUNCH);
-  float* partial = nullptr;
-  {
-    // One-time set-up per device, done by the first call on that device with the device current:
-    // in host code the array's name is only a handle, the kernels need its device address.
-    std::lock_guard<std::mutex> lock(g_quant_static_mutex);
-    if (!g_quant_static_ptr[dev_id]) {
-      float* ptr = nullptr;
-      if (cudaGetSymbolAddress(reinterpret_cast<void**>(&ptr), g_quant_partial_static) != cudaSuccess || !ptr) {
-        cudaGetLastError();
-        return finish(FMHA_I8_ERR_LAUNCH);
-      }
-      g_quant_static_ptr[dev_id] = ptr;
-    }
-    partial = g_quant_static_ptr[dev_id];
-  }
-  // Nothing in the scratch has to start at zero: pass 1 overwrites every slot that pass 2 reads
-  // (slots [0, n_chunks)); what an earlier, larger call left beyond them is never looked at.
-  return finish(launch_quantize(static_cast<cudaStream_t>(stream), x, n, out, amax_out, partial, n_chunks));
+  return finish(quantize_impl(stream, x, n, out, amax_out));
 }
 
 int fmha_i8_sm100_device_status(unsigned words[8]) {
@@ -694,6 +677,10 @@ int fmha_i8_sm100_device_status(unsigned words[8]) {
   if (cudaMemcpyFromSymbol(words, g_status_words, sizeof(unsigned) * 8) != cudaSuccess) return finish(FMHA_I8_ERR_LAUNCH);
   const unsigned zeros[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (cudaMemcpyToSymbol(g_status_words, zeros, sizeof zeros) != cudaSuccess) return finish(FMHA_I8_ERR_LAUNCH);
+  if (words[0] == FMHA_I8_DEV_WAIT_QUANT) {      // that call did not clear its slot; the device is idle here
+    static const QuantSlot clean[kQuantSlots] = {};
+    if (cudaMemcpyToSymbol(g_quant_slots, clean, sizeof clean) != cudaSuccess) return finish(FMHA_I8_ERR_LAUNCH);
+  }
   {
     int dev_id = 0;
     if (cudaGetDevice(&dev_id) == cudaSuccess && dev_id >= 0 && dev_id < kMaxDevices) {

@@ -1,90 +1,249 @@
 // Per-tensor symmetric int8 quantisation on the device: the step the reference project performs on
 // the host before the attention call (abs_max + float_quant2_int8, inc/utils.hpp:23-39, driven by
-// test_fmha_i8.cpp:95-110).  Two bandwidth-bound kernels over fixed chunks of the tensor:
-//   1. quant_absmax_kernel  one CTA per 65536-element chunk -> max|x| of the chunk into partial[chunk]
-//   2. quant_apply_kernel   every CTA first reduces partial[] to the tensor's amax (<= 4096 floats, L2
-//                           resident), then writes q = clamp(floor(x * (127/amax) + 0.5), -127, 127)
-// The partial maxima are scratch memory: global memory that is neither input nor output.
-// Algorithmic traffic: 4 B read (pass 1) + 4 B read + 1 B written (pass 2) = 9 bytes per element.
+// test_fmha_i8.cpp:95-110).  The scale is known only when every element has been seen, so the tensor is needed twice;
+// ONE launch does both passes and keeps as much of it on the chip in between as fits:
+//   quant_cluster_kernel  up to 524,288 elements: one cluster of 1..16 CTAs holds the whole tensor in registers, the
+//                         CTAs exchange their maxima through distributed shared memory.  5 bytes moved per element.
+//   quant_grid_kernel     larger: one CTA per SM (cooperative launch), every warp streams its tiles through a private
+//                         ring of bulk copies.  At the end of pass 1 the ring still holds each warp's last tiles and its
+//                         registers the first ones (53 MB over the chip); pass 2 takes those from there and walks the
+//                         others from the last to the first, so that it meets what the L2 still has.
+// Two launches over 65,536-element chunks, which these replace, took 16.5 us for 255,749 elements (four CTAs) and 107 us
+// for 67,108,864; these take 5.5 and 100 us.  The large case is bound by DRAM: 468 of the 537 MB of the two passes are
+// read from there (ncu, without the register tiles), plus the output.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "fmha_fwd_sm100.cuh"
+#include "ptx.cuh"
+#include "../../include/fmha_i8_c.h"
 
 namespace fmha {
 
-constexpr int kQuantChunk = 65536;       // elements per CTA
-constexpr int kQuantThreads = 256;
-
-__global__ void __launch_bounds__(kQuantThreads)
-quant_absmax_kernel(const float* __restrict__ x, long long n, float* __restrict__ partial) {
-  const long long base = static_cast<long long>(blockIdx.x) * kQuantChunk;
-  const long long end = min(base + kQuantChunk, n);
-  float m = 0.f;
-  // 16-byte loads while a whole float4 fits, scalar tail
-  const long long n4 = (end - base) / 4;
-  const float4* x4 = reinterpret_cast<const float4*>(x + base);
-  for (long long i = threadIdx.x; i < n4; i += kQuantThreads) {
-    const float4 v = __ldg(x4 + i);
-    m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-  }
-  for (long long i = base + n4 * 4 + threadIdx.x; i < end; i += kQuantThreads) m = fmaxf(m, fabsf(x[i]));
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, s));
-  __shared__ float warp_max[kQuantThreads / 32];
-  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float b = warp_max[0];
-#pragma unroll
-    for (int i = 1; i < kQuantThreads / 32; ++i) b = fmaxf(b, warp_max[i]);
-    partial[blockIdx.x] = b;
-  }
+__device__ __forceinline__ float abs_max4(float m, const float4& v) {
+  return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
 }
-
 __device__ __forceinline__ int quant_one(float v, float scale) {
   // float_quant2_int8: floorf(x*scale + 0.5) with the sum rounded once to float, clamp to +-127
   const float f = floorf(__fadd_rn(__fmul_rn(v, scale), 0.5f));
   return static_cast<int>(fminf(fmaxf(f, -127.f), 127.f));
 }
+__device__ __forceinline__ uint32_t quant_four(const float4& v, float scale) {
+  return (static_cast<uint32_t>(quant_one(v.x, scale)) & 0xFFu) | ((static_cast<uint32_t>(quant_one(v.y, scale)) & 0xFFu) << 8) |
+         ((static_cast<uint32_t>(quant_one(v.z, scale)) & 0xFFu) << 16) | (static_cast<uint32_t>(quant_one(v.w, scale)) << 24);
+}
+__device__ __forceinline__ float quant_scale(float amax) {
+  return (amax > 0.f) ? __fdiv_rn(127.0f, amax) : 0.f;     // an all-zero tensor quantises to zeros
+}
+// Largest of a block's values; `scratch` holds one float per warp.
+template <int kThreads>
+__device__ __forceinline__ float block_max(float m, float* scratch) {
+  // magnitudes are non-negative: they order like their bit patterns
+  m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = (threadIdx.x & 31) < kThreads / 32 ? scratch[threadIdx.x & 31] : 0.f;
+  return __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
+}
 
-__global__ void __launch_bounds__(kQuantThreads)
-quant_apply_kernel(const float* __restrict__ x, long long n, const float* __restrict__ partial, int n_chunks,
-                   int8_t* __restrict__ out, float* __restrict__ amax_out) {
-  float m = 0.f;
-  for (int i = threadIdx.x; i < n_chunks; i += kQuantThreads) m = fmaxf(m, partial[i]);
+// ------------------------------------------------------------------------------------------ up to 524,288 elements
+constexpr int kQuantClusterThreads = 1024;
+constexpr int kQuantClusterVec = 8;            // float4 per thread, all loads in flight at once
+constexpr int kQuantClusterMax = 16;
+constexpr long long kQuantPerCta = 4LL * kQuantClusterThreads * kQuantClusterVec;    // 32,768 elements
+
+// CTAs for n elements: two float4 per thread are enough to cover the latency of memory, more CTAs than that only make
+// the exchange longer; beyond 8 CTAs (the portable cluster size) only what the registers of 8 cannot hold.
+inline int quant_cluster_size(long long n) {
+  int c = 1;
+  while (c < 8 && n > c * (kQuantPerCta / 4)) c *= 2;
+  return n > 8 * kQuantPerCta ? 16 : c;
+}
+
+__global__ void __launch_bounds__(kQuantClusterThreads, 1)
+quant_cluster_kernel(const float* __restrict__ x, int n, int8_t* __restrict__ out, float* __restrict__ amax_out) {
+  __shared__ float warp_max[kQuantClusterThreads / 32];
+  __shared__ float cta_max[kQuantClusterMax];
+  grid_launch_dependents();
+  const uint32_t ctas = cluster_ctas(), rank = cluster_rank();
+  cluster_arrive();                                   // every CTA of the cluster runs before its memory is written
+  grid_dependency_wait();
+  const int n4 = n / 4, per_cta = (n4 + static_cast<int>(ctas) - 1) / static_cast<int>(ctas);
+  const int begin = static_cast<int>(rank) * per_cta, end = min(begin + per_cta, n4);
+  const float4* x4 = reinterpret_cast<const float4*>(x);
+  float4 v[kQuantClusterVec];
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, s));
-  __shared__ float warp_max[kQuantThreads / 32];
+  for (int k = 0; k < kQuantClusterVec; ++k) {
+    const int i = begin + k * kQuantClusterThreads + static_cast<int>(threadIdx.x);
+    v[k] = i < end ? __ldg(x4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  // up to three elements behind the last float4
+  const int tail = n4 * 4 + static_cast<int>(threadIdx.x);
+  const bool has_tail = rank == 0 && tail < n;
+  const float t = has_tail ? x[tail] : 0.f;
+  float m = fabsf(t);
+#pragma unroll
+  for (int k = 0; k < kQuantClusterVec; ++k) m = abs_max4(m, v[k]);
+  m = block_max<kQuantClusterThreads>(m, warp_max);
+  cluster_wait();
+  if (threadIdx.x < ctas) st_cluster_f32(smem_u32(&cta_max[rank]), threadIdx.x, m);
+  cluster_arrive();
+  cluster_wait();
+  float amax = 0.f;
+  for (uint32_t i = 0; i < ctas; ++i) amax = fmaxf(amax, cta_max[i]);
+  if (rank == 0 && threadIdx.x == 0 && amax_out) *amax_out = amax;
+  const float scale = quant_scale(amax);
+  uint32_t* o4 = reinterpret_cast<uint32_t*>(out);
+#pragma unroll
+  for (int k = 0; k < kQuantClusterVec; ++k) {
+    const int i = begin + k * kQuantClusterThreads + static_cast<int>(threadIdx.x);
+    if (i < end) o4[i] = quant_four(v[k], scale);
+  }
+  if (has_tail) out[tail] = static_cast<int8_t>(quant_one(t, scale));
+}
+
+// ------------------------------------------------------------------------------------------ larger tensors
+constexpr int kQuantThreads = 256;
+constexpr int kQuantWarps = kQuantThreads / 32;
+constexpr int kQuantTile = 1024;               // elements per tile: 8 float4 per lane
+constexpr int kQuantVec = kQuantTile / 128;
+constexpr int kQuantStages = 7;                // ring of 7 x 4 KB per warp: all of shared memory
+constexpr int kQuantKeep = 4;                  // tiles a warp keeps in registers (128 of them)
+constexpr size_t kQuantGridSmem = static_cast<size_t>(kQuantWarps) * kQuantStages * kQuantTile * sizeof(float);
+
+// What the CTAs of one call share.  All zero between calls: the last CTA to leave clears it.
+struct QuantSlot {
+  unsigned amax_bits, arrived, left, pad[29];  // one 128-byte line
+};
+constexpr int kQuantSlots = 64;                // calls take them in turn: that many may be in flight at once
+__device__ QuantSlot g_quant_slots[kQuantSlots];
+
+__global__ void __launch_bounds__(kQuantThreads, 1)
+quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__ out, float* __restrict__ amax_out, int slot_index,
+                  unsigned* __restrict__ status) {
+  extern __shared__ __align__(128) uint8_t ring_raw[];
+  __shared__ uint64_t bars[kQuantWarps][kQuantStages];
+  __shared__ float warp_max[kQuantWarps];
   __shared__ float s_amax;
-  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float b = warp_max[0];
-#pragma unroll
-    for (int i = 1; i < kQuantThreads / 32; ++i) b = fmaxf(b, warp_max[i]);
-    s_amax = b;
-    if (blockIdx.x == 0 && amax_out) *amax_out = b;
-  }
-  __syncthreads();
-  const float amax = s_amax;
-  const float scale = (amax > 0.f) ? __fdiv_rn(127.0f, amax) : 0.f;     // an all-zero tensor quantises to zeros
+  __shared__ int s_abort;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* ring = reinterpret_cast<float*>(ring_raw) + warp * (kQuantStages * kQuantTile);
+  uint64_t* bar = bars[warp];
+  QuantSlot* slot = &g_quant_slots[slot_index];
 
-  const long long base = static_cast<long long>(blockIdx.x) * kQuantChunk;
-  const long long end = min(base + kQuantChunk, n);
-  const long long n16 = (end - base) / 16;
-  const float4* x4 = reinterpret_cast<const float4*>(x + base);
-  uint4* o16 = reinterpret_cast<uint4*>(out + base);
-  for (long long i = threadIdx.x; i < n16; i += kQuantThreads) {
-    uint32_t w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float4 v = __ldg(x4 + i * 4 + k);
-      w[k] = (static_cast<uint32_t>(quant_one(v.x, scale)) & 0xFFu) | ((static_cast<uint32_t>(quant_one(v.y, scale)) & 0xFFu) << 8) |
-             ((static_cast<uint32_t>(quant_one(v.z, scale)) & 0xFFu) << 16) | ((static_cast<uint32_t>(quant_one(v.w, scale)) & 0xFFu) << 24);
-    }
-    o16[i] = make_uint4(w[0], w[1], w[2], w[3]);
+  // warp w of CTA c takes tiles w * CTAs + c, then every (warps * CTAs)-th: the whole chip reads one stretch of memory
+  // at a time, and the last stretch is the one that pass 2 begins with
+  const int n_tiles = static_cast<int>(n / kQuantTile);
+  const int stride = static_cast<int>(gridDim.x) * kQuantWarps, first = warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+  const int mine = first < n_tiles ? (n_tiles - first + stride - 1) / stride : 0;
+  auto tile_at = [&](int i) { return (static_cast<long long>(first) + static_cast<long long>(i) * stride) * kQuantTile; };
+
+  if (threadIdx.x == 0) s_abort = 0;
+  if (lane == 0) {
+    for (int s = 0; s < kQuantStages; ++s) mbar_init(smem_u32(&bar[s]), 1);
+    mbar_init_fence();
   }
-  for (long long i = base + n16 * 16 + threadIdx.x; i < end; i += kQuantThreads) out[i] = static_cast<int8_t>(quant_one(x[i], scale));
+  __syncthreads();
+  volatile int* abort_flag = &s_abort;
+  auto load = [&](int i, int s) {
+    mbar_arrive_expect_tx(smem_u32(&bar[s]), kQuantTile * sizeof(float));
+    bulk_load(smem_u32(ring + s * kQuantTile), x + tile_at(i), kQuantTile * sizeof(float), smem_u32(&bar[s]));
+  };
+  bool ok = true;
+  uint32_t parity_bits = 0u;                   // bit s: parity of the next completion of ring slot s
+  auto landed = [&](int s) {
+    ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&bar[s]), (parity_bits >> s) & 1u, abort_flag));
+    parity_bits ^= 1u << s;
+    return reinterpret_cast<const float4*>(ring + s * kQuantTile);
+  };
+
+  // ---- pass 1: the largest magnitude
+  if (lane == 0)
+    for (int i = 0; i < kQuantStages && i < mine; ++i) load(i, i);
+  float m = 0.f;
+  float4 keep[kQuantKeep][kQuantVec];
+#pragma unroll
+  for (int i = 0; i < kQuantKeep; ++i) {
+#pragma unroll
+    for (int k = 0; k < kQuantVec; ++k) keep[i][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < mine) {
+      const float4* t = landed(i);
+#pragma unroll
+      for (int k = 0; k < kQuantVec; ++k) {
+        keep[i][k] = t[lane + 32 * k];
+        m = abs_max4(m, keep[i][k]);
+      }
+      __syncwarp();
+      if (lane == 0 && i + kQuantStages < mine) load(i + kQuantStages, i);
+    }
+  }
+  for (int i = kQuantKeep, s = kQuantKeep; i < mine; ++i) {
+    const float4* t = landed(s);
+#pragma unroll
+    for (int k = 0; k < kQuantVec; ++k) m = abs_max4(m, t[lane + 32 * k]);
+    __syncwarp();
+    if (lane == 0 && i + kQuantStages < mine) load(i + kQuantStages, s);
+    if (++s == kQuantStages) s = 0;
+  }
+  // what is left behind the last whole tile: the last CTA reads it, twice
+  const long long rest = static_cast<long long>(n_tiles) * kQuantTile;
+  const bool has_rest = blockIdx.x == gridDim.x - 1;
+  if (has_rest)
+    for (long long i = rest + threadIdx.x; i < n; i += kQuantThreads) m = fmaxf(m, fabsf(x[i]));
+
+  // ---- the largest of all CTAs (they are all resident: cooperative launch)
+  m = block_max<kQuantThreads>(m, warp_max);
+  if (threadIdx.x == 0) {
+    atomicMax(&slot->amax_bits, __float_as_uint(m));
+    __threadfence();
+    atomicAdd(&slot->arrived, 1u);
+    const long long t0 = clock64();
+    uint32_t probes = 0;
+    while (ok && ld_acquire_gpu(&slot->arrived) < gridDim.x) {
+      if (++probes >= kMinProbes && clock64() - t0 > kWaitLimitCycles) ok = false;
+    }
+    s_amax = __uint_as_float(ld_acquire_gpu(&slot->amax_bits));
+    if (!ok) raise_status(abort_flag, status, FMHA_I8_DEV_WAIT_QUANT, blockIdx.x);
+    if (atomicAdd(&slot->left, 1u) == gridDim.x - 1) {
+      slot->amax_bits = 0u;
+      slot->arrived = 0u;
+      slot->left = 0u;
+    }
+    if (blockIdx.x == 0 && amax_out) *amax_out = s_amax;
+  }
+  __syncthreads();
+  const float scale = quant_scale(s_amax);
+
+  // ---- pass 2: quantise, from the last tile to the first
+  auto store = [&](int i, int k, const float4& v) { reinterpret_cast<uint32_t*>(out + tile_at(i))[lane + 32 * k] = quant_four(v, scale); };
+  auto from_ring = [&](int i, int s, const float4* t) {
+#pragma unroll
+    for (int k = 0; k < kQuantVec; ++k) store(i, k, t[lane + 32 * k]);
+    __syncwarp();
+    if (lane == 0 && i - kQuantStages >= kQuantKeep) load(i - kQuantStages, s);
+  };
+  const int still_there = max(mine - kQuantStages, kQuantKeep);    // tiles [still_there, mine) are still in the ring
+  for (int i = mine - 1; i >= still_there; --i) {
+    const int s = i % kQuantStages;
+    from_ring(i, s, reinterpret_cast<const float4*>(ring + s * kQuantTile));
+  }
+#pragma unroll
+  for (int i = 0; i < kQuantKeep; ++i)
+    if (i < mine) {
+#pragma unroll
+      for (int k = 0; k < kQuantVec; ++k) store(i, k, keep[i][k]);
+    }
+  for (int i = still_there - 1; i >= kQuantKeep; --i) {
+    const int s = i % kQuantStages;
+    from_ring(i, s, landed(s));
+  }
+  if (has_rest)
+    for (long long i = rest + threadIdx.x; i < n; i += kQuantThreads) out[i] = static_cast<int8_t>(quant_one(x[i], scale));
+  if (!ok && lane == 0) {
+    raise_status(abort_flag, status, FMHA_I8_DEV_WAIT_QUANT, blockIdx.x);
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) { /* copies still in flight land before the CTA may exit */ }
+  }
 }
 
 }  // namespace fmha

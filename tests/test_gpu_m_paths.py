@@ -48,3 +48,40 @@ def torch_cuda():
     import torch
     torch.cuda.set_device(0)
     return torch
+
+
+# One cluster of 1, 2, 4, 8 and 16 CTAs; then the whole chip, where a warp has 0, 1, 4 (all kept in registers), 7 and 8 (one
+# ring), 12 tiles of 1024 elements, with and without a remainder.
+SWEEP = 148 * 8 * 1024
+@pytest.mark.parametrize("n", [1, 3, 8192, 8193, 32771, 65536, 65537, 262144, 262147, 524288, 524289, SWEEP - 1, SWEEP, 4 * SWEEP + 1,
+                               5 * SWEEP, 7 * SWEEP + 1023, 8 * SWEEP, 12 * SWEEP + 1025])
+def test_quantize_sizes(pkg, oracle, torch_cuda, n):
+    torch = torch_cuda
+    x = np.random.default_rng(n).standard_normal(n, dtype=np.float32)
+    for at in sorted({0, n // 2, n - 1}):                   # wherever the largest magnitude sits, it is found
+        y = x.copy()
+        y[at] = -7.5 - np.abs(x).max()
+        out = torch.full((n + 64,), 0x5A, dtype=torch.int8, device="cuda")
+        amax = torch.zeros(1, device="cuda")
+        pkg.quantize_f32(None, torch.from_numpy(y).cuda(), out, amax, n=n)
+        host = out.cpu().numpy()
+        assert np.float32(amax.item()) == np.abs(y).max()
+        assert np.array_equal(host[:n], oracle.quantize(y, np.abs(y).max())), (n, at)
+        assert np.all(host[n:] == 0x5A)
+    assert pkg.device_status()[0] == pkg.OK
+
+
+def test_quantize_calls_overlap_on_two_streams(pkg, oracle, torch_cuda):
+    torch = torch_cuda
+    n = 3 * SWEEP + 5
+    xs = [torch.randn(n, device="cuda") * s for s in (1.0, 30.0)]
+    want = [oracle.quantize(x.cpu().numpy(), float(x.abs().max())) for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    outs = [torch.empty(n, dtype=torch.int8, device="cuda") for _ in range(24)]
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        pkg.quantize_f32(streams[i % 2], xs[i % 2], o)
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        assert np.array_equal(o.cpu().numpy(), want[i % 2]), i
+    assert pkg.device_status()[0] == pkg.OK
