@@ -8,10 +8,12 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "../../include/fmha_i8_c.h"
 #include "fmha_debug_sm100.cuh"
+#include "fmha_decode_sm100.cuh"
 #include "fmha_fwd_sm100.cuh"
 #include "fmha_quant_sm100.cuh"
 
@@ -91,6 +93,22 @@ template <int D> size_t fwd_smem_bytes() {
 template <int D> size_t qk_smem_bytes() { return 1024 + 2 * kTile * D + sizeof(DebugCtl); }
 template <int D> size_t pv_smem_bytes() { return 1024 + kTile * D + kTile * kTile + sizeof(DebugCtl); }
 
+template <typename Set> void set_decode_attributes(Set set) {
+  auto both = [&](auto d, auto r) {
+    constexpr int D = decltype(d)::value, R = decltype(r)::value;
+    set(reinterpret_cast<const void*>(&fmha_decode_kernel<D, R, false>), sizeof(DecodeSmem<D, R>));
+    set(reinterpret_cast<const void*>(&fmha_decode_kernel<D, R, true>), sizeof(DecodeSmem<D, R>));
+  };
+  auto rows = [&](auto d) {
+    both(d, std::integral_constant<int, 1>());
+    both(d, std::integral_constant<int, 2>());
+    both(d, std::integral_constant<int, 4>());
+    both(d, std::integral_constant<int, 8>());
+  };
+  rows(std::integral_constant<int, 64>());
+  rows(std::integral_constant<int, 128>());
+}
+
 int set_kernel_attributes(DeviceInfo* d) {
   if (d->attr_set) return FMHA_I8_OK;
   cudaError_t e = cudaSuccess;
@@ -101,6 +119,7 @@ int set_kernel_attributes(DeviceInfo* d) {
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, false>), fwd_smem_bytes<128>());
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>), fwd_smem_bytes<64>());
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>), fwd_smem_bytes<128>());
+  set_decode_attributes(set);
   set(reinterpret_cast<const void*>(&quant_grid_kernel), kQuantGridSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&quant_cluster_kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   set(reinterpret_cast<const void*>(&debug_qk_kernel<64>), qk_smem_bytes<64>());
@@ -264,6 +283,36 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q,
   return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
 
+// The few-rows kernel.  CTAs per head: enough for two rounds of the 3 CTAs that an SM holds, so that heads of different
+// length even out, as long as a warp keeps two tiles (B16 H32, 1025..4096 keys, one row: 60.3 us with one round, 58.6 with
+// two, 70 with four, 112 with eight, where the set-up of a CTA outweighs its tiles); where even that leaves SMs idle, down
+// to one tile per warp.
+template <int D, int R, bool kUnsigned>
+int launch_decode_rows(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v) {
+  constexpr int W = DecodeCfg<D>::kWarps;
+  p.q_tiles = (p.Sq + R - 1) / R;
+  const long long units = static_cast<long long>(p.bh_count) * p.q_tiles;
+  const int n_tiles = (p.S + kTile - 1) / kTile;
+  const long long resident = 3LL * dev->sm_count;
+  int c = 1;
+  constexpr int kMaxCtas = R == 8 ? kDecodeMaxCluster / 2 : kDecodeMaxCluster;      // their partial results fit into the tiles of one CTA
+  static_assert(kMaxCtas * W * R * DecodeCfg<D>::kPartFloats * 4 <= DecodeCfg<D>::kRingBytes, "partial results do not fit");
+  while (c < kMaxCtas && ((units * c < 2 * resident && n_tiles >= 4 * c * W) || (units * c * 2 <= resident && n_tiles >= 2 * c * W))) c *= 2;
+  if (units * c > 0x7FFFFFFFLL) return FMHA_I8_ERR_BAD_SHAPE;
+  LaunchHow how;
+  how.cluster = static_cast<unsigned>(c);
+  how.overlap = true;
+  return launch_kernel(fmha_decode_kernel<D, R, kUnsigned>, dim3(static_cast<unsigned>(units * c)), dim3(DecodeCfg<D>::kThreads),
+                       sizeof(DecodeSmem<D, R>), stream, how, static_cast<const int8_t*>(q), static_cast<const int8_t*>(k),
+                       static_cast<const int8_t*>(v), p);
+}
+template <int D>
+int launch_decode(cudaStream_t s, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v) {
+  if (p.Sq == 1) return p.p_unsigned ? launch_decode_rows<D, 1, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 1, false>(s, dev, p, q, k, v);
+  if (p.Sq == 2) return p.p_unsigned ? launch_decode_rows<D, 2, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 2, false>(s, dev, p, q, k, v);
+  if (p.Sq <= 4) return p.p_unsigned ? launch_decode_rows<D, 4, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 4, false>(s, dev, p, q, k, v);
+  return p.p_unsigned ? launch_decode_rows<D, 8, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 8, false>(s, dev, p, q, k, v);
+}
 // calib == nullptr: the forward pass into o.  calib != nullptr: calibration, o is not touched (may be null).
 // Which of the three uses of the forward kernel a launch is.
 struct LaunchMode {
@@ -335,6 +384,10 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   }
   p.status = dev->status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // Few query rows: up to eight the dp4a kernel is faster or as fast at every length and number of heads measured (B16 H32
+  // D128, 1025..4096 keys: 1 row 104 -> 59 us, 2 rows 61, 4 rows 68, 8 rows 100; B128 H32 D64, 256 keys, 8 rows 72 -> 71).
+  if (!mode && !calib && sh.Sq <= kDecodeMaxRows)
+    return sh.D == 128 ? launch_decode<128>(s, dev, p, q, k, v) : launch_decode<64>(s, dev, p, q, k, v);
   if (policy_launch) return sh.D == 128 ? launch_fwd<128, true>(s, dev, p, q, k, v) : launch_fwd<64, true>(s, dev, p, q, k, v);
   return sh.D == 128 ? launch_fwd<128>(s, dev, p, q, k, v) : launch_fwd<64>(s, dev, p, q, k, v);
 }

@@ -153,6 +153,10 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, uint32_t rank, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(addr, rank)), "f"(v) : "memory");
 }
+// Two floats to a cluster address (8-byte aligned).
+__device__ __forceinline__ void st_cluster_v2(uint32_t cluster_addr, float a, float b) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr), "f"(a), "f"(b) : "memory");
+}
 
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
   unsigned v;

@@ -85,3 +85,34 @@ def test_quantize_calls_overlap_on_two_streams(pkg, oracle, torch_cuda):
     for i, o in enumerate(outs):
         assert np.array_equal(o.cpu().numpy(), want[i % 2]), i
     assert pkg.device_status()[0] == pkg.OK
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,B,H,Sk,valid", [
+    (1, 1, 1, 64, None),                     # half a key tile, most warps and CTAs idle
+    (1, 2, 3, 192, (1, 192)),                # one key only; half a tile behind a whole one
+    (1, 3, 2, 1088, (1088, 0, 129)),         # a batch without any key: zeros
+    (1, 1, 2, 8192, (8000,)),                # eight CTAs per head, several tiles per warp
+    (1, 40, 16, 320, None),                  # many heads
+    (2, 2, 2, 704, (640, 513)), (3, 2, 2, 1024, (900, 1024)), (4, 1, 3, 2048, None), (5, 2, 2, 448, (448, 77)),
+    (7, 1, 2, 4096, (3001,)), (8, 3, 3, 640, (640, 64, 500)), (9, 1, 2, 512, None)])
+@pytest.mark.parametrize("uint8_p", [False, True])
+def test_few_query_rows(pkg, wl, oracle, torch_cuda, D, Sq, B, H, Sk, valid, uint8_p):
+    torch = torch_cuda
+    q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, D, seed=Sq * Sk + D, mask_p=0.1 if Sk > 192 else 0.0, valid=valid)
+    want = oracle.q128(q8, k8, v8, mask, amax, p_levels=255 if uint8_p else 128)
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    buf = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    desc, param = pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), pkg.FMHAParamI8(*amax, 1.0)
+    pkg.FMHAInferI8Cross(None, param, desc, q, k, v, m, buf[128:-128], uint8_p=uint8_p)
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    host = buf.cpu().numpy()
+    assert np.all(host[:128] == 0x5A) and np.all(host[-128:] == 0x5A)
+    assert_parity(host[128:-128].reshape(q8.shape), want, f"Sq{Sq} B{B}H{H}Sk{Sk}D{D}")
+    if B * H > 3:                            # a slice that begins inside a batch
+        begin, count = 1, B * H - 2
+        part = torch.zeros(count * Sq * D, dtype=torch.int8, device="cuda")
+        view = [x.reshape(B * H, -1, D)[begin:begin + count].contiguous() for x in (q, k, v)]
+        pkg.FMHAInferI8Cross(None, param, desc, *view, m, part, bh_begin=begin, bh_count=count, uint8_p=uint8_p)
+        assert np.array_equal(part.cpu().numpy(), host[128:-128].reshape(B * H, -1)[begin:begin + count].ravel())
