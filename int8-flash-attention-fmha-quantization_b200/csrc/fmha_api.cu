@@ -88,7 +88,7 @@ DeviceInfo* current_device(int* err) {
 }
 
 template <int D> size_t fwd_smem_bytes() {
-  return 1024 + FwdCfg<D>::kTilesBytesTotal + 2 * kBiasBytes + sizeof(FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>);
+  return 1024 + FwdCfg<D>::kTilesBytesTotal + bias_bytes<D>() + sizeof(FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>);
 }
 template <int D> size_t qk_smem_bytes() { return 1024 + 2 * kTile * D + sizeof(DebugCtl); }
 template <int D> size_t pv_smem_bytes() { return 1024 + kTile * D + kTile * kTile + sizeof(DebugCtl); }

@@ -41,11 +41,18 @@
 //                and leaves it in [112,128)).
 //                These threads hold no output row, so they are light (64 registers).
 //
-// The bias: every accumulator is first written by a one-step fp16 MMA whose operands hold 4096 and
+// The bias: every accumulator is first written by a one-step bf16 MMA whose operands hold 4096 and
 // 3072, i.e. the fp32 value 1.5*2^23 (bits 0x4B400000); the int8 MMAs then add their integer result
 // to that bit pattern.  Read back as a float the accumulator is exactly 1.5*2^23 + s, so no thread
 // ever converts integers to floats: one fused multiply-add turns the raw accumulator into the
 // exponent argument (or into the rescaled partial output).
+//
+// The padding mask goes the same way: where a key tile has masked keys, the issuer of S presets their columns to -2^127
+// instead (a second product, 2^100 * -2^27, that swallows the first).  The scores added to that bit pattern leave a float
+// of the same size, below every real score as an integer and as a float, and its exponential is exactly zero: the softmax
+// threads treat every tile alike.  Before, they tested a mask bit per score in a loop that was not pipelined: B256 H16 S256
+// D64 with lengths 64..256 took 132 us instead of 115, B24 H16 S576 D64 with lengths 300..576 66 instead of 59, and the
+// smaller code makes unmasked head_dim-64 calls faster too (B8 H32 S2048: 430 -> 400 us).
 //
 // Tensor memory (512 columns x 128 lanes x 32 bit): accumulator b at columns [128 b, 128 b + 128).
 // head_dim 128: annex b at [384 + 32 b, 384 + 32 b + 32) holds P (four int8 per column, keys in order), the partial
@@ -148,7 +155,8 @@ template <int D> struct FwdRegs {
 constexpr uint32_t kTmemCols = 512;
 constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23: float whose ulp is 1 over [2^23, 2^24)
 constexpr uint32_t kMagicBits = 0x4B400000u;
-constexpr int kBiasBytes = 4096;               // 128 rows x 16 fp16, unswizzled core-matrix layout
+constexpr int kBiasBytes = 4096;               // 128 rows x 16 bf16, unswizzled core-matrix layout
+template <int D> __host__ __device__ constexpr int bias_bytes() { return (2 + SBufs<D>::n) * kBiasBytes; }
 
 template <int D> struct FwdCfg {
   static_assert(D == 64 || D == 128, "head_dim must be 64 or 128");
@@ -198,8 +206,7 @@ struct FwdParams {
 // memory: the scanner warp fills the ones of coming units while the current unit is being processed.
 struct UnitInfo {
   int n_live;                         // key tiles with at least one unmasked key
-  uint32_t maskbits[kMaxTiles * 4];   // bit set = key masked (or beyond seq_len)
-  uint16_t live[kMaxTiles];           // indices of the live key tiles, ascending
+  uint8_t live[kMaxTiles];            // indices of the live key tiles, ascending
   uint8_t mixed[kMaxTiles];           // 1 = that live tile has masked keys too
 };
 
@@ -247,41 +254,31 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// Builds one unit's view of its batch's padding mask: 128-bit masks per key tile, the list of live
-// tiles and whether each needs the per-key path.  Executed by ONE warp.
+// Builds one unit's view of its batch's padding mask: the list of live tiles and whether each has masked keys too.
+// Executed by ONE warp; a lane looks at 32 keys, four lanes make a tile.
 __device__ __forceinline__ void scan_mask_warp(UnitInfo* info, const int8_t* mask_row, int S, int n_tiles) {
   const int lane = threadIdx.x & 31;
   const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
-  for (int g = lane; g < n_tiles * 4; g += 32) {
-    const int key0 = g * 32;
-    uint32_t bits = 0xFFFFFFFFu;
+  int n = 0;
+  for (int base = 0; base < n_tiles; base += 8) {
+    const int key0 = base * kTile + lane * 32;
+    uint32_t open = 0u, masked = 0xFFFFFFFFu;            // any unmasked key; any masked key (keys beyond S count as masked)
     if (key0 < S) {  // S is a multiple of 64, so a 32-key group is entirely inside or outside
-      bits = 0u;
+      masked = 0u;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const uint32_t wv = __ldg(words + (key0 >> 2) + i);
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          if ((wv >> (8 * b)) & 0xFFu) bits |= 1u << (4 * i + b);
+        masked |= wv;
+        open |= __vcmpeq4(wv, 0u);
       }
     }
-    info->maskbits[g] = bits;
-  }
-  __syncwarp();
-  int n = 0;
-  for (int base = 0; base < n_tiles; base += 32) {
-    const int t = base + lane;
-    bool is_live = false, is_mixed = false;
-    if (t < n_tiles) {
-      const uint32_t a = info->maskbits[4 * t], b = info->maskbits[4 * t + 1], c = info->maskbits[4 * t + 2], d = info->maskbits[4 * t + 3];
-      is_live = (a & b & c & d) != 0xFFFFFFFFu;
-      is_mixed = (a | b | c | d) != 0u;
-    }
+    const uint32_t any_open = __ballot_sync(0xFFFFFFFFu, open != 0u), any_masked = __ballot_sync(0xFFFFFFFFu, masked != 0u);
+    const bool is_live = lane < 8 && ((any_open >> (4 * lane)) & 0xFu) != 0u;
     const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, is_live);
     if (is_live) {
       const int pos = n + __popc(ballot & ((1u << lane) - 1u));
-      info->live[pos] = static_cast<uint16_t>(t);
-      info->mixed[pos] = is_mixed ? 1 : 0;
+      info->live[pos] = static_cast<uint8_t>(base + lane);
+      info->mixed[pos] = ((any_masked >> (4 * lane)) & 0xFu) != 0u ? 1 : 0;
     }
     n += __popc(ballot);
   }
@@ -289,57 +286,48 @@ __device__ __forceinline__ void scan_mask_warp(UnitInfo* info, const int8_t* mas
   __syncwarp();
 }
 
-// Writes the two constant fp16 operands of the bias MMA: A[m][0] = 4096, B[n][0] = 3072, all other
-// elements zero, in the unswizzled K-major layout (core matrix = 8 rows x 16 bytes, the two K halves
-// of a row group 128 bytes apart, row groups 256 bytes apart).
-__device__ __forceinline__ void fill_bias_operands(uint8_t* bias_a, uint8_t* bias_b) {
-  for (int i = threadIdx.x; i < 2 * kBiasBytes / 16; i += blockDim.x)
-    reinterpret_cast<uint4*>(bias_a)[i] = make_uint4(0u, 0u, 0u, 0u);   // bias_b follows bias_a
-  __syncthreads();
-  if (threadIdx.x < kTile) {
-    const int m = threadIdx.x;
-    const int off = (m >> 3) * 256 + (m & 7) * 16;
-    *reinterpret_cast<uint16_t*>(bias_a + off) = 0x6C00u;   // 4096.0 in fp16
-    *reinterpret_cast<uint16_t*>(bias_b + off) = 0x6A00u;   // 3072.0 in fp16
-  }
+// The bf16 operands of the bias MMA in the unswizzled K-major layout (core matrix = 8 rows x 16 bytes, the two K halves
+// of a row group 128 bytes apart, row groups 256 bytes apart).  A: every row holds 4096 and 2^100.  B: row n = key n holds
+// 3072 and 0, or 3072 and -2^27 where the key is masked; one B for tiles without masked keys, one per S accumulator for the others.
+constexpr uint32_t kBiasA = 0x71804580u;         // {4096, 2^100}
+constexpr uint32_t kBiasB = 0x00004540u;         // {3072, 0}
+constexpr uint32_t kBiasBMasked = 0xCD004540u;   // {3072, -2^27}
+__device__ __forceinline__ int bias_row_offset(int row) { return (row >> 3) * 256 + (row & 7) * 16; }
+__device__ __forceinline__ void fill_bias_operands(uint8_t* bias_a, int n_b) {
+  for (int i = threadIdx.x; i < (1 + n_b) * kBiasBytes / 16; i += blockDim.x)      // the B operands follow A
+    reinterpret_cast<uint4*>(bias_a)[i] = make_uint4((i & 8) ? 0u : i < kBiasBytes / 16 ? kBiasA : kBiasB, 0u, 0u, 0u);
   fence_proxy_async_smem();
+}
+// Executed by one warp, lane l for keys l, 32 + l, 64 + l and 96 + l: the B operand of a tile with masked keys.
+__device__ __forceinline__ void fill_mask_operand(uint8_t* bias_b, const bool (&masked)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<uint32_t*>(bias_b + bias_row_offset(32 * i + (threadIdx.x & 31))) = masked[i] ? kBiasBMasked : kBiasB;
+  fence_proxy_async_smem();
+  __syncwarp();
 }
 
 // Row maximum over N raw accumulator words (biased integers compare like the integers themselves).
-// mw: bit i set = key i of this chunk is masked.
-template <bool kMixed, int N>
-__device__ __forceinline__ void chunk_max(const uint32_t (&r)[N], uint32_t mw, int& max_a, int& max_b) {
+template <int N>
+__device__ __forceinline__ void chunk_max(const uint32_t (&r)[N], int& max_a, int& max_b) {
 #pragma unroll
   for (int i = 0; i < N; i += 4) {
-    int a = static_cast<int>(r[i]), b = static_cast<int>(r[i + 1]), c = static_cast<int>(r[i + 2]), d = static_cast<int>(r[i + 3]);
-    if (kMixed) {
-      if ((mw >> i) & 1u) a = INT_MIN;
-      if ((mw >> (i + 1)) & 1u) b = INT_MIN;
-      if ((mw >> (i + 2)) & 1u) c = INT_MIN;
-      if ((mw >> (i + 3)) & 1u) d = INT_MIN;
-    }
-    max_a = max(max_a, max(a, b));
-    max_b = max(max_b, max(c, d));
+    max_a = max(max_a, max(static_cast<int>(r[i]), static_cast<int>(r[i + 1])));
+    max_b = max(max_b, max(static_cast<int>(r[i + 2]), static_cast<int>(r[i + 3])));
   }
 }
 
 // N scores -> N probabilities (summed into two independent packed accumulators) -> N/4 words of
 // packed bytes holding -rn(128 p) (or rn(255 p)).  x = raw accumulator read as float = kMagic + s.
 // kCap: p is limited to p_cap before it is quantised (the static policy clips at its top level, fmha_i8_quant_deviation.py:38-43).
-template <bool kMixed, int N, bool kCap = false>
-__device__ __forceinline__ void chunk_exp_pack(const uint32_t (&r)[N], uint32_t mw, const float2 c2, const float2 neg_hi,
+template <int N, bool kCap = false>
+__device__ __forceinline__ void chunk_exp_pack(const uint32_t (&r)[N], const float2 c2, const float2 neg_hi,
                                                const float2 p_mul_f, float2 (&sum)[2], uint32_t (&packed)[N / 4], const float p_cap = 0.f) {
   const float2 magic2 = make_float2(kMagic, kMagic);
 #pragma unroll
   for (int g = 0; g < N / 4; ++g) {
-    float2 x01 = make_float2(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]));
-    float2 x23 = make_float2(__uint_as_float(r[4 * g + 2]), __uint_as_float(r[4 * g + 3]));
-    if (kMixed) {
-      if ((mw >> (4 * g)) & 1u) x01.x = -INFINITY;
-      if ((mw >> (4 * g + 1)) & 1u) x01.y = -INFINITY;
-      if ((mw >> (4 * g + 2)) & 1u) x23.x = -INFINITY;
-      if ((mw >> (4 * g + 3)) & 1u) x23.y = -INFINITY;
-    }
+    const float2 x01 = make_float2(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]));
+    const float2 x23 = make_float2(__uint_as_float(r[4 * g + 2]), __uint_as_float(r[4 * g + 3]));
     const float2 a01 = __ffma2_rn(x01, c2, neg_hi);
     const float2 a23 = __ffma2_rn(x23, c2, neg_hi);
     float2 p01 = make_float2(ex2_approx(a01.x), ex2_approx(a01.y));
@@ -432,8 +420,9 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it);
       return;
     }
-    const UnitInfo* info = &ctl->info[buf];
-    const int n_live = info->n_live;
+    const int n_live = ctl->info[buf].n_live;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));     // only the tile count is needed here
     // Policy launch: the row's maximum over ALL keys and its exp-sum come from the statistics launch; one scale per
     // row for the whole unit, no tile maximum, no exchange (fmha_i8_quant_deviation.py:62-121).
     RowConsts kp;
@@ -454,10 +443,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       const uint32_t g = g0 + static_cast<uint32_t>(j);
       const uint32_t sb = g % SBufs<D>::n;                       // S accumulator of this step
       const uint32_t tS = tS0 + sb * kTile;
-      // (read before the wait: none of it depends on S)
-      const bool mixed = info->mixed[j] != 0;
-      // the 64 mask bits of my keys (only looked at on the mixed path)
-      const uint32_t* mwords = &info->maskbits[4 * info->live[j] + 2 * half];
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->s_full[sb]), (g / SBufs<D>::n) & 1u, abort_flag))) {
         raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_S_READY, g);
         return;
@@ -482,30 +467,20 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       } else {
       // ---- pass 1: biased integer maximum of my 64 columns (inc/fmha_i8.cuh:183-206)
       int max_a = INT_MIN, max_b = INT_MIN;
-      if (!mixed) {
-        // two tensor-memory round trips (a round trip costs about as much as the whole arithmetic of this pass), two
-        // 16-column loads in flight each time: 32 registers of data live instead of the 48 that one 32-column load
-        // plus the prefetch for pass 2 would need
-        tmem_ld16_issue(tS, ra);
-        tmem_ld16_issue(tS + 16, rb);
-        tmem_ld_fence(ra); tmem_ld_fence(rb);
-        chunk_max<false, 16>(ra, 0u, max_a, max_b);
-        tmem_ld16_issue(tS + 32, ra);
-        chunk_max<false, 16>(rb, 0u, max_a, max_b);
-        tmem_ld16_issue(tS + 48, rb);
-        tmem_ld_fence(ra); tmem_ld_fence(rb);
-        chunk_max<false, 16>(ra, 0u, max_a, max_b);
-        tmem_ld16_issue(tS + c0 * 16, ra);                             // first chunk of pass 2, in flight during the exchange
-        chunk_max<false, 16>(rb, 0u, max_a, max_b);
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          tmem_ld16_issue(tS + c * 16, ra);
-          tmem_ld_fence(ra);
-          chunk_max<true, 16>(ra, (mwords[c >> 1] >> ((c & 1) * 16)) & 0xFFFFu, max_a, max_b);
-        }
-        tmem_ld16_issue(tS + c0 * 16, ra);
-      }
+      // two tensor-memory round trips (a round trip costs about as much as the whole arithmetic of this pass), two
+      // 16-column loads in flight each time: 32 registers of data live instead of the 48 that one 32-column load
+      // plus the prefetch for pass 2 would need
+      tmem_ld16_issue(tS, ra);
+      tmem_ld16_issue(tS + 16, rb);
+      tmem_ld_fence(ra); tmem_ld_fence(rb);
+      chunk_max<16>(ra, max_a, max_b);
+      tmem_ld16_issue(tS + 32, ra);
+      chunk_max<16>(rb, max_a, max_b);
+      tmem_ld16_issue(tS + 48, rb);
+      tmem_ld_fence(ra); tmem_ld_fence(rb);
+      chunk_max<16>(ra, max_a, max_b);
+      tmem_ld16_issue(tS + c0 * 16, ra);                             // first chunk of pass 2, in flight during the exchange
+      chunk_max<16>(rb, max_a, max_b);
       const int mine = max(max_a, max_b);
       // ---- exchange with the thread that owns the other half of this row
       int* xrow = &ctl->xmax[chain][n & 1u][0][row];
@@ -525,25 +500,14 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       // ---- pass 2: exp, row sum, requantise, P over columns already consumed (inc/fmha_i8.cuh:208-253)
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t packed[4];
-      if (!mixed) {
-        tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + cs) * 16, rb);
-        chunk_exp_pack<false, 16, kPolicy>(ra, 0u, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + c0 * 4, packed);
-        tmem_ld_fence(rb); tmem_ld16_issue(tS + (c0 + 2 * cs) * 16, ra);
-        chunk_exp_pack<false, 16, kPolicy>(rb, 0u, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + cs) * 4, packed);
-        tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + 3 * cs) * 16, rb);
-        chunk_exp_pack<false, 16, kPolicy>(ra, 0u, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 2 * cs) * 4, packed);
-        tmem_ld_fence(rb);
-        chunk_exp_pack<false, 16, kPolicy>(rb, 0u, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 3 * cs) * 4, packed);
-      } else {
-        tmem_ld_fence(ra);
-#pragma unroll 1
-        for (int i = 0; i < 4; ++i) {
-          const int c = c0 + i * cs;
-          if (i > 0) { tmem_ld16_issue(tS + c * 16, ra); tmem_ld_fence(ra); }
-          chunk_exp_pack<true, 16, kPolicy>(ra, (mwords[c >> 1] >> ((c & 1) * 16)) & 0xFFFFu, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
-          tmem_st4(tP + c * 4, packed);
-        }
-      }
+      tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + cs) * 16, rb);
+      chunk_exp_pack<16, kPolicy>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + c0 * 4, packed);
+      tmem_ld_fence(rb); tmem_ld16_issue(tS + (c0 + 2 * cs) * 16, ra);
+      chunk_exp_pack<16, kPolicy>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + cs) * 4, packed);
+      tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + 3 * cs) * 16, rb);
+      chunk_exp_pack<16, kPolicy>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 2 * cs) * 4, packed);
+      tmem_ld_fence(rb);
+      chunk_exp_pack<16, kPolicy>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 3 * cs) * 4, packed);
       // ---- publish the row statistics of this step for the merge threads
       const int slot = static_cast<int>(g & 3u);
       const float part = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
@@ -561,8 +525,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       FMHA_STAMP(16 + warp, n);
     }
     g0 += static_cast<uint32_t>(n_live);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));     // this warp is done with the unit's mask information
   }
 }
 
@@ -810,15 +772,14 @@ __device__ __forceinline__ bool issuer_wait(IssuerErr& e, uint32_t bar, uint32_t
 
 template <int D>
 __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
-                                              const uint32_t q_smem, const uint32_t k_smem, const uint32_t bias_a_smem, const uint32_t bias_b_smem,
+                                              const uint32_t q_smem, const uint32_t k_smem, uint8_t* bias_a,
                                               const int first_unit, const int unit_step) {
   using Cfg = FwdCfg<D>;
   constexpr uint32_t NK = Cfg::kStagesK, NQ = Cfg::kQBufs;
   volatile int* abort_flag = &ctl->abort;
   constexpr uint32_t idesc_s = make_idesc_i8(kTile, false);   // S = Q.K^T : N = 128 keys, both K-major
-  constexpr uint32_t idesc_bias_s = make_idesc_f16(kTile);
-  const uint64_t d_bias_a = make_smem_desc_noswizzle(bias_a_smem, 128, 256);
-  const uint64_t d_bias_b = make_smem_desc_noswizzle(bias_b_smem, 128, 256);
+  constexpr uint32_t idesc_bias_s = make_idesc_bf16(kTile);
+  const uint64_t d_bias_a = make_smem_desc_noswizzle(smem_u32(bias_a), 128, 256);
   IssuerErr err;
   uint32_t g = 0, qn = 0;
   int it = 0;
@@ -826,25 +787,40 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   for (int u = first_unit; u < p.n_units && ok; u += unit_step, ++it) {
     const int buf = it % kInfoBufs;
     if (!issuer_wait<true>(err, smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO, it, abort_flag)) break;
-    const int n_live = ctl->info[buf].n_live;
-    __syncwarp();
-    if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));            // only the tile count is needed here
-    if (n_live == 0) continue;
+    const UnitInfo* info = &ctl->info[buf];
+    const int n_live = info->n_live;
     const uint32_t qb = qn % NQ;
+    if (n_live == 0) {
+      __syncwarp();
+      if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
+      continue;
+    }
     if (!issuer_wait<true>(err, smem_u32(&ctl->q_full[qb]), (qn / NQ) & 1u, FMHA_I8_DEV_WAIT_Q_LOAD, g, abort_flag)) break;
     const uint64_t dq = make_smem_desc(q_smem + qb * Cfg::kTileBytes, D);
+    const int8_t* mask_row = p.mask + static_cast<int64_t>(unit_geom(p, u).batch) * p.S;
     for (int j = 0; j < n_live; ++j, ++g) {
       const uint32_t sb = g % SBufs<D>::n, stage = g % NK;
       const uint64_t dk = make_smem_desc(k_smem + stage * Cfg::kTileBytes, D);
       const uint32_t tS = tmem_base + sb * kTile;
+      const bool mixed = info->mixed[j] != 0;
+      bool masked[4] = {};
+      if (mixed) {
+        const int key0 = info->live[j] * kTile + static_cast<int>(threadIdx.x & 31);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || __ldg(mask_row + key0 + 32 * i) != 0;
+      }
       // K first (it has normally been there for a while), then the accumulator: it still holds the partial output of
       // step g - n until the merge warps have drained it, and that hand-off is on the step-to-step critical path
       if (!issuer_wait<true>(err, smem_u32(&ctl->k_full[stage]), (g / NK) & 1u, FMHA_I8_DEV_WAIT_K_LOAD, g, abort_flag)) { ok = false; break; }
       if (g >= SBufs<D>::n && !issuer_wait(err, smem_u32(&ctl->s_free[sb]), ((g / SBufs<D>::n) - 1) & 1u, FMHA_I8_DEV_WAIT_O_FREE, g, abort_flag)) { ok = false; break; }
       FMHA_STAMP(15, g);
       tc_fence_after();
+      // the tile's preset operand: the common one, or this accumulator's own, which nothing has read since step g - n
+      const uint32_t b_index = mixed ? 1 + sb : 0u;
+      if (mixed) fill_mask_operand(bias_a + (1 + b_index) * kBiasBytes, masked);
+      const uint64_t d_bias_b = make_smem_desc_noswizzle(smem_u32(bias_a) + (1 + b_index) * kBiasBytes, 128, 256);
       if (elect_one()) {
-        mma_f16_ss(tS, d_bias_a, d_bias_b, idesc_bias_s, 0u);      // accumulator := 0x4B400000
+        mma_f16_ss(tS, d_bias_a, d_bias_b, idesc_bias_s, 0u);      // accumulator := 0x4B400000, masked keys -2^127
 #pragma unroll
         for (int kk = 0; kk < D / 32; ++kk)
           mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(dk, kk * 32), idesc_s, 1u);
@@ -855,6 +831,8 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       FMHA_STAMP(12, g);
     }
     if (!ok) break;
+    __syncwarp();
+    if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
     ++qn;
   }
   if (err.code != 0u && elect_one()) raise_status(abort_flag, p.status, err.code, err.tile);
@@ -870,7 +848,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   // O = P.V : V is an MN-major operand; one group of MMAs with N = head_dim output columns
   const uint32_t idesc_o = p.p_unsigned ? make_idesc_i8(D, true, true) : make_idesc_i8(D, true, false);
 #if FMHA_PV_BIAS_MMA
-  constexpr uint32_t idesc_bias = make_idesc_f16(D);
+  constexpr uint32_t idesc_bias = make_idesc_bf16(D);
   const uint64_t d_bias_a = make_smem_desc_noswizzle(bias_a_smem, 128, 256);
   const uint64_t d_bias_b = make_smem_desc_noswizzle(bias_b_smem, 128, 256);
 #endif
@@ -930,7 +908,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   uint8_t* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* bias_a = tiles + Cfg::kTilesBytesTotal;
   uint8_t* bias_b = bias_a + kBiasBytes;
-  Ctl* ctl = reinterpret_cast<Ctl*>(bias_b + kBiasBytes);
+  Ctl* ctl = reinterpret_cast<Ctl*>(bias_a + bias_bytes<D>());
   const uint32_t q_smem = smem_u32(tiles);
   const uint32_t k_smem = q_smem + NQ * Cfg::kTileBytes;
   const uint32_t v_smem = k_smem + NK * Cfg::kTileBytes;
@@ -978,7 +956,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
     tmem_relinquish();
   }
-  fill_bias_operands(bias_a, bias_b);
+  fill_bias_operands(bias_a, 1 + SBufs<D>::n);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1000,7 +978,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (warp == kWarpLoad) {
       loader_role<D>(p, ctl, &map_q, &map_k, &map_v, q_smem, k_smem, v_smem, first_unit, unit_step);
     } else if (warp == kWarpMmaS) {
-      s_issuer_role<D>(p, ctl, tmem_base, q_smem, k_smem, smem_u32(bias_a), smem_u32(bias_b), first_unit, unit_step);
+      s_issuer_role<D>(p, ctl, tmem_base, q_smem, k_smem, bias_a, first_unit, unit_step);
     } else if (warp == kWarpMmaO) {
       o_issuer_role<D>(p, ctl, tmem_base, v_smem, smem_u32(bias_a), smem_u32(bias_b), first_unit, unit_step);
     } else if (warp == kWarpScan) {

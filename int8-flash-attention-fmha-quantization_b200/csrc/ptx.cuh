@@ -318,7 +318,8 @@ __device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem] with fp16 operands and an fp32 accumulator (K = 16 per instruction).
+// D[tmem] (+)= A[smem] * B[smem] with fp16 (or bf16: the instruction descriptor says) operands and an fp32 accumulator
+// (K = 16 per instruction).
 __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -360,6 +361,8 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, int row_b
 __host__ __device__ constexpr uint32_t make_idesc_f16(int n) {
   return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
 }
+// The same with bf16 A and B (format 1).
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int n) { return make_idesc_f16(n) | (1u << 7) | (1u << 10); }
 // Descriptor of an unswizzled K-major operand made of 8-row x 16-byte core matrices (128 contiguous
 // bytes each): `lbo` = byte distance between core matrices that follow each other along K,
 // `sbo` = along M/N.

@@ -116,3 +116,26 @@ def test_few_query_rows(pkg, wl, oracle, torch_cuda, D, Sq, B, H, Sk, valid, uin
         view = [x.reshape(B * H, -1, D)[begin:begin + count].contiguous() for x in (q, k, v)]
         pkg.FMHAInferI8Cross(None, param, desc, *view, m, part, bh_begin=begin, bh_count=count, uint8_p=uint8_p)
         assert np.array_equal(part.cpu().numpy(), host[128:-128].reshape(B * H, -1)[begin:begin + count].ravel())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("amax_scale", [1e-6, 1.0, 1e4])
+def test_masked_keys_vanish_at_every_scale(pkg, wl, oracle, torch_cuda, D, amax_scale):
+    """Masked keys are pushed out of the scores by the preset of the accumulator: whatever the scale of the scores, and
+    where the masked keys hold the largest scores of all, they count for nothing.  Every pattern of the mask inside a tile."""
+    torch = torch_cuda
+    B, H, S = 6, 2, 448
+    q8, k8, v8, mask, amax = _tensors(wl, B, H, S, S, D, seed=D)
+    mask[0, 1:] = 1                                   # one key
+    mask[1, :-1] = 1                                  # the last key
+    mask[2, ::2] = 1
+    mask[3, 100:300] = 1                              # a whole tile and the ends of two
+    mask[4] = np.random.default_rng(0).random(S) < 0.97
+    k8 = np.where(mask[:, None, :, None] != 0, np.sign(q8.mean(2, keepdims=True)).astype(np.int8) * 127, k8)
+    v8 = np.where(mask[:, None, :, None] != 0, np.int8(127), v8)
+    amax = (amax[0] * amax_scale, amax[1], amax[2], amax[2])
+    q, k, v, m = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (q8, k8, v8, mask))
+    o = torch.zeros_like(q)
+    pkg.FMHAInferI8(None, pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptor(B, S, H, D), q, k, v, m, o)
+    assert pkg.device_status()[0] == pkg.OK
+    assert_parity(o.cpu().numpy(), oracle.q128(q8, np.ascontiguousarray(k8), np.ascontiguousarray(v8), mask, amax))
