@@ -14,6 +14,7 @@
 #include "../../include/fmha_i8_c.h"
 #include "fmha_debug_sm100.cuh"
 #include "fmha_decode_sm100.cuh"
+#include "fmha_fwd64_sm100.cuh"
 #include "fmha_fwd_sm100.cuh"
 #include "fmha_quant_sm100.cuh"
 
@@ -120,6 +121,8 @@ int set_kernel_attributes(DeviceInfo* d) {
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>), fwd_smem_bytes<64>());
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>), fwd_smem_bytes<128>());
   set_decode_attributes(set);
+  set(reinterpret_cast<const void*>(&w64::fwd_kernel<false>), w64::kSmemBytes);
+  set(reinterpret_cast<const void*>(&w64::fwd_kernel<true>), w64::kSmemBytes);
   set(reinterpret_cast<const void*>(&quant_grid_kernel), kQuantGridSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&quant_cluster_kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   set(reinterpret_cast<const void*>(&debug_qk_kernel<64>), qk_smem_bytes<64>());
@@ -131,15 +134,18 @@ int set_kernel_attributes(DeviceInfo* d) {
   if (e != cudaSuccess) { cudaGetLastError(); return FMHA_I8_ERR_LAUNCH; }
   // The forward kernel redistributes registers with setmaxnreg; that only terminates if the launch
   // allocation is the one the targets were sized for.
-  cudaFuncAttributes fa64{}, fa128{}, fp64{}, fp128{};
+  cudaFuncAttributes fa64{}, fa128{}, fp64{}, fp128{}, fw{}, fwp{};
   if (cudaFuncGetAttributes(&fa64, reinterpret_cast<const void*>(&fmha_fwd_kernel<64, false>)) != cudaSuccess ||
       cudaFuncGetAttributes(&fa128, reinterpret_cast<const void*>(&fmha_fwd_kernel<128, false>)) != cudaSuccess ||
       cudaFuncGetAttributes(&fp64, reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>)) != cudaSuccess ||
       cudaFuncGetAttributes(&fp128, reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>)) != cudaSuccess ||
+      cudaFuncGetAttributes(&fw, reinterpret_cast<const void*>(&w64::fwd_kernel<false>)) != cudaSuccess ||
+      cudaFuncGetAttributes(&fwp, reinterpret_cast<const void*>(&w64::fwd_kernel<true>)) != cudaSuccess ||
+      fw.numRegs != w64::kLaunchRegs || fwp.numRegs != w64::kLaunchRegs ||
       fa64.numRegs != kLaunchRegs || fa128.numRegs != kLaunchRegs || fp64.numRegs != kLaunchRegs || fp128.numRegs != kLaunchRegs) {
     cudaGetLastError();
-    std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d/%d registers per thread, expected %d; refusing to launch\n",
-                 fa64.numRegs, fa128.numRegs, kLaunchRegs);
+    std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d/%d registers per thread, expected %d, and %d, expected %d; refusing to launch\n",
+                 fa64.numRegs, fa128.numRegs, kLaunchRegs, fw.numRegs, w64::kLaunchRegs);
     return FMHA_I8_ERR_LAUNCH;
   }
   d->attr_set = true;
@@ -265,6 +271,17 @@ int launch_kernel(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cud
   return FMHA_I8_ERR_LAUNCH;
 }
 
+// Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  Cycles per key tile, measured: a CTA of
+// fmha_fwd_sm100.cuh works on one unit at a time, 1700 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5800 per
+// tile for all four, 5300 / 4700 / 3900 with three, two or one left in the last round.  (B16 H16 S256: 12.8 / 11.6 us; B8 H12
+// S512: 16.3 / 16.0; B4 H12 S512: 12.2 / 13.7; B2 H12 S1024: 19.5 / 23.3; B1 H8 S16384: 778 / 779.)
+bool use_workers(const FwdParams& p, int sm_count) {
+  const long long tiles = (p.S + kTile - 1) / kTile, round = static_cast<long long>(sm_count) * w64::kWorkers;
+  const long long last[w64::kWorkers + 1] = {0, 3900, 4700, 5300, 5800};
+  const long long rounds = p.n_units / round, left = (p.n_units % round + sm_count - 1) / sm_count;
+  return (rounds * 5800 + last[left]) * tiles < ((p.n_units + sm_count - 1) / sm_count) * (1700 * tiles + 1200);
+}
+
 template <int D, bool kPolicy = false>
 int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v) {
   CUtensorMap mq, mk, mv;
@@ -272,14 +289,18 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q,
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mk, k, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mv, v, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
-  // persistent CTAs: one per SM (tensor memory is allocated whole), each walking its share of the units
-  const unsigned grid = static_cast<unsigned>(p.n_units < dev->sm_count ? p.n_units : dev->sm_count);
   // Overlap pays where the launch latency is a visible part of the launch: up to four rounds of units (512 units of a
   // whole-row policy 65.0 -> 62.5 us).  Beyond that it gives nothing (B8 H32 S2048: 461 us either way) and where whole
   // K/V tiles stream through every few hundred ns it costs: CTAs then land on SMs in the order the launch before frees
   // them, neighbours that share a head are no longer neighbours on the chip (B256 H16 S256 D64: 132 -> 141 us).
   LaunchHow how;
   how.overlap = p.n_units <= 4 * dev->sm_count;
+  // persistent CTAs: one per SM (tensor memory is allocated whole), each walking its share of the units
+  const unsigned grid = static_cast<unsigned>(p.n_units < dev->sm_count ? p.n_units : dev->sm_count);
+  if constexpr (D == 64) {
+    if (use_workers(p, dev->sm_count))
+      return launch_kernel(w64::fwd_kernel<kPolicy>, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
+  }
   return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
 

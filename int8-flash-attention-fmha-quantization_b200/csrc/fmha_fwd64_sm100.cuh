@@ -1,0 +1,467 @@
+// The forward kernel at head_dim 64 for calls with many query tiles (use_workers() in fmha_api.cu draws the line; the others,
+// and head_dim 128, whose output row does not fit beside the scores, run fmha_fwd_sm100.cuh).  Same arithmetic, another
+// division of the work:
+//
+//   worker  = four warps that do everything for a query tile of their own: row maximum, exponentials, the fp32 running row
+//             and the epilogue, one thread per query row, nothing handed from thread to thread.  Four workers to a CTA, one CTA to
+//             an SM; worker w of CTA c walks units c + grid * w, then every (4 grid)-th.
+//   driver  = one warp per worker: mask scan, TMA copies, S = Q.K^T, P.V.
+//   tensor memory: 128 columns per worker.  S of a step; then its 8-bit P over the first 32 columns and P.V over the last 64.
+//
+// A worker's step is one serial chain -- S, maximum, exponentials, P.V, fold -- of 3600 cycles when it runs alone.  Four of them
+// on an SM hide each other's latencies; nobody waits for a stage that other threads own, which is what bounds the other kernel
+// on short sequences (its merge warps need 4500 cycles per unit of two steps whatever the other warps do).  What bounds this
+// one: issue slots and the exponential unit, 57 % and 55 % busy on long sequences, where a step takes 5800 cycles, i.e. 1450 per
+// SM.  An eighth of the exponentials is computed on the multiply-add pipe (all on the exponential unit: 2.5 % slower on
+// B8 H32 S2048; a quarter: 3 % slower).  Pass 2 reads eight columns at a time: with sixteen the 104 registers of a softmax
+// thread do not suffice, and the spills cost 4 to 9 %.
+// Measured against the other kernel: B32 H12 S512 (lengths 256..512) 45.2 -> 41.8 us, B256 H16 S256 (64..256) 115 -> 99,
+// B8 H32 S2048 401 -> 372, B4 H16 S1024 with the per-row policy 55 -> 47.8.
+#pragma once
+#include "fmha_fwd_sm100.cuh"
+
+namespace fmha {
+namespace w64 {
+constexpr int kD = 64;
+constexpr int kWorkers = 4;          // per CTA
+// Warps: four softmax warps per worker (their number modulo 4 is their lane quarter of tensor memory), then one driver per worker.
+constexpr int kSoftmaxWarps = 4 * kWorkers;
+constexpr int kWarps = kSoftmaxWarps + kWorkers;
+constexpr int kThreads = kWarps * 32;          // 640
+constexpr int kInfoBufs = 4;         // units of a worker whose information is resident at once
+// setmaxnreg moves registers inside the CTA's own launch allocation (registers per thread at launch x threads): a request
+// that does not fit blocks forever.  640 threads start with 96 registers each (the host checks this).
+constexpr int kLaunchRegs = 96;
+constexpr int kSoftmaxRegs = 104, kDriverRegs = 64;
+static_assert(kSoftmaxWarps * kSoftmaxRegs + kWorkers * kDriverRegs <= kWarps * kLaunchRegs,
+              "setmaxnreg targets exceed the CTA's register allocation: the kernel would hang");
+static_assert(kSoftmaxRegs >= kLaunchRegs && kDriverRegs <= kLaunchRegs, "the softmax warps gain registers, the drivers give");
+
+constexpr int kTileBytes = kTile * kD;
+constexpr int kStages = 2;                                     // K, V and Q tiles per worker
+constexpr int kWorkerBytes = 3 * kStages * kTileBytes;
+// A worker's tensor memory: 128 columns.  S of a step; then P over its first 32 columns and P.V over its last 64.
+constexpr uint32_t kOCol = 64;
+
+// What the workers need to know about a unit.  The list of key tiles is only used by the driver that writes it.
+struct UnitInfo {
+  int n_live;                         // key tiles with at least one unmasked key
+  int rows;                           // query rows of the unit: 128, fewer in a head's last tile
+  int64_t first_row;                  // of the slice's query rows, the unit's first
+  uint8_t live[kMaxTiles];            // indices of the live key tiles, ascending
+  uint8_t mixed[kMaxTiles];           // 1 = that live tile has masked keys too
+};
+struct WorkerCtl {
+  uint64_t q_full[kStages], k_full[kStages], v_full[kStages];
+  uint64_t s_full, s_free;            // S has completed / its P.V has been drained
+  uint64_t p_ready, o_full;           // P is written (and S consumed) / P.V has completed
+  uint64_t info_full[kInfoBufs], info_empty[kInfoBufs];
+  UnitInfo info[kInfoBufs];
+};
+struct Ctl {
+  uint32_t tmem_base;
+  int abort;
+  WorkerCtl w[kWorkers];
+};
+
+// Operands of the preset MMA (see fill_bias_operands): A, B, and one B per worker for tiles with masked keys.  Only the first
+// two of the K = 16 columns are not zero, so the second core matrix of every row group is one and the same stretch of zeros.
+constexpr int kPresetBytes = kTile * 16;
+constexpr int kPresets = 2 + kWorkers, kPresetBytesTotal = (kPresets + 1) * kPresetBytes;
+__device__ __forceinline__ void fill_presets(uint8_t* preset) {
+  for (int i = threadIdx.x; i < (kPresets + 1) * kTile; i += blockDim.x)
+    reinterpret_cast<uint4*>(preset)[i] = make_uint4(i < kTile ? kBiasA : i < kPresets * kTile ? kBiasB : 0u, 0u, 0u, 0u);
+  fence_proxy_async_smem();
+}
+__device__ __forceinline__ uint64_t preset_desc(uint32_t preset_smem, uint32_t operand) {
+  return make_smem_desc_noswizzle(preset_smem + operand * kPresetBytes, (kPresets - operand) * kPresetBytes, 128);
+}
+
+constexpr size_t kSmemBytes = 1024 + kWorkers * kWorkerBytes + kPresetBytesTotal + sizeof(Ctl);
+
+// The sequence of units one worker walks.
+struct UnitWalk {
+  int first, step;
+};
+
+// ---------------------------------------------------------------------------------------------- softmax role
+// One thread = one query row: its scores, probabilities, fp32 running output row, maximum and sum.
+template <bool kPolicy>
+__device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_worker, const UnitWalk walk) {
+  WorkerCtl* ctl = &all->w[worker];
+  const int lane = threadIdx.x & 31, quad = (threadIdx.x >> 5) & 3;
+  const int row = quad * 32 + lane;
+  const uint32_t tS = tmem_worker + (static_cast<uint32_t>(quad * 32) << 16);
+  volatile int* abort_flag = &all->abort;
+  const bool stats_only = !kPolicy && p.row_stats_out != nullptr;
+
+  uint32_t g = 0;                               // steps so far
+  auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
+    if (__all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag))) return true;
+    raise_status(abort_flag, p.status, code, g);
+    return false;
+  };
+  int it = 0;
+#pragma unroll 1
+  for (int u = walk.first; u < p.n_units; u += walk.step, ++it) {
+    const int buf = it % kInfoBufs;
+    if (!wait_or_fail(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO)) return;
+    const int n_live = ctl->info[buf].n_live;
+    float2 o2[kD / 2];
+#pragma unroll
+    for (int i = 0; i < kD / 2; ++i) o2[i] = make_float2(0.f, 0.f);
+    float m_run = -INFINITY, l_run = 0.f;
+    int imax_run = static_cast<int>(kMagicBits);          // statistics launch: biased integer row maximum over all tiles
+    RowConsts k;                                          // (policy launch: constant over a unit)
+    float p_cap = 0.f;
+    // this thread's output row, -1 past the last row of the head (looked up where it is needed: nothing of it stays in registers)
+    auto output_row = [&]() -> int64_t { return row < ctl->info[buf].rows ? ctl->info[buf].first_row + row : -1; };
+    if (kPolicy) {
+      const int64_t out_row = output_row();
+      // Policy launch: the row's maximum over ALL keys and its exp-sum come from the statistics launch; one scale per
+      // row for the whole unit (fmha_i8_quant_deviation.py:62-121).
+      float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
+      if (out_row >= 0) st = __ldg(&p.row_stats_in[out_row]);
+      l_run = st.y;
+      const float l_row = st.y > 0.f ? st.y : 1.f;
+      // dynamic: P8 = rn(levels * e); static: P8 = min(rn(levels * (e / l) / s_max), levels)
+      const float mul = (p.p_static_mul != 0.f) ? p.p_static_mul / l_row : p.p_row_mul;
+      k = row_consts(__float_as_int(st.x), p.c2, p.row_scale, p.scale_qk, mul);
+      p_cap = p.p_levels / k.p_mul_f.x;       // an exponential above this would quantise beyond the top level
+    }
+
+#pragma unroll 1
+    for (int j = 0; j < n_live; ++j, ++g) {
+      if (!wait_or_fail(smem_u32(&ctl->s_full), g & 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
+      tc_fence_after();
+      FMHA_STAMP(quad == 0 ? worker * 4 + 0 : 47, g);
+      if (!kPolicy) {
+        // ---- pass 1: biased integer maximum of the row (inc/fmha_i8.cuh:183-206)
+        int max_a = INT_MIN, max_b = INT_MIN;
+        uint32_t ra[16], rb[16];
+        tmem_ld16_issue(tS, ra);
+        tmem_ld16_issue(tS + 16, rb);
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+          tmem_ld_fence(ra); tmem_ld_fence(rb);
+          chunk_max<16>(ra, max_a, max_b);
+          if (c < 6) tmem_ld16_issue(tS + (c + 2) * 16, ra);
+          chunk_max<16>(rb, max_a, max_b);
+          if (c < 6) tmem_ld16_issue(tS + (c + 3) * 16, rb);
+        }
+        const int imax = max(max_a, max_b);
+        if (stats_only) imax_run = (j == 0) ? imax : max(imax_run, imax);
+        k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, p.p_mul);
+      }
+      FMHA_STAMP(quad == 0 ? worker * 4 + 1 : 47, g);
+
+      // ---- pass 2: exp, row sum, requantise (inc/fmha_i8.cuh:208-253); the bytes go over columns already consumed
+      float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      uint32_t ra[8], rb[8], packed[2];
+      tmem_ld8_issue(tS, ra);
+#pragma unroll
+      for (uint32_t c = 0; c < 16; c += 2) {
+        tmem_ld_fence(ra);
+        tmem_ld8_issue(tS + (c + 1) * 8, rb);
+        chunk_exp_pack<8, kPolicy, 0>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
+        tmem_st2(tS + c * 2, packed);
+        tmem_ld_fence(rb);
+        if (c < 14) tmem_ld8_issue(tS + (c + 2) * 8, ra);
+        chunk_exp_pack<8, kPolicy, 1>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
+        tmem_st2(tS + c * 2 + 2, packed);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(smem_u32(stats_only ? &ctl->s_free : &ctl->p_ready));
+      FMHA_STAMP(quad == 0 ? worker * 4 + 2 : 47, g);
+
+      // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304), while P.V is under way
+      float e_old = 1.f, e_cur = 1.f;                                  // policy launch: every tile of a row has the same scale
+      if (!kPolicy) {
+        const float m_new = fmaxf(m_run, k.m_tile);
+        e_old = __expf(m_run - m_new);                                 // 0 on the first tile (m_run = -inf)
+        e_cur = clear_low2(__expf(k.m_tile - m_new));                  // 22 significant bits: kMagic*e_cur is exact
+        l_run = fmaf(e_old, l_run, e_cur * (k.f * ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y))));
+        m_run = m_new;
+      }
+      if (stats_only) continue;                                        // no output is wanted: there is no P.V
+      const float es = p.o_sign * e_cur;                               // the accumulator holds o_sign * (P.V)
+      const float2 neg_ec = make_float2(es, es), e_bias = make_float2(-es * kMagic, -es * kMagic);
+      const float2 e_old2 = make_float2(e_old, e_old);
+
+      // ---- P.V of this step into the running row (inc/fmha_i8.cuh:306-310)
+      if (!wait_or_fail(smem_u32(&ctl->o_full), g & 1u, FMHA_I8_DEV_WAIT_O_READY)) return;
+      tc_fence_after();
+      FMHA_STAMP(quad == 0 ? worker * 4 + 3 : 47, g);
+#pragma unroll
+      for (int c = 0; c < kD / 16; ++c) {
+        uint32_t r[16];
+        tmem_ld16_issue(tS + kOCol + c * 16, r);
+        tmem_ld_fence(r);
+        if (c == kD / 16 - 1) {
+          // the last columns are in registers: the driver may go on with the next S
+          tc_fence_before();
+          mbar_arrive(smem_u32(&ctl->s_free));
+        }
+        drain_chunk<16>(r, o2 + c * 8, neg_ec, e_bias, e_old2);
+      }
+    }
+
+    // ---- the unit is finished
+    const int64_t out_row = output_row();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
+    if (stats_only) {
+      // the row's maximum and exp-sum over all keys, for the policy launch that follows
+      if (out_row >= 0) p.row_stats_out[out_row] = make_float2(__int_as_float(imax_run), l_run);
+      continue;
+    }
+    // policy launch: the accumulated integer sum becomes the output through one factor per row: out_mul (/ l for the per-row policy)
+    if (kPolicy && p.p_static_mul != 0.f) l_run = l_run > 0.f ? 1.f : 0.f;
+    if (n_live == 0) l_run = 0.f;
+    const float inv = l_run > 0.f ? __frcp_rn(l_run) : 0.f;
+    if (p.amax_out != nullptr) {
+      // calibration: only the largest magnitude of the unquantised output is wanted (the reference takes o_amax from its
+      // fp32 CPU result, test_fmha_i8.cpp:161); non-negative floats order like their bit patterns
+      float mx = 0.f;
+#pragma unroll
+      for (int i = 0; i < kD / 2; ++i) mx = fmaxf(mx, fmaxf(fabsf(o2[i].x * inv), fabsf(o2[i].y * inv)));
+      const unsigned bits = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(out_row >= 0 ? mx * p.amax_scale : 0.f));
+      if (lane == 0 && bits != 0u) atomicMax(reinterpret_cast<unsigned*>(p.amax_out), bits);
+      continue;
+    }
+    // normalise, requantise, store (inc/fmha_i8.cuh:318-332)
+    if (out_row >= 0) {
+      int8_t* dst = p.o + out_row * kD;
+      // rn(clamp(x)) through the magic number: x + 1.5*2^23 has the integer nearest to x in its low bits (the low byte is the
+      // two's-complement integer), and clamping commutes with the addition; bytes gathered with PRMT
+      const float scale = p.scale_v_out * inv;
+      const float2 sc2 = make_float2(scale, scale), magic2 = make_float2(kMagic, kMagic);
+#pragma unroll
+      for (int c = 0; c < kD / 32; ++c) {
+        uint32_t wide[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float2 a = __ffma2_rn(o2[c * 16 + i * 2], sc2, magic2), b = __ffma2_rn(o2[c * 16 + i * 2 + 1], sc2, magic2);
+          a.x = fminf(fmaxf(a.x, kMagic - 127.f), kMagic + 127.f); a.y = fminf(fmaxf(a.y, kMagic - 127.f), kMagic + 127.f);
+          b.x = fminf(fmaxf(b.x, kMagic - 127.f), kMagic + 127.f); b.y = fminf(fmaxf(b.y, kMagic - 127.f), kMagic + 127.f);
+          wide[i] = __byte_perm(__byte_perm(__float_as_uint(a.x), __float_as_uint(a.y), 0x0040),
+                                __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x0040), 0x5410);
+        }
+        // 32-byte stores: a warp's rows are 64 bytes apart, so every store touches 32 lines whatever its width
+        if (p.o_wide) {
+          st_global_v8(dst + c * 32, wide);
+        } else {
+          *reinterpret_cast<uint4*>(dst + c * 32) = make_uint4(wide[0], wide[1], wide[2], wide[3]);
+          *reinterpret_cast<uint4*>(dst + c * 32 + 16) = make_uint4(wide[4], wide[5], wide[6], wide[7]);
+        }
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- driver
+// One warp per worker, run warp-wide (every lane waits and counts, one elected lane issues).  Per step: S of the step, then --
+// while the softmax warps work -- the mask scan and the copies of the step after it, then P.V.  No barrier guards the reuse of
+// a stage: when step g + 1 is loaded, P.V of step g - 1 has been drained.
+struct DriverStep {
+  int tile;                  // key tile, -1: no more steps
+  bool mixed;                // it has masked keys
+  uint32_t q_use;            // which Q tile of the worker it uses
+  const int8_t* mask_row;
+};
+__device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const int worker, const CUtensorMap* map_q, const CUtensorMap* map_k,
+                                            const CUtensorMap* map_v, const uint32_t tmem_worker, const uint32_t worker_smem, uint8_t* presets,
+                                            const UnitWalk walk) {
+  WorkerCtl* ctl = &all->w[worker];
+  volatile int* abort_flag = &all->abort;
+  const int lane = threadIdx.x & 31;
+  const uint32_t k_smem = worker_smem, v_smem = worker_smem + kStages * kTileBytes, q_smem = worker_smem + 2 * kStages * kTileBytes;
+  constexpr uint32_t idesc_s = make_idesc_i8(kTile, false);       // S = Q.K^T : N = 128 keys, both K-major
+  constexpr uint32_t idesc_preset_s = make_idesc_bf16(kTile), idesc_preset_o = make_idesc_bf16(kD);
+  const uint32_t idesc_o = p.p_unsigned ? make_idesc_i8(kD, true, true) : make_idesc_i8(kD, true, false);     // P.V : V is an MN-major operand
+  const uint32_t preset_smem = smem_u32(presets);
+  const uint64_t d_a = preset_desc(preset_smem, 0), d_b = preset_desc(preset_smem, 1);
+  const bool no_pv = p.row_stats_out != nullptr;
+  const int n_tiles = (p.S + kTile - 1) / kTile;
+  uint32_t fail = 0u, g = 0;
+  auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
+    if (__all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag))) return true;
+    fail = code;
+    return false;
+  };
+
+  // the step being loaded
+  int u = walk.first - walk.step, it = -1, j = 0, n_live = 0;
+  UnitGeom geo{};
+  uint32_t loaded = 0, q_loaded = 0;
+  auto load_next = [&]() -> DriverStep {
+    DriverStep s{-1, false, 0u, nullptr};
+    while (j >= n_live) {
+      u += walk.step;
+      if (u >= p.n_units) { u = p.n_units - walk.step; n_live = 0; return s; }
+      ++it;
+      const int buf = it % kInfoBufs;
+      if (it >= kInfoBufs && !wait(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), FMHA_I8_DEV_WAIT_INFO)) return s;
+      geo = unit_geom(p, u);
+      UnitInfo* info = &ctl->info[buf];
+      scan_mask_warp(info, p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
+      if (elect_one()) {
+        info->rows = min(kTile, p.Sq - geo.q_row0);
+        info->first_row = static_cast<int64_t>(geo.bh_local) * p.Sq + geo.q_row0;
+      }
+      __syncwarp();
+      if (elect_one()) mbar_arrive(smem_u32(&ctl->info_full[buf]));
+      n_live = info->n_live;
+      j = 0;
+    }
+    const UnitInfo* info = &ctl->info[it % kInfoBufs];
+    s.tile = info->live[j];
+    s.mixed = info->mixed[j] != 0;
+    s.mask_row = p.mask + static_cast<int64_t>(geo.batch) * p.S;
+    const uint32_t st = loaded % kStages;
+    if (j == 0) ++q_loaded;
+    s.q_use = q_loaded - 1u;
+    if (elect_one()) {
+      mbar_arrive_expect_tx(smem_u32(&ctl->k_full[st]), kTileBytes);
+      tma_load_3d(k_smem + st * kTileBytes, map_k, smem_u32(&ctl->k_full[st]), 0, s.tile * kTile, geo.bh_local);
+      if (j == 0) {
+        const uint32_t bar_q = smem_u32(&ctl->q_full[s.q_use % kStages]);
+        mbar_arrive_expect_tx(bar_q, kTileBytes);
+        tma_load_3d(q_smem + (s.q_use % kStages) * kTileBytes, map_q, bar_q, 0, geo.q_row0, geo.bh_local);
+      }
+      if (!no_pv) {
+        mbar_arrive_expect_tx(smem_u32(&ctl->v_full[st]), kTileBytes);
+        tma_load_3d(v_smem + st * kTileBytes, map_v, smem_u32(&ctl->v_full[st]), 0, s.tile * kTile, geo.bh_local);
+      }
+    }
+    __syncwarp();
+    ++j;
+    ++loaded;
+    return s;
+  };
+
+  DriverStep cur = load_next();
+  while (cur.tile >= 0 && fail == 0u) {
+    const uint32_t st = g % kStages;
+    bool masked[4] = {};
+    if (cur.mixed) {
+      const int key0 = cur.tile * kTile + lane;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || __ldg(cur.mask_row + key0 + 32 * i) != 0;
+    }
+    if (!wait(smem_u32(&ctl->q_full[cur.q_use % kStages]), (cur.q_use / kStages) & 1u, FMHA_I8_DEV_WAIT_Q_LOAD)) break;
+    if (!wait(smem_u32(&ctl->k_full[st]), (g / kStages) & 1u, FMHA_I8_DEV_WAIT_K_LOAD)) break;
+    if (g > 0u && !wait(smem_u32(&ctl->s_free), (g - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
+    tc_fence_after();
+    FMHA_STAMP(16 + worker * 4 + 0, g);
+    // the tile's preset operand: the common one, or this worker's own, which nothing has read since the last S
+    const uint32_t operand = cur.mixed ? 2u + static_cast<uint32_t>(worker) : 1u;
+    if (cur.mixed) fill_mask_operand(presets + operand * kPresetBytes, masked, 128);
+    const uint64_t d_preset = preset_desc(preset_smem, operand);
+    const uint64_t dq = make_smem_desc(q_smem + (cur.q_use % kStages) * kTileBytes, kD), dk = make_smem_desc(k_smem + st * kTileBytes, kD);
+    if (elect_one()) {
+      mma_f16_ss(tmem_worker, d_a, d_preset, idesc_preset_s, 0u);      // accumulator := 0x4B400000, masked keys -2^127
+#pragma unroll
+      for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tmem_worker, desc_advance(dq, kk * 32), desc_advance(dk, kk * 32), idesc_s, 1u);
+      mma_commit(smem_u32(&ctl->s_full));
+    }
+    FMHA_STAMP(16 + worker * 4 + 1, g);
+    const DriverStep next = load_next();
+    if (fail != 0u) break;
+    if (!no_pv) {
+      const uint64_t dv = make_smem_desc(v_smem + st * kTileBytes, kD);
+      if (!wait(smem_u32(&ctl->v_full[st]), (g / kStages) & 1u, FMHA_I8_DEV_WAIT_V_LOAD)) break;
+      if (!wait(smem_u32(&ctl->p_ready), g & 1u, FMHA_I8_DEV_WAIT_P_READY)) break;
+      tc_fence_after();
+      FMHA_STAMP(16 + worker * 4 + 2, g);
+      if (elect_one()) {
+        mma_f16_ss(tmem_worker + kOCol, d_a, d_b, idesc_preset_o, 0u);
+#pragma unroll
+        for (int kk = 0; kk < kTile / 32; ++kk) mma_i8_ts(tmem_worker + kOCol, tmem_worker + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);
+        mma_commit(smem_u32(&ctl->o_full));
+      }
+      FMHA_STAMP(16 + worker * 4 + 3, g);
+    }
+    cur = next;
+    ++g;
+  }
+  if (fail != 0u) {
+    if (elect_one()) raise_status(abort_flag, p.status, fail, g);
+    // unwinding: let copies that are still in flight land before the CTA may exit
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) { /* about a millisecond */ }
+  }
+}
+
+// kPolicy: the launch that applies a whole-row P scaling policy from row statistics (see FwdParams::row_stats_in);
+// the product default, and the statistics launch, are kPolicy = false.
+template <bool kPolicy>
+__global__ void __launch_bounds__(kThreads, 1)
+fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+           const FwdParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  // The next launch of the stream may set itself up on SMs this one leaves free, and waits below for this one to finish
+  // before it reads anything.
+  grid_launch_dependents();
+  // tiles need 1024-byte alignment (swizzle atoms); the launch reserves the slack (pointer arithmetic on the shared array:
+  // the compiler then knows that everything derived from it is shared memory)
+  uint8_t* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* presets = tiles + kWorkers * kWorkerBytes;
+  Ctl* ctl = reinterpret_cast<Ctl*>(presets + kPresetBytesTotal);
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    ctl->abort = 0;
+    for (WorkerCtl& w : ctl->w) {
+      for (int s = 0; s < kStages; ++s) {
+        mbar_init(smem_u32(&w.q_full[s]), 1);
+        mbar_init(smem_u32(&w.k_full[s]), 1);
+        mbar_init(smem_u32(&w.v_full[s]), 1);
+      }
+      mbar_init(smem_u32(&w.s_full), 1);
+      mbar_init(smem_u32(&w.s_free), kTile);
+      mbar_init(smem_u32(&w.p_ready), kTile);
+      mbar_init(smem_u32(&w.o_full), 1);
+      for (int b = 0; b < kInfoBufs; ++b) {
+        mbar_init(smem_u32(&w.info_full[b]), 1);
+        mbar_init(smem_u32(&w.info_empty[b]), 4);
+      }
+    }
+    mbar_init_fence();
+    tma_prefetch_desc(&map_q);
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+  }
+  if (warp == kWarps - 1) {
+    __syncwarp();
+    tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
+    tmem_relinquish();
+  }
+  fill_presets(presets);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&ctl->tmem_base);
+  grid_dependency_wait();      // nothing above touches global memory
+
+  const int worker = warp < kSoftmaxWarps ? warp >> 2 : warp - kSoftmaxWarps;
+  const UnitWalk walk = {static_cast<int>(blockIdx.x + gridDim.x * worker), static_cast<int>(gridDim.x) * kWorkers};
+  const uint32_t tmem_worker = tmem_base + static_cast<uint32_t>(worker * kTile);
+  uint8_t* worker_smem = tiles + worker * kWorkerBytes;
+  if (warp < kSoftmaxWarps) {
+    setmaxnreg_inc<kSoftmaxRegs>();
+    w64::softmax_role<kPolicy>(p, ctl, worker, tmem_worker, walk);
+  } else {
+    setmaxnreg_dec<kDriverRegs>();
+    driver_role(p, ctl, worker, &map_q, &map_k, &map_v, tmem_worker, smem_u32(worker_smem), presets, walk);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kWarps - 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+}  // namespace w64
+}  // namespace fmha

@@ -143,10 +143,10 @@ constexpr int kInfoConsumers = 3 + kSoftmaxWarps + kMergeWarps;   // loader, two
 // launch and refuses otherwise); the targets per role (FwdRegs) add up to 28 x 72.
 constexpr int kLaunchRegs = 72;
 template <int D> struct FwdRegs {
-  // head_dim 128: the merge threads hold a 64-register half output row, the one-warp roles run lean (measured on C3:
-  // 104/40 is 2 % faster than 96/56).  head_dim 64: the output row is 32 registers; 88/72 is the split at which
+  // head_dim 128: the merge threads hold a 64-register half output row (B8 H32 S2048: 96/56 is 1.3 % faster than 104/40
+  // and as fast as 88/72).  head_dim 64: the output row is 32 registers; 88/72 is the split at which
   // ptxas reports no spills at all, and C5 runs 5 % faster with it than with 80/88 or 96/56, which both spill.
-  static constexpr int kSoftmax = 64, kMerge = (D == 128) ? 104 : 88, kOther = (D == 128) ? 40 : 72;
+  static constexpr int kSoftmax = 64, kMerge = (D == 128) ? 96 : 88, kOther = (D == 128) ? 56 : 72;
   static_assert(kSoftmaxWarps * kSoftmax + kMergeWarps * kMerge + 4 * kOther <= kFwdWarps * kLaunchRegs,
                 "setmaxnreg targets exceed the CTA's register allocation: the kernel would hang");
   static_assert(kSoftmax <= kLaunchRegs && kMerge >= kLaunchRegs, "the softmax warps give registers, the merge warps gain");
@@ -179,7 +179,7 @@ struct FwdParams {
   int S;                // keys per head (seq_len; seq_len_k when queries and keys differ in number)
   int Sq;               // query rows per head (== S for self-attention)
   int H, bh_begin, bh_count, q_tiles;
-  int n_units;          // bh_count * q_tiles work units, taken round-robin by the resident CTAs
+  int n_units;          // bh_count * q_tiles work units
   float row_scale;      // 1/sqrt(D), the reference's constant (inc/fmha_i8.cuh:71)
   float scale_qk;       // q_amax*k_amax/127^2 (inc/fmha_i8.cuh:72)
   float scale_v_out;    // v_amax/(o_amax*128) (inc/fmha_i8.cuh:318)
@@ -256,7 +256,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 // Builds one unit's view of its batch's padding mask: the list of live tiles and whether each has masked keys too.
 // Executed by ONE warp; a lane looks at 32 keys, four lanes make a tile.
-__device__ __forceinline__ void scan_mask_warp(UnitInfo* info, const int8_t* mask_row, int S, int n_tiles) {
+template <typename Info>
+__device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_row, int S, int n_tiles) {
   const int lane = threadIdx.x & 31;
   const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
   int n = 0;
@@ -299,10 +300,12 @@ __device__ __forceinline__ void fill_bias_operands(uint8_t* bias_a, int n_b) {
   fence_proxy_async_smem();
 }
 // Executed by one warp, lane l for keys l, 32 + l, 64 + l and 96 + l: the B operand of a tile with masked keys.
-__device__ __forceinline__ void fill_mask_operand(uint8_t* bias_b, const bool (&masked)[4]) {
+__device__ __forceinline__ void fill_mask_operand(uint8_t* bias_b, const bool (&masked)[4], const int group_bytes = 256) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    *reinterpret_cast<uint32_t*>(bias_b + bias_row_offset(32 * i + (threadIdx.x & 31))) = masked[i] ? kBiasBMasked : kBiasB;
+  for (int i = 0; i < 4; ++i) {
+    const int row = 32 * i + static_cast<int>(threadIdx.x & 31);
+    *reinterpret_cast<uint32_t*>(bias_b + (row >> 3) * group_bytes + (row & 7) * 16) = masked[i] ? kBiasBMasked : kBiasB;
+  }
   fence_proxy_async_smem();
   __syncwarp();
 }
@@ -317,10 +320,28 @@ __device__ __forceinline__ void chunk_max(const uint32_t (&r)[N], int& max_a, in
   }
 }
 
+// 2^a for two values a <= 0 on the multiply-add pipe: a = n + f with |f| <= 1/2, a degree-5 minimax polynomial for 2^f (fitted by
+// exchange; 2.1e-7 in fp32 arithmetic, the error bound of ex2.approx is 2^-22 = 2.4e-7), n added to the exponent.
+__device__ __forceinline__ float2 exp2_poly(float2 a) {
+  const float2 magic = make_float2(kMagic, kMagic), neg_magic = make_float2(-kMagic, -kMagic);
+  a.x = fmaxf(a.x, -126.f);
+  a.y = fmaxf(a.y, -126.f);
+  const float2 t = __fadd2_rn(a, magic);                    // n in the low bits
+  const float2 n = __fadd2_rn(t, neg_magic);
+  const float2 f = __fadd2_rn(a, make_float2(-n.x, -n.y));
+  float2 q = __ffma2_rn(f, make_float2(0.0013276472f, 0.0013276472f), make_float2(0.0096755410f, 0.0096755410f));
+  q = __ffma2_rn(q, f, make_float2(0.0555071309f, 0.0555071309f));
+  q = __ffma2_rn(q, f, make_float2(0.2402212024f, 0.2402212024f));
+  q = __ffma2_rn(q, f, make_float2(0.6931469440f, 0.6931469440f));
+  q = __ffma2_rn(q, f, make_float2(1.f, 1.f));
+  return make_float2(__uint_as_float(__float_as_uint(q.x) + (__float_as_uint(t.x) << 23)), __uint_as_float(__float_as_uint(q.y) + (__float_as_uint(t.y) << 23)));
+}
+
 // N scores -> N probabilities (summed into two independent packed accumulators) -> N/4 words of
 // packed bytes holding -rn(128 p) (or rn(255 p)).  x = raw accumulator read as float = kMagic + s.
 // kCap: p is limited to p_cap before it is quantised (the static policy clips at its top level, fmha_i8_quant_deviation.py:38-43).
-template <int N, bool kCap = false>
+// kPolyPairs: that many pairs of values per eight are computed by exp2_poly.
+template <int N, bool kCap = false, int kPolyPairs = 0>
 __device__ __forceinline__ void chunk_exp_pack(const uint32_t (&r)[N], const float2 c2, const float2 neg_hi,
                                                const float2 p_mul_f, float2 (&sum)[2], uint32_t (&packed)[N / 4], const float p_cap = 0.f) {
   const float2 magic2 = make_float2(kMagic, kMagic);
@@ -331,7 +352,7 @@ __device__ __forceinline__ void chunk_exp_pack(const uint32_t (&r)[N], const flo
     const float2 a01 = __ffma2_rn(x01, c2, neg_hi);
     const float2 a23 = __ffma2_rn(x23, c2, neg_hi);
     float2 p01 = make_float2(ex2_approx(a01.x), ex2_approx(a01.y));
-    float2 p23 = make_float2(ex2_approx(a23.x), ex2_approx(a23.y));
+    float2 p23 = (g & 1) < kPolyPairs ? exp2_poly(a23) : make_float2(ex2_approx(a23.x), ex2_approx(a23.y));
     if (kCap) {
       p01.x = fminf(p01.x, p_cap); p01.y = fminf(p01.y, p_cap);
       p23.x = fminf(p23.x, p_cap); p23.y = fminf(p23.y, p_cap);

@@ -139,3 +139,41 @@ def test_masked_keys_vanish_at_every_scale(pkg, wl, oracle, torch_cuda, D, amax_
     pkg.FMHAInferI8(None, pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptor(B, S, H, D), q, k, v, m, o)
     assert pkg.device_status()[0] == pkg.OK
     assert_parity(o.cpu().numpy(), oracle.q128(q8, np.ascontiguousarray(k8), np.ascontiguousarray(v8), mask, amax))
+
+
+# Calls at head_dim 64 with many query tiles run four workers to an SM: fewer units than workers, all workers busy, a last round with
+# one worker, several rounds; key tiles half beyond the sequence, sequences without a key, a mask with holes in every tile.
+@pytest.mark.parametrize("B,H,Sq,Sk,mask_p", [(50, 8, 64, 64, 0.0), (30, 13, 100, 192, 0.3), (37, 16, 128, 128, 0.0), (11, 9, 961, 448, 0.05)])
+@pytest.mark.parametrize("what", ["plain", "uint8", "row", "static", "amax"])
+def test_many_query_tiles_head_dim_64(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk, mask_p, what):
+    torch = torch_cuda
+    valid = np.random.default_rng(B).integers(1, Sk + 1, B)
+    valid[3] = 0
+    valid[4] = Sk
+    q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, 64, seed=B + Sk, mask_p=mask_p, valid=valid)
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    desc, param = pkg.AttnDataDescriptorX(B, Sq, Sk, H, 64), pkg.FMHAParamI8(*amax, 0.25)
+    o = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    scratch = torch.zeros(2 * B * H * Sq, device="cuda")
+    if what == "amax":
+        got = torch.zeros(1, device="cuda")
+        pkg.calibrate_o_amax(None, param, desc, q, k, v, m, got)
+        # the same arithmetic with a known scale: the largest output quantises to 127, and to no more with 1 % of head room
+        tops = []
+        for s in (1.0, 1.01):
+            pkg.FMHAInferI8Cross(None, pkg.FMHAParamI8(*amax[:3], float(got) * s, 1.0), desc, q, k, v, m, o[128:-128])
+            tops.append(int(o[128:-128].abs().max()))
+        assert tops[0] == 127 and tops[1] in (125, 126), tops
+        return
+    if what in ("row", "static"):
+        policy = pkg.POLICY_ROW if what == "row" else pkg.POLICY_STATIC
+        pkg.FMHAInferI8Policy(None, param, desc, q, k, v, m, o[128:-128], policy, scratch)
+        want = oracle.policy(q8, k8, v8, mask, (*amax, 0.25), oracle.POLICY_ROW if what == "row" else oracle.POLICY_STATIC)
+    else:
+        pkg.FMHAInferI8Cross(None, param, desc, q, k, v, m, o[128:-128], uint8_p=what == "uint8")
+        want = oracle.q128(q8, k8, v8, mask, amax, p_levels=255 if what == "uint8" else 128)
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    host = o.cpu().numpy()
+    assert np.all(host[:128] == 0x5A) and np.all(host[-128:] == 0x5A)
+    assert_parity(host[128:-128].reshape(q8.shape), want, what)
