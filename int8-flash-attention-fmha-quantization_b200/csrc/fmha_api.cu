@@ -34,6 +34,7 @@ int finish(int status) {
 
 constexpr int kMaxDevices = 64;
 
+constexpr int kClusterSizes = 3;
 struct DeviceInfo {
   int checked = 0;      // 0 = not yet, 1 = sm_100, -1 = something else
   unsigned* status = nullptr;
@@ -41,6 +42,7 @@ struct DeviceInfo {
   // it (besides the device status words), so the next host call can see the failure without synchronising.
   volatile unsigned* host_flag = nullptr;
   int sm_count = 0;
+  int max_clusters[kClusterSizes] = {};      // clusters of 2, 4, 8 CTAs of the forward kernel that are resident at once
   bool attr_set = false;
 };
 DeviceInfo g_dev[kMaxDevices];
@@ -147,6 +149,24 @@ int set_kernel_attributes(DeviceInfo* d) {
     std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d/%d registers per thread, expected %d, and %d, expected %d; refusing to launch\n",
                  fa64.numRegs, fa128.numRegs, kLaunchRegs, fw.numRegs, w64::kLaunchRegs);
     return FMHA_I8_ERR_LAUNCH;
+  }
+  for (int i = 0; i < kClusterSizes; ++i) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2u << i;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(d->sm_count / (2 << i) * (2 << i)));
+    cfg.blockDim = dim3(kFwdThreads);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n64 = 0, n128 = 0;
+    cfg.dynamicSmemBytes = fwd_smem_bytes<64>();
+    if (cudaOccupancyMaxActiveClusters(&n64, fmha_fwd_kernel<64, false>, &cfg) != cudaSuccess) n64 = 0;
+    cfg.dynamicSmemBytes = fwd_smem_bytes<128>();
+    if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128, false>, &cfg) != cudaSuccess) n128 = 0;
+    cudaGetLastError();
+    d->max_clusters[i] = n64 < n128 ? n64 : n128;
   }
   d->attr_set = true;
   return FMHA_I8_OK;
@@ -282,6 +302,23 @@ bool use_workers(const FwdParams& p, int sm_count) {
   return (rounds * 5800 + last[left]) * tiles < ((p.n_units + sm_count - 1) / sm_count) * (1700 * tiles + 1200);
 }
 
+// CTAs that share one unit (query tile), each with a part of its key tiles: for calls whose units leave most SMs idle, as long as
+// all clusters are resident at once (a second wave of them starts from nothing and costs 10 us).  In nanoseconds, measured: 950
+// per key tile of a CTA, and for cluster launch, two cluster barriers and the merge of the partial results through distributed
+// shared memory 2300 / 3000 / 4300 with 2 / 4 / 8 CTAs.  (Head_dim 64, us without -> with: B1 H8 S1024 Sq256 11.9 -> 9.1, B1 H4
+// S2048 Sq200 19.2 -> 10.5, B1 H2 S4096 34.9 -> 23.4, B1 H8 S8192 Sq64 64 -> 17.7; head_dim 128: B2 H16 S1984 Sq200 21.1 -> 16.8,
+// B1 H2 S16384 Sq128 131 -> 29.)
+int parts_of_a_unit(const FwdParams& p, const DeviceInfo* dev) {
+  constexpr int kOverhead[kClusterSizes] = {2300, 3000, 4300};
+  const int tiles = (p.S + kTile - 1) / kTile;
+  int best = 1, best_ns = 950 * tiles;
+  for (int i = 0; i < kClusterSizes; ++i) {
+    const int c = 2 << i, ns = 950 * ((tiles + c - 1) / c) + kOverhead[i];
+    if (p.n_units <= dev->max_clusters[i] && ns < best_ns) { best = c; best_ns = ns; }
+  }
+  return best;
+}
+
 template <int D, bool kPolicy = false>
 int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v) {
   CUtensorMap mq, mk, mv;
@@ -300,6 +337,14 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q,
   if constexpr (D == 64) {
     if (use_workers(p, dev->sm_count))
       return launch_kernel(w64::fwd_kernel<kPolicy>, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
+  }
+  p.parts = 1;
+  if (!kPolicy && !p.row_stats_out && !p.amax_out) p.parts = parts_of_a_unit(p, dev);
+  if (p.parts > 1) {
+    how.cluster = static_cast<unsigned>(p.parts);
+    how.overlap = true;
+    return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(static_cast<unsigned>(p.n_units * p.parts)), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream,
+                         how, mq, mk, mv, p);
   }
   return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }

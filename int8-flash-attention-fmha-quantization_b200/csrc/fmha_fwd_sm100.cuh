@@ -180,6 +180,7 @@ struct FwdParams {
   int Sq;               // query rows per head (== S for self-attention)
   int H, bh_begin, bh_count, q_tiles;
   int n_units;          // bh_count * q_tiles work units
+  int parts;            // 1: a CTA takes units of its own; more: that many CTAs, a cluster, share one unit, each a part of its key tiles
   float row_scale;      // 1/sqrt(D), the reference's constant (inc/fmha_i8.cuh:71)
   float scale_qk;       // q_amax*k_amax/127^2 (inc/fmha_i8.cuh:72)
   float scale_v_out;    // v_amax/(o_amax*128) (inc/fmha_i8.cuh:318)
@@ -205,7 +206,8 @@ struct FwdParams {
 // What every role needs to know about one work unit's padding mask.  kInfoBufs of these live in shared
 // memory: the scanner warp fills the ones of coming units while the current unit is being processed.
 struct UnitInfo {
-  int n_live;                         // key tiles with at least one unmasked key
+  int n_live;                         // key tiles with at least one unmasked key (of this CTA's part of them)
+  int begin;                          // this CTA's part begins here in the lists below
   uint8_t live[kMaxTiles];            // indices of the live key tiles, ascending
   uint8_t mixed[kMaxTiles];           // 1 = that live tile has masked keys too
 };
@@ -225,6 +227,7 @@ template <int NK, int NV> struct FwdCtl {
   float st_m[4][kTile], st_f[4][kTile], st_s0[4][kTile], st_s1[4][kTile];
   int st_i[4][kTile];                  // biased integer row maximum of the step's tile (for the statistics launch)
   int xmax[2][2][2][kTile];            // [chain][step parity][half][row]: biased integer maximum of that half row
+  float2 part[kTile];                  // row maximum and sum of a partial result (a unit shared by a cluster)
   UnitInfo info[kInfoBufs];
 };
 
@@ -255,35 +258,50 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 
 // Builds one unit's view of its batch's padding mask: the list of live tiles and whether each has masked keys too.
-// Executed by ONE warp; a lane looks at 32 keys, four lanes make a tile.
-template <typename Info>
-__device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_row, int S, int n_tiles) {
+// Executed by ONE warp; a lane looks at 32 keys, four lanes make a tile.  kGroups: groups of eight tiles whose loads are in
+// flight together (four for long masks: 128 tiles one group after the other take 5 us).
+template <int kGroups, typename Info>
+__device__ __forceinline__ int scan_mask_groups(Info* info, const uint32_t* words, int S, int n_tiles) {
   const int lane = threadIdx.x & 31;
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
   int n = 0;
-  for (int base = 0; base < n_tiles; base += 8) {
-    const int key0 = base * kTile + lane * 32;
-    uint32_t open = 0u, masked = 0xFFFFFFFFu;            // any unmasked key; any masked key (keys beyond S count as masked)
-    if (key0 < S) {  // S is a multiple of 64, so a 32-key group is entirely inside or outside
-      masked = 0u;
+#pragma unroll 1
+  for (int base0 = 0; base0 < n_tiles; base0 += 8 * kGroups) {
+    uint32_t open[kGroups], masked[kGroups];                     // any unmasked key; any masked key (keys beyond S count as masked)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t wv = __ldg(words + (key0 >> 2) + i);
-        masked |= wv;
-        open |= __vcmpeq4(wv, 0u);
+    for (int q = 0; q < kGroups; ++q) {
+      const int key0 = (base0 + 8 * q) * kTile + lane * 32;
+      open[q] = 0u;
+      masked[q] = 0xFFFFFFFFu;
+      if (key0 < S) {  // S is a multiple of 64, so a 32-key group is entirely inside or outside
+        masked[q] = 0u;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t wv = __ldg(words + (key0 >> 2) + i);
+          masked[q] |= wv;
+          open[q] |= __vcmpeq4(wv, 0u);
+        }
       }
     }
-    const uint32_t any_open = __ballot_sync(0xFFFFFFFFu, open != 0u), any_masked = __ballot_sync(0xFFFFFFFFu, masked != 0u);
-    const bool is_live = lane < 8 && ((any_open >> (4 * lane)) & 0xFu) != 0u;
-    const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, is_live);
-    if (is_live) {
-      const int pos = n + __popc(ballot & ((1u << lane) - 1u));
-      info->live[pos] = static_cast<uint8_t>(base + lane);
-      info->mixed[pos] = ((any_masked >> (4 * lane)) & 0xFu) != 0u ? 1 : 0;
+#pragma unroll
+    for (int q = 0; q < kGroups; ++q) {
+      const uint32_t any_open = __ballot_sync(0xFFFFFFFFu, open[q] != 0u), any_masked = __ballot_sync(0xFFFFFFFFu, masked[q] != 0u);
+      const bool is_live = lane < 8 && ((any_open >> (4 * lane)) & 0xFu) != 0u;
+      const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, is_live);
+      if (is_live) {
+        const int pos = n + __popc(ballot & ((1u << lane) - 1u));
+        info->live[pos] = static_cast<uint8_t>(base0 + 8 * q + lane);
+        info->mixed[pos] = ((any_masked >> (4 * lane)) & 0xFu) != 0u ? 1 : 0;
+      }
+      n += __popc(ballot);
     }
-    n += __popc(ballot);
   }
-  if (lane == 0) info->n_live = n;
+  return n;
+}
+template <typename Info>
+__device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_row, int S, int n_tiles) {
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
+  const int n = n_tiles <= 32 ? scan_mask_groups<1>(info, words, S, n_tiles) : scan_mask_groups<4>(info, words, S, n_tiles);
+  if ((threadIdx.x & 31) == 0) info->n_live = n;
   __syncwarp();
 }
 
@@ -553,7 +571,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
 // One thread = one half (D/2 columns) of the fp32 running output row of one query row, plus the running
 // maximum and the running sum of that row (kept by both threads of the row).
 template <int D, bool kPolicy>
-__device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
+__device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base, uint8_t* tiles,
                                            const int first_unit, const int unit_step) {
   constexpr int DH = D / 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -673,6 +691,16 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
       continue;
     }
 
+    // ---- a partial result: fp32 half row into the tiles, which nothing uses any more (16-byte chunk c of row r at chunk
+    //      c ^ (r & 15): neither these stores nor the merge's loads meet in a bank), maximum and sum beside it
+    if (!kPolicy && p.parts > 1) {
+      float4* dst = reinterpret_cast<float4*>(tiles) + row * (D / 4);
+#pragma unroll
+      for (int c = 0; c < DH / 4; ++c) dst[(ch * (DH / 4) + c) ^ (row & 15)] = make_float4(o2[2 * c].x, o2[2 * c].y, o2[2 * c + 1].x, o2[2 * c + 1].y);
+      if (ch == 0) ctl->part[row] = make_float2(m_run, l_run);
+      continue;
+    }
+
     // ---- epilogue (inc/fmha_i8.cuh:318-332): normalise, requantise, store
     if (q_row < p.Sq) {
       const float inv = (n_live > 0 && l_run > 0.f) ? 1.0f / l_run : 0.f;
@@ -707,6 +735,57 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
         }
       }
     }
+  }
+}
+
+template <int N> struct Flight { static constexpr int value = N; };
+
+// The CTAs of a cluster have a part of one unit each: their warps merge some of the rows each, normalise, requantise and store
+// them (inc/fmha_i8.cuh:298-332).  A lane holds four columns.
+template <int D>
+__device__ __forceinline__ void merge_parts(const FwdParams& p, const uint32_t part_smem, const uint32_t tiles_smem, const int unit) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, parts = p.parts, rank = static_cast<int>(blockIdx.x) % parts;
+  const UnitGeom geo = unit_geom(p, unit);
+  const int rows = min(kTile, p.Sq - geo.q_row0);
+  constexpr int kLanes = D / 4, kRowsPerWarp = 32 / kLanes;
+  const int c = lane & (kLanes - 1);
+#pragma unroll 1
+  for (int row = (rank * kFwdWarps + warp) * kRowsPerWarp + lane / kLanes; row < rows; row += parts * kFwdWarps * kRowsPerWarp) {
+    float m = -INFINITY, l = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    // two parts (of a pair) or four in flight at a time: a load from another SM takes a good part of a microsecond
+    auto fold = [&](auto flight, int r0) {
+      constexpr int N = decltype(flight)::value;
+      float2 ml[N];
+      float4 x[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        ml[i] = ld_cluster_v2(map_to_rank(part_smem + row * 8, r0 + i));
+        x[i] = ld_cluster_v4(map_to_rank(tiles_smem + (row * kLanes + (c ^ (row & 15))) * 16, r0 + i));
+      }
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (ml[i].y > 0.f) {
+          const float m_new = fmaxf(m, ml[i].x), e = __expf(m - m_new), f = __expf(ml[i].x - m_new);
+          m = m_new;
+          l = fmaf(e, l, f * ml[i].y);
+          o.x = fmaf(e, o.x, f * x[i].x); o.y = fmaf(e, o.y, f * x[i].y); o.z = fmaf(e, o.z, f * x[i].z); o.w = fmaf(e, o.w, f * x[i].w);
+        }
+      }
+    };
+    if (parts == 2) {
+      fold(Flight<2>(), 0);
+    } else {
+#pragma unroll 1
+      for (int r0 = 0; r0 < parts; r0 += 4) fold(Flight<4>(), r0);      // four or eight parts
+    }
+    const float scale = l > 0.f ? p.scale_v_out * __frcp_rn(l) : 0.f;
+    const float v[4] = {o.x, o.y, o.z, o.w};
+    uint32_t word = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      word |= (__float_as_uint(fminf(fmaxf(fmaf(v[i], scale, kMagic), kMagic - 127.f), kMagic + 127.f)) & 0xFFu) << (8 * i);
+    reinterpret_cast<uint32_t*>(p.o + (static_cast<int64_t>(geo.bh_local) * p.Sq + geo.q_row0 + row) * D)[c] = word;
   }
 }
 
@@ -746,7 +825,7 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
       }
       ++qn;
       for (int j = 0; j < n_live; ++j, ++g) {
-        const int t = info->live[j];
+        const int t = info->live[info->begin + j];
         const uint32_t sk = g % NK, rk = g / NK, sv = g % NV, rv = g / NV;
         if (rk > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->k_empty[sk]), (rk - 1) & 1u, abort_flag))) {
           fail = FMHA_I8_DEV_WAIT_K_FREE; fail_tile = g; break;
@@ -823,10 +902,10 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       const uint32_t sb = g % SBufs<D>::n, stage = g % NK;
       const uint64_t dk = make_smem_desc(k_smem + stage * Cfg::kTileBytes, D);
       const uint32_t tS = tmem_base + sb * kTile;
-      const bool mixed = info->mixed[j] != 0;
+      const bool mixed = info->mixed[info->begin + j] != 0;
       bool masked[4] = {};
       if (mixed) {
-        const int key0 = info->live[j] * kTile + static_cast<int>(threadIdx.x & 31);
+        const int key0 = info->live[info->begin + j] * kTile + static_cast<int>(threadIdx.x & 31);
 #pragma unroll
         for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || __ldg(mask_row + key0 + 32 * i) != 0;
       }
@@ -939,7 +1018,8 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_tiles = (p.S + kTile - 1) / kTile;
-  const int first_unit = blockIdx.x, unit_step = gridDim.x;
+  // (a cluster's CTAs have consecutive numbers)
+  const int first_unit = static_cast<int>(blockIdx.x) / p.parts, unit_step = gridDim.x;
 
   if (threadIdx.x == 0) {
     ctl->abort = 0;
@@ -992,7 +1072,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     softmax_role<D, kPolicy>(p, ctl, tmem_base, first_unit, unit_step);
   } else if (warp >= kWarpMerge0) {
     setmaxnreg_inc<FwdRegs<D>::kMerge>();
-    merge_role<D, kPolicy>(p, ctl, tmem_base, first_unit, unit_step);
+    merge_role<D, kPolicy>(p, ctl, tmem_base, tiles, first_unit, unit_step);
   } else {
     if (FwdRegs<D>::kOther < kLaunchRegs) setmaxnreg_dec<FwdRegs<D>::kOther>();
     else if (FwdRegs<D>::kOther > kLaunchRegs) setmaxnreg_inc<FwdRegs<D>::kOther>();
@@ -1015,6 +1095,11 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         const UnitGeom geo = unit_geom(p, u);
         scan_mask_warp(&ctl->info[buf], p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
+        if (lane == 0) {
+          const int n = ctl->info[buf].n_live, parts = p.parts, rank = static_cast<int>(blockIdx.x) % parts;
+          ctl->info[buf].begin = n * rank / parts;
+          ctl->info[buf].n_live = n * (rank + 1) / parts - n * rank / parts;
+        }
         if (lane == 0) mbar_arrive(smem_u32(&ctl->info_full[buf]));
       }
     }
@@ -1022,7 +1107,17 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   // every unit of this CTA has been computed and stored by the time the merge warps leave their loop
   tc_fence_before();
-  __syncthreads();
+  if (p.parts == 1) {
+    __syncthreads();
+  } else {
+    __syncwarp();
+    cluster_arrive();          // every partial result of the unit is in shared memory
+    cluster_wait();
+    merge_parts<D>(p, smem_u32(ctl->part), smem_u32(tiles), first_unit);
+    __syncwarp();
+    cluster_arrive();          // and stays there until everyone has read it
+    cluster_wait();
+  }
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

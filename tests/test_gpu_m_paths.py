@@ -177,3 +177,25 @@ def test_many_query_tiles_head_dim_64(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk,
     host = o.cpu().numpy()
     assert np.all(host[:128] == 0x5A) and np.all(host[-128:] == 0x5A)
     assert_parity(host[128:-128].reshape(q8.shape), want, what)
+
+
+# Few query tiles and many keys: a query tile is shared by a cluster of 2, 4 or 8 CTAs.  Parts without a key, one live tile in all,
+# holes, a sequence without any key, fewer tiles than they divide into evenly.
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,Sq,Sk,valid,mask_p", [
+    (1, 2, 128, 1024, None, 0.0), (2, 1, 100, 2048, (130, 2048), 0.0), (3, 2, 300, 1088, (1, 0, 1025), 0.2), (1, 3, 9, 4096, None, 0.5),
+    (2, 16, 200, 1984, (1984, 1201), 0.0), (1, 1, 640, 8192, (8100,), 0.0)])
+@pytest.mark.parametrize("uint8_p", [False, True])
+def test_few_query_tiles_share_their_keys(pkg, wl, oracle, torch_cuda, D, B, H, Sq, Sk, valid, mask_p, uint8_p):
+    torch = torch_cuda
+    q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, D, seed=Sq + Sk + D, mask_p=mask_p, valid=valid)
+    want = oracle.q128(q8, k8, v8, mask, amax, p_levels=255 if uint8_p else 128)
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    o = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    for _ in range(3):
+        pkg.FMHAInferI8Cross(None, pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), q, k, v, m, o[128:-128], uint8_p=uint8_p)
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    host = o.cpu().numpy()
+    assert np.all(host[:128] == 0x5A) and np.all(host[-128:] == 0x5A)
+    assert_parity(host[128:-128].reshape(q8.shape), want, f"B{B}H{H}Sq{Sq}Sk{Sk}D{D}")
