@@ -129,7 +129,8 @@ int fmha_i8_sm100_calibrate_o_amax(void* stream, const float amax[5], const int 
  * buffer out.  Copies q,k,v,mask to device staging buffers owned by the library (grown on demand,
  * kept for reuse), runs the forward pass, copies o back and synchronises.  The work is pipelined
  * over up to eight ranges of heads on three internal streams, so with pinned host memory the
- * inbound copies, the kernels and the outbound copies overlap; pageable memory works too. */
+ * inbound copies, the kernels and the outbound copies overlap; pageable memory works too.  From pinned
+ * memory, keys and values that the mask excludes are not fetched where that saves time. */
 int fmha_i8_sm100_infer_host(const float amax[5], const int desc[4],
                              const void* host_q, const void* host_k, const void* host_v,
                              const void* host_mask, void* host_o, unsigned flags);

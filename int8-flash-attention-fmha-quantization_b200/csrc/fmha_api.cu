@@ -16,6 +16,7 @@
 #include "fmha_decode_sm100.cuh"
 #include "fmha_fwd64_sm100.cuh"
 #include "fmha_fwd_sm100.cuh"
+#include "fmha_host_sm100.cuh"
 #include "fmha_quant_sm100.cuh"
 
 namespace {
@@ -320,7 +321,7 @@ int parts_of_a_unit(const FwdParams& p, const DeviceInfo* dev) {
 }
 
 template <int D, bool kPolicy = false>
-int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v) {
+int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v, int busy_sms) {
   CUtensorMap mq, mk, mv;
   int st;
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
@@ -333,13 +334,14 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q,
   LaunchHow how;
   how.overlap = p.n_units <= 4 * dev->sm_count;
   // persistent CTAs: one per SM (tensor memory is allocated whole), each walking its share of the units
-  const unsigned grid = static_cast<unsigned>(p.n_units < dev->sm_count ? p.n_units : dev->sm_count);
+  const int sms = dev->sm_count - busy_sms;
+  const unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
   if constexpr (D == 64) {
     if (use_workers(p, dev->sm_count))
       return launch_kernel(w64::fwd_kernel<kPolicy>, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
   }
   p.parts = 1;
-  if (!kPolicy && !p.row_stats_out && !p.amax_out) p.parts = parts_of_a_unit(p, dev);
+  if (!kPolicy && !p.row_stats_out && !p.amax_out && busy_sms == 0) p.parts = parts_of_a_unit(p, dev);
   if (p.parts > 1) {
     how.cluster = static_cast<unsigned>(p.parts);
     how.overlap = true;
@@ -386,6 +388,7 @@ struct LaunchMode {
   float2* stats_out = nullptr;     // statistics launch of a whole-row policy: {row max bits, exp-sum} per query row, o untouched
   const float2* stats_in = nullptr;  // policy launch: those statistics
   int policy = 0;                  // FMHA_I8_POLICY_* of a policy launch
+  int busy_sms = 0;                // SMs that something else is using for longer than this launch
 };
 
 int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void* q, const void* k,
@@ -454,15 +457,16 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   // D128, 1025..4096 keys: 1 row 104 -> 59 us, 2 rows 61, 4 rows 68, 8 rows 100; B128 H32 D64, 256 keys, 8 rows 72 -> 71).
   if (!mode && !calib && sh.Sq <= kDecodeMaxRows)
     return sh.D == 128 ? launch_decode<128>(s, dev, p, q, k, v) : launch_decode<64>(s, dev, p, q, k, v);
-  if (policy_launch) return sh.D == 128 ? launch_fwd<128, true>(s, dev, p, q, k, v) : launch_fwd<64, true>(s, dev, p, q, k, v);
-  return sh.D == 128 ? launch_fwd<128>(s, dev, p, q, k, v) : launch_fwd<64>(s, dev, p, q, k, v);
+  const int busy = mode ? mode->busy_sms : 0;
+  if (policy_launch) return sh.D == 128 ? launch_fwd<128, true>(s, dev, p, q, k, v, busy) : launch_fwd<64, true>(s, dev, p, q, k, v, busy);
+  return sh.D == 128 ? launch_fwd<128>(s, dev, p, q, k, v, busy) : launch_fwd<64>(s, dev, p, q, k, v, busy);
 }
 
 int infer_slice_impl(void* stream, const float amax[5], const int desc[4], const void* q, const void* k,
-                     const void* v, const void* mask, void* o, int bh_begin, int bh_count, unsigned flags) {
+                     const void* v, const void* mask, void* o, int bh_begin, int bh_count, unsigned flags, const LaunchMode* mode = nullptr) {
   if (!desc) return FMHA_I8_ERR_NULL_POINTER;
   const Shape sh{desc[0], desc[1], desc[1], desc[2], desc[3]};
-  return infer_x_impl(stream, amax, sh, q, k, v, mask, o, bh_begin, bh_count, flags);
+  return infer_x_impl(stream, amax, sh, q, k, v, mask, o, bh_begin, bh_count, flags, nullptr, mode);
 }
 
 // Device staging buffers of fmha_i8_sm100_infer_host, one set per device, grown on demand, plus the
@@ -477,6 +481,42 @@ struct HostStaging {
 };
 HostStaging g_staging[kMaxDevices];
 std::mutex g_staging_mutex[kMaxDevices];     // one lock per device: host threads that drive different GPUs do not wait for each other
+
+// How the inputs of a host-buffer call come in.  A kernel can leave rows of masked keys out and costs 5 us per chunk; the copy
+// engine is 7 % faster per byte, 50.7 and 54.7 GB/s, but needs three copies of 4 us each.  (Both ways of the link together carry
+// no more than 70 GB/s, so either pays for the output as well.)  The kernel needs pinned, device-readable, 16-byte aligned buffers,
+// and takes its SMs from the forward kernels, so it is left where those, not the link, take the time: long sequences.
+constexpr int kHostLongSeq = 4096;
+struct FetchPlan {
+  bool by_kernel = false;
+  const void *q = nullptr, *k = nullptr, *v = nullptr;     // device addresses of the host buffers
+};
+FetchPlan plan_fetch(const int desc[4], const void* host_q, const void* host_k, const void* host_v, const int8_t* host_mask, int bh_begin, int bh_count, int n_chunks) {
+  FetchPlan plan;
+  const int S = desc[1], H = desc[2], D = desc[3];
+  if (S > kHostLongSeq) return plan;
+  // rows that come in: all of Q, the groups of keys with an unmasked one (of the batches that the slice touches)
+  double rows = static_cast<double>(bh_count) * S;
+  for (int b = bh_begin / H; b <= (bh_begin + bh_count - 1) / H; ++b) {
+    const int first = b * H > bh_begin ? b * H : bh_begin, last = (b + 1) * H < bh_begin + bh_count ? (b + 1) * H : bh_begin + bh_count;
+    const int8_t* m = host_mask + static_cast<size_t>(b) * S;
+    int groups = 0;
+    for (int g = 0; g < S; g += kFetchRows) groups += std::memchr(m + g, 0, kFetchRows) != nullptr;
+    rows += 2.0 * (last - first) * groups * kFetchRows;
+  }
+  const double us_kernel = rows * D / 50.7e3 + 5.0 * n_chunks, us_copies = 3.0 * bh_count * S * D / 54.7e3 + 12.0 * n_chunks;
+  if (us_kernel > us_copies) return plan;
+  const void* host[3] = {host_q, host_k, host_v};
+  const void** seen[3] = {&plan.q, &plan.k, &plan.v};
+  for (int i = 0; i < 3; ++i) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, host[i]) != cudaSuccess) { cudaGetLastError(); return plan; }
+    if (attr.type != cudaMemoryTypeHost || attr.devicePointer == nullptr || !aligned(attr.devicePointer, 16)) return plan;
+    *seen[i] = attr.devicePointer;
+  }
+  plan.by_kernel = true;
+  return plan;
+}
 
 int check_quant_args(const float* x, long long n, const int8_t* out) {
   if (!x || !out) return FMHA_I8_ERR_NULL_POINTER;
@@ -620,37 +660,51 @@ static int infer_host_slice_impl(const float amax[5], const int desc[4], const v
   }
   // Pipeline over contiguous ranges of heads: while chunk i is computed, chunk i+1 is on its way in and
   // chunk i-1 on its way out (the bus is full duplex).  Each chunk is one forward launch on a sub-slice.
+  // Each piece of the inbound transfer costs some microseconds, so there are few; what follows the last of them -- its kernel
+  // and its outbound copy -- is exposed, so the pieces shrink by halves: a chunk's outbound copy, a third of its inbound
+  // bytes, is hidden behind the next chunk's inbound transfer.  Long sequences, where the kernels take the time, are cut evenly.
+  // (us, eight even chunks of three copies -> this: B32 H12 S512 D64 with lengths 256..512 976 -> 846, without padding 979 -> 890,
+  // B8 H12 S512 with lengths 300..512 340 -> 244, B1 H4 S256 82 -> 36, B4 H32 S2048 D128 2350 -> 2168.)
   const int BH = bh_count;
-  const int n_chunks = BH < kHostChunks ? BH : kHostChunks;
-  // The inbound copies are the bottleneck, so what follows the last of them -- the last chunk's kernel and its
-  // outbound copy -- is exposed: with enough heads the last chunk is made small (1/24 of the heads) and the
-  // others share the rest equally.
+  const size_t bytes_in = 3 * tensor_bytes;
+  const bool even = desc[1] > kHostLongSeq;
+  const int wanted = even ? kHostChunks : bytes_in < (3u << 19) ? 1 : bytes_in < (6u << 20) ? 2 : bytes_in < (64u << 20) ? 4 : 6;
+  const int n_chunks = BH < wanted ? BH : wanted;
   int bounds[kHostChunks + 1];
-  {
-    const int tail = (BH >= 8 * kHostChunks) ? (BH / 24 > 0 ? BH / 24 : 1) : 0;      // 0: equal chunks
-    const int body = BH - tail, n_body = tail ? n_chunks - 1 : n_chunks;
-    for (int i = 0; i <= n_body; ++i) bounds[i] = static_cast<int>(static_cast<long long>(body) * i / n_body);
-    if (tail) bounds[n_chunks] = BH;
+  bounds[0] = 0;
+  for (int i = 1; i <= n_chunks; ++i) {
+    const double done = even ? static_cast<double>(i) / n_chunks : (1.0 - std::ldexp(1.0, -i)) / (1.0 - std::ldexp(1.0, -n_chunks));
+    const int rounded = static_cast<int>(std::lround(done * BH)), least = bounds[i - 1] + 1, most = BH - (n_chunks - i);     // every chunk has a head
+    bounds[i] = rounded < least ? least : rounded > most ? most : rounded;
   }
+  const FetchPlan plan = plan_fetch(desc, host_q, host_k, host_v, static_cast<const int8_t*>(host_mask), bh_begin, bh_count, n_chunks);
+  LaunchMode mode;
+  mode.busy_sms = plan.by_kernel ? kFetchCtas : 0;
   cudaError_t e = cudaMemcpyAsync(s.mask, host_mask, mask_bytes, cudaMemcpyHostToDevice, s.s_in);
   for (int i = 0; i < n_chunks && e == cudaSuccess; ++i) {
     const int begin = bounds[i];
     const int end = bounds[i + 1];
     const size_t off = begin * head_bytes, bytes = (end - begin) * head_bytes;
-    const char* hq = static_cast<const char*>(host_q) + off;
-    const char* hk = static_cast<const char*>(host_k) + off;
-    const char* hv = static_cast<const char*>(host_v) + off;
     char* dq = static_cast<char*>(s.q) + off;
     char* dk = static_cast<char*>(s.k) + off;
     char* dv = static_cast<char*>(s.v) + off;
     char* dout = static_cast<char*>(s.o) + off;
-    e = cudaMemcpyAsync(dq, hq, bytes, cudaMemcpyHostToDevice, s.s_in);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dk, hk, bytes, cudaMemcpyHostToDevice, s.s_in);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dv, hv, bytes, cudaMemcpyHostToDevice, s.s_in);
+    if (plan.by_kernel) {
+      auto* fetch = desc[3] == 128 ? fetch_heads_kernel<128> : fetch_heads_kernel<64>;
+      fetch<<<kFetchCtas, kFetchThreads, 0, s.s_in>>>(static_cast<const uint4*>(plan.q), static_cast<const uint4*>(plan.k), static_cast<const uint4*>(plan.v),
+                                                      static_cast<uint4*>(s.q), static_cast<uint4*>(s.k), static_cast<uint4*>(s.v),
+                                                      static_cast<const int8_t*>(s.mask), desc[1], desc[2], bh_begin, begin, end);
+      g_launch_count.fetch_add(1, std::memory_order_relaxed);
+      e = cudaGetLastError();
+    } else {
+      e = cudaMemcpyAsync(dq, static_cast<const char*>(host_q) + off, bytes, cudaMemcpyHostToDevice, s.s_in);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(dk, static_cast<const char*>(host_k) + off, bytes, cudaMemcpyHostToDevice, s.s_in);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(dv, static_cast<const char*>(host_v) + off, bytes, cudaMemcpyHostToDevice, s.s_in);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(s.landed[i], s.s_in);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s.s_run, s.landed[i], 0);
     if (e != cudaSuccess) break;
-    st = infer_slice_impl(s.s_run, amax, desc, dq, dk, dv, s.mask, dout, bh_begin + begin, end - begin, flags);
+    st = infer_slice_impl(s.s_run, amax, desc, dq, dk, dv, s.mask, dout, bh_begin + begin, end - begin, flags, &mode);
     if (st != FMHA_I8_OK) break;
     e = cudaEventRecord(s.computed[i], s.s_run);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s.s_out, s.computed[i], 0);

@@ -199,3 +199,34 @@ def test_few_query_tiles_share_their_keys(pkg, wl, oracle, torch_cuda, D, B, H, 
     host = o.cpu().numpy()
     assert np.all(host[:128] == 0x5A) and np.all(host[-128:] == 0x5A)
     assert_parity(host[128:-128].reshape(q8.shape), want, f"B{B}H{H}Sq{Sq}Sk{Sk}D{D}")
+
+
+# Host buffers: one, two and four chunks, fewer heads than chunks, copies (no padding, or pageable memory) and the fetching kernel (padding),
+# a slice that begins and ends inside a batch.  Staging memory starts out dirty: the rows that are not fetched must not matter.
+@pytest.mark.parametrize("B,H,S,D,valid,pinned", [
+    (1, 1, 64, 64, None, True), (2, 2, 192, 128, (33, 192), True), (1, 3, 4096, 128, (1000,), True), (6, 11, 640, 64, (1, 0, 640, 320, 97, 96), True),
+    (6, 11, 640, 64, (1, 0, 640, 320, 97, 96), False), (3, 7, 1024, 128, None, True)])
+def test_host_buffers(pkg, wl, oracle, torch_cuda, B, H, S, D, valid, pinned):
+    torch = torch_cuda
+    q8, k8, v8, mask, amax = _tensors(wl, B, H, S, S, D, seed=S + D, valid=valid)
+    param, desc = pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptor(B, S, H, D)
+    host = [torch.from_numpy(x).pin_memory() if pinned else torch.from_numpy(x) for x in (q8, k8, v8, mask)]
+    dirty = [torch.full_like(t, -127).pin_memory() for t in host[:3]]
+    o = torch.zeros_like(host[0]).pin_memory() if pinned else torch.zeros_like(host[0])
+    pkg.FMHAInferI8Host(param, desc, *dirty, torch.zeros_like(host[3]), o)
+    pkg.FMHAInferI8Host(param, desc, *host, o)
+    dev = [t.cuda() for t in host]
+    want = torch.zeros_like(dev[0])
+    pkg.FMHAInferI8(None, param, desc, *dev, want)
+    want = want.cpu().numpy()
+    # another division of the work than the whole call's may pick another kernel: equal up to ties
+    assert_parity(o.numpy(), want, "host against device")
+    assert_parity(o.numpy()[:, :, ::37], oracle.q128(q8, k8, v8, mask, amax)[:, :, ::37], "host against oracle")
+    if B * H > 4:
+        begin, count = 2, B * H - 3
+        part = [t.reshape(B * H, S, D)[begin:begin + count].contiguous() for t in host[:3]]
+        part = [t.pin_memory() for t in part] if pinned else part
+        out = torch.zeros_like(part[0])
+        pkg.FMHAInferI8HostSlice(param, desc, *part, host[3], out, begin, count)
+        assert_parity(out.numpy(), want.reshape(B * H, S, D)[begin:begin + count], "slice")
+    assert pkg.device_status()[0] == pkg.OK
