@@ -38,8 +38,7 @@ static_assert(kSoftmaxWarps * kSoftmaxRegs + kWorkers * kDriverRegs <= kWarps * 
 static_assert(kSoftmaxRegs >= kLaunchRegs && kDriverRegs <= kLaunchRegs, "the softmax warps gain registers, the drivers give");
 
 constexpr int kTileBytes = kTile * kD;
-constexpr int kStages = 2;                                     // K, V and Q tiles per worker
-constexpr int kWorkerBytes = 3 * kStages * kTileBytes;
+constexpr int kWorkerBytes = 3 * kTileBytes;                   // K, V, Q
 // A worker's tensor memory: 128 columns.  S of a step; then P over its first 32 columns and P.V over its last 64.
 constexpr uint32_t kOCol = 64;
 
@@ -52,7 +51,7 @@ struct UnitInfo {
   uint8_t mixed[kMaxTiles];           // 1 = that live tile has masked keys too
 };
 struct WorkerCtl {
-  uint64_t q_full[kStages], k_full[kStages], v_full[kStages];
+  uint64_t q_full, k_full, v_full;    // the tiles have landed
   uint64_t s_full, s_free;            // S has completed / its P.V has been drained
   uint64_t p_ready, o_full;           // P is written (and S consumed) / P.V has completed
   uint64_t info_full[kInfoBufs], info_empty[kInfoBufs];
@@ -87,11 +86,12 @@ struct UnitWalk {
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = one query row: its scores, probabilities, fp32 running output row, maximum and sum.
 template <bool kPolicy>
-__device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_worker, const UnitWalk walk) {
+__device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base, const UnitWalk walk) {
   WorkerCtl* ctl = &all->w[worker];
   const int lane = threadIdx.x & 31, quad = (threadIdx.x >> 5) & 3;
   const int row = quad * 32 + lane;
-  const uint32_t tS = tmem_worker + (static_cast<uint32_t>(quad * 32) << 16);
+  const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+  const uint32_t tS = t_lane + static_cast<uint32_t>(worker * kTile), tP = tS;
   volatile int* abort_flag = &all->abort;
   const bool stats_only = !kPolicy && p.row_stats_out != nullptr;
 
@@ -157,18 +157,18 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
 
       // ---- pass 2: exp, row sum, requantise (inc/fmha_i8.cuh:208-253); the bytes go over columns already consumed
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      uint32_t ra[8], rb[8], packed[2];
-      tmem_ld8_issue(tS, ra);
+      uint32_t sa[8], sb[8], packed[2];
+      tmem_ld8_issue(tS, sa);
 #pragma unroll
       for (uint32_t c = 0; c < 16; c += 2) {
-        tmem_ld_fence(ra);
-        tmem_ld8_issue(tS + (c + 1) * 8, rb);
-        chunk_exp_pack<8, kPolicy, 0>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
-        tmem_st2(tS + c * 2, packed);
-        tmem_ld_fence(rb);
-        if (c < 14) tmem_ld8_issue(tS + (c + 2) * 8, ra);
-        chunk_exp_pack<8, kPolicy, 1>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
-        tmem_st2(tS + c * 2 + 2, packed);
+        tmem_ld_fence(sa);
+        tmem_ld8_issue(tS + (c + 1) * 8, sb);
+        chunk_exp_pack<8, kPolicy, 0>(sa, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
+        tmem_st2(tP + c * 2, packed);
+        tmem_ld_fence(sb);
+        if (c < 14) tmem_ld8_issue(tS + (c + 2) * 8, sa);
+        chunk_exp_pack<8, kPolicy, 1>(sb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
+        tmem_st2(tP + c * 2 + 2, packed);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -193,18 +193,21 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       if (!wait_or_fail(smem_u32(&ctl->o_full), g & 1u, FMHA_I8_DEV_WAIT_O_READY)) return;
       tc_fence_after();
       FMHA_STAMP(quad == 0 ? worker * 4 + 3 : 47, g);
-#pragma unroll
-      for (int c = 0; c < kD / 16; ++c) {
-        uint32_t r[16];
-        tmem_ld16_issue(tS + kOCol + c * 16, r);
-        tmem_ld_fence(r);
-        if (c == kD / 16 - 1) {
-          // the last columns are in registers: the driver may go on with the next S
-          tc_fence_before();
-          mbar_arrive(smem_u32(&ctl->s_free));
-        }
-        drain_chunk<16>(r, o2 + c * 8, neg_ec, e_bias, e_old2);
-      }
+      // (two loads in flight: a round trip to tensor memory costs more than folding a chunk in)
+      uint32_t ra[16], rb[16];
+      tmem_ld16_issue(tS + kOCol, ra);
+      tmem_ld16_issue(tS + kOCol + 16, rb);
+      tmem_ld_fence(ra); tmem_ld_fence(rb);
+      drain_chunk<16>(ra, o2, neg_ec, e_bias, e_old2);
+      tmem_ld16_issue(tS + kOCol + 32, ra);
+      drain_chunk<16>(rb, o2 + 8, neg_ec, e_bias, e_old2);
+      tmem_ld16_issue(tS + kOCol + 48, rb);
+      tmem_ld_fence(ra); tmem_ld_fence(rb);
+      // the last columns are in registers: the driver may go on with the next S
+      tc_fence_before();
+      mbar_arrive(smem_u32(&ctl->s_free));
+      drain_chunk<16>(ra, o2 + 16, neg_ec, e_bias, e_old2);
+      drain_chunk<16>(rb, o2 + 24, neg_ec, e_bias, e_old2);
     }
 
     // ---- the unit is finished
@@ -261,49 +264,53 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
 }
 
 // ---------------------------------------------------------------------------------------------- driver
-// One warp per worker, run warp-wide (every lane waits and counts, one elected lane issues).  Per step: S of the step, then --
-// while the softmax warps work -- the mask scan and the copies of the step after it, then P.V.  No barrier guards the reuse of
-// a stage: when step g + 1 is loaded, P.V of step g - 1 has been drained.
+// One warp per worker, run warp-wide (every lane waits and counts, one elected lane issues).  Per step: S, then -- while the
+// softmax warps work -- V of the step, the mask scan and, S having completed, K (and Q) of the step after it, then P.V.  A
+// worker has one tile of each: a step is long enough (3600 cycles at least) to hide a load behind it, and no barrier guards
+// the reuse of a tile, which the driver itself has seen used.
 struct DriverStep {
   int tile;                  // key tile, -1: no more steps
   bool mixed;                // it has masked keys
-  uint32_t q_use;            // which Q tile of the worker it uses
-  const int8_t* mask_row;
+  bool first;                // of its unit
+  int bh, batch;
 };
 __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const int worker, const CUtensorMap* map_q, const CUtensorMap* map_k,
-                                            const CUtensorMap* map_v, const uint32_t tmem_worker, const uint32_t worker_smem, uint8_t* presets,
+                                            const CUtensorMap* map_v, const uint32_t tmem_base, const uint32_t worker_smem, uint8_t* presets,
                                             const UnitWalk walk) {
   WorkerCtl* ctl = &all->w[worker];
   volatile int* abort_flag = &all->abort;
   const int lane = threadIdx.x & 31;
-  const uint32_t k_smem = worker_smem, v_smem = worker_smem + kStages * kTileBytes, q_smem = worker_smem + 2 * kStages * kTileBytes;
+  const uint32_t tS = tmem_base + static_cast<uint32_t>(worker * kTile), tO = tS + kOCol;
+  const uint32_t k_smem = worker_smem, v_smem = worker_smem + kTileBytes, q_smem = worker_smem + 2 * kTileBytes;
   constexpr uint32_t idesc_s = make_idesc_i8(kTile, false);       // S = Q.K^T : N = 128 keys, both K-major
   constexpr uint32_t idesc_preset_s = make_idesc_bf16(kTile), idesc_preset_o = make_idesc_bf16(kD);
   const uint32_t idesc_o = p.p_unsigned ? make_idesc_i8(kD, true, true) : make_idesc_i8(kD, true, false);     // P.V : V is an MN-major operand
   const uint32_t preset_smem = smem_u32(presets);
   const uint64_t d_a = preset_desc(preset_smem, 0), d_b = preset_desc(preset_smem, 1);
+  const uint64_t dq = make_smem_desc(q_smem, kD), dk = make_smem_desc(k_smem, kD), dv = make_smem_desc(v_smem, kD);
   const bool no_pv = p.row_stats_out != nullptr;
   const int n_tiles = (p.S + kTile - 1) / kTile;
-  uint32_t fail = 0u, g = 0;
+  uint32_t fail = 0u, g = 0, units = 0;
   auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
     if (__all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag))) return true;
     fail = code;
     return false;
   };
 
-  // the step being loaded
   int u = walk.first - walk.step, it = -1, j = 0, n_live = 0;
-  UnitGeom geo{};
-  uint32_t loaded = 0, q_loaded = 0;
-  auto load_next = [&]() -> DriverStep {
-    DriverStep s{-1, false, 0u, nullptr};
+  int bh = 0, batch = 0, q_row0 = 0;          // of the unit of the step handed out last
+  auto next_step = [&]() -> DriverStep {
     while (j >= n_live) {
       u += walk.step;
-      if (u >= p.n_units) { u = p.n_units - walk.step; n_live = 0; return s; }
+      if (u >= p.n_units) { u = p.n_units - walk.step; n_live = 0; return DriverStep{-1, false, false, 0, 0}; }
       ++it;
       const int buf = it % kInfoBufs;
-      if (it >= kInfoBufs && !wait(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), FMHA_I8_DEV_WAIT_INFO)) return s;
-      geo = unit_geom(p, u);
+      if (it >= kInfoBufs && !wait(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), FMHA_I8_DEV_WAIT_INFO))
+        return DriverStep{-1, false, false, 0, 0};
+      const UnitGeom geo = unit_geom(p, u);
+      bh = geo.bh_local;
+      batch = geo.batch;
+      q_row0 = geo.q_row0;
       UnitInfo* info = &ctl->info[buf];
       scan_mask_warp(info, p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
       if (elect_one()) {
@@ -316,42 +323,34 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
       j = 0;
     }
     const UnitInfo* info = &ctl->info[it % kInfoBufs];
-    s.tile = info->live[j];
-    s.mixed = info->mixed[j] != 0;
-    s.mask_row = p.mask + static_cast<int64_t>(geo.batch) * p.S;
-    const uint32_t st = loaded % kStages;
-    if (j == 0) ++q_loaded;
-    s.q_use = q_loaded - 1u;
-    if (elect_one()) {
-      mbar_arrive_expect_tx(smem_u32(&ctl->k_full[st]), kTileBytes);
-      tma_load_3d(k_smem + st * kTileBytes, map_k, smem_u32(&ctl->k_full[st]), 0, s.tile * kTile, geo.bh_local);
-      if (j == 0) {
-        const uint32_t bar_q = smem_u32(&ctl->q_full[s.q_use % kStages]);
-        mbar_arrive_expect_tx(bar_q, kTileBytes);
-        tma_load_3d(q_smem + (s.q_use % kStages) * kTileBytes, map_q, bar_q, 0, geo.q_row0, geo.bh_local);
-      }
-      if (!no_pv) {
-        mbar_arrive_expect_tx(smem_u32(&ctl->v_full[st]), kTileBytes);
-        tma_load_3d(v_smem + st * kTileBytes, map_v, smem_u32(&ctl->v_full[st]), 0, s.tile * kTile, geo.bh_local);
+    const DriverStep s{info->live[j], info->mixed[j] != 0, j == 0, bh, batch};
+    ++j;
+    return s;
+  };
+  auto load_k = [&](const DriverStep& s) {
+    if (s.tile >= 0 && elect_one()) {
+      mbar_arrive_expect_tx(smem_u32(&ctl->k_full), kTileBytes);
+      tma_load_3d(k_smem, map_k, smem_u32(&ctl->k_full), 0, s.tile * kTile, bh);
+      if (s.first) {
+        mbar_arrive_expect_tx(smem_u32(&ctl->q_full), kTileBytes);
+        tma_load_3d(q_smem, map_q, smem_u32(&ctl->q_full), 0, q_row0, bh);
       }
     }
     __syncwarp();
-    ++j;
-    ++loaded;
-    return s;
   };
 
-  DriverStep cur = load_next();
+  DriverStep cur = next_step();
+  load_k(cur);
   while (cur.tile >= 0 && fail == 0u) {
-    const uint32_t st = g % kStages;
     bool masked[4] = {};
     if (cur.mixed) {
+      const int8_t* mask_row = p.mask + static_cast<int64_t>(cur.batch) * p.S;
       const int key0 = cur.tile * kTile + lane;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || __ldg(cur.mask_row + key0 + 32 * i) != 0;
+      for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || __ldg(mask_row + key0 + 32 * i) != 0;
     }
-    if (!wait(smem_u32(&ctl->q_full[cur.q_use % kStages]), (cur.q_use / kStages) & 1u, FMHA_I8_DEV_WAIT_Q_LOAD)) break;
-    if (!wait(smem_u32(&ctl->k_full[st]), (g / kStages) & 1u, FMHA_I8_DEV_WAIT_K_LOAD)) break;
+    if (cur.first && !wait(smem_u32(&ctl->q_full), units++ & 1u, FMHA_I8_DEV_WAIT_Q_LOAD)) break;
+    if (!wait(smem_u32(&ctl->k_full), g & 1u, FMHA_I8_DEV_WAIT_K_LOAD)) break;
     if (g > 0u && !wait(smem_u32(&ctl->s_free), (g - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
     tc_fence_after();
     FMHA_STAMP(16 + worker * 4 + 0, g);
@@ -359,26 +358,29 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
     const uint32_t operand = cur.mixed ? 2u + static_cast<uint32_t>(worker) : 1u;
     if (cur.mixed) fill_mask_operand(presets + operand * kPresetBytes, masked, 128);
     const uint64_t d_preset = preset_desc(preset_smem, operand);
-    const uint64_t dq = make_smem_desc(q_smem + (cur.q_use % kStages) * kTileBytes, kD), dk = make_smem_desc(k_smem + st * kTileBytes, kD);
     if (elect_one()) {
-      mma_f16_ss(tmem_worker, d_a, d_preset, idesc_preset_s, 0u);      // accumulator := 0x4B400000, masked keys -2^127
+      mma_f16_ss(tS, d_a, d_preset, idesc_preset_s, 0u);      // accumulator := 0x4B400000, masked keys -2^127
 #pragma unroll
-      for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tmem_worker, desc_advance(dq, kk * 32), desc_advance(dk, kk * 32), idesc_s, 1u);
+      for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(dk, kk * 32), idesc_s, 1u);
       mma_commit(smem_u32(&ctl->s_full));
+      if (!no_pv) {
+        mbar_arrive_expect_tx(smem_u32(&ctl->v_full), kTileBytes);
+        tma_load_3d(v_smem, map_v, smem_u32(&ctl->v_full), 0, cur.tile * kTile, cur.bh);
+      }
     }
     FMHA_STAMP(16 + worker * 4 + 1, g);
-    const DriverStep next = load_next();
-    if (fail != 0u) break;
+    const DriverStep next = next_step();
+    if (fail != 0u || !wait(smem_u32(&ctl->s_full), g & 1u, FMHA_I8_DEV_WAIT_S_READY)) break;
+    load_k(next);
     if (!no_pv) {
-      const uint64_t dv = make_smem_desc(v_smem + st * kTileBytes, kD);
-      if (!wait(smem_u32(&ctl->v_full[st]), (g / kStages) & 1u, FMHA_I8_DEV_WAIT_V_LOAD)) break;
+      if (!wait(smem_u32(&ctl->v_full), g & 1u, FMHA_I8_DEV_WAIT_V_LOAD)) break;
       if (!wait(smem_u32(&ctl->p_ready), g & 1u, FMHA_I8_DEV_WAIT_P_READY)) break;
       tc_fence_after();
       FMHA_STAMP(16 + worker * 4 + 2, g);
       if (elect_one()) {
-        mma_f16_ss(tmem_worker + kOCol, d_a, d_b, idesc_preset_o, 0u);
+        mma_f16_ss(tO, d_a, d_b, idesc_preset_o, 0u);
 #pragma unroll
-        for (int kk = 0; kk < kTile / 32; ++kk) mma_i8_ts(tmem_worker + kOCol, tmem_worker + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);
+        for (int kk = 0; kk < kTile / 32; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);
         mma_commit(smem_u32(&ctl->o_full));
       }
       FMHA_STAMP(16 + worker * 4 + 3, g);
@@ -413,11 +415,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
   if (threadIdx.x == 0) {
     ctl->abort = 0;
     for (WorkerCtl& w : ctl->w) {
-      for (int s = 0; s < kStages; ++s) {
-        mbar_init(smem_u32(&w.q_full[s]), 1);
-        mbar_init(smem_u32(&w.k_full[s]), 1);
-        mbar_init(smem_u32(&w.v_full[s]), 1);
-      }
+      mbar_init(smem_u32(&w.q_full), 1);
+      mbar_init(smem_u32(&w.k_full), 1);
+      mbar_init(smem_u32(&w.v_full), 1);
       mbar_init(smem_u32(&w.s_full), 1);
       mbar_init(smem_u32(&w.s_free), kTile);
       mbar_init(smem_u32(&w.p_ready), kTile);
@@ -446,14 +446,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
 
   const int worker = warp < kSoftmaxWarps ? warp >> 2 : warp - kSoftmaxWarps;
   const UnitWalk walk = {static_cast<int>(blockIdx.x + gridDim.x * worker), static_cast<int>(gridDim.x) * kWorkers};
-  const uint32_t tmem_worker = tmem_base + static_cast<uint32_t>(worker * kTile);
   uint8_t* worker_smem = tiles + worker * kWorkerBytes;
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
-    w64::softmax_role<kPolicy>(p, ctl, worker, tmem_worker, walk);
+    w64::softmax_role<kPolicy>(p, ctl, worker, tmem_base, walk);
   } else {
     setmaxnreg_dec<kDriverRegs>();
-    driver_role(p, ctl, worker, &map_q, &map_k, &map_v, tmem_worker, smem_u32(worker_smem), presets, walk);
+    driver_role(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets, walk);
   }
   tc_fence_before();
   __syncthreads();
