@@ -292,32 +292,44 @@ int launch_kernel(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cud
   return FMHA_I8_ERR_LAUNCH;
 }
 
-// Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  Cycles per key tile, measured: a CTA of
-// fmha_fwd_sm100.cuh works on one unit at a time, 1700 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5800 per
-// tile for all four, 5300 / 4700 / 3900 with three, two or one left in the last round.  (B16 H16 S256: 12.8 / 11.6 us; B8 H12
-// S512: 16.3 / 16.0; B4 H12 S512: 12.2 / 13.7; B2 H12 S1024: 19.5 / 23.3; B1 H8 S16384: 778 / 779.)
-bool use_workers(const FwdParams& p, int sm_count) {
-  const long long tiles = (p.S + kTile - 1) / kTile, round = static_cast<long long>(sm_count) * w64::kWorkers;
-  const long long last[w64::kWorkers + 1] = {0, 3900, 4700, 5300, 5800};
-  const long long rounds = p.n_units / round, left = (p.n_units % round + sm_count - 1) / sm_count;
-  return (rounds * 5800 + last[left]) * tiles < ((p.n_units + sm_count - 1) / sm_count) * (1700 * tiles + 1200);
-}
-
 // CTAs that share one unit (query tile), each with a part of its key tiles: for calls whose units leave most SMs idle, as long as
 // all clusters are resident at once (a second wave of them starts from nothing and costs 10 us).  In nanoseconds, measured: 950
 // per key tile of a CTA, and for cluster launch, two cluster barriers and the merge of the partial results through distributed
 // shared memory 2300 / 3000 / 4300 with 2 / 4 / 8 CTAs.  (Head_dim 64, us without -> with: B1 H8 S1024 Sq256 11.9 -> 9.1, B1 H4
 // S2048 Sq200 19.2 -> 10.5, B1 H2 S4096 34.9 -> 23.4, B1 H8 S8192 Sq64 64 -> 17.7; head_dim 128: B2 H16 S1984 Sq200 21.1 -> 16.8,
 // B1 H2 S16384 Sq128 131 -> 29.)
-int parts_of_a_unit(const FwdParams& p, const DeviceInfo* dev) {
+//
+// With more units than SMs the same is done for those of the last round: where they are half as many as the SMs or fewer, a pair
+// of CTAs shares each.  (Head_dim 128: B1 H16 S1280 25.6 -> 23.6, B1 H5 S4096 68.9 -> 56.0, B1 H32 S2048 70.9 -> 65.8.)
+bool pairs_share_last_round(const FwdParams& p, const DeviceInfo* dev) {
+  const int last = p.n_units % dev->sm_count, tiles = (p.S + kTile - 1) / kTile;
+  return p.n_units > dev->sm_count && last > 0 && last <= dev->max_clusters[0] && 2 * dev->max_clusters[0] == dev->sm_count && 950 * (tiles / 2) > 2300;
+}
+void plan_parts(FwdParams* p, const DeviceInfo* dev) {
   constexpr int kOverhead[kClusterSizes] = {2300, 3000, 4300};
-  const int tiles = (p.S + kTile - 1) / kTile;
-  int best = 1, best_ns = 950 * tiles;
+  const int tiles = (p->S + kTile - 1) / kTile;
+  p->own_rounds = p->n_units / dev->sm_count;
+  if (p->own_rounds > 0) {
+    if (pairs_share_last_round(*p, dev)) p->parts = 2;
+    return;
+  }
+  int best_ns = 950 * tiles;
   for (int i = 0; i < kClusterSizes; ++i) {
     const int c = 2 << i, ns = 950 * ((tiles + c - 1) / c) + kOverhead[i];
-    if (p.n_units <= dev->max_clusters[i] && ns < best_ns) { best = c; best_ns = ns; }
+    if (p->n_units <= dev->max_clusters[i] && ns < best_ns) { p->parts = c; best_ns = ns; }
   }
-  return best;
+}
+
+// Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  Cycles per key tile, measured: a CTA of
+// fmha_fwd_sm100.cuh works on one unit at a time, 1700 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5800 per
+// tile for all four, 5300 / 4700 / 3900 with three, two or one left in the last round.  (B16 H16 S256: 12.8 / 11.6 us; B8 H12
+// S512: 16.3 / 16.0; B4 H12 S512: 12.2 / 13.7; B2 H12 S1024: 19.5 / 23.3; B1 H8 S16384: 778 / 779.)
+bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
+  const long long sms = dev->sm_count, tiles = (p.S + kTile - 1) / kTile, round = sms * w64::kWorkers;
+  const long long last[w64::kWorkers + 1] = {0, 3900, 4700, 5300, 5800};
+  const long long workers = p.n_units / round * 5800 + last[(p.n_units % round + sms - 1) / sms];
+  const long long own = p.n_units / sms, more = p.n_units % sms != 0, unit = 1700 * tiles + 1200;
+  return workers * tiles < own * unit + more * (pairs_share_last_round(p, dev) ? unit / 2 + 4500 : unit);
 }
 
 template <int D, bool kPolicy = false>
@@ -337,16 +349,16 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q,
   const int sms = dev->sm_count - busy_sms;
   const unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
   if constexpr (D == 64) {
-    if (use_workers(p, dev->sm_count))
+    if (use_workers(p, dev))
       return launch_kernel(w64::fwd_kernel<kPolicy>, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
   }
   p.parts = 1;
-  if (!kPolicy && !p.row_stats_out && !p.amax_out && busy_sms == 0) p.parts = parts_of_a_unit(p, dev);
+  if (!kPolicy && !p.row_stats_out && !p.amax_out && busy_sms == 0) plan_parts(&p, dev);
   if (p.parts > 1) {
     how.cluster = static_cast<unsigned>(p.parts);
     how.overlap = true;
-    return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(static_cast<unsigned>(p.n_units * p.parts)), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream,
-                         how, mq, mk, mv, p);
+    const int ctas = p.own_rounds > 0 ? dev->sm_count : p.n_units * p.parts;
+    return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(static_cast<unsigned>(ctas)), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
   }
   return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }

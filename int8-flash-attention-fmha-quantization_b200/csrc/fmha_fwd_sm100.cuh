@@ -180,7 +180,8 @@ struct FwdParams {
   int Sq;               // query rows per head (== S for self-attention)
   int H, bh_begin, bh_count, q_tiles;
   int n_units;          // bh_count * q_tiles work units
-  int parts;            // 1: a CTA takes units of its own; more: that many CTAs, a cluster, share one unit, each a part of its key tiles
+  int own_rounds;       // units [0, own_rounds * CTAs) are taken round-robin by the CTAs, one CTA each; the others ...
+  int parts;            // ... by clusters of this many CTAs, each CTA a part of the unit's key tiles (1: no clusters, all units are round-robin)
   float row_scale;      // 1/sqrt(D), the reference's constant (inc/fmha_i8.cuh:71)
   float scale_qk;       // q_amax*k_amax/127^2 (inc/fmha_i8.cuh:72)
   float scale_v_out;    // v_amax/(o_amax*128) (inc/fmha_i8.cuh:318)
@@ -423,6 +424,25 @@ __device__ __forceinline__ void drain_chunk(const uint32_t (&r)[N], float2* o2, 
   }
 }
 
+// The units of one CTA in order: `own` round-robin ones, then perhaps one that it shares with its cluster.
+struct UnitWalk {
+  int own, count, shared;
+  __device__ __forceinline__ int unit(int it) const { return it < own ? static_cast<int>(blockIdx.x + it * gridDim.x) : shared; }
+};
+__device__ __forceinline__ UnitWalk unit_walk(const FwdParams& p) {
+  const int b = static_cast<int>(blockIdx.x), ctas = static_cast<int>(gridDim.x);
+  UnitWalk w;
+  if (p.parts == 1) {
+    w.own = w.count = (p.n_units - b + ctas - 1) / ctas;
+    w.shared = 0;
+  } else {
+    w.own = p.own_rounds;
+    w.shared = p.own_rounds * ctas + b / p.parts;           // a cluster's CTAs have consecutive numbers
+    w.count = w.own + (w.shared < p.n_units ? 1 : 0);
+  }
+  return w;
+}
+
 // Geometry of work unit u.
 struct UnitGeom {
   int bh_local, batch, q_row0;
@@ -440,7 +460,7 @@ __device__ __forceinline__ UnitGeom unit_geom(const FwdParams& p, int u) {
 // handles the steps of its chain.
 template <int D, bool kPolicy>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
-                                             const int first_unit, const int unit_step) {
+                                             const UnitWalk walk) {
   const int warp = (threadIdx.x >> 5) - kWarpSoftmax0, lane = threadIdx.x & 31;
   const int chain = warp >> 3, half = (warp >> 2) & 1, quad = warp & 3;
   const int row = quad * 32 + lane;
@@ -452,8 +472,8 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
 
   uint32_t n = 0;     // steps this chain has processed so far (phase of xch)
   uint32_t g0 = 0;    // global index of the current unit's first step
-  int it = 0;
-  for (int u = first_unit; u < p.n_units; u += unit_step, ++it) {
+  for (int it = 0; it < walk.count; ++it) {
+    const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
     if (!__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
       raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it);
@@ -572,7 +592,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
 // maximum and the running sum of that row (kept by both threads of the row).
 template <int D, bool kPolicy>
 __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base, uint8_t* tiles,
-                                           const int first_unit, const int unit_step) {
+                                           const UnitWalk walk) {
   constexpr int DH = D / 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int quad = warp & 3, ch = (warp - kWarpMerge0) >> 2;       // ch = which half of the output columns
@@ -581,8 +601,8 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
   volatile int* abort_flag = &ctl->abort;
 
   uint32_t g0 = 0;
-  int it = 0;
-  for (int u = first_unit; u < p.n_units; u += unit_step, ++it) {
+  for (int it = 0; it < walk.count; ++it) {
+    const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
     if (!__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
       raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it);
@@ -693,7 +713,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
 
     // ---- a partial result: fp32 half row into the tiles, which nothing uses any more (16-byte chunk c of row r at chunk
     //      c ^ (r & 15): neither these stores nor the merge's loads meet in a bank), maximum and sum beside it
-    if (!kPolicy && p.parts > 1) {
+    if (!kPolicy && it >= walk.own) {
       float4* dst = reinterpret_cast<float4*>(tiles) + row * (D / 4);
 #pragma unroll
       for (int c = 0; c < DH / 4; ++c) dst[(ch * (DH / 4) + c) ^ (row & 15)] = make_float4(o2[2 * c].x, o2[2 * c].y, o2[2 * c + 1].x, o2[2 * c + 1].y);
@@ -705,23 +725,22 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
     if (q_row < p.Sq) {
       const float inv = (n_live > 0 && l_run > 0.f) ? 1.0f / l_run : 0.f;
       int8_t* dst = p.o + (static_cast<int64_t>(geo.bh_local) * p.Sq + q_row) * D + ch * DH;
-      // rn(clamp(x)) through the magic-number addition (the low byte of clamp(x) + 1.5*2^23 is the two's-complement
-      // integer), bytes gathered with PRMT: conversions and shifts would cost three times the issue cycles
-      const float2 inv2 = make_float2(inv, inv), sc2 = make_float2(p.scale_v_out, p.scale_v_out);
-      const float2 zero2 = make_float2(0.f, 0.f), magic2 = make_float2(kMagic, kMagic);
+      // rn(clamp(x)) through the magic number: x + 1.5*2^23 has the integer nearest to x in its low bits (the low byte is the
+      // two's-complement integer), and clamping commutes with the addition; bytes gathered with PRMT: conversions and shifts
+      // would cost three times the issue cycles
+      const float scale = p.scale_v_out * inv;
+      const float2 sc2 = make_float2(scale, scale), magic2 = make_float2(kMagic, kMagic);
       uint32_t wide[8];
 #pragma unroll
       for (int c = 0; c < DH / 16; ++c) {
         uint32_t* wds = &wide[(c & 1) * 4];
 #pragma unroll
         for (int gq = 0; gq < 4; ++gq) {
-          float2 a = __ffma2_rn(sc2, __ffma2_rn(o2[c * 8 + gq * 2], inv2, zero2), zero2);        // scale_v_out * (o * inv), each product rounded
-          float2 b = __ffma2_rn(sc2, __ffma2_rn(o2[c * 8 + gq * 2 + 1], inv2, zero2), zero2);
-          a.x = fminf(fmaxf(a.x, -127.f), 127.f); a.y = fminf(fmaxf(a.y, -127.f), 127.f);
-          b.x = fminf(fmaxf(b.x, -127.f), 127.f); b.y = fminf(fmaxf(b.y, -127.f), 127.f);
-          const float2 ya = __fadd2_rn(a, magic2), yb = __fadd2_rn(b, magic2);
-          wds[gq] = __byte_perm(__byte_perm(__float_as_uint(ya.x), __float_as_uint(ya.y), 0x0040),
-                                __byte_perm(__float_as_uint(yb.x), __float_as_uint(yb.y), 0x0040), 0x5410);
+          float2 a = __ffma2_rn(o2[c * 8 + gq * 2], sc2, magic2), b = __ffma2_rn(o2[c * 8 + gq * 2 + 1], sc2, magic2);
+          a.x = fminf(fmaxf(a.x, kMagic - 127.f), kMagic + 127.f); a.y = fminf(fmaxf(a.y, kMagic - 127.f), kMagic + 127.f);
+          b.x = fminf(fmaxf(b.x, kMagic - 127.f), kMagic + 127.f); b.y = fminf(fmaxf(b.y, kMagic - 127.f), kMagic + 127.f);
+          wds[gq] = __byte_perm(__byte_perm(__float_as_uint(a.x), __float_as_uint(a.y), 0x0040),
+                                __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x0040), 0x5410);
         }
         // 32-byte stores: a warp's rows are 128 (or 64) bytes apart, so every store touches 32 lines whatever its
         // width, and the 16-byte version of this loop cost 5 % of the whole kernel at head_dim 128
@@ -796,15 +815,16 @@ template <int D>
 __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl,
                                             const CUtensorMap* map_q, const CUtensorMap* map_k, const CUtensorMap* map_v,
                                             const uint32_t q_smem, const uint32_t k_smem, const uint32_t v_smem,
-                                            const int first_unit, const int unit_step) {
+                                            const UnitWalk walk) {
   using Cfg = FwdCfg<D>;
   constexpr uint32_t NK = Cfg::kStagesK, NV = Cfg::kStagesV, NQ = Cfg::kQBufs;
   volatile int* abort_flag = &ctl->abort;
   uint32_t g = 0;            // steps loaded so far: ring position and phase continue across units
   uint32_t qn = 0;           // non-empty units so far: Q buffer and phase
   uint32_t fail = 0u, fail_tile = 0u;
-  int it = 0;
-  for (int u = first_unit; u < p.n_units && fail == 0u; u += unit_step, ++it) {
+  const bool no_v = p.row_stats_out != nullptr;        // the statistics launch has no P.V
+  for (int it = 0; it < walk.count && fail == 0u; ++it) {
+    const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
     if (!__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
       fail = FMHA_I8_DEV_WAIT_INFO; fail_tile = it; break;
@@ -873,7 +893,7 @@ __device__ __forceinline__ bool issuer_wait(IssuerErr& e, uint32_t bar, uint32_t
 template <int D>
 __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                               const uint32_t q_smem, const uint32_t k_smem, uint8_t* bias_a,
-                                              const int first_unit, const int unit_step) {
+                                              const UnitWalk walk) {
   using Cfg = FwdCfg<D>;
   constexpr uint32_t NK = Cfg::kStagesK, NQ = Cfg::kQBufs;
   volatile int* abort_flag = &ctl->abort;
@@ -882,9 +902,9 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   const uint64_t d_bias_a = make_smem_desc_noswizzle(smem_u32(bias_a), 128, 256);
   IssuerErr err;
   uint32_t g = 0, qn = 0;
-  int it = 0;
   bool ok = true;
-  for (int u = first_unit; u < p.n_units && ok; u += unit_step, ++it) {
+  for (int it = 0; it < walk.count && ok; ++it) {
+    const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
     if (!issuer_wait<true>(err, smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO, it, abort_flag)) break;
     const UnitInfo* info = &ctl->info[buf];
@@ -941,7 +961,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
 template <int D>
 __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                               const uint32_t v_smem, const uint32_t bias_a_smem, const uint32_t bias_b_smem,
-                                              const int first_unit, const int unit_step) {
+                                              const UnitWalk walk) {
   using Cfg = FwdCfg<D>;
   constexpr uint32_t NV = Cfg::kStagesV;
   volatile int* abort_flag = &ctl->abort;
@@ -954,9 +974,9 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
 #endif
   IssuerErr err;
   uint32_t g = 0;
-  int it = 0;
   bool ok = true;
-  for (int u = first_unit; u < p.n_units && ok; u += unit_step, ++it) {
+  for (int it = 0; it < walk.count && ok; ++it) {
+    const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
     if (!issuer_wait<true>(err, smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO, it, abort_flag)) break;
     const int n_live = ctl->info[buf].n_live;
@@ -1018,8 +1038,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_tiles = (p.S + kTile - 1) / kTile;
-  // (a cluster's CTAs have consecutive numbers)
-  const int first_unit = static_cast<int>(blockIdx.x) / p.parts, unit_step = gridDim.x;
+  const UnitWalk walk = unit_walk(p);
 
   if (threadIdx.x == 0) {
     ctl->abort = 0;
@@ -1069,24 +1088,24 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // phase of an info barrier = (it / kInfoBufs) & 1; `g` counts its steps (live key tiles) across units.
   if (warp >= kWarpSoftmax0) {
     setmaxnreg_dec<FwdRegs<D>::kSoftmax>();
-    softmax_role<D, kPolicy>(p, ctl, tmem_base, first_unit, unit_step);
+    softmax_role<D, kPolicy>(p, ctl, tmem_base, walk);
   } else if (warp >= kWarpMerge0) {
     setmaxnreg_inc<FwdRegs<D>::kMerge>();
-    merge_role<D, kPolicy>(p, ctl, tmem_base, tiles, first_unit, unit_step);
+    merge_role<D, kPolicy>(p, ctl, tmem_base, tiles, walk);
   } else {
     if (FwdRegs<D>::kOther < kLaunchRegs) setmaxnreg_dec<FwdRegs<D>::kOther>();
     else if (FwdRegs<D>::kOther > kLaunchRegs) setmaxnreg_inc<FwdRegs<D>::kOther>();
     if (warp == kWarpLoad) {
-      loader_role<D>(p, ctl, &map_q, &map_k, &map_v, q_smem, k_smem, v_smem, first_unit, unit_step);
+      loader_role<D>(p, ctl, &map_q, &map_k, &map_v, q_smem, k_smem, v_smem, walk);
     } else if (warp == kWarpMmaS) {
-      s_issuer_role<D>(p, ctl, tmem_base, q_smem, k_smem, bias_a, first_unit, unit_step);
+      s_issuer_role<D>(p, ctl, tmem_base, q_smem, k_smem, bias_a, walk);
     } else if (warp == kWarpMmaO) {
-      o_issuer_role<D>(p, ctl, tmem_base, v_smem, smem_u32(bias_a), smem_u32(bias_b), first_unit, unit_step);
+      o_issuer_role<D>(p, ctl, tmem_base, v_smem, smem_u32(bias_a), smem_u32(bias_b), walk);
     } else if (warp == kWarpScan) {
       // ---------------------------------------------------------------- scanner: mask information, units ahead
       bool ok = true;
-      int it = 0;
-      for (int u = first_unit; u < p.n_units && ok; u += unit_step, ++it) {
+      for (int it = 0; it < walk.count && ok; ++it) {
+        const int u = walk.unit(it);
         const int buf = it % kInfoBufs;
         // the buffer was used by unit it - kInfoBufs: wait until all its consumers have released it
         if (it >= kInfoBufs) {
@@ -1096,7 +1115,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const UnitGeom geo = unit_geom(p, u);
         scan_mask_warp(&ctl->info[buf], p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
         if (lane == 0) {
-          const int n = ctl->info[buf].n_live, parts = p.parts, rank = static_cast<int>(blockIdx.x) % parts;
+          const int n = ctl->info[buf].n_live, parts = it < walk.own ? 1 : p.parts, rank = static_cast<int>(blockIdx.x) % parts;
           ctl->info[buf].begin = n * rank / parts;
           ctl->info[buf].n_live = n * (rank + 1) / parts - n * rank / parts;
         }
@@ -1107,13 +1126,13 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   // every unit of this CTA has been computed and stored by the time the merge warps leave their loop
   tc_fence_before();
-  if (p.parts == 1) {
+  if (walk.count == walk.own) {      // (the same for all CTAs of a cluster)
     __syncthreads();
   } else {
     __syncwarp();
     cluster_arrive();          // every partial result of the unit is in shared memory
     cluster_wait();
-    merge_parts<D>(p, smem_u32(ctl->part), smem_u32(tiles), first_unit);
+    merge_parts<D>(p, smem_u32(ctl->part), smem_u32(tiles), walk.shared);
     __syncwarp();
     cluster_arrive();          // and stays there until everyone has read it
     cluster_wait();

@@ -230,3 +230,23 @@ def test_host_buffers(pkg, wl, oracle, torch_cuda, B, H, S, D, valid, pinned):
         pkg.FMHAInferI8HostSlice(param, desc, *part, host[3], out, begin, count)
         assert_parity(out.numpy(), want.reshape(B * H, S, D)[begin:begin + count], "slice")
     assert pkg.device_status()[0] == pkg.OK
+
+
+# More query tiles than SMs: those of a last round of at most half the SMs are shared by pairs of CTAs.  148 + 2, 148 + 74 (the most), 2 * 148 + 64
+# query tiles; the last of them beyond the sequence's end, a sequence without a key among them.
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,Sq,Sk,valid,mask_p", [
+    (3, 10, 600, 704, (704, 650, 0), 0.0), (2, 37, 300, 1024, (1000, 129), 0.0), (1, 24, 1900, 640, None, 0.1)])
+def test_pairs_share_the_last_round(pkg, wl, oracle, torch_cuda, D, B, H, Sq, Sk, valid, mask_p):
+    torch = torch_cuda
+    q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, D, seed=Sq + Sk + D, mask_p=mask_p, valid=valid)
+    want = oracle.q128(q8, k8, v8, mask, amax)
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    o = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    for _ in range(3):
+        pkg.FMHAInferI8Cross(None, pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), q, k, v, m, o[128:-128])
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    host = o.cpu().numpy()
+    assert np.all(host[:128] == 0x5A) and np.all(host[-128:] == 0x5A)
+    assert_parity(host[128:-128].reshape(q8.shape), want, f"B{B}H{H}Sq{Sq}Sk{Sk}D{D}")
