@@ -305,6 +305,14 @@ bool pairs_share_last_round(const FwdParams& p, const DeviceInfo* dev) {
   const int last = p.n_units % dev->sm_count, tiles = (p.S + kTile - 1) / kTile;
   return p.n_units > dev->sm_count && last > 0 && last <= dev->max_clusters[0] && 2 * dev->max_clusters[0] == dev->sm_count && 950 * (tiles / 2) > 2300;
 }
+// ceil(2^(31 + bits) / d) with 2^bits >= d > 2^(bits - 1): the quotient is exact for every dividend below 2^31.
+FastDiv fast_div_by(int d) {
+  int bits = 0;
+  while ((1ll << bits) < d) ++bits;
+  const uint64_t one = 1ull << (31 + bits);
+  return FastDiv{static_cast<uint32_t>((one + static_cast<uint64_t>(d) - 1) / static_cast<uint64_t>(d)), 31 + bits};
+}
+
 void plan_parts(FwdParams* p, const DeviceInfo* dev) {
   constexpr int kOverhead[kClusterSizes] = {2300, 3000, 4300};
   const int tiles = (p->S + kTile - 1) / kTile;
@@ -458,6 +466,8 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   p.bh_begin = bh_begin;
   p.bh_count = bh_count;
   p.q_tiles = (p.Sq + kTile - 1) / kTile;
+  p.by_q_tiles = fast_div_by(p.q_tiles);
+  p.by_heads = fast_div_by(p.H);
   {
     const long long units = static_cast<long long>(bh_count) * p.q_tiles;
     if (units > 0x7FFFFFFFLL) return FMHA_I8_ERR_BAD_SHAPE;

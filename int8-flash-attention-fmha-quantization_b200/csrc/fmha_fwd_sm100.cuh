@@ -172,6 +172,16 @@ template <int D> struct FwdCfg {
   static constexpr int kTilesBytesTotal = (kQBufs + kStagesK + kStagesV) * kTileBytes;
 };
 
+// u / d = u * mul >> shift for every u < 2^31, without a division's twenty instructions: all roles take units apart, and short
+// units wait for it (B64 H32 S256 D128 81.9 -> 78.2 us).
+struct FastDiv {
+  uint32_t mul;
+  int shift;
+};
+__device__ __forceinline__ int fast_div(int u, const FastDiv d) {
+  return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(u)) * d.mul) >> d.shift);
+}
+
 struct FwdParams {
   const int8_t* mask;   // [B,S] whole mask
   int8_t* o;            // first head of the slice
@@ -179,6 +189,7 @@ struct FwdParams {
   int S;                // keys per head (seq_len; seq_len_k when queries and keys differ in number)
   int Sq;               // query rows per head (== S for self-attention)
   int H, bh_begin, bh_count, q_tiles;
+  FastDiv by_q_tiles, by_heads;
   int n_units;          // bh_count * q_tiles work units
   int own_rounds;       // units [0, own_rounds * CTAs) are taken round-robin by the CTAs, one CTA each; the others ...
   int parts;            // ... by clusters of this many CTAs, each CTA a part of the unit's key tiles (1: no clusters, all units are round-robin)
@@ -410,6 +421,32 @@ __device__ __forceinline__ RowConsts row_consts(const int imax, const float c2s,
 // o2 (+)= e_cur * (P8 . V) for N output columns.  r = accumulator: either preset by the bias MMA, so that it reads
 // as the float kMagic + (P8 . V), or a raw int32 (|r| < 2^22) that becomes that float by adding the bit pattern
 // of 1.5*2^23 -- no conversion instruction either way.
+// Does any of N pairs of the unnormalised output leave [-127, 127] when it is multiplied by `scale` and rounded?
+template <int N> __device__ __forceinline__ bool needs_clamp(const float2* o2, const float scale) {
+  float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; i += 2) { m0 = max3_abs(m0, o2[i].x, o2[i].y); m1 = max3_abs(m1, o2[i + 1].x, o2[i + 1].y); }
+  return !(fmaxf(m0, m1) * scale < 127.25f);
+}
+// Eight pairs to sixteen bytes: rn(clamp(x * scale)) through the magic number (x + 1.5*2^23 has the integer nearest to x in its
+// low bits, the low byte is the two's-complement integer), bytes gathered with PRMT.
+__device__ __forceinline__ void requantise16(const float2* o2, const float2 scale, const bool clamp, uint32_t* words) {
+  float2 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __ffma2_rn(o2[i], scale, make_float2(kMagic, kMagic));
+  if (clamp) {      // (clamping commutes with the addition)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i].x = fminf(fmaxf(v[i].x, kMagic - 127.f), kMagic + 127.f);
+      v[i].y = fminf(fmaxf(v[i].y, kMagic - 127.f), kMagic + 127.f);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    words[i] = __byte_perm(__byte_perm(__float_as_uint(v[2 * i].x), __float_as_uint(v[2 * i].y), 0x0040),
+                           __byte_perm(__float_as_uint(v[2 * i + 1].x), __float_as_uint(v[2 * i + 1].y), 0x0040), 0x5410);
+}
+
 template <int N>
 __device__ __forceinline__ void drain_chunk(const uint32_t (&r)[N], float2* o2, const float2 neg_ec, const float2 e_bias, const float2 e_old) {
 #pragma unroll
@@ -449,8 +486,8 @@ struct UnitGeom {
 };
 __device__ __forceinline__ UnitGeom unit_geom(const FwdParams& p, int u) {
   UnitGeom g;
-  g.bh_local = u / p.q_tiles;
-  g.batch = (p.bh_begin + g.bh_local) / p.H;
+  g.bh_local = fast_div(u, p.by_q_tiles);
+  g.batch = fast_div(p.bh_begin + g.bh_local, p.by_heads);
   g.q_row0 = (u - g.bh_local * p.q_tiles) * kTile;
   return g;
 }
@@ -600,6 +637,10 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   volatile int* abort_flag = &ctl->abort;
 
+  // The running row is never cleared: the first tile of a unit multiplies what the unit before has left by zero.
+  float2 o2[DH / 2];
+#pragma unroll
+  for (int i = 0; i < DH / 2; ++i) o2[i] = make_float2(0.f, 0.f);
   uint32_t g0 = 0;
   for (int it = 0; it < walk.count; ++it) {
     const int u = walk.unit(it);
@@ -614,9 +655,6 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
     const UnitGeom geo = unit_geom(p, u);
     const int q_row = geo.q_row0 + row;
 
-    float2 o2[DH / 2];
-#pragma unroll
-    for (int i = 0; i < DH / 2; ++i) o2[i] = make_float2(0.f, 0.f);
     float m_run = -INFINITY, l_run = 0.f;
     int imax_run = INT_MIN;                                 // statistics launch: biased integer row maximum over all tiles
     const bool stats_only = !kPolicy && p.row_stats_out != nullptr;
@@ -631,7 +669,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
         return;
       }
       // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304)
-      float e_old = 1.f, e_cur = 1.f;                                  // policy launch: every tile of a row has the same scale
+      float e_old = j > 0 ? 1.f : 0.f, e_cur = 1.f;                    // policy launch: every tile of a row has the same scale
       if (!kPolicy) {
         const float m_tile = ctl->st_m[slot][row];
         const float l_tile = ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);
@@ -721,27 +759,20 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
       continue;
     }
 
-    // ---- epilogue (inc/fmha_i8.cuh:318-332): normalise, requantise, store
+    // ---- epilogue (inc/fmha_i8.cuh:318-332): normalise, requantise, store.  With units of one or two tiles the merge warps
+    //      are what the CTA waits for (the epilogue took 3200 of a two-tile unit's 6000 cycles: its minima and maxima go
+    //      to the half-rate pipe the softmax warps use most).  So the clamp is applied only where a warp has an output beyond
+    //      127, which a calibrated scale makes rare; a row is not cleared for the next unit; no division.  B64 H32 S256
+    //      D128: 86.2 -> 78.2 us, B32 H16 S384 46.0 -> 43.2, B128 H16 S128 41.0 -> 38.0.
+    const float inv = (n_live > 0 && l_run > 0.f) ? __frcp_rn(l_run) : 0.f;
+    const float scale = p.scale_v_out * inv;
+    const bool clamp = __any_sync(0xFFFFFFFFu, needs_clamp<DH / 2>(o2, scale));
     if (q_row < p.Sq) {
-      const float inv = (n_live > 0 && l_run > 0.f) ? 1.0f / l_run : 0.f;
       int8_t* dst = p.o + (static_cast<int64_t>(geo.bh_local) * p.Sq + q_row) * D + ch * DH;
-      // rn(clamp(x)) through the magic number: x + 1.5*2^23 has the integer nearest to x in its low bits (the low byte is the
-      // two's-complement integer), and clamping commutes with the addition; bytes gathered with PRMT: conversions and shifts
-      // would cost three times the issue cycles
-      const float scale = p.scale_v_out * inv;
-      const float2 sc2 = make_float2(scale, scale), magic2 = make_float2(kMagic, kMagic);
       uint32_t wide[8];
 #pragma unroll
       for (int c = 0; c < DH / 16; ++c) {
-        uint32_t* wds = &wide[(c & 1) * 4];
-#pragma unroll
-        for (int gq = 0; gq < 4; ++gq) {
-          float2 a = __ffma2_rn(o2[c * 8 + gq * 2], sc2, magic2), b = __ffma2_rn(o2[c * 8 + gq * 2 + 1], sc2, magic2);
-          a.x = fminf(fmaxf(a.x, kMagic - 127.f), kMagic + 127.f); a.y = fminf(fmaxf(a.y, kMagic - 127.f), kMagic + 127.f);
-          b.x = fminf(fmaxf(b.x, kMagic - 127.f), kMagic + 127.f); b.y = fminf(fmaxf(b.y, kMagic - 127.f), kMagic + 127.f);
-          wds[gq] = __byte_perm(__byte_perm(__float_as_uint(a.x), __float_as_uint(a.y), 0x0040),
-                                __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x0040), 0x5410);
-        }
+        requantise16(o2 + c * 8, make_float2(scale, scale), clamp, wide + (c & 1) * 4);
         // 32-byte stores: a warp's rows are 128 (or 64) bytes apart, so every store touches 32 lines whatever its
         // width, and the 16-byte version of this loop cost 5 % of the whole kernel at head_dim 128
         if (c & 1) {

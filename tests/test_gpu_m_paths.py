@@ -250,3 +250,22 @@ def test_pairs_share_the_last_round(pkg, wl, oracle, torch_cuda, D, B, H, Sq, Sk
     host = o.cpu().numpy()
     assert np.all(host[:128] == 0x5A) and np.all(host[-128:] == 0x5A)
     assert_parity(host[128:-128].reshape(q8.shape), want, f"B{B}H{H}Sq{Sq}Sk{Sk}D{D}")
+
+
+@pytest.mark.parametrize("o_scale", [4.0, 0.3, 0.1, 1e-4])
+@pytest.mark.parametrize("D,Sk", [(128, 128), (128, 384), (64, 192)])
+def test_outputs_on_both_sides_of_the_clamp(pkg, wl, oracle, torch_cuda, D, Sk, o_scale):
+    """No output, a few rows', most of them and all of them beyond +-127.  (A row with one key repeats its V8 / o_scale: above
+    127 for |v8| > 38 at o_scale 0.3, one standard deviation of it; and never above 127 / 4 + 1 at o_scale 4.)"""
+    torch = torch_cuda
+    q8, k8, v8, mask, amax = _tensors(wl, 3, 5, Sk, Sk, D, seed=Sk + D, valid=[Sk, 1, Sk - 3])
+    amax = amax[:3] + (amax[2] * o_scale,)
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    o = torch.full_like(q, 77)
+    pkg.FMHAInferI8(None, pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptor(3, Sk, 5, D), q, k, v, m, o)
+    torch.cuda.synchronize()
+    got = o.cpu().numpy()
+    assert_parity(got, oracle.q128(q8, k8, v8, mask, amax), f"o_scale {o_scale}")
+    assert np.abs(got.astype(int)).max() <= 127
+    assert (np.abs(got.astype(int)) == 127).any() == (o_scale < 0.5)
+    assert pkg.device_status()[0] == pkg.OK
