@@ -88,7 +88,7 @@ struct UnitWalk {
 template <bool kPolicy>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base, const UnitWalk walk) {
   WorkerCtl* ctl = &all->w[worker];
-  const int lane = threadIdx.x & 31, quad = (threadIdx.x >> 5) & 3;
+  const int lane = threadIdx.x & 31, quad = warp_index() & 3;
   const int row = quad * 32 + lane;
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   const uint32_t tS = t_lane + static_cast<uint32_t>(worker * kTile), tP = tS;
@@ -411,7 +411,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
   uint8_t* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* presets = tiles + kWorkers * kWorkerBytes;
   Ctl* ctl = reinterpret_cast<Ctl*>(presets + kPresetBytesTotal);
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   if (threadIdx.x == 0) {
     ctl->abort = 0;
     for (WorkerCtl& w : ctl->w) {

@@ -498,7 +498,7 @@ __device__ __forceinline__ UnitGeom unit_geom(const FwdParams& p, int u) {
 template <int D, bool kPolicy>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                              const UnitWalk walk) {
-  const int warp = (threadIdx.x >> 5) - kWarpSoftmax0, lane = threadIdx.x & 31;
+  const int warp = warp_index() - kWarpSoftmax0, lane = threadIdx.x & 31;
   const int chain = warp >> 3, half = (warp >> 2) & 1, quad = warp & 3;
   const int row = quad * 32 + lane;
   // my 64 columns of S buffer 0; my P bytes go over their first 16 columns
@@ -546,10 +546,10 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       tc_fence_after();
       if (half == 0 && quad == 0) FMHA_STAMP(chain * 4 + 0, n);
 
-      // Order of my four 16-column chunks: the lower half row walks up, the upper half row walks DOWN.  At head_dim 64
-      // that lets each leave its P bytes over columns it has already consumed (the first 16 and the last 16 of the
+      // Order of my four 16-column chunks: at head_dim 64 the lower half row walks up, the upper half row walks DOWN, which
+      // lets each leave its P bytes over columns it has already consumed (the first 16 and the last 16 of the
       // accumulator); columns [16,112) stay untouched, and P.V of this step puts the partial output there.
-      const int c0 = half ? 3 : 0, cs = half ? -1 : 1;                 // first chunk and direction
+      const int c0 = !PLayout<D>::kAnnex && half ? 3 : 0, cs = !PLayout<D>::kAnnex && half ? -1 : 1;      // first chunk and direction
       // my 16 columns of P: inside the accumulator (head_dim 64) or in the annex of the buffer set (head_dim 128)
       const uint32_t tP = PLayout<D>::kAnnex
           ? tS0 - static_cast<uint32_t>(half * kHalf) + SBufs<D>::n * kTile + sb * PLayout<D>::kAnnexCols + static_cast<uint32_t>(half * 16)
@@ -631,7 +631,7 @@ template <int D, bool kPolicy>
 __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base, uint8_t* tiles,
                                            const UnitWalk walk) {
   constexpr int DH = D / 2;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int quad = warp & 3, ch = (warp - kWarpMerge0) >> 2;       // ch = which half of the output columns
   const int row = quad * 32 + lane;
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
@@ -794,7 +794,7 @@ template <int N> struct Flight { static constexpr int value = N; };
 // them (inc/fmha_i8.cuh:298-332).  A lane holds four columns.
 template <int D>
 __device__ __forceinline__ void merge_parts(const FwdParams& p, const uint32_t part_smem, const uint32_t tiles_smem, const int unit) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, parts = p.parts, rank = static_cast<int>(blockIdx.x) % parts;
+  const int lane = threadIdx.x & 31, warp = warp_index(), parts = p.parts, rank = static_cast<int>(blockIdx.x) % parts;
   const UnitGeom geo = unit_geom(p, unit);
   const int rows = min(kTile, p.Sq - geo.q_row0);
   constexpr int kLanes = D / 4, kRowsPerWarp = 32 / kLanes;
@@ -1067,7 +1067,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // The next launch of the stream may set itself up (barriers, tensor memory, constant operands: about 1.5 us with the
   // launch latency) on SMs this one leaves free, and waits below for this one to finish before it reads anything.
   grid_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = (p.S + kTile - 1) / kTile;
   const UnitWalk walk = unit_walk(p);
 

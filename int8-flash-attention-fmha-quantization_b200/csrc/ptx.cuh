@@ -7,6 +7,12 @@
 
 namespace fmha {
 
+// A value that is the same in all lanes, in a form from which the compiler can see it (all 32 lanes call this together).  What
+// is derived from it -- addresses of tensor memory and of barriers, descriptors, ring positions -- then lives in uniform registers
+// and on the uniform datapath; otherwise every tcgen05 instruction has its address brought over lane by lane, and the issue
+// slots this takes are what the forward kernels are short of.
+template <typename T> __device__ __forceinline__ T uniform(T v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+__device__ __forceinline__ int warp_index() { return uniform(static_cast<int>(threadIdx.x >> 5)); }
 // max(a, |b|, |c|) for a >= 0
 __device__ __forceinline__ float max3_abs(float a, float b, float c) {
   float r;
