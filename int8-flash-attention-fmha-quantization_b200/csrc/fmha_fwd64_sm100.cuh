@@ -97,7 +97,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
 
   uint32_t g = 0;                               // steps so far
   auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
-    if (__all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag))) return true;
+    if (warp_wait(bar, parity, abort_flag)) return true;
     raise_status(abort_flag, p.status, code, g);
     return false;
   };
@@ -292,7 +292,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   const int n_tiles = (p.S + kTile - 1) / kTile;
   uint32_t fail = 0u, g = 0, units = 0;
   auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
-    if (__all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag))) return true;
+    if (warp_wait(bar, parity, abort_flag)) return true;
     fail = code;
     return false;
   };

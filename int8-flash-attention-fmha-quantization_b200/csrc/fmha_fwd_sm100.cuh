@@ -143,10 +143,10 @@ constexpr int kInfoConsumers = 3 + kSoftmaxWarps + kMergeWarps;   // loader, two
 // launch and refuses otherwise); the targets per role (FwdRegs) add up to 28 x 72.
 constexpr int kLaunchRegs = 72;
 template <int D> struct FwdRegs {
-  // head_dim 128: the merge threads hold a 64-register half output row (B8 H32 S2048: 96/56 is 1.3 % faster than 104/40
-  // and as fast as 88/72).  head_dim 64: the output row is 32 registers; 88/72 is the split at which
+  // head_dim 128: the merge threads hold a 64-register half output row (B8 H32 S2048: 104/40 takes 405 us, 96/56
+  // 410, 88/72 427).  head_dim 64: the output row is 32 registers; 88/72 is the split at which
   // ptxas reports no spills at all, and C5 runs 5 % faster with it than with 80/88 or 96/56, which both spill.
-  static constexpr int kSoftmax = 64, kMerge = (D == 128) ? 96 : 88, kOther = (D == 128) ? 56 : 72;
+  static constexpr int kSoftmax = 64, kMerge = (D == 128) ? 104 : 88, kOther = (D == 128) ? 40 : 72;
   static_assert(kSoftmaxWarps * kSoftmax + kMergeWarps * kMerge + 4 * kOther <= kFwdWarps * kLaunchRegs,
                 "setmaxnreg targets exceed the CTA's register allocation: the kernel would hang");
   static_assert(kSoftmax <= kLaunchRegs && kMerge >= kLaunchRegs, "the softmax warps give registers, the merge warps gain");

@@ -113,6 +113,14 @@ __device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, co
   return mbar_wait_backoff<FMHA_SLEEP_SLOW>(bar, parity, abort_flag, kWaitLimitCycles, kMinProbes);
 }
 
+// Warp-wide wait of the head_dim-64 workers: most of their waits find the phase complete, and without the loop around the
+// first probe that costs three instructions (B8 H32 S2048: 345 -> 342 us).  Not for the other kernel: at head_dim 128 it is as
+// fast for long sequences, but its short units get 3 % slower.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag));
+}
+
 // One lane of a converged warp (the same one every time).  The single-thread roles of the forward kernel run
 // warp-wide with only their side-effecting instructions behind this predicate: addresses, descriptors and loop
 // counters are then warp-uniform values.
