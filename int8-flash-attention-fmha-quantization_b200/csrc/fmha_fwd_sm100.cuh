@@ -22,8 +22,8 @@
 //   warp 0       loader: TMA brings Q (once per unit, in a small ring) and rings of K and of V tiles into
 //                swizzled shared memory, running ahead into the next units.
 //   warp 1       S issuer:  S_b = bias + Q . K_g^T  (tcgen05.mma smem x smem -> int32 in tensor memory).
-//   warp 2       scanner: turns the coming units' padding-mask rows into per-tile bit masks and the list of
-//                key tiles that hold at least one unmasked key (ring of four).
+//   warp 2       scanner: turns the coming units' padding-mask rows into the list of key tiles that hold at least
+//                one unmasked key, each marked if it has masked keys too (ring of four).
 //   warp 3       P.V issuer:  O~ = bias + P_b . V_g  (tcgen05.mma tmem x smem -> int32 in tensor memory) when the
 //                softmax warps have written P_b.
 //                These four run warp-wide -- every lane waits and counts, one elected lane issues -- so that
@@ -40,6 +40,10 @@
 //                consumed (the lower half row walks up and leaves P in columns [0,16), the upper one walks down
 //                and leaves it in [112,128)).
 //                These threads hold no output row, so they are light (64 registers).
+//
+// What bounds it: issue slots (64 % busy; 4300 warp instructions for a step of 128 x 128 scores at head_dim 128, 2700 of them
+// arithmetic) and the exponential unit (63 %), on a chain of hand-offs that the sets of buffers overlap; in units of one or two
+// steps the merge warps, which spend more on a unit's epilogue than on a step.  B8 H32 S2048 D128: 405 us.
 //
 // The bias: every accumulator is first written by a one-step bf16 MMA whose operands hold 4096 and
 // 3072, i.e. the fp32 value 1.5*2^23 (bits 0x4B400000); the int8 MMAs then add their integer result
@@ -71,12 +75,6 @@
 #include "ptx.cuh"
 #include "../../include/fmha_i8_c.h"
 
-// 1: the partial-output accumulators are preset to the bit pattern of 1.5*2^23 by a one-step fp16 MMA (as the S
-//    accumulators are), so the merge threads read floats; 0: they add that bit pattern themselves, one integer
-//    addition per element.
-#ifndef FMHA_PV_BIAS_MMA
-#define FMHA_PV_BIAS_MMA 1
-#endif
 // Ring depths can be overridden at compile time for tuning runs.
 #ifndef FMHA_STAGES_K128
 #define FMHA_STAGES_K128 3
@@ -323,7 +321,6 @@ __device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_ro
 constexpr uint32_t kBiasA = 0x71804580u;         // {4096, 2^100}
 constexpr uint32_t kBiasB = 0x00004540u;         // {3072, 0}
 constexpr uint32_t kBiasBMasked = 0xCD004540u;   // {3072, -2^27}
-__device__ __forceinline__ int bias_row_offset(int row) { return (row >> 3) * 256 + (row & 7) * 16; }
 __device__ __forceinline__ void fill_bias_operands(uint8_t* bias_a, int n_b) {
   for (int i = threadIdx.x; i < (1 + n_b) * kBiasBytes / 16; i += blockDim.x)      // the B operands follow A
     reinterpret_cast<uint4*>(bias_a)[i] = make_uint4((i & 8) ? 0u : i < kBiasBytes / 16 ? kBiasA : kBiasB, 0u, 0u, 0u);
@@ -418,9 +415,6 @@ __device__ __forceinline__ RowConsts row_consts(const int imax, const float c2s,
   return k;
 }
 
-// o2 (+)= e_cur * (P8 . V) for N output columns.  r = accumulator: either preset by the bias MMA, so that it reads
-// as the float kMagic + (P8 . V), or a raw int32 (|r| < 2^22) that becomes that float by adding the bit pattern
-// of 1.5*2^23 -- no conversion instruction either way.
 // Does any of N pairs of the unnormalised output leave [-127, 127] when it is multiplied by `scale` and rounded?
 template <int N> __device__ __forceinline__ bool needs_clamp(const float2* o2, const float scale) {
   float m0 = 0.f, m1 = 0.f;
@@ -447,15 +441,13 @@ __device__ __forceinline__ void requantise16(const float2* o2, const float2 scal
                            __byte_perm(__float_as_uint(v[2 * i + 1].x), __float_as_uint(v[2 * i + 1].y), 0x0040), 0x5410);
 }
 
+// o2 = e_old * o2 + e_cur * (P8 . V) for N output columns.  r = accumulator, preset by the bias MMA, so that it reads as the float
+// kMagic + (P8 . V).
 template <int N>
 __device__ __forceinline__ void drain_chunk(const uint32_t (&r)[N], float2* o2, const float2 neg_ec, const float2 e_bias, const float2 e_old) {
 #pragma unroll
   for (int i = 0; i < N / 2; ++i) {
-#if FMHA_PV_BIAS_MMA
     const float2 x = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-#else
-    const float2 x = make_float2(__uint_as_float(r[2 * i] + kMagicBits), __uint_as_float(r[2 * i + 1] + kMagicBits));
-#endif
     const float2 t = __ffma2_rn(x, neg_ec, e_bias);          // e_cur * (P8 . V), exact product before rounding
     o2[i] = __ffma2_rn(o2[i], e_old, t);
   }
@@ -998,11 +990,9 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   volatile int* abort_flag = &ctl->abort;
   // O = P.V : V is an MN-major operand; one group of MMAs with N = head_dim output columns
   const uint32_t idesc_o = p.p_unsigned ? make_idesc_i8(D, true, true) : make_idesc_i8(D, true, false);
-#if FMHA_PV_BIAS_MMA
   constexpr uint32_t idesc_bias = make_idesc_bf16(D);
   const uint64_t d_bias_a = make_smem_desc_noswizzle(bias_a_smem, 128, 256);
   const uint64_t d_bias_b = make_smem_desc_noswizzle(bias_b_smem, 128, 256);
-#endif
   IssuerErr err;
   uint32_t g = 0;
   bool ok = true;
@@ -1027,12 +1017,10 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       // The accumulator of this step is S(g)'s own buffer (free since the softmax threads have read S(g)), minus the
       // columns that hold P bytes at head_dim 64.
       if (elect_one()) {
-#if FMHA_PV_BIAS_MMA
         mma_f16_ss(tO, d_bias_a, d_bias_b, idesc_bias, 0u);      // accumulator := 0x4B400000
-#endif
 #pragma unroll
         for (int kk = 0; kk < kTile / 32; ++kk)
-          mma_i8_ts(tO, tP + PLayout<D>::p_col(kk), desc_advance(dv, kk * 32 * D), idesc_o, (FMHA_PV_BIAS_MMA || kk > 0) ? 1u : 0u);
+          mma_i8_ts(tO, tP + PLayout<D>::p_col(kk), desc_advance(dv, kk * 32 * D), idesc_o, 1u);
         mma_commit(smem_u32(&ctl->o_full[sb]));
         mma_commit(smem_u32(&ctl->v_empty[stage]));
       }
