@@ -15,8 +15,9 @@
 //     bytes of four keys transposed with eight byte permutations.  About 770 warp instructions per tile of 32 KB and one
 //     row, an eighth of what the SM can issue while that tile arrives.
 // Measured against the tensor-core kernel, cross attention B16 H32 D128, 1025..4096 keys of 4096 per sequence, one row
-// per head (336 MB): 104.3 -> 52.6 us,
-// 98 % of the measured copy bandwidth.
+// per head (336 MB): 104.3 -> 50.8 us,
+// the measured copy bandwidth.  (52.9 of it with a warp index that the compiler could not see to be uniform; B1 H32 with 16384
+// keys 31.0 -> 28.4.)
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -63,7 +64,7 @@ fmha_decode_kernel(const int8_t* __restrict__ q, const int8_t* __restrict__ k, c
   extern __shared__ __align__(128) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   grid_launch_dependents();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_index();
   const int ctas = static_cast<int>(cluster_ctas()), rank = static_cast<int>(cluster_rank());
   const int unit = static_cast<int>(blockIdx.x) / ctas;
   const int bh = unit / p.q_tiles, row0 = (unit - bh * p.q_tiles) * R;

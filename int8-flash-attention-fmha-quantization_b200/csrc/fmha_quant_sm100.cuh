@@ -9,7 +9,7 @@
 //                         registers the first ones (53 MB over the chip); pass 2 takes those from there and walks the
 //                         others from the last to the first, so that it meets what the L2 still has.
 // Two launches over 65,536-element chunks, which these replace, took 16.5 us for 255,749 elements (four CTAs) and 107 us
-// for 67,108,864; these take 5.5 and 95 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
+// for 67,108,864; these take 5.5 and 93.5 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
 // what neither the SMs (50 MB) nor the L2 kept.
 #pragma once
 #include <cuda_runtime.h>
@@ -127,7 +127,7 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
   __shared__ float warp_max[kQuantWarps];
   __shared__ float s_amax;
   __shared__ int s_abort;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_index();
   float* ring = reinterpret_cast<float*>(ring_raw) + warp * (kQuantStages * kQuantTile);
   uint64_t* bar = bars[warp];
   QuantSlot* slot = &g_quant_slots[slot_index];
