@@ -329,14 +329,15 @@ void plan_parts(FwdParams* p, const DeviceInfo* dev) {
 }
 
 // Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  Cycles per key tile, measured: a CTA of
-// fmha_fwd_sm100.cuh works on one unit at a time, 1700 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5800 per
-// tile for all four, 5300 / 4700 / 3900 with three, two or one left in the last round.  (B16 H16 S256: 12.8 / 11.6 us; B8 H12
-// S512: 16.3 / 16.0; B4 H12 S512: 12.2 / 13.7; B2 H12 S1024: 19.5 / 23.3; B1 H8 S16384: 778 / 779.)
+// fmha_fwd_sm100.cuh works on one unit at a time, 1600 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5850 per
+// tile for all four, 4900 / 4350 / 3400 with three, two or one left in the last round.  (B12 H12 S256: 8.2 / 7.9 us; B6 H12
+// S512: 11.6 / 12.5; B16 H12 S512: 26.8 / 26.2; B3 H12 S1024: 18.4 / 21.5; B8 H12 S1024: 44.2 / 46.2; B1 H24 S2048: 45.0 / 44.4;
+// B1 H40 S2048: 66.7 / 80.4.)
 bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
   const long long sms = dev->sm_count, tiles = (p.S + kTile - 1) / kTile, round = sms * w64::kWorkers;
-  const long long last[w64::kWorkers + 1] = {0, 3900, 4700, 5300, 5800};
-  const long long workers = p.n_units / round * 5800 + last[(p.n_units % round + sms - 1) / sms];
-  const long long own = p.n_units / sms, more = p.n_units % sms != 0, unit = 1700 * tiles + 1200;
+  const long long last[w64::kWorkers + 1] = {0, 3400, 4350, 4900, 5850};
+  const long long workers = p.n_units / round * 5850 + last[(p.n_units % round + sms - 1) / sms];
+  const long long own = p.n_units / sms, more = p.n_units % sms != 0, unit = 1600 * tiles + 1200;
   return workers * tiles < own * unit + more * (pairs_share_last_round(p, dev) ? unit / 2 + 4500 : unit);
 }
 
