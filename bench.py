@@ -535,8 +535,10 @@ def main():
             o_ref = torch.empty_like(data["q8"])
             pkg.FMHAInferI8(stream, param, desc, data["q8"], data["k8"], data["v8"], mask, o_ref, True)
             torch.cuda.synchronize()
-            same = bool(torch.equal(whole.reshape(o_ref.shape), o_ref))
-            partition_check = {"slices_equal_whole_problem_run": same, "coverage": cov,
+            diff = (whole.reshape(o_ref.shape).to(torch.int16) - o_ref.to(torch.int16)).abs()
+            partition_check = {"slices_equal_whole_problem_run": not bool(diff.any()),
+                               # (a slice may share the keys of its last units among CTAs where the whole does not)
+                               "difference": {"elements": int((diff != 0).sum()), "max_lsb": int(diff.max())}, "coverage": cov,
                                "heads_per_rank": [part.slice_bounds(BH, r, world)[1] for r in range(world)]}
             o8_whole = o_ref
     elif rank == 0:
@@ -577,10 +579,13 @@ def main():
         for _ in range(n_e2e):
             pkg.FMHAInferI8HostSlice(param, desc, hq, hk, hv, hm, ho, begin, count)
         dt = max_ranks((time.perf_counter() - t0) / n_e2e)
-        same = bool(torch.equal(ho, o8s.cpu()))
+        host_diff = (ho.to(torch.int16) - o8s.cpu().to(torch.int16)).abs()
+        same = not bool(host_diff.any())
         e2e = {"value": job_ops / dt / 1e12, "unit": UNIT, "h2d_bytes_per_step": int(3 * q8s.numel() + mask.numel()),
                "d2h_bytes_per_step": int(o8s.numel()), "ms_per_step": dt * 1e3, "steps": n_e2e,
-               "bytes_are": "per rank", "matches_device_resident_result": same}
+               "bytes_are": "per rank", "matches_device_resident_result": same,
+               # (pieces of the host path may share the keys of their last units among CTAs where the whole does not)
+               "difference_from_device_resident_result": {"elements": int((host_diff != 0).sum()), "max_lsb": int(host_diff.max())}}
         del hq, hk, hv, ho
 
     # ---- the same step back to back for at least a second, with the clocks of that second
