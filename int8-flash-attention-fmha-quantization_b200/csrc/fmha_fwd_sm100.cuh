@@ -53,8 +53,9 @@
 //
 // The padding mask goes the same way: where a key tile has masked keys, the issuer of S presets their columns to -2^127
 // instead (a second product, 2^100 * -2^27, that swallows the first).  The scores added to that bit pattern leave a float
-// of the same size, below every real score as an integer and as a float, and its exponential is exactly zero: the softmax
-// threads treat every tile alike.  Before, they tested a mask bit per score in a loop that was not pipelined: B256 H16 S256
+// of the same size (-2^126 at the least), below every real score as an integer and as a float.  Its exponential is zero,
+// or 2^-126 where the workers of fmha_fwd64_sm100.cuh compute it on the multiply-add pipe: nothing beside the row maximum's 1, and
+// quantised to zero.  (As long as 2^126 * c2 is large: kMinC2.)  The softmax threads treat every tile alike.  Before, they tested a mask bit per score in a loop that was not pipelined: B256 H16 S256
 // D64 with lengths 64..256 took 132 us instead of 115, B24 H16 S576 D64 with lengths 300..576 66 instead of 59, and the
 // smaller code makes unmasked head_dim-64 calls faster too (B8 H32 S2048: 430 -> 400 us).
 //
@@ -153,6 +154,11 @@ template <int D> struct FwdRegs {
 constexpr uint32_t kTmemCols = 512;
 constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23: float whose ulp is 1 over [2^23, 2^24)
 constexpr uint32_t kMagicBits = 0x4B400000u;
+// Smallest factor from scores to exponents that the kernels work with, far from both of its limits.  A masked key's score is -2^126
+// or less, and its exponent has to be below -150 for the exponential to be zero: 2^126 * 2^-100 = 2^26.  The scores of a row differ by
+// at most 2 * 128 * 128 * head_dim = 2^22, and 2^22 * 2^-100 = 2^-78 is far below half an ulp of 1 (2^-25): the exponentials of a
+// call whose own factor is smaller are all 1, and they are with this one.
+constexpr float kMinC2 = 0x1p-100f;
 constexpr int kBiasBytes = 4096;               // 128 rows x 16 bf16, unswizzled core-matrix layout
 template <int D> __host__ __device__ constexpr int bias_bytes() { return (2 + SBufs<D>::n) * kBiasBytes; }
 

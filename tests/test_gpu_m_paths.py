@@ -141,6 +141,40 @@ def test_masked_keys_vanish_at_every_scale(pkg, wl, oracle, torch_cuda, D, amax_
     assert_parity(o.cpu().numpy(), oracle.q128(q8, np.ascontiguousarray(k8), np.ascontiguousarray(v8), mask, amax))
 
 
+# Scores so small that all probabilities of a row are equal: masked keys still count for nothing.  Scales on both sides of the
+# smallest factor from scores to exponents that the kernels work with (2^-100), where a masked key's preset alone would no longer
+# vanish, and close to the smallest that a call accepts; on every kernel that presets masked keys, and on the one that does not.
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("c2", [2.0 ** -99.9, 2.0 ** -100.1, 2.0 ** -126, 2.0 ** -145])
+@pytest.mark.parametrize("what,B,H,Sq,Sk", [("plain", 2, 3, 320, 320), ("many", 30, 13, 100, 192), ("few_rows", 2, 2, 4, 704), ("shared", 2, 16, 200, 1984),
+                                            ("row", 2, 3, 320, 320), ("row", 30, 13, 100, 192), ("host", 6, 11, 640, 640)])
+def test_masked_keys_vanish_at_the_smallest_scales(pkg, wl, oracle, torch_cuda, D, c2, what, B, H, Sq, Sk):
+    torch = torch_cuda
+    valid = np.random.default_rng(B).integers(1, Sk, B)
+    q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, D, seed=D + Sk, mask_p=0.1, valid=valid)
+    v8 = np.where(mask[:, None, :, None] != 0, np.int8(127), v8)                 # what masked keys would add shows
+    each = float(np.sqrt(c2 * np.sqrt(D) * 127.0 ** 2 / np.log2(np.e)))          # q_amax and k_amax for that factor
+    amax = (each, each, amax[2], amax[3])
+    param = pkg.FMHAParamI8(*amax, 1.0)
+    desc, desc_x = pkg.AttnDataDescriptor(B, Sk, H, D), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D)
+    want = (oracle.policy(q8, k8, v8, mask, (*amax, 1.0), oracle.POLICY_ROW) if what == "row" else oracle.q128(q8, k8, v8, mask, amax))
+    if what == "host":
+        host = [torch.from_numpy(x).pin_memory() for x in (q8, k8, v8, mask)]
+        o = torch.zeros_like(host[0]).pin_memory()
+        dirty = [torch.full_like(t, 111).pin_memory() for t in host[:3]]         # what the staging rows of keys that are not fetched hold
+        pkg.FMHAInferI8Host(param, desc, *dirty, torch.zeros_like(host[3]), o)
+        pkg.FMHAInferI8Host(param, desc, *host, o)
+    else:
+        q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+        o = torch.zeros_like(q)
+        if what == "row":
+            pkg.FMHAInferI8Policy(None, param, desc_x, q, k, v, m, o, pkg.POLICY_ROW, torch.zeros(2 * B * H * Sq, device="cuda"))
+        else:
+            pkg.FMHAInferI8Cross(None, param, desc_x, q, k, v, m, o)
+    assert pkg.device_status()[0] == pkg.OK
+    assert_parity(o.cpu().numpy(), want, f"{what} D{D} c2 {c2}")
+
+
 # Calls at head_dim 64 with many query tiles run four workers to an SM: fewer units than workers, all workers busy, a last round with
 # one worker, several rounds; key tiles half beyond the sequence, sequences without a key, a mask with holes in every tile.
 @pytest.mark.parametrize("B,H,Sq,Sk,mask_p", [(50, 8, 64, 64, 0.0), (30, 13, 100, 192, 0.3), (37, 16, 128, 128, 0.0), (11, 9, 961, 448, 0.05)])
