@@ -144,6 +144,11 @@ int fmha_i8_sm100_infer_host_slice(const float amax[5], const int desc[4],
                                    const void* host_mask, void* host_o, int bh_begin, int bh_count,
                                    unsigned flags);
 
+/* Debug: how fmha_i8_sm100_infer_host would bring these inputs in, without doing it: 1 = a kernel reads the host buffers (all of q, k
+ * and v lie in pinned memory), 0 = copies, negative = FMHA_I8_ERR_*.  Reads the mask, launches nothing. */
+int fmha_i8_sm100_debug_host_fetch(const int desc[4], const void* host_q, const void* host_k, const void* host_v,
+                                   const void* host_mask);
+
 /* Debug: S_int32[bh, i, j] = sum_d q[bh,i,d] k[bh,j,d] written as int32 [B*H, S, S] through the
  * same TMA + tensor-core stage the forward pass uses (GEMM 1, inc/fmha_i8.cuh:120-172).  For
  * bit-exact checks against cpuGEMM<int32_t,int32_t,int8_t,int32_t>; small shapes only. */

@@ -37,7 +37,7 @@ FLAG_UINT8_P = 2     # P quantised as unsigned 8 bit, 255 levels (the reference 
 EXPORTS = (
     "fmha_i8_sm100_infer", "fmha_i8_sm100_infer_slice", "fmha_i8_sm100_infer_cross", "fmha_i8_sm100_calibrate_o_amax", "fmha_i8_sm100_infer_host",
     "fmha_i8_sm100_infer_host_slice", "fmha_i8_sm100_infer_policy",
-    "fmha_i8_sm100_debug_qk", "fmha_i8_sm100_debug_pv", "fmha_i8_sm100_debug_simt", "fmha_i8_sm100_debug_simt_x", "fmha_i8_sm100_debug_wait_probe",
+    "fmha_i8_sm100_debug_host_fetch", "fmha_i8_sm100_debug_qk", "fmha_i8_sm100_debug_pv", "fmha_i8_sm100_debug_simt", "fmha_i8_sm100_debug_simt_x", "fmha_i8_sm100_debug_wait_probe",
     "fmha_i8_sm100_quantize_f32", "fmha_i8_sm100_quantize_f32_noalloc", "fmha_i8_sm100_device_status", "fmha_i8_sm100_last_status", "fmha_i8_sm100_status_string",
     "fmha_i8_sm100_launch_count", "fmha_i8_sm100_version",
 )
@@ -106,6 +106,7 @@ def lib():
         L.fmha_i8_sm100_infer_policy.argtypes = [vp, fp, ip, vp, vp, vp, vp, vp, ctypes.c_int, ctypes.c_int, u, ctypes.c_int, vp]
         L.fmha_i8_sm100_infer_host.argtypes = [fp, ip, vp, vp, vp, vp, vp, u]
         L.fmha_i8_sm100_infer_host_slice.argtypes = [fp, ip, vp, vp, vp, vp, vp, ctypes.c_int, ctypes.c_int, u]
+        L.fmha_i8_sm100_debug_host_fetch.argtypes = [ip, vp, vp, vp, vp]
         L.fmha_i8_sm100_debug_qk.argtypes = [vp, ip, vp, vp, vp]
         L.fmha_i8_sm100_debug_pv.argtypes = [vp, ip, vp, vp, vp, u]
         L.fmha_i8_sm100_debug_simt.argtypes = [vp, fp, ip, vp, vp, vp, vp, vp]
@@ -257,6 +258,14 @@ def FMHAInferI8HostSlice(fmha_param, attn_desc, host_q, host_k, host_v, host_mas
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8HostSlice")
     return st
+
+
+def debug_host_fetch(attn_desc, host_q, host_k, host_v, host_mask):
+    """Would FMHAInferI8Host have a kernel read these host buffers (True) or copy them (False)?  Launches nothing."""
+    st = lib().fmha_i8_sm100_debug_host_fetch(attn_desc.as_c(), _ptr(host_q), _ptr(host_k), _ptr(host_v), _ptr(host_mask))
+    if st < 0:
+        raise FmhaError(st, "debug_host_fetch")
+    return st == 1
 
 
 def debug_qk(stream, attn_desc, q, k, s_out):

@@ -173,19 +173,23 @@ int set_kernel_attributes(DeviceInfo* d) {
   return FMHA_I8_OK;
 }
 
-// cuTensorMapEncodeTiled, fetched through the runtime so the library has no link-time libcuda dependency.
+// Driver entry points, fetched through the runtime so the library has no link-time libcuda dependency.
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+using PointerAttributeFn = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+template <typename Fn> Fn driver_fn(const char* name) {
+  void* f = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return nullptr;
+  return reinterpret_cast<Fn>(f);
+}
 EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
+  static EncodeTiledFn fn = driver_fn<EncodeTiledFn>("cuTensorMapEncodeTiled");
+  return fn;
+}
+PointerAttributeFn pointer_attribute_fn() {
+  static PointerAttributeFn fn = driver_fn<PointerAttributeFn>("cuPointerGetAttribute");
   return fn;
 }
 
@@ -515,6 +519,22 @@ struct FetchPlan {
   bool by_kernel = false;
   const void *q = nullptr, *k = nullptr, *v = nullptr;     // device addresses of the host buffers
 };
+// Device address of a host buffer, if all of it lies in one pinned, device-readable block (allocated or registered) and is 16-byte
+// aligned; nullptr otherwise.  A kernel that reads past the registered part of a buffer faults, a copy is refused by the runtime.
+const void* device_view(const void* host, size_t bytes) {
+  cudaPointerAttributes attr{};
+  if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (attr.type != cudaMemoryTypeHost || attr.devicePointer == nullptr || !aligned(attr.devicePointer, 16)) return nullptr;
+  const PointerAttributeFn query = pointer_attribute_fn();
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(attr.devicePointer);
+  CUdeviceptr block = 0;
+  size_t block_bytes = 0;
+  if (!query || query(&block, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+      query(&block_bytes, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS || at < block || at - block > block_bytes ||
+      bytes > block_bytes - (at - block))
+    return nullptr;
+  return attr.devicePointer;
+}
 FetchPlan plan_fetch(const int desc[4], const void* host_q, const void* host_k, const void* host_v, const int8_t* host_mask, int bh_begin, int bh_count, int n_chunks) {
   FetchPlan plan;
   const int S = desc[1], H = desc[2], D = desc[3];
@@ -530,16 +550,33 @@ FetchPlan plan_fetch(const int desc[4], const void* host_q, const void* host_k, 
   }
   const double us_kernel = rows * D / 50.7e3 + 5.0 * n_chunks, us_copies = 3.0 * bh_count * S * D / 54.7e3 + 12.0 * n_chunks;
   if (us_kernel > us_copies) return plan;
-  const void* host[3] = {host_q, host_k, host_v};
-  const void** seen[3] = {&plan.q, &plan.k, &plan.v};
-  for (int i = 0; i < 3; ++i) {
-    cudaPointerAttributes attr{};
-    if (cudaPointerGetAttributes(&attr, host[i]) != cudaSuccess) { cudaGetLastError(); return plan; }
-    if (attr.type != cudaMemoryTypeHost || attr.devicePointer == nullptr || !aligned(attr.devicePointer, 16)) return plan;
-    *seen[i] = attr.devicePointer;
-  }
-  plan.by_kernel = true;
+  const size_t bytes = static_cast<size_t>(bh_count) * S * D;
+  plan.q = device_view(host_q, bytes);
+  plan.k = plan.q ? device_view(host_k, bytes) : nullptr;
+  plan.v = plan.k ? device_view(host_v, bytes) : nullptr;
+  plan.by_kernel = plan.v != nullptr;
   return plan;
+}
+
+// Cuts the heads of a host-buffer call into the chunks of its pipeline; returns their number.
+// Each piece of the inbound transfer costs some microseconds, so there are few; what follows the last of them -- its kernel
+// and its outbound copy -- is exposed, so the pieces shrink by halves: a chunk's outbound copy, a third of its inbound
+// bytes, is hidden behind the next chunk's inbound transfer.  Long sequences, where the kernels take the time, are cut evenly.
+// (us, eight even chunks of three copies -> this: B32 H12 S512 D64 with lengths 256..512 976 -> 846, without padding 979 -> 890,
+// B8 H12 S512 with lengths 300..512 340 -> 244, B1 H4 S256 82 -> 36, B4 H32 S2048 D128 2350 -> 2168.)
+int cut_heads(const int desc[4], int bh_count, int (&bounds)[kHostChunks + 1]) {
+  const int BH = bh_count;
+  const size_t bytes_in = 3 * static_cast<size_t>(bh_count) * desc[1] * desc[3];
+  const bool even = desc[1] > kHostLongSeq;
+  const int wanted = even ? kHostChunks : bytes_in < (3u << 19) ? 1 : bytes_in < (6u << 20) ? 2 : bytes_in < (64u << 20) ? 4 : 6;
+  const int n_chunks = BH < wanted ? BH : wanted;
+  bounds[0] = 0;
+  for (int i = 1; i <= n_chunks; ++i) {
+    const double done = even ? static_cast<double>(i) / n_chunks : (1.0 - std::ldexp(1.0, -i)) / (1.0 - std::ldexp(1.0, -n_chunks));
+    const int rounded = static_cast<int>(std::lround(done * BH)), least = bounds[i - 1] + 1, most = BH - (n_chunks - i);     // every chunk has a head
+    bounds[i] = rounded < least ? least : rounded > most ? most : rounded;
+  }
+  return n_chunks;
 }
 
 int check_quant_args(const float* x, long long n, const int8_t* out) {
@@ -684,23 +721,8 @@ static int infer_host_slice_impl(const float amax[5], const int desc[4], const v
   }
   // Pipeline over contiguous ranges of heads: while chunk i is computed, chunk i+1 is on its way in and
   // chunk i-1 on its way out (the bus is full duplex).  Each chunk is one forward launch on a sub-slice.
-  // Each piece of the inbound transfer costs some microseconds, so there are few; what follows the last of them -- its kernel
-  // and its outbound copy -- is exposed, so the pieces shrink by halves: a chunk's outbound copy, a third of its inbound
-  // bytes, is hidden behind the next chunk's inbound transfer.  Long sequences, where the kernels take the time, are cut evenly.
-  // (us, eight even chunks of three copies -> this: B32 H12 S512 D64 with lengths 256..512 976 -> 846, without padding 979 -> 890,
-  // B8 H12 S512 with lengths 300..512 340 -> 244, B1 H4 S256 82 -> 36, B4 H32 S2048 D128 2350 -> 2168.)
-  const int BH = bh_count;
-  const size_t bytes_in = 3 * tensor_bytes;
-  const bool even = desc[1] > kHostLongSeq;
-  const int wanted = even ? kHostChunks : bytes_in < (3u << 19) ? 1 : bytes_in < (6u << 20) ? 2 : bytes_in < (64u << 20) ? 4 : 6;
-  const int n_chunks = BH < wanted ? BH : wanted;
   int bounds[kHostChunks + 1];
-  bounds[0] = 0;
-  for (int i = 1; i <= n_chunks; ++i) {
-    const double done = even ? static_cast<double>(i) / n_chunks : (1.0 - std::ldexp(1.0, -i)) / (1.0 - std::ldexp(1.0, -n_chunks));
-    const int rounded = static_cast<int>(std::lround(done * BH)), least = bounds[i - 1] + 1, most = BH - (n_chunks - i);     // every chunk has a head
-    bounds[i] = rounded < least ? least : rounded > most ? most : rounded;
-  }
+  const int n_chunks = cut_heads(desc, bh_count, bounds);
   const FetchPlan plan = plan_fetch(desc, host_q, host_k, host_v, static_cast<const int8_t*>(host_mask), bh_begin, bh_count, n_chunks);
   LaunchMode mode;
   mode.busy_sms = plan.by_kernel ? kFetchCtas : 0;
@@ -753,6 +775,18 @@ int fmha_i8_sm100_infer_host_slice(const float amax[5], const int desc[4], const
                                    const void* host_v, const void* host_mask, void* host_o, int bh_begin, int bh_count,
                                    unsigned flags) {
   return finish(infer_host_slice_impl(amax, desc, host_q, host_k, host_v, host_mask, host_o, bh_begin, bh_count, flags));
+}
+
+int fmha_i8_sm100_debug_host_fetch(const int desc[4], const void* host_q, const void* host_k, const void* host_v, const void* host_mask) {
+  if (!desc || !host_q || !host_k || !host_v || !host_mask) return finish(FMHA_I8_ERR_NULL_POINTER);
+  const int st = check_shape(desc);
+  if (st != FMHA_I8_OK) return finish(st);
+  const long long BH = static_cast<long long>(desc[0]) * desc[2];
+  if (BH > 0x7FFFFFFFLL) return finish(FMHA_I8_ERR_BAD_SHAPE);
+  int bounds[kHostChunks + 1];
+  const int n_chunks = cut_heads(desc, static_cast<int>(BH), bounds);
+  finish(FMHA_I8_OK);
+  return plan_fetch(desc, host_q, host_k, host_v, static_cast<const int8_t*>(host_mask), 0, static_cast<int>(BH), n_chunks).by_kernel ? 1 : 0;
 }
 
 int fmha_i8_sm100_debug_qk(void* stream, const int desc[4], const void* q, const void* k, int32_t* s_out) {

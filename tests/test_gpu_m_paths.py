@@ -266,6 +266,41 @@ def test_host_buffers(pkg, wl, oracle, torch_cuda, B, H, S, D, valid, pinned):
     assert pkg.device_status()[0] == pkg.OK
 
 
+def test_only_wholly_pinned_buffers_are_read_by_a_kernel(pkg, torch_cuda):
+    """A kernel that reads host memory must find every byte of it pinned.  Only the decision is looked at; nothing is launched."""
+    torch = torch_cuda
+    B, H, S, D = 6, 11, 640, 64
+    n, page = B * H * S * D, 4096
+    desc, mask = pkg.AttnDataDescriptor(B, S, H, D), torch.ones((B, S), dtype=torch.int8)
+    mask[:, :64] = 0                                     # so much padding that the kernel is worth it
+    pinned = [torch.zeros(n + page, dtype=torch.int8).pin_memory() for _ in range(3)]
+    q, k, v = (t[:n] for t in pinned)
+    assert pkg.debug_host_fetch(desc, q, k, v, mask)
+    assert pkg.debug_host_fetch(desc, pinned[0][page:], k, v, mask)                  # up to the end of its block
+    assert not pkg.debug_host_fetch(desc, pinned[0][8:], k, v, mask)                 # not 16-byte aligned
+    plain = np.zeros(n + 3 * page, np.int8)
+    first = (plain.ctypes.data + page - 1) // page * page
+    assert not pkg.debug_host_fetch(desc, q, first, v, mask)                         # pageable
+    rt = torch.cuda.cudart()
+
+    def with_registered(ranges):
+        """The decision for q, k or v at `first`, with these byte ranges behind it registered."""
+        try:
+            done = []
+            for begin, end in ranges:
+                assert int(rt.cudaHostRegister(first + begin, end - begin, 0)) == 0
+                done.append(begin)
+            return [pkg.debug_host_fetch(desc, *(first if i == j else t for j, t in enumerate((q, k, v))), mask) for i in range(3)]
+        finally:
+            for begin in done:
+                rt.cudaHostUnregister(first + begin)
+
+    whole = (n + page - 1) // page * page
+    assert with_registered([(0, whole)]) == [True] * 3
+    assert with_registered([(0, whole - page)]) == [False] * 3                       # all but the end
+    assert with_registered([(0, page), (whole - page, whole)]) == [False] * 3        # both ends, a hole between them
+
+
 # More query tiles than SMs: those of a last round of at most half the SMs are shared by pairs of CTAs.  148 + 2, 148 + 74 (the most), 2 * 148 + 64
 # query tiles; the last of them beyond the sequence's end, a sequence without a key among them.
 @pytest.mark.parametrize("D", [64, 128])
