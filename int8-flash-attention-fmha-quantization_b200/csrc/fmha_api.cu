@@ -539,6 +539,10 @@ FetchPlan plan_fetch(const int desc[4], const void* host_q, const void* host_k, 
   FetchPlan plan;
   const int S = desc[1], H = desc[2], D = desc[3];
   if (S > kHostLongSeq) return plan;
+  // (the mask is read here by the host; one that lives on the device is left to the copies and what the runtime says to them)
+  cudaPointerAttributes of_mask{};
+  if (cudaPointerGetAttributes(&of_mask, host_mask) != cudaSuccess) { cudaGetLastError(); return plan; }
+  if (of_mask.type == cudaMemoryTypeDevice) return plan;
   // rows that come in: all of Q, the groups of keys with an unmasked one (of the batches that the slice touches)
   double rows = static_cast<double>(bh_count) * S;
   for (int b = bh_begin / H; b <= (bh_begin + bh_count - 1) / H; ++b) {

@@ -301,6 +301,16 @@ def test_only_wholly_pinned_buffers_are_read_by_a_kernel(pkg, torch_cuda):
     assert with_registered([(0, page), (whole - page, whole)]) == [False] * 3        # both ends, a hole between them
 
 
+def test_a_mask_on_the_device_is_not_read_by_the_host(pkg, torch_cuda):
+    """The choice between copies and the fetching kernel looks at the mask, unless the host cannot."""
+    torch = torch_cuda
+    desc, mask = pkg.AttnDataDescriptor(2, 256, 4, 64), torch.ones((2, 256), dtype=torch.int8)
+    mask[:, :32] = 0
+    q, k, v = (torch.zeros(2 * 4 * 256 * 64, dtype=torch.int8).pin_memory() for _ in range(3))
+    assert pkg.debug_host_fetch(desc, q, k, v, mask) and pkg.debug_host_fetch(desc, q, k, v, mask.pin_memory())
+    assert not pkg.debug_host_fetch(desc, q, k, v, mask.cuda())
+
+
 # More query tiles than SMs: those of a last round of at most half the SMs are shared by pairs of CTAs.  148 + 2, 148 + 74 (the most), 2 * 148 + 64
 # query tiles; the last of them beyond the sequence's end, a sequence without a key among them.
 @pytest.mark.parametrize("D", [64, 128])
