@@ -57,7 +57,7 @@ __device__ __forceinline__ int dot4(uint32_t p, uint32_t v, int acc) {
 // grid = (clusters of c CTAs) x (bh_count * row groups); R = query rows per group (rows past Sq are computed and dropped).
 template <int D, int R, bool kUnsigned>
 __global__ void __launch_bounds__(DecodeCfg<D>::kThreads, 3)
-fmha_decode_kernel(const int8_t* __restrict__ q, const int8_t* __restrict__ k, const int8_t* __restrict__ v, const FwdParams p) {
+fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdParams p) {
   using Cfg = DecodeCfg<D>;
   using Smem = DecodeSmem<D, R>;
   constexpr int W = Cfg::kWarps;
@@ -87,11 +87,11 @@ fmha_decode_kernel(const int8_t* __restrict__ q, const int8_t* __restrict__ k, c
   // ---- query rows; key tiles with at least one unmasked key (a word of the mask = four keys; S is a multiple of 64)
   for (int i = threadIdx.x; i < R * (D / 4); i += Cfg::kThreads) {
     const int r = i / (D / 4);
-    sm.q[r][i % (D / 4)] = (row0 + r < p.Sq) ? __ldg(reinterpret_cast<const uint32_t*>(q + (static_cast<int64_t>(bh) * p.Sq + row0) * D) + i) : 0u;
+    sm.q[r][i % (D / 4)] = (row0 + r < p.Sq) ? reinterpret_cast<const uint32_t*>(q + (static_cast<int64_t>(bh) * p.Sq + row0) * D)[i] : 0u;
   }
   auto has_key = [&](int t) -> bool {
     const int key = t * kTile + 4 * lane;
-    const uint32_t m4 = key < p.S ? __ldg(mask4 + (key >> 2)) : 0xFFFFFFFFu;
+    const uint32_t m4 = key < p.S ? mask4[key >> 2] : 0xFFFFFFFFu;
     return __any_sync(0xFFFFFFFFu, __vcmpeq4(m4, 0u) != 0u);                // a mask byte that is zero
   };
   if (n_tiles <= 2 * W) {
@@ -152,7 +152,7 @@ fmha_decode_kernel(const int8_t* __restrict__ q, const int8_t* __restrict__ k, c
   }
   for (int i = begin + warp; i < end; i += W, ++n) {
     const int key0 = sm.live[i] * kTile + 4 * lane;         // my four keys
-    const uint32_t masked = key0 < p.S ? ~__vcmpeq4(__ldg(mask4 + (key0 >> 2)), 0u) : 0xFFFFFFFFu;    // byte = 0xFF: masked
+    const uint32_t masked = key0 < p.S ? ~__vcmpeq4(mask4[key0 >> 2], 0u) : 0xFFFFFFFFu;    // byte = 0xFF: masked
 
     // ---- scores of my four keys (inc/fmha_i8.cuh:120-172)
     if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar_k, n & 1u, abort_flag)))) break;

@@ -121,7 +121,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       // Policy launch: the row's maximum over ALL keys and its exp-sum come from the statistics launch; one scale per
       // row for the whole unit (fmha_i8_quant_deviation.py:62-121).
       float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
-      if (out_row >= 0) st = __ldg(&p.row_stats_in[out_row]);
+      if (out_row >= 0) st = p.row_stats_in[out_row];
       l_run = st.y;
       const float l_row = st.y > 0.f ? st.y : 1.f;
       // dynamic: P8 = rn(levels * e); static: P8 = min(rn(levels * (e / l) / s_max), levels)
@@ -341,7 +341,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
       const int8_t* mask_row = p.mask + static_cast<int64_t>(cur.batch) * p.S;
       const int key0 = cur.tile * kTile + lane;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || __ldg(mask_row + key0 + 32 * i) != 0;
+      for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || mask_row[key0 + 32 * i] != 0;
     }
     if (cur.first && !wait(smem_u32(&ctl->q_full), units++ & 1u, FMHA_I8_DEV_WAIT_Q_LOAD)) break;
     if (!wait(smem_u32(&ctl->k_full), g & 1u, FMHA_I8_DEV_WAIT_K_LOAD)) break;

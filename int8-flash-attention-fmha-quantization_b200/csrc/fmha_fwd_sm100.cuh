@@ -292,7 +292,7 @@ __device__ __forceinline__ int scan_mask_groups(Info* info, const uint32_t* word
         masked[q] = 0u;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const uint32_t wv = __ldg(words + (key0 >> 2) + i);
+          const uint32_t wv = words[(key0 >> 2) + i];
           masked[q] |= wv;
           open[q] |= __vcmpeq4(wv, 0u);
         }
@@ -525,7 +525,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       const UnitGeom geo = unit_geom(p, u);
       const int q_row = geo.q_row0 + row;
       float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 1.f);
-      if (q_row < p.Sq) st = __ldg(&p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row]);
+      if (q_row < p.Sq) st = p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row];
       const float l_row = st.y > 0.f ? st.y : 1.f;
       // dynamic: P8 = rn(levels * e); static: P8 = min(rn(levels * (e / l) / s_max), levels)
       const float mul = (p.p_static_mul != 0.f) ? p.p_static_mul / l_row : p.p_row_mul;
@@ -728,7 +728,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
     if (kPolicy) {
       // the accumulated integer sum becomes the output through one factor per row: out_mul (/ l for the per-row policy)
       float l_row = 0.f;
-      if (q_row < p.Sq) l_row = __ldg(&p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row]).y;
+      if (q_row < p.Sq) l_row = p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row].y;
       l_run = (p.p_static_mul != 0.f) ? (l_row > 0.f ? 1.f : 0.f) : l_row;
     }
 
@@ -956,7 +956,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       if (mixed) {
         const int key0 = info->live[info->begin + j] * kTile + static_cast<int>(threadIdx.x & 31);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || __ldg(mask_row + key0 + 32 * i) != 0;
+        for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || mask_row[key0 + 32 * i] != 0;
       }
       // K first (it has normally been there for a while), then the accumulator: it still holds the partial output of
       // step g - n until the merge warps have drained it, and that hand-off is on the step-to-step critical path

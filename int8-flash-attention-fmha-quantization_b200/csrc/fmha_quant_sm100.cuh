@@ -61,7 +61,7 @@ inline int quant_cluster_size(long long n) {
 }
 
 __global__ void __launch_bounds__(kQuantClusterThreads, 1)
-quant_cluster_kernel(const float* __restrict__ x, int n, int8_t* __restrict__ out, float* __restrict__ amax_out) {
+quant_cluster_kernel(const float* x, int n, int8_t* out, float* amax_out) {
   __shared__ float warp_max[kQuantClusterThreads / 32];
   __shared__ float cta_max[kQuantClusterMax];
   grid_launch_dependents();
@@ -75,7 +75,7 @@ quant_cluster_kernel(const float* __restrict__ x, int n, int8_t* __restrict__ ou
 #pragma unroll
   for (int k = 0; k < kQuantClusterVec; ++k) {
     const int i = begin + k * kQuantClusterThreads + static_cast<int>(threadIdx.x);
-    v[k] = i < end ? __ldg(x4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[k] = i < end ? x4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   // up to three elements behind the last float4
   const int tail = n4 * 4 + static_cast<int>(threadIdx.x);

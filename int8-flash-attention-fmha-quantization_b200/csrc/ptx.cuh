@@ -131,6 +131,9 @@ __device__ __forceinline__ void st_global_v8(void* ptr, const uint32_t (&r)[8]) 
 // Blocks until every kernel before this one in the stream has finished and its writes are visible.  With the launch
 // attribute that allows it, a kernel starts before that: what precedes this instruction must not touch global memory
 // that an earlier kernel may write or still read.
+// What comes after it reads global memory with ordinary loads: __ldg and loads through const __restrict__ parameters are for memory
+// that nobody writes while the kernel runs, and the kernel before may still be writing when this one has begun.  (The compiler may
+// move such a load in front of the wait, and the L1 may answer it with what another kernel on that SM has left there.)
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the next kernel of the stream start (up to its own grid_dependency_wait) once all CTAs have executed this.
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -43,6 +43,36 @@ def test_back_to_back_calls_see_each_others_output(pkg, wl, torch_cuda, S, D):
     assert pkg.device_status()[0] == pkg.OK
 
 
+@pytest.mark.parametrize("what", ["few_rows", "policy", "policy_many"])
+def test_buffers_rewritten_between_overlapping_launches(pkg, wl, torch_cuda, what):
+    """One set of buffers, filled anew by every step's launches while the launches of the step before may still drain: the quantised
+    query of a decoding step, the row statistics of a policy.  The outputs are those of steps with a synchronisation between them."""
+    torch = torch_cuda
+    B, H, Sq, Sk, D = {"few_rows": (3, 5, 1, 704, 128), "policy": (1, 5, 100, 320, 64), "policy_many": (30, 13, 100, 192, 64)}[what]
+    _, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, D, seed=Sq, valid=np.random.default_rng(B).integers(1, Sk, B))
+    k, v, m = (torch.from_numpy(x).cuda() for x in (k8, v8, mask))
+    desc, param = pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), pkg.FMHAParamI8(*amax, 1.0)
+    xs = [torch.randn((B, H, Sq, D), device="cuda") for _ in range(40)]
+    q, scratch = torch.zeros((B, H, Sq, D), dtype=torch.int8, device="cuda"), torch.zeros(2 * B * H * Sq, device="cuda")
+    results = []
+    for wait in (True, False):
+        outs = [torch.zeros_like(q) for _ in xs]
+        torch.cuda.synchronize()
+        for x, o in zip(xs, outs):
+            pkg.quantize_f32(None, x, q)
+            if what == "few_rows":
+                pkg.FMHAInferI8Cross(None, param, desc, q, k, v, m, o)
+            else:
+                pkg.FMHAInferI8Policy(None, param, desc, q, k, v, m, o, pkg.POLICY_ROW, scratch)
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        results.append([o.cpu().numpy() for o in outs])
+    for i, (a, b) in enumerate(zip(*results)):
+        assert np.array_equal(a, b), f"step {i} read what another step had left"
+    assert pkg.device_status()[0] == pkg.OK
+
+
 @pytest.fixture(scope="module")
 def torch_cuda():
     import torch

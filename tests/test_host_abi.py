@@ -108,3 +108,20 @@ def test_workload_table_and_mask_polarity(wl):
     assert v.shape == (32,) and set(v.tolist()) <= {256, 320, 384, 448, 512}
     assert np.array_equal(v, wl.valid_lengths(c["C2"], 2023))
     assert wl.valid_lengths(c["C4"], 1).tolist() == [15360]
+
+
+def test_kernels_that_may_start_early_use_ordinary_loads():
+    """A kernel that waits for the one before it (grid_dependency_wait) has begun while that one may still be writing: no load of
+    such a kernel, or of the roles it is made of, may be declared read-only for the kernel's whole life."""
+    csrc = os.path.join(ROOT, "int8-flash-attention-fmha-quantization_b200", "csrc")
+    seen = 0
+    for name in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        if "grid_dependency_wait();" not in text:
+            continue
+        assert "__ldg" not in text, name
+        for kernel in re.split(r"__global__", text)[1:]:
+            if "grid_dependency_wait();" in kernel:
+                seen += 1
+                assert "__restrict__" not in kernel[:kernel.index("{")], (name, kernel[:120])
+    assert seen == 4                                    # the general, the head_dim-64 and the few-rows kernel, the quantiser's cluster
