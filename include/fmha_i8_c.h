@@ -59,7 +59,7 @@ enum {
   FMHA_I8_DEV_WAIT_O_FREE = 9,     /* MMA issuer waiting for the previous P.V to be drained */
   FMHA_I8_DEV_WAIT_DEBUG = 10,     /* a wait inside a debug kernel */
   FMHA_I8_DEV_WAIT_INFO = 11,      /* a role waiting for (or the scanner waiting to reuse) a unit's mask information */
-  FMHA_I8_DEV_WAIT_QUANT = 12      /* quantiser: a tile of the tensor, or the other CTAs' maxima */
+  FMHA_I8_DEV_WAIT_QUANT = 12      /* quantiser: a tile of the tensor */
 };
 
 #define FMHA_I8_FLAG_USE_TCU 1u    /* mirrors the reference's use_tcu argument; must be set */
@@ -185,7 +185,8 @@ int fmha_i8_sm100_debug_wait_probe(void* stream, long long limit_cycles);
  * (float_quant2_int8, inc/utils.hpp:23-29; the reference does both on the host, test_fmha_i8.cpp:95-110).
  * x: n floats (device, 16-byte aligned), out: n int8 (device, 16-byte aligned), amax_out: one float on
  * the device (may be NULL).  One kernel on `stream`, no synchronisation, nothing allocated.  Calls on different
- * streams may overlap (up to 64 in flight on one device). */
+ * streams may overlap, any number of them, and so may replays of captured ones: a call keeps all it needs in its own `out`,
+ * whose content is undefined until the kernel has finished. */
 int fmha_i8_sm100_quantize_f32(void* stream, const float* x, long long n, int8_t* out, float* amax_out);
 
 /* The same quantisation under a name that promises what some callers need: it never allocates device memory.  (No

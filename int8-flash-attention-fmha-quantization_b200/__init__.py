@@ -304,8 +304,8 @@ def debug_wait_probe(stream, limit_cycles):
 def quantize_f32(stream, x, out, amax_out=None, n=None, entry="fmha_i8_sm100_quantize_f32"):
     """Device-side abs_max + float_quant2_int8 (reference inc/utils.hpp:23-39): x float32 -> out int8,
     amax written to the one-element device tensor `amax_out`.  Enqueues on `stream`, no synchronisation.
-    entry="fmha_i8_sm100_quantize_f32_noalloc" selects the variant that never allocates device memory
-    (built-in scratch, at most 268,435,456 elements, calls on one device must not overlap)."""
+    Neither entry allocates device memory, and calls may overlap; entry="fmha_i8_sm100_quantize_f32_noalloc" selects the
+    one whose contract promises the former (at most 268,435,456 elements)."""
     if entry not in ("fmha_i8_sm100_quantize_f32", "fmha_i8_sm100_quantize_f32_noalloc"):
         raise AttributeError(entry)
     st = (_binding or _native()).quantize(stream, x, int(n if n is not None else x.numel()), out, amax_out,

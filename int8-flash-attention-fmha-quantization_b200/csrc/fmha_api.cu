@@ -592,7 +592,6 @@ int check_quant_args(const float* x, long long n, const int8_t* out) {
 
 // The largest tensor of fmha_i8_sm100_quantize_f32_noalloc (1 GiB of fp32), part of its contract.
 constexpr long long kNoAllocMaxElements = 268435456LL;
-std::atomic<unsigned> g_quant_calls{0};
 
 // Up to what the registers of one cluster hold: one cluster.  Beyond: the whole chip, every CTA with work for all its warps.
 int launch_quantize(cudaStream_t stream, DeviceInfo* dev, const float* x, long long n, int8_t* out, float* amax_out) {
@@ -604,10 +603,10 @@ int launch_quantize(cudaStream_t stream, DeviceInfo* dev, const float* x, long l
   }
   if (n / kQuantTile > 0x7FFFFFFFLL) return FMHA_I8_ERR_TOO_LARGE;
   how.cooperative = true;
-  const long long ctas = (n / kQuantTile + kQuantWarps - 1) / kQuantWarps;
-  const int slot = static_cast<int>(g_quant_calls.fetch_add(1, std::memory_order_relaxed) % kQuantSlots);
-  return launch_kernel(quant_grid_kernel, dim3(static_cast<unsigned>(ctas < dev->sm_count ? ctas : dev->sm_count)), dim3(kQuantThreads), kQuantGridSmem,
-                       stream, how, x, n, out, amax_out, slot, dev->status);
+  const long long wanted = (n / kQuantTile + kQuantWarps - 1) / kQuantWarps;
+  const int most = dev->sm_count < kQuantMaxCtas ? dev->sm_count : kQuantMaxCtas;
+  return launch_kernel(quant_grid_kernel, dim3(static_cast<unsigned>(wanted < most ? wanted : most)), dim3(kQuantThreads), kQuantGridSmem,
+                       stream, how, x, n, out, amax_out, dev->status);
 }
 
 int quantize_impl(void* stream, const float* x, long long n, int8_t* out, float* amax_out) {
@@ -912,10 +911,6 @@ int fmha_i8_sm100_device_status(unsigned words[8]) {
   if (cudaMemcpyFromSymbol(words, g_status_words, sizeof(unsigned) * 8) != cudaSuccess) return finish(FMHA_I8_ERR_LAUNCH);
   const unsigned zeros[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (cudaMemcpyToSymbol(g_status_words, zeros, sizeof zeros) != cudaSuccess) return finish(FMHA_I8_ERR_LAUNCH);
-  if (words[0] == FMHA_I8_DEV_WAIT_QUANT) {      // that call did not clear its slot; the device is idle here
-    static const QuantSlot clean[kQuantSlots] = {};
-    if (cudaMemcpyToSymbol(g_quant_slots, clean, sizeof clean) != cudaSuccess) return finish(FMHA_I8_ERR_LAUNCH);
-  }
   {
     int dev_id = 0;
     if (cudaGetDevice(&dev_id) == cudaSuccess && dev_id >= 0 && dev_id < kMaxDevices) {

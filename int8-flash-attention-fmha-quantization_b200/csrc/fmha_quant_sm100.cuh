@@ -12,6 +12,7 @@
 // for 67,108,864; these take 5.5 and 93.5 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
 // what neither the SMs (50 MB) nor the L2 kept.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "fmha_fwd_sm100.cuh"
@@ -112,25 +113,21 @@ constexpr int kQuantKeep = 4;                  // tiles a warp keeps in register
 constexpr long long kQuantHoldBytes = 40000000;
 constexpr size_t kQuantGridSmem = static_cast<size_t>(kQuantWarps) * kQuantStages * kQuantTile * sizeof(float);
 
-// What the CTAs of one call share.  All zero between calls: the last CTA to leave clears it.
-struct QuantSlot {
-  unsigned amax_bits, arrived, left, pad[29];  // one 128-byte line
-};
-constexpr int kQuantSlots = 64;                // calls take them in turn: that many may be in flight at once
-__device__ QuantSlot g_quant_slots[kQuantSlots];
+// What the CTAs of one call exchange, their maxima, lies in the call's own output until the result goes there: nothing is shared with
+// another call, however many are in flight and whether they are captured or not.  The first 4 bytes x CTAs of a CTA's first tile are its
+// copy of the list; every CTA writes its entry into all copies, and reads and later overwrites only its own.
+constexpr int kQuantMaxCtas = kQuantTile / 4;  // the list fits into a tile of output
+static_assert(kQuantMaxCtas <= kQuantThreads, "one thread per entry");
 
 __global__ void __launch_bounds__(kQuantThreads, 1)
-quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__ out, float* __restrict__ amax_out, int slot_index,
-                  unsigned* __restrict__ status) {
+quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__ out, float* __restrict__ amax_out, unsigned* __restrict__ status) {
   extern __shared__ __align__(128) uint8_t ring_raw[];
   __shared__ uint64_t bars[kQuantWarps][kQuantStages];
   __shared__ float warp_max[kQuantWarps];
-  __shared__ float s_amax;
   __shared__ int s_abort;
   const int lane = threadIdx.x & 31, warp = warp_index();
   float* ring = reinterpret_cast<float*>(ring_raw) + warp * (kQuantStages * kQuantTile);
   uint64_t* bar = bars[warp];
-  QuantSlot* slot = &g_quant_slots[slot_index];
 
   // warp w of CTA c takes tiles w * CTAs + c, then every (warps * CTAs)-th: the whole chip reads one stretch of memory
   // at a time, and the last stretch is the one that pass 2 begins with
@@ -198,28 +195,16 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
   if (has_rest)
     for (long long i = rest + threadIdx.x; i < n; i += kQuantThreads) m = fmaxf(m, fabsf(x[i]));
 
-  // ---- the largest of all CTAs (they are all resident: cooperative launch)
+  // ---- the largest of all CTAs.  The grid's barrier is the one of the cooperative launch, whose CTAs are all resident and all come
+  // here: no wait above is longer than its limit.
   m = block_max<kQuantThreads>(m, warp_max);
-  if (threadIdx.x == 0) {
-    atomicMax(&slot->amax_bits, __float_as_uint(m));
-    __threadfence();
-    atomicAdd(&slot->arrived, 1u);
-    const long long t0 = clock64();
-    uint32_t probes = 0;
-    while (ok && ld_acquire_gpu(&slot->arrived) < gridDim.x) {
-      if (++probes >= kMinProbes && clock64() - t0 > kWaitLimitCycles) ok = false;
-    }
-    s_amax = __uint_as_float(ld_acquire_gpu(&slot->amax_bits));
-    if (!ok) raise_status(abort_flag, status, FMHA_I8_DEV_WAIT_QUANT, blockIdx.x);
-    if (atomicAdd(&slot->left, 1u) == gridDim.x - 1) {
-      slot->amax_bits = 0u;
-      slot->arrived = 0u;
-      slot->left = 0u;
-    }
-    if (blockIdx.x == 0 && amax_out) *amax_out = s_amax;
-  }
-  __syncthreads();
-  const float scale = quant_scale(s_amax);
+  const int ctas = static_cast<int>(gridDim.x), t = static_cast<int>(threadIdx.x);
+  if (t < ctas) __stcg(reinterpret_cast<float*>(out + static_cast<long long>(t) * kQuantTile) + blockIdx.x, m);
+  cooperative_groups::this_grid().sync();
+  m = t < ctas ? __ldcg(reinterpret_cast<const float*>(out + static_cast<long long>(blockIdx.x) * kQuantTile) + t) : 0.f;
+  const float amax = block_max<kQuantThreads>(m, warp_max);      // (its barrier: the list has been read before the tile is written)
+  if (blockIdx.x == 0 && t == 0 && amax_out) *amax_out = amax;
+  const float scale = quant_scale(amax);
 
   // ---- pass 2: quantise, from the last tile to the first
   auto store = [&](int i, int k, const float4& v) { __stcs(reinterpret_cast<uint32_t*>(out + tile_at(i)) + lane + 32 * k, quant_four(v, scale)); };

@@ -176,12 +176,6 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
   return v;
 }
 
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 // ---------------------------------------------------------------- TMA
 // L2 replacement policies for such copies.
 __device__ __forceinline__ uint64_t l2_evict_first() {

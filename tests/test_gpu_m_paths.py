@@ -117,6 +117,43 @@ def test_quantize_calls_overlap_on_two_streams(pkg, oracle, torch_cuda):
     assert pkg.device_status()[0] == pkg.OK
 
 
+# Just beyond what one cluster holds: 65 and 74 CTAs, so that two calls fit on the chip side by side.
+@pytest.mark.parametrize("apart", [1, 63, 64, 128])
+def test_quantize_calls_in_flight_share_nothing(pkg, oracle, torch_cuda, apart):
+    """Two captured calls, `apart` calls after one another, replayed on two streams at once, and eager calls on a third: however their
+    kernels meet, each finds its own largest magnitude."""
+    torch = torch_cuda
+    sizes, scales = (524288 + 37, 74 * 8192 - 5, 600001), (1.0, 30.0, 0.05)
+    xs = [torch.randn(n, device="cuda") * s for n, s in zip(sizes, scales)]
+    outs = [torch.zeros(n, dtype=torch.int8, device="cuda") for n in sizes]
+    amaxs = [torch.zeros(1, device="cuda") for _ in sizes]
+    want = [torch.from_numpy(oracle.quantize(x.cpu().numpy(), float(x.abs().max()))).cuda() for x in xs]
+    pkg.quantize_f32(None, xs[2], outs[2], amaxs[2])
+    graphs = []
+    for i in range(2):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[i]):
+            pkg.quantize_f32(None, xs[i], outs[i], amaxs[i])
+        for _ in range(apart - 1):
+            pkg.quantize_f32(None, xs[2], outs[2], amaxs[2])
+    streams = [torch.cuda.Stream() for _ in sizes]
+    torch.cuda.synchronize()
+    for _ in range(8):
+        for o, a in zip(outs, amaxs):
+            o.zero_()
+            a.zero_()
+        torch.cuda.synchronize()
+        for _ in range(10):
+            for i in range(2):
+                with torch.cuda.stream(streams[i]):
+                    graphs[i].replay()
+            pkg.quantize_f32(streams[2], xs[2], outs[2], amaxs[2])
+        torch.cuda.synchronize()
+        for i in range(3):
+            assert float(amaxs[i]) == float(xs[i].abs().max()) and torch.equal(outs[i], want[i]), i
+    assert pkg.device_status()[0] == pkg.OK
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("Sq,B,H,Sk,valid", [
     (1, 1, 1, 64, None),                     # half a key tile, most warps and CTAs idle
