@@ -198,6 +198,10 @@ int fmha_i8_sm100_quantize_f32(void* stream, const float* x, long long n, int8_t
  * Arguments and results are those of fmha_i8_sm100_quantize_f32. */
 int fmha_i8_sm100_quantize_f32_noalloc(void* stream, const float* x, long long n, int8_t* out, float* amax_out);
 
+/* Debug: the quantiser's whole-chip kernel for a size (n > 262,144) that one cluster of 16 CTAs would hold: what a device runs that
+ * has no room for such a cluster.  Arguments and results are those of fmha_i8_sm100_quantize_f32. */
+int fmha_i8_sm100_debug_quantize_whole_chip(void* stream, const float* x, long long n, int8_t* out, float* amax_out);
+
 /* Synchronises the current device, copies out and clears the eight device status words.
  * words[0] == 0 means no kernel of this library gave up on a bounded wait since the last call.
  * Otherwise words[0] = which wait gave up (FMHA_I8_DEV_*), words[1] = block index, words[2] = warp,

@@ -38,7 +38,7 @@ EXPORTS = (
     "fmha_i8_sm100_infer", "fmha_i8_sm100_infer_slice", "fmha_i8_sm100_infer_cross", "fmha_i8_sm100_calibrate_o_amax", "fmha_i8_sm100_infer_host",
     "fmha_i8_sm100_infer_host_slice", "fmha_i8_sm100_infer_policy",
     "fmha_i8_sm100_debug_host_fetch", "fmha_i8_sm100_debug_qk", "fmha_i8_sm100_debug_pv", "fmha_i8_sm100_debug_simt", "fmha_i8_sm100_debug_simt_x", "fmha_i8_sm100_debug_wait_probe",
-    "fmha_i8_sm100_quantize_f32", "fmha_i8_sm100_quantize_f32_noalloc", "fmha_i8_sm100_device_status", "fmha_i8_sm100_last_status", "fmha_i8_sm100_status_string",
+    "fmha_i8_sm100_quantize_f32", "fmha_i8_sm100_quantize_f32_noalloc", "fmha_i8_sm100_debug_quantize_whole_chip", "fmha_i8_sm100_device_status", "fmha_i8_sm100_last_status", "fmha_i8_sm100_status_string",
     "fmha_i8_sm100_launch_count", "fmha_i8_sm100_version",
 )
 
@@ -114,6 +114,7 @@ def lib():
         L.fmha_i8_sm100_debug_wait_probe.argtypes = [vp, ctypes.c_longlong]
         L.fmha_i8_sm100_quantize_f32.argtypes = [vp, vp, ctypes.c_longlong, vp, vp]
         L.fmha_i8_sm100_quantize_f32_noalloc.argtypes = [vp, vp, ctypes.c_longlong, vp, vp]
+        L.fmha_i8_sm100_debug_quantize_whole_chip.argtypes = [vp, vp, ctypes.c_longlong, vp, vp]
         L.fmha_i8_sm100_device_status.argtypes = [ctypes.POINTER(ctypes.c_uint)]
         L.fmha_i8_sm100_status_string.restype = ctypes.c_char_p
         L.fmha_i8_sm100_status_string.argtypes = [ctypes.c_int]
@@ -312,6 +313,13 @@ def quantize_f32(stream, x, out, amax_out=None, n=None, entry="fmha_i8_sm100_qua
                                           entry == "fmha_i8_sm100_quantize_f32_noalloc")
     if st != OK:
         raise FmhaError(st, entry)
+
+
+def debug_quantize_whole_chip(stream, x, out, amax_out=None, n=None):
+    """quantize_f32 with the kernel for large tensors, also where one cluster would hold the tensor (n > 262,144)."""
+    st = lib().fmha_i8_sm100_debug_quantize_whole_chip(_stream_handle(stream), _ptr(x), int(n if n is not None else x.numel()), _ptr(out), _ptr(amax_out))
+    if st != OK:
+        raise FmhaError(st, "debug_quantize_whole_chip")
 
 
 def device_status():

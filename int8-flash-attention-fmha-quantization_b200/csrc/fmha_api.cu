@@ -44,6 +44,7 @@ struct DeviceInfo {
   volatile unsigned* host_flag = nullptr;
   int sm_count = 0;
   int max_clusters[kClusterSizes] = {};      // clusters of 2, 4, 8 CTAs of the forward kernel that are resident at once
+  bool quant_clusters_of_16 = false;         // one cluster of 16 CTAs of the quantiser can be resident
   bool attr_set = false;
 };
 DeviceInfo g_dev[kMaxDevices];
@@ -168,6 +169,20 @@ int set_kernel_attributes(DeviceInfo* d) {
     if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128, false>, &cfg) != cudaSuccess) n128 = 0;
     cudaGetLastError();
     d->max_clusters[i] = n64 < n128 ? n64 : n128;
+  }
+  {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kQuantClusterMax;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(kQuantClusterMax);
+    cfg.blockDim = dim3(kQuantClusterThreads);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    d->quant_clusters_of_16 = cudaOccupancyMaxActiveClusters(&n, quant_cluster_kernel, &cfg) == cudaSuccess && n >= 1;
+    cudaGetLastError();
   }
   d->attr_set = true;
   return FMHA_I8_OK;
@@ -593,10 +608,11 @@ int check_quant_args(const float* x, long long n, const int8_t* out) {
 // The largest tensor of fmha_i8_sm100_quantize_f32_noalloc (1 GiB of fp32), part of its contract.
 constexpr long long kNoAllocMaxElements = 268435456LL;
 
-// Up to what the registers of one cluster hold: one cluster.  Beyond: the whole chip, every CTA with work for all its warps.
-int launch_quantize(cudaStream_t stream, DeviceInfo* dev, const float* x, long long n, int8_t* out, float* amax_out) {
+// Up to what the registers of one cluster hold: one cluster -- of 16 CTAs where the device has room for one together (more than 8 is
+// not a size that every device or partition of one offers), of 8 otherwise.  Beyond: the whole chip, every CTA with work for all its warps.
+int launch_quantize(cudaStream_t stream, DeviceInfo* dev, const float* x, long long n, int8_t* out, float* amax_out, bool whole_chip) {
   LaunchHow how;
-  if (n <= kQuantClusterMax * kQuantPerCta) {
+  if (!whole_chip && n <= (dev->quant_clusters_of_16 ? kQuantClusterMax : kQuantClusterPortable) * kQuantPerCta) {
     how.cluster = static_cast<unsigned>(quant_cluster_size(n));
     how.overlap = true;
     return launch_kernel(quant_cluster_kernel, dim3(how.cluster), dim3(kQuantClusterThreads), 0, stream, how, x, static_cast<int>(n), out, amax_out);
@@ -609,12 +625,12 @@ int launch_quantize(cudaStream_t stream, DeviceInfo* dev, const float* x, long l
                        stream, how, x, n, out, amax_out, dev->status);
 }
 
-int quantize_impl(void* stream, const float* x, long long n, int8_t* out, float* amax_out) {
+int quantize_impl(void* stream, const float* x, long long n, int8_t* out, float* amax_out, bool whole_chip = false) {
   int err = FMHA_I8_OK;
   DeviceInfo* dev = current_device(&err);
   if (!dev) return err;
   const int st = set_kernel_attributes(dev);
-  return st != FMHA_I8_OK ? st : launch_quantize(static_cast<cudaStream_t>(stream), dev, x, n, out, amax_out);
+  return st != FMHA_I8_OK ? st : launch_quantize(static_cast<cudaStream_t>(stream), dev, x, n, out, amax_out, whole_chip);
 }
 
 }  // namespace
@@ -903,6 +919,13 @@ int fmha_i8_sm100_quantize_f32_noalloc(void* stream, const float* x, long long n
     return finish(FMHA_I8_ERR_TOO_LARGE);
   }
   return finish(quantize_impl(stream, x, n, out, amax_out));
+}
+
+int fmha_i8_sm100_debug_quantize_whole_chip(void* stream, const float* x, long long n, int8_t* out, float* amax_out) {
+  const int st = check_quant_args(x, n, out);
+  if (st != FMHA_I8_OK) return finish(st);
+  if (n <= kQuantClusterPortable * kQuantPerCta) return finish(FMHA_I8_ERR_BAD_SHAPE);
+  return finish(quantize_impl(stream, x, n, out, amax_out, true));
 }
 
 int fmha_i8_sm100_device_status(unsigned words[8]) {

@@ -50,15 +50,15 @@ __device__ __forceinline__ float block_max(float m, float* scratch) {
 // ------------------------------------------------------------------------------------------ up to 524,288 elements
 constexpr int kQuantClusterThreads = 1024;
 constexpr int kQuantClusterVec = 8;            // float4 per thread, all loads in flight at once
-constexpr int kQuantClusterMax = 16;
+constexpr int kQuantClusterMax = 16, kQuantClusterPortable = 8;
 constexpr long long kQuantPerCta = 4LL * kQuantClusterThreads * kQuantClusterVec;    // 32,768 elements
 
 // CTAs for n elements: two float4 per thread are enough to cover the latency of memory, more CTAs than that only make
 // the exchange longer; beyond 8 CTAs (the portable cluster size) only what the registers of 8 cannot hold.
 inline int quant_cluster_size(long long n) {
   int c = 1;
-  while (c < 8 && n > c * (kQuantPerCta / 4)) c *= 2;
-  return n > 8 * kQuantPerCta ? 16 : c;
+  while (c < kQuantClusterPortable && n > c * (kQuantPerCta / 4)) c *= 2;
+  return n > kQuantClusterPortable * kQuantPerCta ? kQuantClusterMax : c;
 }
 
 __global__ void __launch_bounds__(kQuantClusterThreads, 1)

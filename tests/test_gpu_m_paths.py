@@ -101,6 +101,23 @@ def test_quantize_sizes(pkg, oracle, torch_cuda, n):
     assert pkg.device_status()[0] == pkg.OK
 
 
+# The sizes that one cluster of 16 CTAs holds, on a device that has no room for one: from 256 tiles for 32 CTAs to 512 for 64.
+@pytest.mark.parametrize("n", [262145, 262144 + 1023, 300007, 524288])
+def test_quantize_without_clusters_of_16(pkg, oracle, torch_cuda, n):
+    torch = torch_cuda
+    x = np.random.default_rng(n).standard_normal(n, dtype=np.float32)
+    x[n - 1] = 9.25
+    out, amax = torch.full((n + 64,), 0x5A, dtype=torch.int8, device="cuda"), torch.zeros(1, device="cuda")
+    on_gpu = torch.from_numpy(x).cuda()
+    pkg.debug_quantize_whole_chip(None, on_gpu, out, amax, n=n)
+    host = out.cpu().numpy()
+    assert np.float32(amax.item()) == np.abs(x).max()
+    assert np.array_equal(host[:n], oracle.quantize(x, np.abs(x).max())) and np.all(host[n:] == 0x5A)
+    with pytest.raises(pkg.FmhaError):
+        pkg.debug_quantize_whole_chip(None, on_gpu, out, amax, n=262144)
+    assert pkg.device_status()[0] == pkg.OK
+
+
 def test_quantize_calls_overlap_on_two_streams(pkg, oracle, torch_cuda):
     torch = torch_cuda
     n = 3 * SWEEP + 5
