@@ -94,6 +94,23 @@ def test_python_mirror_raises(pkg):
     assert st == pkg.ERR_NO_CUDA_CORE_PATH
 
 
+def test_python_mirror_takes_whatever_int_takes_for_heads_and_policy(pkg):
+    """Slice bounds and policies computed with floats or numpy: they get as far as the library's own checks (here: its answer to a
+    sequence length that is no multiple of 64)."""
+    param, desc, desc_x = pkg.FMHAParamI8(1, 1, 1, 1, 1), pkg.AttnDataDescriptor(1, 100, 2, 64), pkg.AttnDataDescriptorX(1, 7, 100, 2, 64)
+    p = (256, 512, 768, 1024, 1280)
+    for begin, count in ((0.0, 2.0), (np.float64(1), np.float32(1)), (np.int64(0), np.int32(2)), ("0", "1")):
+        assert pkg.FMHAInferI8Slice(0, param, desc, *p, begin, count, check=False) == pkg.ERR_BAD_SHAPE
+        assert pkg.FMHAInferI8Cross(0, param, desc_x, *p, bh_begin=begin, bh_count=count, check=False) == pkg.ERR_BAD_SHAPE
+        assert pkg.FMHAInferI8Cross(0, param, desc_x, *p, bh_begin=begin, check=False) == pkg.ERR_BAD_SHAPE
+        assert pkg.FMHAInferI8Policy(0, param, desc_x, *p, float(pkg.POLICY_ROW), 2048, begin, count, check=False) == pkg.ERR_BAD_SHAPE
+        assert pkg.FMHAInferI8HostSlice(param, desc, *p, begin, count, check=False) == pkg.ERR_BAD_SHAPE
+    with pytest.raises((TypeError, ValueError)):
+        pkg.FMHAInferI8Slice(0, param, desc, *p, None, 1, check=False)
+    with pytest.raises((TypeError, ValueError)):
+        pkg.FMHAInferI8HostSlice(param, desc, *p, None, None, check=False)
+
+
 def test_workload_table_and_mask_polarity(wl):
     c = wl.CONFIGS
     assert (c["C2"].B, c["C2"].H, c["C2"].S, c["C2"].D) == (32, 12, 512, 64)
