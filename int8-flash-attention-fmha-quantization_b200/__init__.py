@@ -37,7 +37,7 @@ FLAG_UINT8_P = 2     # P quantised as unsigned 8 bit, 255 levels (the reference 
 EXPORTS = (
     "fmha_i8_sm100_infer", "fmha_i8_sm100_infer_slice", "fmha_i8_sm100_infer_cross", "fmha_i8_sm100_calibrate_o_amax", "fmha_i8_sm100_infer_host",
     "fmha_i8_sm100_infer_host_slice", "fmha_i8_sm100_infer_policy",
-    "fmha_i8_sm100_debug_host_fetch", "fmha_i8_sm100_debug_qk", "fmha_i8_sm100_debug_pv", "fmha_i8_sm100_debug_simt", "fmha_i8_sm100_debug_simt_x", "fmha_i8_sm100_debug_wait_probe",
+    "fmha_i8_sm100_debug_plan", "fmha_i8_sm100_debug_host_fetch", "fmha_i8_sm100_debug_qk", "fmha_i8_sm100_debug_pv", "fmha_i8_sm100_debug_simt", "fmha_i8_sm100_debug_simt_x", "fmha_i8_sm100_debug_wait_probe",
     "fmha_i8_sm100_quantize_f32", "fmha_i8_sm100_quantize_f32_noalloc", "fmha_i8_sm100_debug_quantize_whole_chip", "fmha_i8_sm100_device_status", "fmha_i8_sm100_last_status", "fmha_i8_sm100_status_string",
     "fmha_i8_sm100_launch_count", "fmha_i8_sm100_version",
 )
@@ -106,6 +106,7 @@ def lib():
         L.fmha_i8_sm100_infer_policy.argtypes = [vp, fp, ip, vp, vp, vp, vp, vp, ctypes.c_int, ctypes.c_int, u, ctypes.c_int, vp]
         L.fmha_i8_sm100_infer_host.argtypes = [fp, ip, vp, vp, vp, vp, vp, u]
         L.fmha_i8_sm100_infer_host_slice.argtypes = [fp, ip, vp, vp, vp, vp, vp, ctypes.c_int, ctypes.c_int, u]
+        L.fmha_i8_sm100_debug_plan.argtypes = [ip, ctypes.c_int, ip]
         L.fmha_i8_sm100_debug_host_fetch.argtypes = [ip, vp, vp, vp, vp]
         L.fmha_i8_sm100_debug_qk.argtypes = [vp, ip, vp, vp, vp]
         L.fmha_i8_sm100_debug_pv.argtypes = [vp, ip, vp, vp, vp, u]
@@ -259,6 +260,18 @@ def FMHAInferI8HostSlice(fmha_param, attn_desc, host_q, host_k, host_v, host_mas
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8HostSlice")
     return st
+
+
+KERNEL_FEW_ROWS, KERNEL_GENERAL, KERNEL_WORKERS = 0, 1, 2
+
+
+def debug_plan(attn_desc_x, policy=POLICY_TILE):
+    """(kernel, CTAs that share a query tile, rounds before those) of a call of that shape on the current device.  Launches nothing."""
+    plan = (ctypes.c_int * 3)()
+    st = lib().fmha_i8_sm100_debug_plan(attn_desc_x.as_c(), int(policy), plan)
+    if st != OK:
+        raise FmhaError(st, "debug_plan")
+    return tuple(plan)
 
 
 def debug_host_fetch(attn_desc, host_q, host_k, host_v, host_mask):

@@ -108,10 +108,10 @@ template <typename Set> void set_decode_attributes(Set set) {
     both(d, std::integral_constant<int, 1>());
     both(d, std::integral_constant<int, 2>());
     both(d, std::integral_constant<int, 4>());
-    both(d, std::integral_constant<int, 8>());
   };
   rows(std::integral_constant<int, 64>());
   rows(std::integral_constant<int, 128>());
+  both(std::integral_constant<int, 64>(), std::integral_constant<int, 8>());
 }
 
 int set_kernel_attributes(DeviceInfo* d) {
@@ -361,8 +361,28 @@ bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
   return workers * tiles < own * unit + more * (pairs_share_last_round(p, dev) ? unit / 2 + 4500 : unit);
 }
 
+// Few query rows run the few-rows kernel.  Up to four rows it is bound by reading K and V; from five on (computed as eight) its integer dot
+// products take as long or longer.  us, few-rows / general kernel:
+//   D128, 1 row   B16 H32 S4096 (1025..4096 keys) 55 / 104
+//   D128, 8 rows  B128 H32 S64 90.9 / 62.0, B64 H32 S256 50.1 / 40.2, B32 H32 S1024 71.8 / 61.5, B8 H32 S4096 83.3 / 63.2, B1 H8 S16384
+//                 77.3 / 25.3, and so on: the general one at every length and number of heads measured
+//   D64, 8 rows   B128 H32 S128 61.0 / 32.9, B1 H4 S128 5.9 / 4.7: the general one for a single key tile; beyond, with many heads, the
+//                 few-rows one (B32 H32 S512 23.9 / 29.9, B8 H32 S4096 47.5 / 60.2), with few heads either (B1 H32 S2048 13.3 / 9.9)
+//   D64, 4 rows   B128 H32 S128 42.6 / 32.9, S256 and beyond the few-rows one or within a few per cent
+bool few_rows(int Sq, int S, int D) { return Sq <= 4 || (D == 64 && Sq <= kDecodeMaxRows && S > kTile); }
+
+// Chooses the kernel of a call and how its units are divided: fills p->parts and p->own_rounds.  `plain`: neither calibration nor a
+// launch of a whole-row policy; `busy_sms`: SMs that something else is using.
+int plan_call(FwdParams* p, int D, bool plain, int busy_sms, const DeviceInfo* dev) {
+  p->parts = 1;
+  if (plain && few_rows(p->Sq, p->S, D)) return FMHA_I8_KERNEL_FEW_ROWS;
+  if (D == 64 && use_workers(*p, dev)) return FMHA_I8_KERNEL_WORKERS;
+  if (plain && busy_sms == 0) plan_parts(p, dev);
+  return FMHA_I8_KERNEL_GENERAL;
+}
+
 template <int D, bool kPolicy = false>
-int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v, int busy_sms) {
+int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v, int kernel, int busy_sms) {
   CUtensorMap mq, mk, mv;
   int st;
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
@@ -376,18 +396,15 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q,
   how.overlap = p.n_units <= 4 * dev->sm_count;
   // persistent CTAs: one per SM (tensor memory is allocated whole), each walking its share of the units
   const int sms = dev->sm_count - busy_sms;
-  const unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
+  unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
   if constexpr (D == 64) {
-    if (use_workers(p, dev))
+    if (kernel == FMHA_I8_KERNEL_WORKERS)
       return launch_kernel(w64::fwd_kernel<kPolicy>, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
   }
-  p.parts = 1;
-  if (!kPolicy && !p.row_stats_out && !p.amax_out && busy_sms == 0) plan_parts(&p, dev);
   if (p.parts > 1) {
     how.cluster = static_cast<unsigned>(p.parts);
     how.overlap = true;
-    const int ctas = p.own_rounds > 0 ? dev->sm_count : p.n_units * p.parts;
-    return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(static_cast<unsigned>(ctas)), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
+    grid = static_cast<unsigned>(p.own_rounds > 0 ? dev->sm_count : p.n_units * p.parts);
   }
   return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
@@ -419,11 +436,12 @@ template <int D>
 int launch_decode(cudaStream_t s, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v) {
   if (p.Sq == 1) return p.p_unsigned ? launch_decode_rows<D, 1, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 1, false>(s, dev, p, q, k, v);
   if (p.Sq == 2) return p.p_unsigned ? launch_decode_rows<D, 2, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 2, false>(s, dev, p, q, k, v);
-  if (p.Sq <= 4) return p.p_unsigned ? launch_decode_rows<D, 4, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 4, false>(s, dev, p, q, k, v);
-  return p.p_unsigned ? launch_decode_rows<D, 8, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 8, false>(s, dev, p, q, k, v);
+  if constexpr (D == 64) {
+    if (p.Sq > 4) return p.p_unsigned ? launch_decode_rows<D, 8, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 8, false>(s, dev, p, q, k, v);
+  }
+  return p.p_unsigned ? launch_decode_rows<D, 4, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 4, false>(s, dev, p, q, k, v);
 }
-// calib == nullptr: the forward pass into o.  calib != nullptr: calibration, o is not touched (may be null).
-// Which of the three uses of the forward kernel a launch is.
+// Which of the uses of the forward kernel a launch is.
 struct LaunchMode {
   float* calib = nullptr;          // calibration: largest |output| to this device float, o untouched
   float2* stats_out = nullptr;     // statistics launch of a whole-row policy: {row max bits, exp-sum} per query row, o untouched
@@ -431,6 +449,20 @@ struct LaunchMode {
   int policy = 0;                  // FMHA_I8_POLICY_* of a policy launch
   int busy_sms = 0;                // SMs that something else is using for longer than this launch
 };
+
+int fill_units(FwdParams* p, const Shape& sh, int bh_count) {
+  p->S = sh.Sk;
+  p->Sq = sh.Sq;
+  p->H = sh.H;
+  p->bh_count = bh_count;
+  p->q_tiles = (p->Sq + kTile - 1) / kTile;
+  p->by_q_tiles = fast_div_by(p->q_tiles);
+  p->by_heads = fast_div_by(p->H);
+  const long long units = static_cast<long long>(bh_count) * p->q_tiles;
+  if (units > 0x7FFFFFFFLL) return FMHA_I8_ERR_BAD_SHAPE;
+  p->n_units = static_cast<int>(units);
+  return FMHA_I8_OK;
+}
 
 int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void* q, const void* k,
                  const void* v, const void* mask, void* o, int bh_begin, int bh_count, unsigned flags,
@@ -481,28 +513,17 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   p.mask = static_cast<const int8_t*>(mask);
   p.o = static_cast<int8_t*>(o);
   p.o_wide = aligned(o, 32) ? 1 : 0;
-  p.S = sh.Sk;
-  p.Sq = sh.Sq;
-  p.H = sh.H;
   p.bh_begin = bh_begin;
-  p.bh_count = bh_count;
-  p.q_tiles = (p.Sq + kTile - 1) / kTile;
-  p.by_q_tiles = fast_div_by(p.q_tiles);
-  p.by_heads = fast_div_by(p.H);
-  {
-    const long long units = static_cast<long long>(bh_count) * p.q_tiles;
-    if (units > 0x7FFFFFFFLL) return FMHA_I8_ERR_BAD_SHAPE;
-    p.n_units = static_cast<int>(units);
-  }
+  if ((st = fill_units(&p, sh, bh_count)) != FMHA_I8_OK) return st;
   p.status = dev->status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Few query rows: up to eight the dp4a kernel is faster or as fast at every length and number of heads measured (B16 H32
-  // D128, 1025..4096 keys: 1 row 104 -> 59 us, 2 rows 61, 4 rows 68, 8 rows 100; B128 H32 D64, 256 keys, 8 rows 72 -> 71).
-  if (!mode && !calib && sh.Sq <= kDecodeMaxRows)
-    return sh.D == 128 ? launch_decode<128>(s, dev, p, q, k, v) : launch_decode<64>(s, dev, p, q, k, v);
   const int busy = mode ? mode->busy_sms : 0;
-  if (policy_launch) return sh.D == 128 ? launch_fwd<128, true>(s, dev, p, q, k, v, busy) : launch_fwd<64, true>(s, dev, p, q, k, v, busy);
-  return sh.D == 128 ? launch_fwd<128>(s, dev, p, q, k, v, busy) : launch_fwd<64>(s, dev, p, q, k, v, busy);
+  const bool plain = !calib && !(mode && (mode->stats_out || mode->stats_in));
+  const int kernel = plan_call(&p, sh.D, plain, busy, dev);
+  if (kernel == FMHA_I8_KERNEL_FEW_ROWS) return sh.D == 128 ? launch_decode<128>(s, dev, p, q, k, v) : launch_decode<64>(s, dev, p, q, k, v);
+  if (policy_launch)
+    return sh.D == 128 ? launch_fwd<128, true>(s, dev, p, q, k, v, kernel, busy) : launch_fwd<64, true>(s, dev, p, q, k, v, kernel, busy);
+  return sh.D == 128 ? launch_fwd<128>(s, dev, p, q, k, v, kernel, busy) : launch_fwd<64>(s, dev, p, q, k, v, kernel, busy);
 }
 
 int infer_slice_impl(void* stream, const float amax[5], const int desc[4], const void* q, const void* k,
@@ -794,6 +815,24 @@ int fmha_i8_sm100_infer_host_slice(const float amax[5], const int desc[4], const
                                    const void* host_v, const void* host_mask, void* host_o, int bh_begin, int bh_count,
                                    unsigned flags) {
   return finish(infer_host_slice_impl(amax, desc, host_q, host_k, host_v, host_mask, host_o, bh_begin, bh_count, flags));
+}
+
+int fmha_i8_sm100_debug_plan(const int desc5[5], int policy, int plan[3]) {
+  if (!desc5 || !plan) return finish(FMHA_I8_ERR_NULL_POINTER);
+  const Shape sh{desc5[0], desc5[1], desc5[2], desc5[3], desc5[4]};
+  int st = check_shape_x(sh);
+  if (st != FMHA_I8_OK) return finish(st);
+  if (policy < FMHA_I8_POLICY_TILE || policy > FMHA_I8_POLICY_STATIC) return finish(FMHA_I8_ERR_BAD_FLAGS);
+  int err = FMHA_I8_OK;
+  DeviceInfo* dev = current_device(&err);
+  if (!dev) return finish(err);
+  if ((st = set_kernel_attributes(dev)) != FMHA_I8_OK) return finish(st);
+  FwdParams p{};
+  if ((st = fill_units(&p, sh, sh.B * sh.H)) != FMHA_I8_OK) return finish(st);
+  plan[0] = plan_call(&p, sh.D, policy == FMHA_I8_POLICY_TILE, 0, dev);
+  plan[1] = p.parts;
+  plan[2] = p.parts > 1 ? p.own_rounds : 0;
+  return finish(FMHA_I8_OK);
 }
 
 int fmha_i8_sm100_debug_host_fetch(const int desc[4], const void* host_q, const void* host_k, const void* host_v, const void* host_mask) {

@@ -1,5 +1,5 @@
-// Attention of a few query rows per head (decoding against a cache): fmha_i8_sm100_infer_cross with at most
-// kDecodeMaxRows rows.  Same arithmetic as the forward kernel (fmha_fwd_sm100.cuh): key tiles of 128 starting at key 0, P
+// Attention of a few query rows per head (decoding against a cache): fmha_i8_sm100_infer_cross with up to four rows, at head_dim 64
+// up to kDecodeMaxRows (few_rows() in fmha_api.cu draws the line).  Same arithmetic as the forward kernel (fmha_fwd_sm100.cuh): key tiles of 128 starting at key 0, P
 // quantised to 8 bits against each tile's own row maximum, tiles merged in fp32; key tiles without an unmasked key are
 // skipped.
 //
