@@ -45,7 +45,7 @@ struct DeviceInfo {
   int sm_count = 0;
   int max_clusters[kClusterSizes] = {};      // clusters of 2, 4, 8 CTAs of the forward kernel that are resident at once
   bool quant_clusters_of_16 = false;         // one cluster of 16 CTAs of the quantiser can be resident
-  bool attr_set = false;
+  std::atomic<bool> attr_set{false};         // the kernel attributes are set and what the device was asked about them is filled in
 };
 DeviceInfo g_dev[kMaxDevices];
 std::mutex g_dev_mutex;
@@ -115,7 +115,9 @@ template <typename Set> void set_decode_attributes(Set set) {
 }
 
 int set_kernel_attributes(DeviceInfo* d) {
-  if (d->attr_set) return FMHA_I8_OK;
+  if (d->attr_set.load(std::memory_order_acquire)) return FMHA_I8_OK;
+  std::lock_guard<std::mutex> lock(g_dev_mutex);
+  if (d->attr_set.load(std::memory_order_relaxed)) return FMHA_I8_OK;
   cudaError_t e = cudaSuccess;
   auto set = [&](const void* fn, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
@@ -184,7 +186,7 @@ int set_kernel_attributes(DeviceInfo* d) {
     d->quant_clusters_of_16 = cudaOccupancyMaxActiveClusters(&n, quant_cluster_kernel, &cfg) == cudaSuccess && n >= 1;
     cudaGetLastError();
   }
-  d->attr_set = true;
+  d->attr_set.store(true, std::memory_order_release);
   return FMHA_I8_OK;
 }
 
