@@ -443,9 +443,10 @@ int launch_decode(cudaStream_t s, DeviceInfo* dev, const FwdParams& p, const voi
   }
   return p.p_unsigned ? launch_decode_rows<D, 4, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 4, false>(s, dev, p, q, k, v);
 }
-// Which of the uses of the forward kernel a launch is.
+
+// What a launch of the forward kernels is beside the plain forward pass into o.  (Calibration comes as infer_x_impl's `calib`: the
+// largest |output| goes to that device float and o, which may be null, is not touched.)
 struct LaunchMode {
-  float* calib = nullptr;          // calibration: largest |output| to this device float, o untouched
   float2* stats_out = nullptr;     // statistics launch of a whole-row policy: {row max bits, exp-sum} per query row, o untouched
   const float2* stats_in = nullptr;  // policy launch: those statistics
   int policy = 0;                  // FMHA_I8_POLICY_* of a policy launch

@@ -95,7 +95,7 @@ debug_pv_kernel(const __grid_constant__ CUtensorMap map_v, const int8_t* p8, int
   uint8_t* p_tile = tiles + kTileBytes;                       // 128 x 128 bytes
   DebugCtl* ctl = reinterpret_cast<DebugCtl*>(tiles + kTileBytes + kTile * kTile);
   const uint32_t v_smem = smem_u32(tiles), p_smem = smem_u32(p_tile);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
   const int qt = blockIdx.x, bh = blockIdx.y;
   const int row = qt * kTile + threadIdx.x;
   const int n_tiles = (S + kTile - 1) / kTile;

@@ -76,20 +76,6 @@
 #include "ptx.cuh"
 #include "../../include/fmha_i8_c.h"
 
-// Ring depths can be overridden at compile time for tuning runs.
-#ifndef FMHA_STAGES_K128
-#define FMHA_STAGES_K128 3
-#endif
-#ifndef FMHA_STAGES_V128
-#define FMHA_STAGES_V128 6
-#endif
-#ifndef FMHA_STAGES_K64
-#define FMHA_STAGES_K64 4
-#endif
-#ifndef FMHA_STAGES_V64
-#define FMHA_STAGES_V64 8
-#endif
-
 namespace fmha {
 
 // Optional timeline tracing for performance work: with -DFMHA_TRACE the first CTA records clock64()
@@ -164,10 +150,10 @@ template <int D> __host__ __device__ constexpr int bias_bytes() { return (2 + SB
 
 template <int D> struct FwdCfg {
   static_assert(D == 64 || D == 128, "head_dim must be 64 or 128");
-  static constexpr int kStagesK = (D == 128) ? FMHA_STAGES_K128 : FMHA_STAGES_K64;   // ring depth of K
+  static constexpr int kStagesK = (D == 128) ? 3 : 4;   // ring depth of K
   // ring depth of V: one thread loads K(g), V(g), K(g+1), ... in order, and V(g) is consumed a few steps (the number of S accumulators) after
   // K(g), so the V ring has to be that much deeper than the K ring
-  static constexpr int kStagesV = (D == 128) ? FMHA_STAGES_V128 : FMHA_STAGES_V64;
+  static constexpr int kStagesV = (D == 128) ? 6 : 8;
   static_assert(kStagesV >= kStagesK + SBufs<D>::n, "V ring too shallow for the in-order loader");
   // Q tiles resident at once: the S cursor runs three steps ahead, which with one-tile units means three
   // units ahead, so short-sequence shapes want more than two (head_dim 128 has no shared memory to spare)
@@ -510,7 +496,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
   for (int it = 0; it < walk.count; ++it) {
     const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
-    if (!__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
       raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it);
       return;
     }
@@ -643,7 +629,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
   for (int it = 0; it < walk.count; ++it) {
     const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
-    if (!__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
       raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it);
       return;
     }
@@ -662,7 +648,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
       const uint32_t g = g0 + static_cast<uint32_t>(j);
       const int slot = static_cast<int>(g & 3u);
       const uint32_t sb = g % SBufs<D>::n;
-      if (!__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->p_ready[slot]), (g >> 2) & 1u, abort_flag))) {
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->p_ready[slot]), (g >> 2) & 1u, abort_flag))) {
         raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_P_READY, g);
         return;
       }
@@ -840,6 +826,7 @@ __device__ __forceinline__ void merge_parts(const FwdParams& p, const uint32_t p
 // ---------------------------------------------------------------------------------------------- loader
 // One warp, run warp-wide (every lane waits and counts, one elected lane issues the copies): the Q tile of every
 // non-empty unit, then per step the K tile and the V tile, in step order.
+// (In a statistics launch, too: this kernel multiplies P and V there like anywhere else, and the merge warps drop the product.)
 template <int D>
 __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl,
                                             const CUtensorMap* map_q, const CUtensorMap* map_k, const CUtensorMap* map_v,
@@ -851,11 +838,10 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
   uint32_t g = 0;            // steps loaded so far: ring position and phase continue across units
   uint32_t qn = 0;           // non-empty units so far: Q buffer and phase
   uint32_t fail = 0u, fail_tile = 0u;
-  const bool no_v = p.row_stats_out != nullptr;        // the statistics launch has no P.V
   for (int it = 0; it < walk.count && fail == 0u; ++it) {
     const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
-    if (!__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
       fail = FMHA_I8_DEV_WAIT_INFO; fail_tile = it; break;
     }
     const UnitGeom geo = unit_geom(p, u);
@@ -864,7 +850,7 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
     if (n_live > 0) {
       const uint32_t qb = qn % NQ;
       // the Q buffer is free once the last S = Q.K^T of the unit that used it NQ units ago has completed
-      if (qn >= NQ && !__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->q_empty[qb]), ((qn / NQ) - 1) & 1u, abort_flag))) {
+      if (qn >= NQ && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->q_empty[qb]), ((qn / NQ) - 1) & 1u, abort_flag))) {
         fail = FMHA_I8_DEV_WAIT_K_FREE; fail_tile = it; break;
       }
       if (elect_one()) {
@@ -876,14 +862,14 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
       for (int j = 0; j < n_live; ++j, ++g) {
         const int t = info->live[info->begin + j];
         const uint32_t sk = g % NK, rk = g / NK, sv = g % NV, rv = g / NV;
-        if (rk > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->k_empty[sk]), (rk - 1) & 1u, abort_flag))) {
+        if (rk > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->k_empty[sk]), (rk - 1) & 1u, abort_flag))) {
           fail = FMHA_I8_DEV_WAIT_K_FREE; fail_tile = g; break;
         }
         if (elect_one()) {
           mbar_arrive_expect_tx(smem_u32(&ctl->k_full[sk]), Cfg::kTileBytes);
           tma_load_3d(k_smem + sk * Cfg::kTileBytes, map_k, smem_u32(&ctl->k_full[sk]), 0, t * kTile, geo.bh_local);
         }
-        if (rv > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->v_empty[sv]), (rv - 1) & 1u, abort_flag))) {
+        if (rv > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->v_empty[sv]), (rv - 1) & 1u, abort_flag))) {
           fail = FMHA_I8_DEV_WAIT_V_FREE; fail_tile = g; break;
         }
         if (elect_one()) {
@@ -911,9 +897,8 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
 struct IssuerErr {
   uint32_t code = 0u, tile = 0u;
 };
-template <bool kSlow = false>
 __device__ __forceinline__ bool issuer_wait(IssuerErr& e, uint32_t bar, uint32_t parity, uint32_t code, uint32_t tile, const volatile int* abort_flag) {
-  if (__all_sync(0xFFFFFFFFu, kSlow ? mbar_wait_slow(bar, parity, abort_flag) : mbar_wait(bar, parity, abort_flag))) return true;
+  if (__all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag))) return true;
   e.code = code;
   e.tile = tile;
   return false;
@@ -935,7 +920,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   for (int it = 0; it < walk.count && ok; ++it) {
     const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
-    if (!issuer_wait<true>(err, smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO, it, abort_flag)) break;
+    if (!issuer_wait(err, smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO, it, abort_flag)) break;
     const UnitInfo* info = &ctl->info[buf];
     const int n_live = info->n_live;
     const uint32_t qb = qn % NQ;
@@ -944,7 +929,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
       continue;
     }
-    if (!issuer_wait<true>(err, smem_u32(&ctl->q_full[qb]), (qn / NQ) & 1u, FMHA_I8_DEV_WAIT_Q_LOAD, g, abort_flag)) break;
+    if (!issuer_wait(err, smem_u32(&ctl->q_full[qb]), (qn / NQ) & 1u, FMHA_I8_DEV_WAIT_Q_LOAD, g, abort_flag)) break;
     const uint64_t dq = make_smem_desc(q_smem + qb * Cfg::kTileBytes, D);
     const int8_t* mask_row = p.mask + static_cast<int64_t>(unit_geom(p, u).batch) * p.S;
     for (int j = 0; j < n_live; ++j, ++g) {
@@ -960,7 +945,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       }
       // K first (it has normally been there for a while), then the accumulator: it still holds the partial output of
       // step g - n until the merge warps have drained it, and that hand-off is on the step-to-step critical path
-      if (!issuer_wait<true>(err, smem_u32(&ctl->k_full[stage]), (g / NK) & 1u, FMHA_I8_DEV_WAIT_K_LOAD, g, abort_flag)) { ok = false; break; }
+      if (!issuer_wait(err, smem_u32(&ctl->k_full[stage]), (g / NK) & 1u, FMHA_I8_DEV_WAIT_K_LOAD, g, abort_flag)) { ok = false; break; }
       if (g >= SBufs<D>::n && !issuer_wait(err, smem_u32(&ctl->s_free[sb]), ((g / SBufs<D>::n) - 1) & 1u, FMHA_I8_DEV_WAIT_O_FREE, g, abort_flag)) { ok = false; break; }
       FMHA_STAMP(15, g);
       tc_fence_after();
@@ -1005,7 +990,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   for (int it = 0; it < walk.count && ok; ++it) {
     const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
-    if (!issuer_wait<true>(err, smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO, it, abort_flag)) break;
+    if (!issuer_wait(err, smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO, it, abort_flag)) break;
     const int n_live = ctl->info[buf].n_live;
     __syncwarp();
     if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));            // only the tile count is needed here
@@ -1016,7 +1001,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       const uint32_t tP = PLayout<D>::kAnnex ? tmem_base + SBufs<D>::n * kTile + sb * PLayout<D>::kAnnexCols : tS;
       const uint32_t tO = tS + PLayout<D>::kOOff;
       // V first (loaded steps ago), then P: the MMAs go out as soon as the last softmax warp has arrived
-      if (!issuer_wait<true>(err, smem_u32(&ctl->v_full[stage]), (g / NV) & 1u, FMHA_I8_DEV_WAIT_V_LOAD, g, abort_flag)) { ok = false; break; }
+      if (!issuer_wait(err, smem_u32(&ctl->v_full[stage]), (g / NV) & 1u, FMHA_I8_DEV_WAIT_V_LOAD, g, abort_flag)) { ok = false; break; }
       if (!issuer_wait(err, smem_u32(&ctl->p_ready[g & 3u]), (g >> 2) & 1u, FMHA_I8_DEV_WAIT_P_READY, g, abort_flag)) { ok = false; break; }
       FMHA_STAMP(13, g);
       tc_fence_after();
@@ -1134,7 +1119,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const int buf = it % kInfoBufs;
         // the buffer was used by unit it - kInfoBufs: wait until all its consumers have released it
         if (it >= kInfoBufs) {
-          ok = __all_sync(0xFFFFFFFFu, mbar_wait_slow(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), abort_flag));
+          ok = __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), abort_flag));
           if (!ok) { if (lane == 0) raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it); break; }
         }
         const UnitGeom geo = unit_geom(p, u);

@@ -57,30 +57,17 @@ constexpr long long kWaitLimitCycles = 2000000000LL;
 // switched out on a shared GPU, probes do not, so a long time slice elsewhere cannot by itself end a wait.
 constexpr uint32_t kMinProbes = 4096u;
 
-// Back-off between probes, in nanoseconds (0 = none, the default and the measured best).  mbarrier.try_wait returns
-// after a short, hardware-defined time when the phase is not complete, so a waiting warp keeps issuing its polling
-// loop.  nanosleep between probes was measured on B200 to cost more on the hand-offs than the freed issue slots are
-// worth (and every argument up to 80 ns sleeps equally long); the two classes of waits -- on the step-to-step
-// critical path, and normally satisfied long before they are needed -- are kept apart for further tuning.
-#ifndef FMHA_SLEEP_FAST
-#define FMHA_SLEEP_FAST 0
-#endif
-#ifndef FMHA_SLEEP_SLOW
-#define FMHA_SLEEP_SLOW 0
-#endif
-
 // Waits for the phase with the given parity to complete.  Gives up when the cycle limit is reached (and at
 // least min_probes probes were made) or when another thread of the CTA has already raised *abort_flag.
-// The loop is deliberately not tight: measured on B200, a waiting warp that probes as fast as it can (three
-// instructions per probe) slows the working warps of its SM down more than this one does, and nanosleep between
-// probes costs more latency on the hand-offs than it saves (any argument up to 80 ns sleeps equally long).
-template <uint32_t kSleepNs>
-__device__ __forceinline__ bool mbar_wait_backoff(uint32_t bar, uint32_t parity, const volatile int* abort_flag, long long limit_cycles,
-                                                  uint32_t min_probes) {
+// The loop is deliberately not tight: mbarrier.try_wait returns after a short, hardware-defined time when the phase is not
+// complete, and measured on B200 a waiting warp that probes as fast as it can (three instructions per probe) slows the working warps
+// of its SM down more than this one does, while nanosleep between probes costs more latency on the hand-offs than it saves
+// (any argument up to 80 ns sleeps equally long).
+__device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, const volatile int* abort_flag, long long limit_cycles,
+                                                  uint32_t min_probes = 0u) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   for (uint32_t it = 1;; ++it) {
-    if (kSleepNs != 0u) __nanosleep(kSleepNs);
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 31u) == 0u) {
       if (*abort_flag) return false;
@@ -88,14 +75,8 @@ __device__ __forceinline__ bool mbar_wait_backoff(uint32_t bar, uint32_t parity,
     }
   }
 }
-__device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, const volatile int* abort_flag, long long limit_cycles) {
-  return mbar_wait_backoff<0u>(bar, parity, abort_flag, limit_cycles, 0u);
-}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
-  return mbar_wait_backoff<FMHA_SLEEP_FAST>(bar, parity, abort_flag, kWaitLimitCycles, kMinProbes);
-}
-__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
-  return mbar_wait_backoff<FMHA_SLEEP_SLOW>(bar, parity, abort_flag, kWaitLimitCycles, kMinProbes);
+  return mbar_wait_limited(bar, parity, abort_flag, kWaitLimitCycles, kMinProbes);
 }
 
 // Warp-wide wait of the head_dim-64 workers: most of their waits find the phase complete, and without the loop around the
