@@ -295,6 +295,7 @@ def test_many_query_tiles_head_dim_64(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk,
     q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, 64, seed=B + Sk, mask_p=mask_p, valid=valid)
     q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
     desc, param = pkg.AttnDataDescriptorX(B, Sq, Sk, H, 64), pkg.FMHAParamI8(*amax, 0.25)
+    assert pkg.debug_plan(desc)[0] == pkg.KERNEL_WORKERS and pkg.debug_plan(desc, pkg.POLICY_ROW)[0] == pkg.KERNEL_WORKERS
     o = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
     scratch = torch.zeros(2 * B * H * Sq, device="cuda")
     if what == "amax":
@@ -334,8 +335,10 @@ def test_few_query_tiles_share_their_keys(pkg, wl, oracle, torch_cuda, D, B, H, 
     want = oracle.q128(q8, k8, v8, mask, amax, p_levels=255 if uint8_p else 128)
     q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
     o = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    desc = pkg.AttnDataDescriptorX(B, Sq, Sk, H, D)
+    assert pkg.debug_plan(desc)[0] == pkg.KERNEL_GENERAL and pkg.debug_plan(desc)[1] in (2, 4, 8) and pkg.debug_plan(desc)[2] == 0
     for _ in range(3):
-        pkg.FMHAInferI8Cross(None, pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), q, k, v, m, o[128:-128], uint8_p=uint8_p)
+        pkg.FMHAInferI8Cross(None, pkg.FMHAParamI8(*amax, 1.0), desc, q, k, v, m, o[128:-128], uint8_p=uint8_p)
     st, words = pkg.device_status()
     assert st == pkg.OK, words
     host = o.cpu().numpy()
@@ -419,19 +422,23 @@ def test_a_mask_on_the_device_is_not_read_by_the_host(pkg, torch_cuda):
     assert not pkg.debug_host_fetch(desc, q, k, v, mask.cuda())
 
 
-# More query tiles than SMs: those of a last round of at most half the SMs are shared by pairs of CTAs.  148 + 2, 148 + 74 (the most), 2 * 148 + 64
-# query tiles; the last of them beyond the sequence's end, a sequence without a key among them.
+# More query tiles than SMs: those of a last round of at most half the SMs are shared by pairs of CTAs.  148 + 2, 148 + 74 (the most) and
+# 2 * 148 + 64 query tiles; the last of them beyond the sequence's end.  Where two whole rounds come first, the shared tiles belong to a
+# sequence whose keys divide unevenly, leave one CTA of a pair without any, or leave none at all.
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("B,H,Sq,Sk,valid,mask_p", [
-    (3, 10, 600, 704, (704, 650, 0), 0.0), (2, 37, 300, 1024, (1000, 129), 0.0), (1, 24, 1900, 640, None, 0.1)])
-def test_pairs_share_the_last_round(pkg, wl, oracle, torch_cuda, D, B, H, Sq, Sk, valid, mask_p):
+@pytest.mark.parametrize("B,H,Sq,Sk,valid,mask_p,rounds", [
+    (3, 10, 600, 704, (704, 650, 0), 0.0, 1), (2, 37, 300, 1024, (1000, 129), 0.0, 1),
+    (2, 12, 1900, 1280, (1280, 700), 0.1, 2), (2, 12, 1900, 1280, (900, 100), 0.0, 2), (2, 12, 1900, 1280, (1280, 0), 0.0, 2)])
+def test_pairs_share_the_last_round(pkg, wl, oracle, torch_cuda, D, B, H, Sq, Sk, valid, mask_p, rounds):
     torch = torch_cuda
     q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, D, seed=Sq + Sk + D, mask_p=mask_p, valid=valid)
     want = oracle.q128(q8, k8, v8, mask, amax)
     q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
     o = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    desc = pkg.AttnDataDescriptorX(B, Sq, Sk, H, D)
+    assert pkg.debug_plan(desc) == (pkg.KERNEL_GENERAL, 2, rounds)
     for _ in range(3):
-        pkg.FMHAInferI8Cross(None, pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), q, k, v, m, o[128:-128])
+        pkg.FMHAInferI8Cross(None, pkg.FMHAParamI8(*amax, 1.0), desc, q, k, v, m, o[128:-128])
     st, words = pkg.device_status()
     assert st == pkg.OK, words
     host = o.cpu().numpy()
