@@ -315,17 +315,23 @@ int launch_kernel(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cud
 }
 
 // CTAs that share one unit (query tile), each with a part of its key tiles: for calls whose units leave most SMs idle, as long as
-// all clusters are resident at once (a second wave of them starts from nothing and costs 10 us).  In nanoseconds, measured: 950
+// all clusters are resident at once (a second wave of them starts from nothing and costs 10 us).  In nanoseconds, measured: 860
 // per key tile of a CTA, and for cluster launch, two cluster barriers and the merge of the partial results through distributed
-// shared memory 2300 / 3000 / 4300 with 2 / 4 / 8 CTAs.  (Head_dim 64, us without -> with: B1 H8 S1024 Sq256 11.9 -> 9.1, B1 H4
-// S2048 Sq200 19.2 -> 10.5, B1 H2 S4096 34.9 -> 23.4, B1 H8 S8192 Sq64 64 -> 17.7; head_dim 128: B2 H16 S1984 Sq200 21.1 -> 16.8,
-// B1 H2 S16384 Sq128 131 -> 29.)
+// shared memory, at head_dim 64 and (rows twice as long) 128, with 2, 4 and 8 CTAs:
+constexpr int kTileNs = 860;
+constexpr int kShareNs[2][kClusterSizes] = {{2400, 2900, 4700}, {3100, 4800, 6000}};
+// us without -> with.  Head_dim 64: B1 H8 S1024 Sq256 10.9 -> 8.7, B1 H4 S2048 Sq200 17.6 -> 10.2, B1 H2 S4096 32.1 -> 21.3, B1 H8 S8192
+// Sq64 57.9 -> 16.9; head_dim 128: B2 H16 S1984 Sq200 19.1 -> 15.6, B1 H2 S16384 Sq128 114 -> 27.  Where the line lies, 12 units, 1 / 2 / 4
+// CTAs each: head_dim 64, 5 tiles 8.3 / 8.8 / 8.5, 6 tiles 9.1 / 8.9 / 8.6; head_dim 128, 6 tiles 9.8 / 10.1 / 11.1, 8 tiles 11.5 / 11.1 /
+// 11.2, 12 tiles 15.1 / 13.0 / 12.2.
 //
 // With more units than SMs the same is done for those of the last round: where they are half as many as the SMs or fewer, a pair
-// of CTAs shares each.  (Head_dim 128: B1 H16 S1280 25.6 -> 23.6, B1 H5 S4096 68.9 -> 56.0, B1 H32 S2048 70.9 -> 65.8.)
-bool pairs_share_last_round(const FwdParams& p, const DeviceInfo* dev) {
+// of CTAs shares each.  (Head_dim 128: B1 H16 S1280 23.1 -> 21.8, B1 H5 S4096 60.9 -> 50.2, B1 H32 S2048 61.7 -> 58.0; 208 units of
+// 6 tiles 16.3 -> 16.5, of 8 tiles 19.8 -> 19.4.  Head_dim 64: 5 tiles 13.1 -> 13.8, 6 tiles 14.9 -> 14.7.)
+bool pairs_share_last_round(const FwdParams& p, int D, const DeviceInfo* dev) {
   const int last = p.n_units % dev->sm_count, tiles = (p.S + kTile - 1) / kTile;
-  return p.n_units > dev->sm_count && last > 0 && last <= dev->max_clusters[0] && 2 * dev->max_clusters[0] == dev->sm_count && 950 * (tiles / 2) > 2300;
+  return p.n_units > dev->sm_count && last > 0 && last <= dev->max_clusters[0] && 2 * dev->max_clusters[0] == dev->sm_count &&
+         kTileNs * (tiles / 2) > kShareNs[D == 128][0];
 }
 // ceil(2^(31 + bits) / d) with 2^bits >= d > 2^(bits - 1): the quotient is exact for every dividend below 2^31.
 FastDiv fast_div_by(int d) {
@@ -335,32 +341,31 @@ FastDiv fast_div_by(int d) {
   return FastDiv{static_cast<uint32_t>((one + static_cast<uint64_t>(d) - 1) / static_cast<uint64_t>(d)), 31 + bits};
 }
 
-void plan_parts(FwdParams* p, const DeviceInfo* dev) {
-  constexpr int kOverhead[kClusterSizes] = {2300, 3000, 4300};
+void plan_parts(FwdParams* p, int D, const DeviceInfo* dev) {
   const int tiles = (p->S + kTile - 1) / kTile;
   p->own_rounds = p->n_units / dev->sm_count;
   if (p->own_rounds > 0) {
-    if (pairs_share_last_round(*p, dev)) p->parts = 2;
+    if (pairs_share_last_round(*p, D, dev)) p->parts = 2;
     return;
   }
-  int best_ns = 950 * tiles;
+  int best_ns = kTileNs * tiles;
   for (int i = 0; i < kClusterSizes; ++i) {
-    const int c = 2 << i, ns = 950 * ((tiles + c - 1) / c) + kOverhead[i];
+    const int c = 2 << i, ns = kTileNs * ((tiles + c - 1) / c) + kShareNs[D == 128][i];
     if (p->n_units <= dev->max_clusters[i] && ns < best_ns) { p->parts = c; best_ns = ns; }
   }
 }
 
 // Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  Cycles per key tile, measured: a CTA of
 // fmha_fwd_sm100.cuh works on one unit at a time, 1600 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5850 per
-// tile for all four, 4900 / 4350 / 3400 with three, two or one left in the last round.  (B12 H12 S256: 8.2 / 7.9 us; B6 H12
-// S512: 11.6 / 12.5; B16 H12 S512: 26.8 / 26.2; B3 H12 S1024: 18.4 / 21.5; B8 H12 S1024: 44.2 / 46.2; B1 H24 S2048: 45.0 / 44.4;
-// B1 H40 S2048: 66.7 / 80.4.)
+// tile for all four, 4900 / 4350 / 3400 with three, two or one left in the last round.  (us, fmha_fwd_sm100.cuh / fmha_fwd64_sm100.cuh: B64 H16 S64
+// 14.9 / 12.5; B12 H12 S256 8.1 / 8.5, the estimate's worst error among these; B6 H12 S512 11.6 / 13.0; B16 H12 S512 28.8 / 27.8; B3 H12
+// S1024 18.4 / 22.0; B8 H12 S1024 44.3 / 47.7; B1 H24 S2048 45.5 / 45.2; B1 H40 S2048 67.2 / 82.1; B8 H32 S2048 368 / 343.)
 bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
   const long long sms = dev->sm_count, tiles = (p.S + kTile - 1) / kTile, round = sms * w64::kWorkers;
   const long long last[w64::kWorkers + 1] = {0, 3400, 4350, 4900, 5850};
   const long long workers = p.n_units / round * 5850 + last[(p.n_units % round + sms - 1) / sms];
   const long long own = p.n_units / sms, more = p.n_units % sms != 0, unit = 1600 * tiles + 1200;
-  return workers * tiles < own * unit + more * (pairs_share_last_round(p, dev) ? unit / 2 + 4500 : unit);
+  return workers * tiles < own * unit + more * (pairs_share_last_round(p, 64, dev) ? unit / 2 + 4500 : unit);
 }
 
 // Few query rows run the few-rows kernel.  Up to four rows it is bound by reading K and V; from five on (computed as eight) its integer dot
@@ -379,7 +384,7 @@ int plan_call(FwdParams* p, int D, bool plain, int busy_sms, const DeviceInfo* d
   p->parts = 1;
   if (plain && few_rows(p->Sq, p->S, D)) return FMHA_I8_KERNEL_FEW_ROWS;
   if (D == 64 && use_workers(*p, dev)) return FMHA_I8_KERNEL_WORKERS;
-  if (plain && busy_sms == 0) plan_parts(p, dev);
+  if (plain && busy_sms == 0) plan_parts(p, D, dev);
   return FMHA_I8_KERNEL_GENERAL;
 }
 

@@ -422,12 +422,21 @@ def test_a_mask_on_the_device_is_not_read_by_the_host(pkg, torch_cuda):
     assert not pkg.debug_host_fetch(desc, q, k, v, mask.cuda())
 
 
+def test_where_a_query_tile_is_shared(pkg, torch_cuda):
+    """Either side of the lines: 12 query tiles of so many key tiles, and 148 + 60."""
+    for D, tiles, shared in [(64, 5, False), (64, 6, True), (128, 6, False), (128, 7, False), (128, 8, True), (64, 64, True), (128, 64, True)]:
+        assert (pkg.debug_plan(pkg.AttnDataDescriptorX(1, 128, 128 * tiles, 12, D))[1] > 1) == shared, (D, tiles)
+    for D, tiles, shared in [(64, 5, False), (64, 6, True), (128, 7, False), (128, 8, True)]:
+        plan = pkg.debug_plan(pkg.AttnDataDescriptorX(1, 2048, 128 * tiles, 13, D))
+        assert plan == ((pkg.KERNEL_GENERAL, 2, 1) if shared else (pkg.KERNEL_GENERAL, 1, 0)), (D, tiles)
+
+
 # More query tiles than SMs: those of a last round of at most half the SMs are shared by pairs of CTAs.  148 + 2, 148 + 74 (the most) and
 # 2 * 148 + 64 query tiles; the last of them beyond the sequence's end.  Where two whole rounds come first, the shared tiles belong to a
 # sequence whose keys divide unevenly, leave one CTA of a pair without any, or leave none at all.
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,H,Sq,Sk,valid,mask_p,rounds", [
-    (3, 10, 600, 704, (704, 650, 0), 0.0, 1), (2, 37, 300, 1024, (1000, 129), 0.0, 1),
+    (3, 10, 600, 1088, (1088, 650, 0), 0.0, 1), (2, 37, 300, 1024, (1000, 129), 0.0, 1),
     (2, 12, 1900, 1280, (1280, 700), 0.1, 2), (2, 12, 1900, 1280, (900, 100), 0.0, 2), (2, 12, 1900, 1280, (1280, 0), 0.0, 2)])
 def test_pairs_share_the_last_round(pkg, wl, oracle, torch_cuda, D, B, H, Sq, Sk, valid, mask_p, rounds):
     torch = torch_cuda
