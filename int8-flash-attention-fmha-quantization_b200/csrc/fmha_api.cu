@@ -370,7 +370,7 @@ bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
 
 // Few query rows run the few-rows kernel.  Up to four rows it is bound by reading K and V; from five on (computed as eight) its integer dot
 // products take as long or longer.  us, few-rows / general kernel:
-//   D128, 1 row   B16 H32 S4096 (1025..4096 keys) 55 / 104
+//   D128, 1 row   B16 H32 S4096 (1025..4096 keys) 55.3 / 82.9
 //   D128, 8 rows  B128 H32 S64 90.9 / 62.0, B64 H32 S256 50.1 / 40.2, B32 H32 S1024 71.8 / 61.5, B8 H32 S4096 83.3 / 63.2, B1 H8 S16384
 //                 77.3 / 25.3, and so on: the general one at every length and number of heads measured
 //   D64, 8 rows   B128 H32 S128 61.0 / 32.9, B1 H4 S128 5.9 / 4.7: the general one for a single key tile; beyond, with many heads, the
@@ -396,9 +396,10 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   if ((st = make_map(&mk, k, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mv, v, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
   // Overlap pays where the launch latency is a visible part of the launch: up to four rounds of units (512 units of a
-  // whole-row policy 65.0 -> 62.5 us).  Beyond that it gives nothing (B8 H32 S2048: 461 us either way) and where whole
-  // K/V tiles stream through every few hundred ns it costs: CTAs then land on SMs in the order the launch before frees
-  // them, neighbours that share a head are no longer neighbours on the chip (B256 H16 S256 D64: 132 -> 141 us).
+  // whole-row policy 49.5 -> 46.2 us).  Far beyond that it gives nothing (B8 H32 S2048 415 and 412, B256 H16 S256 D64 with lengths 64..256
+  // 90.1 and 91.0, repeats differ by more), and CTAs then land on SMs in the order the launch before frees them, where neighbours
+  // that share a head are no longer neighbours on the chip.  (Between four and thirty rounds it would still gain: B4 H32 S1024
+  // D128, seven rounds, 61.5 -> 58.2; B64 H32 S256 D128, 28 rounds, 87 -> 83.)
   LaunchHow how;
   how.overlap = p.n_units <= 4 * dev->sm_count;
   // persistent CTAs: one per SM (tensor memory is allocated whole), each walking its share of the units
@@ -417,8 +418,8 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
 }
 
 // The few-rows kernel.  CTAs per head: enough for two rounds of the 3 CTAs that an SM holds, so that heads of different
-// length even out, as long as a warp keeps two tiles (B16 H32, 1025..4096 keys, one row: 60.3 us with one round, 58.6 with
-// two, 70 with four, 112 with eight, where the set-up of a CTA outweighs its tiles); where even that leaves SMs idle, down
+// length even out, as long as a warp keeps two tiles (B16 H32, 1025..4096 keys, one row, clusters of 1 / 2 / 4 / 8: 60.9 / 55.3 / 59.0 /
+// 80.2 us, the last where the set-up of a CTA outweighs its tiles); where even that leaves SMs idle, down
 // to one tile per warp.
 template <int D, int R, bool kUnsigned>
 int launch_decode_rows(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v) {

@@ -11,12 +11,12 @@
 // A worker's step is one serial chain -- S, maximum, exponentials, P.V, fold -- of 3600 cycles when it runs alone.  Four of them
 // on an SM hide each other's latencies; nobody waits for a stage that other threads own, which is what bounds the other kernel
 // on short sequences (its merge warps need 4500 cycles per unit of two steps whatever the other warps do).  What bounds this
-// one: issue slots and the exponential unit, 57 % and 55 % busy on long sequences, where a step takes 5800 cycles, i.e. 1450 per
+// one: issue slots and the exponential unit, 61 % and 66 % busy on long sequences, where a step takes 5520 cycles, i.e. 1380 per
 // SM.  An eighth of the exponentials is computed on the multiply-add pipe (all on the exponential unit: 2.5 % slower on
 // B8 H32 S2048; a quarter: 3 % slower).  Pass 2 reads eight columns at a time: with sixteen the 104 registers of a softmax
 // thread do not suffice, and the spills cost 4 to 9 %.
-// Measured against the other kernel: B32 H12 S512 (lengths 256..512) 45.2 -> 41.8 us, B256 H16 S256 (64..256) 115 -> 99,
-// B8 H32 S2048 401 -> 372, B4 H16 S1024 with the per-row policy 55 -> 47.8.
+// Measured against the other kernel: B32 H12 S512 (lengths 256..512) 42.1 -> 39.3 us, B256 H16 S256 (64..256) 98 -> 90,
+// B8 H32 S2048 368 -> 343, B4 H16 S1024 with the per-row policy 52.4 -> 46.2.
 #pragma once
 #include "fmha_fwd_sm100.cuh"
 

@@ -43,7 +43,8 @@
 //
 // What bounds it: issue slots (64 % busy; 4300 warp instructions for a step of 128 x 128 scores at head_dim 128, 2700 of them
 // arithmetic) and the exponential unit (63 %), on a chain of hand-offs that the sets of buffers overlap; in units of one or two
-// steps the merge warps, which spend more on a unit's epilogue than on a step.  B8 H32 S2048 D128: 405 us.
+// steps the merge warps, which spend more on a unit's epilogue than on a step.  B8 H32 S2048 D128: 405 us while the chip is cool enough
+// for 1965 MHz, 430 to 440 back to back, where the power limit holds it at 1820 to 1860.
 //
 // The bias: every accumulator is first written by a one-step bf16 MMA whose operands hold 4096 and
 // 3072, i.e. the fp32 value 1.5*2^23 (bits 0x4B400000); the int8 MMAs then add their integer result
@@ -128,8 +129,8 @@ constexpr int kInfoConsumers = 3 + kSoftmaxWarps + kMergeWarps;   // loader, two
 // launch and refuses otherwise); the targets per role (FwdRegs) add up to 28 x 72.
 constexpr int kLaunchRegs = 72;
 template <int D> struct FwdRegs {
-  // head_dim 128: the merge threads hold a 64-register half output row (B8 H32 S2048: 104/40 takes 405 us, 96/56
-  // 410, 88/72 427).  head_dim 64: the output row is 32 registers; 88/72 is the split at which
+  // head_dim 128: the merge threads hold a 64-register half output row (B8 H32 S2048 at 1965 MHz: 104/40 takes 405 us,
+  // 96/56 410, 88/72 427).  head_dim 64: the output row is 32 registers; 88/72 is the split at which
   // ptxas reports no spills at all, and C5 runs 5 % faster with it than with 80/88 or 96/56, which both spill.
   static constexpr int kSoftmax = 64, kMerge = (D == 128) ? 104 : 88, kOther = (D == 128) ? 40 : 72;
   static_assert(kSoftmaxWarps * kSoftmax + kMergeWarps * kMerge + 4 * kOther <= kFwdWarps * kLaunchRegs,

@@ -9,8 +9,8 @@
 //                         registers the first ones (53 MB over the chip); pass 2 takes those from there and walks the
 //                         others from the last to the first, so that it meets what the L2 still has.
 // Two launches over 65,536-element chunks, which these replace, took 16.5 us for 255,749 elements (four CTAs) and 107 us
-// for 67,108,864; these take 5.5 and 93.5 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
-// what neither the SMs (50 MB) nor the L2 kept.
+// for 67,108,864; these take 5.5 and 95 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
+// what neither the SMs (50 MB) nor the L2 (44 MB) kept.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
