@@ -317,21 +317,23 @@ int launch_kernel(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cud
 // CTAs that share one unit (query tile), each with a part of its key tiles: for calls whose units leave most SMs idle, as long as
 // all clusters are resident at once (a second wave of them starts from nothing and costs 10 us).  In nanoseconds, measured: 860
 // per key tile of a CTA, and for cluster launch, two cluster barriers and the merge of the partial results through distributed
-// shared memory, at head_dim 64 and (rows twice as long) 128, with 2, 4 and 8 CTAs:
+// shared memory, with 2, 4 and 8 CTAs, kShareNs for up to 64 rows at head_dim 128 or 128 at 64, kShareMoreNs more for twice as many:
 constexpr int kTileNs = 860;
-constexpr int kShareNs[2][kClusterSizes] = {{2400, 2900, 4700}, {3100, 4800, 6000}};
+constexpr int kShareNs[kClusterSizes] = {2400, 2900, 4300}, kShareMoreNs[kClusterSizes] = {700, 1900, 1700};
 // us without -> with.  Head_dim 64: B1 H8 S1024 Sq256 10.9 -> 8.7, B1 H4 S2048 Sq200 17.6 -> 10.2, B1 H2 S4096 32.1 -> 21.3, B1 H8 S8192
 // Sq64 57.9 -> 16.9; head_dim 128: B2 H16 S1984 Sq200 19.1 -> 15.6, B1 H2 S16384 Sq128 114 -> 27.  Where the line lies, 12 units, 1 / 2 / 4
-// CTAs each: head_dim 64, 5 tiles 8.3 / 8.8 / 8.5, 6 tiles 9.1 / 8.9 / 8.6; head_dim 128, 6 tiles 9.8 / 10.1 / 11.1, 8 tiles 11.5 / 11.1 /
-// 11.2, 12 tiles 15.1 / 13.0 / 12.2.
+// CTAs each: head_dim 64, 128 rows, 5 tiles 8.3 / 8.9 / 8.5, 6 tiles 9.1 / 8.9 / 8.6; head_dim 128, 33 rows, 5 tiles 9.0 / 8.9 / 9.4,
+// 6 tiles 9.8 / 9.0 / 9.5; 96 rows, 6 tiles 9.8 / 9.7 / 10.2, 7 tiles 10.7 / 10.6 / 10.3; 128 rows, 7 tiles 10.7 / 11.0 / 11.2, 8 tiles 11.6 / 11.2 / 11.2, 12 tiles 15.1 / 13.1 / 12.1.
 //
 // With more units than SMs the same is done for those of the last round: where they are half as many as the SMs or fewer, a pair
 // of CTAs shares each.  (Head_dim 128: B1 H16 S1280 23.1 -> 21.8, B1 H5 S4096 60.9 -> 50.2, B1 H32 S2048 61.7 -> 58.0; 208 units of
-// 6 tiles 16.3 -> 16.5, of 8 tiles 19.8 -> 19.4.  Head_dim 64: 5 tiles 13.1 -> 13.8, 6 tiles 14.9 -> 14.7.)
-bool pairs_share_last_round(const FwdParams& p, int D, const DeviceInfo* dev) {
+// 6 tiles 16.3 -> 16.5, of 8 tiles 19.8 -> 19.4; 1072 units of 6 tiles 53.5 -> 50.7, with what overlapping launches give, see
+// launch_fwd.  Head_dim 64: 208 units of 5 tiles 13.1 -> 13.8, of 6 tiles 14.9 -> 14.7.)
+constexpr int kPairNs = 2400;
+bool pairs_share_last_round(const FwdParams& p, const DeviceInfo* dev) {
   const int last = p.n_units % dev->sm_count, tiles = (p.S + kTile - 1) / kTile;
   return p.n_units > dev->sm_count && last > 0 && last <= dev->max_clusters[0] && 2 * dev->max_clusters[0] == dev->sm_count &&
-         kTileNs * (tiles / 2) > kShareNs[D == 128][0];
+         kTileNs * (tiles / 2) > kPairNs;
 }
 // ceil(2^(31 + bits) / d) with 2^bits >= d > 2^(bits - 1): the quotient is exact for every dividend below 2^31.
 FastDiv fast_div_by(int d) {
@@ -345,12 +347,13 @@ void plan_parts(FwdParams* p, int D, const DeviceInfo* dev) {
   const int tiles = (p->S + kTile - 1) / kTile;
   p->own_rounds = p->n_units / dev->sm_count;
   if (p->own_rounds > 0) {
-    if (pairs_share_last_round(*p, D, dev)) p->parts = 2;
+    if (pairs_share_last_round(*p, dev)) p->parts = 2;
     return;
   }
+  const int outputs = (p->Sq < kTile ? p->Sq : kTile) * D, more = outputs > 8192 ? outputs - 8192 : 0;
   int best_ns = kTileNs * tiles;
   for (int i = 0; i < kClusterSizes; ++i) {
-    const int c = 2 << i, ns = kTileNs * ((tiles + c - 1) / c) + kShareNs[D == 128][i];
+    const int c = 2 << i, ns = kTileNs * ((tiles + c - 1) / c) + kShareNs[i] + kShareMoreNs[i] * more / 8192;
     if (p->n_units <= dev->max_clusters[i] && ns < best_ns) { p->parts = c; best_ns = ns; }
   }
 }
@@ -365,7 +368,7 @@ bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
   const long long last[w64::kWorkers + 1] = {0, 3400, 4350, 4900, 5850};
   const long long workers = p.n_units / round * 5850 + last[(p.n_units % round + sms - 1) / sms];
   const long long own = p.n_units / sms, more = p.n_units % sms != 0, unit = 1600 * tiles + 1200;
-  return workers * tiles < own * unit + more * (pairs_share_last_round(p, 64, dev) ? unit / 2 + 4500 : unit);
+  return workers * tiles < own * unit + more * (pairs_share_last_round(p, dev) ? unit / 2 + 4500 : unit);
 }
 
 // Few query rows run the few-rows kernel.  Up to four rows it is bound by reading K and V; from five on (computed as eight) its integer dot

@@ -423,12 +423,14 @@ def test_a_mask_on_the_device_is_not_read_by_the_host(pkg, torch_cuda):
 
 
 def test_where_a_query_tile_is_shared(pkg, torch_cuda):
-    """Either side of the lines: 12 query tiles of so many key tiles, and 148 + 60."""
-    for D, tiles, shared in [(64, 5, False), (64, 6, True), (128, 6, False), (128, 7, False), (128, 8, True), (64, 64, True), (128, 64, True)]:
-        assert (pkg.debug_plan(pkg.AttnDataDescriptorX(1, 128, 128 * tiles, 12, D))[1] > 1) == shared, (D, tiles)
-    for D, tiles, shared in [(64, 5, False), (64, 6, True), (128, 7, False), (128, 8, True)]:
-        plan = pkg.debug_plan(pkg.AttnDataDescriptorX(1, 2048, 128 * tiles, 13, D))
-        assert plan == ((pkg.KERNEL_GENERAL, 2, 1) if shared else (pkg.KERNEL_GENERAL, 1, 0)), (D, tiles)
+    """Either side of the lines: 12 query tiles of so many rows and key tiles, and 148 + 60."""
+    for D, Sq, tiles, shared in [(64, 128, 5, False), (64, 128, 6, True), (128, 64, 5, False), (128, 64, 6, True), (128, 96, 6, False), (128, 96, 7, True), (128, 128, 7, False),
+                                 (128, 128, 8, True), (64, 128, 64, True), (128, 128, 64, True)]:
+        assert (pkg.debug_plan(pkg.AttnDataDescriptorX(1, Sq, 128 * tiles, 12, D))[1] > 1) == shared, (D, Sq, tiles)
+    for D in (64, 128):
+        for tiles, shared in [(5, False), (6, True)]:
+            plan = pkg.debug_plan(pkg.AttnDataDescriptorX(1, 2048, 128 * tiles, 13, D))
+            assert plan == ((pkg.KERNEL_GENERAL, 2, 1) if shared else (pkg.KERNEL_GENERAL, 1, 0)), (D, tiles)
 
 
 # More query tiles than SMs: those of a last round of at most half the SMs are shared by pairs of CTAs.  148 + 2, 148 + 74 (the most) and
