@@ -202,8 +202,8 @@ def FMHAInferI8Cross(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, 
                      use_tcu=True, check=True, uint8_p=False):
     """Query rows and keys differ in number: q, o int8 [B,H,Sq,D]; k, v int8 [B,H,Sk,D]; padding_mask int8
     [B,Sk].  attn_desc_x is an AttnDataDescriptorX.  bh_begin/bh_count select heads as in FMHAInferI8Slice."""
-    st = (_binding or _native()).infer_cross(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, int(bh_begin),
-                                             None if bh_count is None else int(bh_count), _flags(use_tcu, uint8_p))
+    st = (_binding or _native()).infer_cross(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, bh_begin, bh_count,
+                                             _flags(use_tcu, uint8_p))
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8Cross")
     return st
@@ -217,8 +217,8 @@ def FMHAInferI8Policy(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o,
     """Whole-row scaling policies for the 8-bit P (reference fmha_i8_quant_deviation.py:57-121): POLICY_ROW = per-row
     ("dynamic") scale, POLICY_STATIC = one calibrated scale fmha_param.s_max for all rows, POLICY_TILE = the reference
     kernel's tile-local scale.  row_scratch: float32 device tensor with 2 elements per query row of the slice."""
-    st = (_binding or _native()).infer_policy(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, int(bh_begin),
-                                              None if bh_count is None else int(bh_count), FLAG_USE_TCU, int(policy), row_scratch)
+    st = (_binding or _native()).infer_policy(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o, bh_begin, bh_count,
+                                              FLAG_USE_TCU, policy, row_scratch)
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8Policy")
     return st
@@ -236,7 +236,7 @@ def calibrate_o_amax(stream, fmha_param, attn_desc_x, q, k, v, padding_mask, o_a
 
 def FMHAInferI8Slice(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, bh_begin, bh_count, check=True, uint8_p=False):
     """Heads [bh_begin, bh_begin+bh_count) of the flattened batch*head axis; q,k,v,o hold only the slice."""
-    st = (_binding or _native()).infer_slice(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, int(bh_begin), int(bh_count),
+    st = (_binding or _native()).infer_slice(stream, fmha_param, attn_desc, q, k, v, padding_mask, o, bh_begin, bh_count,
                                              _flags(True, uint8_p))
     if check and st != OK:
         raise FmhaError(st, "FMHAInferI8Slice")

@@ -40,8 +40,9 @@ bool get_int(PyObject* obj, PyObject* name, int* out) {
   Py_DECREF(i);
   return true;
 }
+// Whatever int() takes.
 bool as_int(PyObject* v, int* out) {
-  PyObject* i = PyNumber_Index(v);
+  PyObject* i = PyNumber_Long(v);
   if (!i) return false;
   *out = static_cast<int>(PyLong_AsUnsignedLongLongMask(i));
   Py_DECREF(i);
