@@ -87,15 +87,15 @@ fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdP
     const int r = i / (D / 4);
     sm.q[r][i % (D / 4)] = (row0 + r < p.Sq) ? reinterpret_cast<const uint32_t*>(q + (static_cast<int64_t>(bh) * p.Sq + row0) * D)[i] : 0u;
   }
-  auto has_key = [&](int t) -> bool {
+  auto mask_word = [&](int t) -> uint32_t {
     const int key = t * kTile + 4 * lane;
-    const uint32_t m4 = key < p.S ? mask4[key >> 2] : 0xFFFFFFFFu;
-    return __any_sync(0xFFFFFFFFu, __vcmpeq4(m4, 0u) != 0u);                // a mask byte that is zero
+    return key < p.S ? mask4[key >> 2] : 0xFFFFFFFFu;
   };
+  auto has_key = [&](uint32_t m4) -> bool { return __any_sync(0xFFFFFFFFu, __vcmpeq4(m4, 0u) != 0u); };      // a mask byte that is zero
   if (n_tiles <= 2 * W) {
 #pragma unroll 1
     for (int t = warp; t < n_tiles; t += W)
-      if (has_key(t) && lane == 0) atomicOr(&sm.live_bits[0], 1u << t);
+      if (has_key(mask_word(t)) && lane == 0) atomicOr(&sm.live_bits[0], 1u << t);
   } else {
     // A warp takes a run of tiles inside one 32-bit word of the list, with eight loads in flight: one tile after the other,
     // which is what a CTA would wait for before its first copy, took 6 us of the call above.
@@ -103,9 +103,15 @@ fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdP
     for (int t0 = warp * run; t0 < n_tiles; t0 += W * run) {
       const int t1 = min(t0 + run, n_tiles);
       uint32_t bits = 0u;
-#pragma unroll 8
-      for (int t = t0; t < t1; ++t)
-        if (has_key(t)) bits |= 1u << (t & 31);
+#pragma unroll 1
+      for (int t = t0; t < t1; t += 8) {
+        uint32_t m4[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m4[i] = mask_word(t + i);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (has_key(m4[i]) && t + i < t1) bits |= 1u << ((t + i) & 31);
+      }
       if (lane == 0) atomicOr(&sm.live_bits[t0 >> 5], bits);
     }
   }

@@ -121,7 +121,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       // Policy launch: the row's maximum over ALL keys and its exp-sum come from the statistics launch; one scale per
       // row for the whole unit (fmha_i8_quant_deviation.py:62-121).
       float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
-      if (out_row >= 0) st = p.row_stats_in[out_row];
+      if (out_row >= 0) st = __ldcg(&p.row_stats_in[out_row]);       // (through the L1, 48.1 -> 48.4 us for B4 H16 S1024)
       l_run = st.y;
       const float l_row = st.y > 0.f ? st.y : 1.f;
       // dynamic: P8 = rn(levels * e); static: P8 = min(rn(levels * (e / l) / s_max), levels)
