@@ -9,8 +9,8 @@
 //                         registers the first ones (53 MB over the chip); pass 2 takes those from there and walks the
 //                         others from the last to the first, so that it meets what the L2 still has.
 // Two launches over 65,536-element chunks, which these replace, took 16.5 us for 255,749 elements (four CTAs) and 107 us
-// for 67,108,864; these take 5.5 and 95 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
-// what neither the SMs (50 MB) nor the L2 (44 MB) kept.
+// for 67,108,864; these take 5.5 and 90 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
+// what neither the SMs (50 MB) nor the L2 kept.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -110,7 +110,7 @@ constexpr int kQuantTile = 1024;               // elements per tile: 8 float4 pe
 constexpr int kQuantVec = kQuantTile / 128;
 constexpr int kQuantStages = 7;                // ring of 7 x 4 KB per warp: all of shared memory
 constexpr int kQuantKeep = 4;                  // tiles a warp keeps in registers (128 of them)
-constexpr long long kQuantHoldBytes = 40000000;
+constexpr long long kQuantHoldBytes = 50000000;
 constexpr size_t kQuantGridSmem = static_cast<size_t>(kQuantWarps) * kQuantStages * kQuantTile * sizeof(float);
 
 // What the CTAs of one call exchange, their maxima, lies in the call's own output until the result goes there: nothing is shared with
@@ -144,8 +144,8 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
   __syncthreads();
   volatile int* abort_flag = &s_abort;
   // The L2 is asked to hold on to the stretch that pass 2 meets first and to nothing else: what pass 2 reads or writes is
-  // not used again.  67,108,864 elements: 100.0 us without policies, 96.6 with 20 MB, 94.7 with 35, 95.0 with 50, 95.4
-  // with 70 (the L2 is two halves, and what is read from the other half takes room in both).
+  // not used again.  67,108,864 elements: 94.7 us with nothing held, 91.9 with 40 MB, 89.4 with 49, 89.3 with 52 or 58, 90.1 with
+  // 70 (the L2 is two halves, and what is read from the other half takes room in both); 33,554,432: 45.2, 46.4, 47.1, 47.1, 47.2, 47.6.
   const uint64_t evict_first = l2_evict_first(), evict_last = l2_evict_last();
   const int hold_from = mine - kQuantStages - static_cast<int>(kQuantHoldBytes / (static_cast<long long>(kQuantTile) * 4 * stride));
   auto load = [&](int i, int s, bool first_pass) {
