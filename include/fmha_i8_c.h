@@ -19,6 +19,8 @@
  *             themselves never look at the status words: one failure does not switch the
  *             library off.
  * All device-pointer entry points enqueue on the stream and return without synchronising.
+ * Calls of the same shape give the same bytes every time.  A head's output may differ by 1 in a few elements of a million between
+ * calls with different numbers of heads (slices, batches): the order of fp32 additions follows the division of the work.
  */
 #ifndef FMHA_I8_C_H_
 #define FMHA_I8_C_H_
