@@ -99,19 +99,18 @@ template <int D> size_t qk_smem_bytes() { return 1024 + 2 * kTile * D + sizeof(D
 template <int D> size_t pv_smem_bytes() { return 1024 + kTile * D + kTile * kTile + sizeof(DebugCtl); }
 
 template <typename Set> void set_decode_attributes(Set set) {
-  auto both = [&](auto d, auto r) {
+  auto one = [&](auto d, auto r) {
     constexpr int D = decltype(d)::value, R = decltype(r)::value;
-    set(reinterpret_cast<const void*>(&fmha_decode_kernel<D, R, false>), sizeof(DecodeSmem<D, R>));
-    set(reinterpret_cast<const void*>(&fmha_decode_kernel<D, R, true>), sizeof(DecodeSmem<D, R>));
+    set(reinterpret_cast<const void*>(&fmha_decode_kernel<D, R>), sizeof(DecodeSmem<D, R>));
   };
   auto rows = [&](auto d) {
-    both(d, std::integral_constant<int, 1>());
-    both(d, std::integral_constant<int, 2>());
-    both(d, std::integral_constant<int, 4>());
+    one(d, std::integral_constant<int, 1>());
+    one(d, std::integral_constant<int, 2>());
+    one(d, std::integral_constant<int, 4>());
   };
   rows(std::integral_constant<int, 64>());
   rows(std::integral_constant<int, 128>());
-  both(std::integral_constant<int, 64>(), std::integral_constant<int, 8>());
+  one(std::integral_constant<int, 64>(), std::integral_constant<int, 8>());
 }
 
 int set_kernel_attributes(DeviceInfo* d) {
@@ -266,9 +265,7 @@ int fill_params(FwdParams* p, const float amax[5], int D, unsigned flags = 0u) {
   p->row_scale = reference_row_scale(D);
   p->scale_qk = amax[0] * amax[1] / (127.f * 127.f);
   p->scale_v_out = amax[2] * (1.0f / (amax[3] * (up ? 255.f : 128.f)));
-  p->p_mul = up ? 255.f : -128.f;
-  p->o_sign = up ? 1.f : -1.f;
-  p->p_unsigned = up ? 1u : 0u;
+  p->p_mul = up ? 255.f : 128.f;
   p->amax_out = nullptr;
   p->amax_scale = amax[2] / ((up ? 255.f : 128.f) * 127.f);   // O~/l counts P in 1/128 (1/255) and V in v_amax/127
   p->c2 = static_cast<float>(static_cast<double>(p->row_scale) * static_cast<double>(p->scale_qk) * 1.4426950408889634);
@@ -424,7 +421,7 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
 // length even out, as long as a warp keeps two tiles (B16 H32, 1025..4096 keys, one row, clusters of 1 / 2 / 4 / 8: 60.9 / 55.3 / 59.0 /
 // 80.2 us, the last where the set-up of a CTA outweighs its tiles); where even that leaves SMs idle, down
 // to one tile per warp.
-template <int D, int R, bool kUnsigned>
+template <int D, int R>
 int launch_decode_rows(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const void* q, const void* k, const void* v) {
   constexpr int W = DecodeCfg<D>::kWarps;
   p.q_tiles = (p.Sq + R - 1) / R;
@@ -439,18 +436,18 @@ int launch_decode_rows(cudaStream_t stream, DeviceInfo* dev, FwdParams p, const 
   LaunchHow how;
   how.cluster = static_cast<unsigned>(c);
   how.overlap = true;
-  return launch_kernel(fmha_decode_kernel<D, R, kUnsigned>, dim3(static_cast<unsigned>(units * c)), dim3(DecodeCfg<D>::kThreads),
+  return launch_kernel(fmha_decode_kernel<D, R>, dim3(static_cast<unsigned>(units * c)), dim3(DecodeCfg<D>::kThreads),
                        sizeof(DecodeSmem<D, R>), stream, how, static_cast<const int8_t*>(q), static_cast<const int8_t*>(k),
                        static_cast<const int8_t*>(v), p);
 }
 template <int D>
 int launch_decode(cudaStream_t s, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v) {
-  if (p.Sq == 1) return p.p_unsigned ? launch_decode_rows<D, 1, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 1, false>(s, dev, p, q, k, v);
-  if (p.Sq == 2) return p.p_unsigned ? launch_decode_rows<D, 2, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 2, false>(s, dev, p, q, k, v);
+  if (p.Sq == 1) return launch_decode_rows<D, 1>(s, dev, p, q, k, v);
+  if (p.Sq == 2) return launch_decode_rows<D, 2>(s, dev, p, q, k, v);
   if constexpr (D == 64) {
-    if (p.Sq > 4) return p.p_unsigned ? launch_decode_rows<D, 8, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 8, false>(s, dev, p, q, k, v);
+    if (p.Sq > 4) return launch_decode_rows<D, 8>(s, dev, p, q, k, v);
   }
-  return p.p_unsigned ? launch_decode_rows<D, 4, true>(s, dev, p, q, k, v) : launch_decode_rows<D, 4, false>(s, dev, p, q, k, v);
+  return launch_decode_rows<D, 4>(s, dev, p, q, k, v);
 }
 
 // What a launch of the forward kernels is beside the plain forward pass into o.  (Calibration comes as infer_x_impl's `calib`: the
@@ -507,8 +504,6 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
       p.p_row_mul = levels;
       p.p_static_mul = (mode->policy == FMHA_I8_POLICY_STATIC) ? levels / amax[4] : 0.f;
       p.p_mul = levels;
-      p.o_sign = 1.f;
-      p.p_unsigned = 1u;
       p.scale_v_out = (mode->policy == FMHA_I8_POLICY_STATIC) ? amax[4] * amax[2] / (levels * amax[3]) : amax[2] / (levels * amax[3]);
     }
   }
@@ -932,9 +927,9 @@ int fmha_i8_sm100_debug_simt_x(void* stream, const float amax[5], const int desc
   const int8_t* m8 = static_cast<const int8_t*>(mask);
   int8_t* o8 = static_cast<int8_t*>(o);
   if (sh.D == 128)
-    simt_check_kernel<128><<<grid, 128, 0, s>>>(q8, k8, v8, m8, o8, sh.Sq, sh.Sk, sh.H, 0, p.row_scale, p.scale_qk, p.scale_v_out, p.p_mul, p.o_sign);
+    simt_check_kernel<128><<<grid, 128, 0, s>>>(q8, k8, v8, m8, o8, sh.Sq, sh.Sk, sh.H, 0, p.row_scale, p.scale_qk, p.scale_v_out, p.p_mul);
   else
-    simt_check_kernel<64><<<grid, 128, 0, s>>>(q8, k8, v8, m8, o8, sh.Sq, sh.Sk, sh.H, 0, p.row_scale, p.scale_qk, p.scale_v_out, p.p_mul, p.o_sign);
+    simt_check_kernel<64><<<grid, 128, 0, s>>>(q8, k8, v8, m8, o8, sh.Sq, sh.Sk, sh.H, 0, p.row_scale, p.scale_qk, p.scale_v_out, p.p_mul);
   g_launch_count.fetch_add(1, std::memory_order_relaxed);
   return finish(cudaGetLastError() == cudaSuccess ? FMHA_I8_OK : FMHA_I8_ERR_LAUNCH);
 }

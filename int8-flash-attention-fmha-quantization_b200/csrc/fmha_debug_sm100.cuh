@@ -214,7 +214,7 @@ template <int D>
 __global__ void __launch_bounds__(128)
 simt_check_kernel(const int8_t* __restrict__ q, const int8_t* __restrict__ k, const int8_t* __restrict__ v,
                   const int8_t* __restrict__ mask, int8_t* __restrict__ o, int Sq, int S, int H, int bh_begin,
-                  float row_scale, float scale_qk, float scale_v_out, float p_mul, float o_sign) {
+                  float row_scale, float scale_qk, float scale_v_out, float p_mul) {
   __shared__ __align__(16) int8_t ks[kTile * D];
   __shared__ __align__(16) int8_t vs[kTile * D];
   __shared__ int8_t ms[kTile];
@@ -278,7 +278,7 @@ simt_check_kernel(const int8_t* __restrict__ q, const int8_t* __restrict__ k, co
       const float sf = __fmul_rn(__fmul_rn(row_scale, static_cast<float>(s_loc[c])), scale_qk);
       const float pe = (ms[c] != 0) ? 0.f : expf(__fsub_rn(sf, m_t));
       l_t = __fadd_rn(l_t, pe);
-      const int p8 = __float2int_rn(fmaxf(fminf(__fmul_rn(p_mul, pe), fmaxf(p_mul, 0.f)), fminf(p_mul, 0.f)));   // -rn(128 p) or rn(255 p)
+      const int p8 = __float2int_rn(fminf(__fmul_rn(p_mul, pe), p_mul));   // rn(128 p) or rn(255 p)
       if (p8 != 0) {
         const int8_t* vr = vs + c * D;
 #pragma unroll
@@ -293,7 +293,7 @@ simt_check_kernel(const int8_t* __restrict__ q, const int8_t* __restrict__ k, co
     const float a = __fmul_rn(l_run, e_old);
 #pragma unroll
     for (int i = 0; i < D; ++i)
-      oacc[i] = __fmul_rn(rcp, __fadd_rn(__fmul_rn(a, oacc[i]), __fmul_rn(e_cur, __fmul_rn(o_sign, static_cast<float>(ot[i])))));
+      oacc[i] = __fmul_rn(rcp, __fadd_rn(__fmul_rn(a, oacc[i]), __fmul_rn(e_cur, static_cast<float>(ot[i]))));
     l_run = l_new;
     m_run = m_new;
   }

@@ -44,16 +44,15 @@ template <int D, int R> struct DecodeSmem {
   int n_live, abort;
 };
 
-template <bool kUnsigned>
+// acc + the dot product of four unsigned bytes with four signed ones
 __device__ __forceinline__ int dot4(uint32_t p, uint32_t v, int acc) {
   int d;
-  if (kUnsigned) asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(p), "r"(v), "r"(acc));
-  else asm("dp4a.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(p), "r"(v), "r"(acc));
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(p), "r"(v), "r"(acc));
   return d;
 }
 
 // grid = (clusters of c CTAs) x (bh_count * row groups); R = query rows per group (rows past Sq are computed and dropped).
-template <int D, int R, bool kUnsigned>
+template <int D, int R>
 __global__ void __launch_bounds__(DecodeCfg<D>::kThreads, 3)
 fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdParams p) {
   using Cfg = DecodeCfg<D>;
@@ -255,10 +254,10 @@ fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdP
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const uint32_t pr = h == 0 ? pw[r].x : h == 1 ? pw[r].y : h == 2 ? pw[r].z : pw[r].w;
-          acc[r][0] = dot4<kUnsigned>(pr, w0, acc[r][0]);
-          acc[r][1] = dot4<kUnsigned>(pr, w1, acc[r][1]);
-          acc[r][2] = dot4<kUnsigned>(pr, w2, acc[r][2]);
-          acc[r][3] = dot4<kUnsigned>(pr, w3, acc[r][3]);
+          acc[r][0] = dot4(pr, w0, acc[r][0]);
+          acc[r][1] = dot4(pr, w1, acc[r][1]);
+          acc[r][2] = dot4(pr, w2, acc[r][2]);
+          acc[r][3] = dot4(pr, w3, acc[r][3]);
         }
       }
     }
@@ -267,7 +266,7 @@ fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdP
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) o[r][c] = fmaf(o[r][c], e_old[r], e_cur[r] * (p.o_sign * static_cast<float>(acc[r][c])));
+      for (int c = 0; c < 4; ++c) o[r][c] = fmaf(o[r][c], e_old[r], e_cur[r] * static_cast<float>(acc[r][c]));
   }
   if (!ok) {
     if (lane == 0) {

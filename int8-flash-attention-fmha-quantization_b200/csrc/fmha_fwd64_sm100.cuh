@@ -185,8 +185,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
         m_run = m_new;
       }
       if (stats_only) continue;                                        // no output is wanted: there is no P.V
-      const float es = p.o_sign * e_cur;                               // the accumulator holds o_sign * (P.V)
-      const float2 neg_ec = make_float2(es, es), e_bias = make_float2(-es * kMagic, -es * kMagic);
+      const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
       const float2 e_old2 = make_float2(e_old, e_old);
 
       // ---- P.V of this step into the running row (inc/fmha_i8.cuh:306-310)
@@ -198,16 +197,16 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       tmem_ld16_issue(tS + kOCol, ra);
       tmem_ld16_issue(tS + kOCol + 16, rb);
       tmem_ld_fence(ra); tmem_ld_fence(rb);
-      drain_chunk<16>(ra, o2, neg_ec, e_bias, e_old2);
+      drain_chunk<16>(ra, o2, e_cur2, e_bias, e_old2);
       tmem_ld16_issue(tS + kOCol + 32, ra);
-      drain_chunk<16>(rb, o2 + 8, neg_ec, e_bias, e_old2);
+      drain_chunk<16>(rb, o2 + 8, e_cur2, e_bias, e_old2);
       tmem_ld16_issue(tS + kOCol + 48, rb);
       tmem_ld_fence(ra); tmem_ld_fence(rb);
       // the last columns are in registers: the driver may go on with the next S
       tc_fence_before();
       mbar_arrive(smem_u32(&ctl->s_free));
-      drain_chunk<16>(ra, o2 + 16, neg_ec, e_bias, e_old2);
-      drain_chunk<16>(rb, o2 + 24, neg_ec, e_bias, e_old2);
+      drain_chunk<16>(ra, o2 + 16, e_cur2, e_bias, e_old2);
+      drain_chunk<16>(rb, o2 + 24, e_cur2, e_bias, e_old2);
     }
 
     // ---- the unit is finished
@@ -278,7 +277,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   const uint32_t k_smem = worker_smem, v_smem = worker_smem + kTileBytes, q_smem = worker_smem + 2 * kTileBytes;
   constexpr uint32_t idesc_s = make_idesc_i8(kTile, false);       // S = Q.K^T : N = 128 keys, both K-major
   constexpr uint32_t idesc_preset_s = make_idesc_bf16(kTile), idesc_preset_o = make_idesc_bf16(kD);
-  const uint32_t idesc_o = p.p_unsigned ? make_idesc_i8(kD, true, true) : make_idesc_i8(kD, true, false);     // P.V : V is an MN-major operand
+  constexpr uint32_t idesc_o = make_idesc_i8(kD, true, true);     // P.V : P unsigned, V an MN-major operand
   const uint32_t preset_smem = smem_u32(presets);
   const uint64_t d_a = preset_desc(preset_smem, 0), d_b = preset_desc(preset_smem, 1);
   const uint64_t dq = make_smem_desc(q_smem, kD), dk = make_smem_desc(k_smem, kD), dv = make_smem_desc(v_smem, kD);

@@ -188,10 +188,9 @@ struct FwdParams {
   float scale_qk;       // q_amax*k_amax/127^2 (inc/fmha_i8.cuh:72)
   float scale_v_out;    // v_amax/(o_amax*128) (inc/fmha_i8.cuh:318)
   float c2;             // row_scale*scale_qk*log2(e)
-  float p_mul;          // -128: P8 = -rn(128 p) signed, the reference's quantisation (inc/fmha_i8.cuh:241-250);
-                        // +255: P8 = rn(255 p) unsigned (the reference README's planned UINT8 x INT8 variant)
-  float o_sign;         // -1 when the accumulator holds -(P.V) (signed P), +1 when it holds +(P.V)
-  unsigned p_unsigned;  // 1 = the tensor core reads P as unsigned bytes
+  float p_mul;          // 128: P8 = rn(128 p), the reference's quantisation (inc/fmha_i8.cuh:241-250, which keeps -rn(128 p) in a
+                        // signed byte); 255: P8 = rn(255 p) (the reference README's planned UINT8 x INT8 variant).  P8 is an unsigned
+                        // byte in all kernels.
   float* amax_out;      // calibration mode when not null: nothing is stored to o; instead the largest |output|
                         // in real units, max |O~ / l| * amax_scale, is folded into this device float
   float amax_scale;     // v_amax / (127 * 128)  (127 * 255 with unsigned P)
@@ -358,7 +357,11 @@ __device__ __forceinline__ float2 exp2_poly(float2 a) {
 }
 
 // N scores -> N probabilities (summed into two independent packed accumulators) -> N/4 words of
-// packed bytes holding -rn(128 p) (or rn(255 p)).  x = raw accumulator read as float = kMagic + s.
+// packed bytes holding rn(128 p) (or rn(255 p)).  x = raw accumulator read as float = kMagic + s.
+// A word's bytes are put together in pairs by the arithmetic that rounds them: kMagic + n1, times 256 and less 255 kMagic, is
+// kMagic + 256 n1, all exact, and adding 128 p0 to that rounds to kMagic + 256 n1 + n0, where 128 p0 alone would round (256 n1 is
+// even).  The two low bytes are the pair, as long as no byte is negative.  One byte permutation then makes a word of two pairs:
+// four instructions per word against two multiply-adds and three permutations, which run at half rate.
 // kCap: p is limited to p_cap before it is quantised (the static policy clips at its top level, fmha_i8_quant_deviation.py:38-43).
 // kPolyPairs: that many pairs of values per eight are computed by exp2_poly.
 template <int N, bool kCap = false, int kPolyPairs = 0>
@@ -377,12 +380,12 @@ __device__ __forceinline__ void chunk_exp_pack(const uint32_t (&r)[N], const flo
       p01.x = fminf(p01.x, p_cap); p01.y = fminf(p01.y, p_cap);
       p23.x = fminf(p23.x, p_cap); p23.y = fminf(p23.y, p_cap);
     }
-    sum[0] = __fadd2_rn(sum[0], p01);
-    sum[1] = __fadd2_rn(sum[1], p23);
-    const float2 y01 = __ffma2_rn(p01, p_mul_f, magic2);      // low byte = the two's-complement P8
-    const float2 y23 = __ffma2_rn(p23, p_mul_f, magic2);
-    packed[g] = __byte_perm(__byte_perm(__float_as_uint(y01.x), __float_as_uint(y01.y), 0x0040),
-                            __byte_perm(__float_as_uint(y23.x), __float_as_uint(y23.y), 0x0040), 0x5410);
+    const float2 even = make_float2(p01.x, p23.x), odd = make_float2(p01.y, p23.y);
+    sum[0] = __fadd2_rn(sum[0], even);
+    sum[1] = __fadd2_rn(sum[1], odd);
+    const float2 high = __ffma2_rn(__ffma2_rn(odd, p_mul_f, magic2), make_float2(256.f, 256.f), make_float2(-255.f * kMagic, -255.f * kMagic));
+    const float2 y = __ffma2_rn(even, p_mul_f, high);
+    packed[g] = __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x5410);
   }
 }
 
@@ -402,7 +405,7 @@ __device__ __forceinline__ RowConsts row_consts(const int imax, const float c2s,
   k.f = fmaf(-lo, 0.6931471805599453f, 1.0f);
   k.c2 = make_float2(c2s, c2s);
   k.neg_hi = make_float2(-hi, -hi);
-  k.p_mul_f = make_float2(p_mul * k.f, p_mul * k.f);        // -128 f (or +255 f): quantisation multiplier
+  k.p_mul_f = make_float2(p_mul * k.f, p_mul * k.f);        // 128 f (or 255 f): quantisation multiplier
   // the value the reference computes for the maximal element (inc/fmha_i8.cuh:196)
   k.m_tile = (row_scale * static_cast<float>(imax - static_cast<int>(kMagicBits))) * scale_qk;
   return k;
@@ -437,11 +440,11 @@ __device__ __forceinline__ void requantise16(const float2* o2, const float2 scal
 // o2 = e_old * o2 + e_cur * (P8 . V) for N output columns.  r = accumulator, preset by the bias MMA, so that it reads as the float
 // kMagic + (P8 . V).
 template <int N>
-__device__ __forceinline__ void drain_chunk(const uint32_t (&r)[N], float2* o2, const float2 neg_ec, const float2 e_bias, const float2 e_old) {
+__device__ __forceinline__ void drain_chunk(const uint32_t (&r)[N], float2* o2, const float2 e_cur, const float2 e_bias, const float2 e_old) {
 #pragma unroll
   for (int i = 0; i < N / 2; ++i) {
     const float2 x = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-    const float2 t = __ffma2_rn(x, neg_ec, e_bias);          // e_cur * (P8 . V), exact product before rounding
+    const float2 t = __ffma2_rn(x, e_cur, e_bias);          // e_cur * (P8 . V), exact product before rounding
     o2[i] = __ffma2_rn(o2[i], e_old, t);
   }
 }
@@ -665,8 +668,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
         m_run = m_new;
         imax_run = max(imax_run, ctl->st_i[slot][row]);
       }
-      const float es = p.o_sign * e_cur;                               // the accumulator holds o_sign * (P.V)
-      const float2 neg_ec = make_float2(es, es), e_bias = make_float2(-es * kMagic, -es * kMagic);
+      const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
       const float2 e_old2 = make_float2(e_old, e_old);
 
       // ---- drain my half of O~ = bias -/+ (P8 . V) into the fp32 running row.  The partial output of step g lives in
@@ -692,9 +694,9 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
             tc_fence_before();
             mbar_arrive(smem_u32(&ctl->s_free[sb]));
           }
-          drain_chunk<16>(ra, o2 + c * 8, neg_ec, e_bias, e_old2);
+          drain_chunk<16>(ra, o2 + c * 8, e_cur2, e_bias, e_old2);
           if (c + 2 < DH / 16) tmem_ld16_issue(chunk_col(c + 2), ra);
-          drain_chunk<16>(rb, o2 + (c + 1) * 8, neg_ec, e_bias, e_old2);
+          drain_chunk<16>(rb, o2 + (c + 1) * 8, e_cur2, e_bias, e_old2);
           if (c + 3 < DH / 16) tmem_ld16_issue(chunk_col(c + 3), rb);
         }
       } else {
@@ -981,7 +983,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   constexpr uint32_t NV = Cfg::kStagesV;
   volatile int* abort_flag = &ctl->abort;
   // O = P.V : V is an MN-major operand; one group of MMAs with N = head_dim output columns
-  const uint32_t idesc_o = p.p_unsigned ? make_idesc_i8(D, true, true) : make_idesc_i8(D, true, false);
+  constexpr uint32_t idesc_o = make_idesc_i8(D, true, true);
   constexpr uint32_t idesc_bias = make_idesc_bf16(D);
   const uint64_t d_bias_a = make_smem_desc_noswizzle(bias_a_smem, 128, 256);
   const uint64_t d_bias_b = make_smem_desc_noswizzle(bias_b_smem, 128, 256);
