@@ -128,7 +128,8 @@ int set_kernel_attributes(DeviceInfo* d) {
   set_decode_attributes(set);
   set(reinterpret_cast<const void*>(&w64::fwd_kernel<false>), w64::kSmemBytes);
   set(reinterpret_cast<const void*>(&w64::fwd_kernel<true>), w64::kSmemBytes);
-  set(reinterpret_cast<const void*>(&quant_grid_kernel), kQuantGridSmem);
+  set(reinterpret_cast<const void*>(&quant_grid_kernel<false>), kQuantGridSmem);
+  set(reinterpret_cast<const void*>(&quant_grid_kernel<true>), kQuantGridSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&quant_cluster_kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   set(reinterpret_cast<const void*>(&debug_qk_kernel<64>), qk_smem_bytes<64>());
   set(reinterpret_cast<const void*>(&debug_qk_kernel<128>), qk_smem_bytes<128>());
@@ -649,8 +650,9 @@ int launch_quantize(cudaStream_t stream, DeviceInfo* dev, const float* x, long l
   how.cooperative = true;
   const long long wanted = (n / kQuantTile + kQuantWarps - 1) / kQuantWarps;
   const int most = dev->sm_count < kQuantMaxCtas ? dev->sm_count : kQuantMaxCtas;
-  return launch_kernel(quant_grid_kernel, dim3(static_cast<unsigned>(wanted < most ? wanted : most)), dim3(kQuantThreads), kQuantGridSmem,
-                       stream, how, x, n, out, amax_out, dev->status);
+  const int ctas = static_cast<int>(wanted < most ? wanted : most);
+  auto* kernel = quant_needs_tmem(n, ctas) ? quant_grid_kernel<true> : quant_grid_kernel<false>;
+  return launch_kernel(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kQuantThreads), kQuantGridSmem, stream, how, x, n, out, amax_out, dev->status);
 }
 
 int quantize_impl(void* stream, const float* x, long long n, int8_t* out, float* amax_out, bool whole_chip = false) {

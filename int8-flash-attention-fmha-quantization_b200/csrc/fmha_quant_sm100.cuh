@@ -5,12 +5,11 @@
 //   quant_cluster_kernel  up to 524,288 elements: one cluster of 1..16 CTAs holds the whole tensor in registers, the
 //                         CTAs exchange their maxima through distributed shared memory.  5 bytes moved per element.
 //   quant_grid_kernel     larger: one CTA per SM (cooperative launch), every warp streams its tiles through a private
-//                         ring of bulk copies.  At the end of pass 1 the ring still holds each warp's last tiles and its
-//                         registers the first ones (53 MB over the chip); pass 2 takes those from there and walks the
-//                         others from the last to the first, so that it meets what the L2 still has.
-// Two launches over 65,536-element chunks, which these replace, took 16.5 us for 255,749 elements (four CTAs) and 107 us
-// for 67,108,864; these take 5.5 and 90 us.  The large case is bound by DRAM: pass 1 reads all 268 MB from there, pass 2
-// what neither the SMs (50 MB) nor the L2 kept.
+//                         ring of bulk copies.  At the end of pass 1 the ring still holds each warp's last tiles, its
+//                         registers the first ones and its part of tensor memory the next (92 MB over the chip); pass 2
+//                         takes those from there and reads the others again, as far as it can from the L2.
+// 255,749 elements take 4.2 us, 67,108,864 take 78.4: DRAM, since pass 1 reads all 268 MB from there and pass 2 what neither the SMs
+// (92 MB) nor the L2 (50) kept.  Without tensor memory the latter take 84.2 us, and 33,554,432 elements 37.7 instead of 35.6.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -21,13 +20,30 @@
 
 namespace fmha {
 
-__device__ __forceinline__ float abs_max4(float m, const float4& v) {
-  return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-}
+__device__ __forceinline__ float abs_max4(float m, const float4& v) { return max3_abs(max3_abs(m, v.x, v.y), v.z, v.w); }
 __device__ __forceinline__ int quant_one(float v, float scale) {
   // float_quant2_int8: floorf(x*scale + 0.5) with the sum rounded once to float, clamp to +-127
   const float f = floorf(__fadd_rn(__fmul_rn(v, scale), 0.5f));
   return static_cast<int>(fminf(fmaxf(f, -127.f), 127.f));
+}
+// The same for N float4, a word of bytes each.  floorf and the conversion to an integer are instructions of the unit that also
+// has the exponentials, 16 lanes a cycle on an SM; with them it, not memory, was what quantising waited for (67,108,864 elements: 29
+// us of that unit; 89.5 -> 84.2 us in all, 33,554,432 elements 47.2 -> 37.7, 255,749 5.6 -> 4.2).  Here the floor comes from an addition to 1.5 * 2^23 that
+// rounds down.  That needs x*scale + 0.5 to be a number in [-127, 128), which it is unless x is not a number or the scale is not
+// finite: false is returned if it may not be, and the words are then quant_one's to make.
+template <int N>
+__device__ __forceinline__ bool quant_words(const float4 (&v)[N], float scale, uint32_t (&words)[N]) {
+  const float2 s2 = make_float2(scale, scale), half = make_float2(0.5f, 0.5f), magic = make_float2(kMagic, kMagic);
+  float most = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float2 y01 = __fadd2_rn(__fmul2_rn(make_float2(v[i].x, v[i].y), s2), half), y23 = __fadd2_rn(__fmul2_rn(make_float2(v[i].z, v[i].w), s2), half);
+    most = max3_abs_nan(max3_abs_nan(most, y01.x, y01.y), y23.x, y23.y);
+    const float2 n01 = __fadd2_rd(y01, magic), n23 = __fadd2_rd(y23, magic);
+    words[i] = __byte_perm(__byte_perm(__float_as_uint(n01.x), __float_as_uint(n01.y), 0x0040),
+                           __byte_perm(__float_as_uint(n23.x), __float_as_uint(n23.y), 0x0040), 0x5410);
+  }
+  return most < 127.75f;
 }
 __device__ __forceinline__ uint32_t quant_four(const float4& v, float scale) {
   return (static_cast<uint32_t>(quant_one(v.x, scale)) & 0xFFu) | ((static_cast<uint32_t>(quant_one(v.y, scale)) & 0xFFu) << 8) |
@@ -95,10 +111,15 @@ quant_cluster_kernel(const float* x, int n, int8_t* out, float* amax_out) {
   if (rank == 0 && threadIdx.x == 0 && amax_out) *amax_out = amax;
   const float scale = quant_scale(amax);
   uint32_t* o4 = reinterpret_cast<uint32_t*>(out);
+  uint32_t words[kQuantClusterVec];
+  if (!quant_words(v, scale, words)) {
+#pragma unroll
+    for (int k = 0; k < kQuantClusterVec; ++k) words[k] = quant_four(v[k], scale);
+  }
 #pragma unroll
   for (int k = 0; k < kQuantClusterVec; ++k) {
     const int i = begin + k * kQuantClusterThreads + static_cast<int>(threadIdx.x);
-    if (i < end) o4[i] = quant_four(v[k], scale);
+    if (i < end) o4[i] = words[k];
   }
   if (has_tail) out[tail] = static_cast<int8_t>(quant_one(t, scale));
 }
@@ -109,7 +130,10 @@ constexpr int kQuantWarps = kQuantThreads / 32;
 constexpr int kQuantTile = 1024;               // elements per tile: 8 float4 per lane
 constexpr int kQuantVec = kQuantTile / 128;
 constexpr int kQuantStages = 7;                // ring of 7 x 4 KB per warp: all of shared memory
-constexpr int kQuantKeep = 4;                  // tiles a warp keeps in registers (128 of them)
+constexpr int kQuantKeep = 4;                  // tiles a warp keeps in registers (128 of them): its first
+constexpr int kQuantTmem = 8;                  // tiles a warp keeps in tensor memory, 32 columns each: the next
+constexpr uint32_t kQuantTmemCols = 32 * kQuantTmem * kQuantWarps / 4;      // two warps to a lane quarter
+static_assert(kQuantTmemCols <= 512, "tensor memory has 512 columns");
 constexpr long long kQuantHoldBytes = 50000000;
 constexpr size_t kQuantGridSmem = static_cast<size_t>(kQuantWarps) * kQuantStages * kQuantTile * sizeof(float);
 
@@ -119,12 +143,16 @@ constexpr size_t kQuantGridSmem = static_cast<size_t>(kQuantWarps) * kQuantStage
 constexpr int kQuantMaxCtas = kQuantTile / 4;  // the list fits into a tile of output
 static_assert(kQuantMaxCtas <= kQuantThreads, "one thread per entry");
 
+// kTmem: some warp has more tiles than its registers and its ring hold (quant_needs_tmem).
+inline bool quant_needs_tmem(long long n, int ctas) { return n / kQuantTile > static_cast<long long>(kQuantKeep + kQuantStages) * kQuantWarps * ctas; }
+template <bool kTmem>
 __global__ void __launch_bounds__(kQuantThreads, 1)
 quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__ out, float* __restrict__ amax_out, unsigned* __restrict__ status) {
   extern __shared__ __align__(128) uint8_t ring_raw[];
   __shared__ uint64_t bars[kQuantWarps][kQuantStages];
   __shared__ float warp_max[kQuantWarps];
   __shared__ int s_abort;
+  __shared__ uint32_t s_tmem;
   const int lane = threadIdx.x & 31, warp = warp_index();
   float* ring = reinterpret_cast<float*>(ring_raw) + warp * (kQuantStages * kQuantTile);
   uint64_t* bar = bars[warp];
@@ -141,18 +169,42 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
     for (int s = 0; s < kQuantStages; ++s) mbar_init(smem_u32(&bar[s]), 1);
     mbar_init_fence();
   }
-  __syncthreads();
-  volatile int* abort_flag = &s_abort;
-  // The L2 is asked to hold on to the stretch that pass 2 meets first and to nothing else: what pass 2 reads or writes is
-  // not used again.  67,108,864 elements: 94.7 us with nothing held, 91.9 with 40 MB, 89.4 with 49, 89.3 with 52 or 58, 90.1 with
-  // 70 (the L2 is two halves, and what is read from the other half takes room in both); 33,554,432: 45.2, 46.4, 47.1, 47.1, 47.2, 47.6.
+  // The L2 is asked to hold on to the last of the tiles that are read again and to nothing else: what pass 2 reads or writes is
+  // not used again.  67,108,864 elements: 79.5 us with 30 MB held, 78.9 with 45, 78.4 with 50, 78.0 with 58 or 64 (the L2 is two halves,
+  // and what is read from the other half takes room in both); 33,554,432: 34.7, 35.4, 35.6, 35.6, 35.6.  Tiles for pass 2 asked into the
+  // L2 before the grid's barrier: 2 a warp 78.0 and 35.9, 8 a warp 80.7 and 36.2.
   const uint64_t evict_first = l2_evict_first(), evict_last = l2_evict_last();
-  const int hold_from = mine - kQuantStages - static_cast<int>(kQuantHoldBytes / (static_cast<long long>(kQuantTile) * 4 * stride));
+  // Pass 2 finds tiles [still_there, mine) in the ring, the first on_chip in registers and tensor memory, and reads the others
+  // again: those from `held` on from the L2, those below from DRAM.
+  const int on_chip = min(mine, kTmem ? kQuantKeep + kQuantTmem : kQuantKeep), still_there = max(mine - kQuantStages, on_chip);
+  const int hold = static_cast<int>(kQuantHoldBytes / (static_cast<long long>(kQuantTile) * 4 * stride));
+  const int held = max(still_there - hold, on_chip);
   auto load = [&](int i, int s, bool first_pass) {
     mbar_arrive_expect_tx(smem_u32(&bar[s]), kQuantTile * sizeof(float));
     bulk_load(smem_u32(ring + s * kQuantTile), x + tile_at(i), kQuantTile * sizeof(float), smem_u32(&bar[s]),
-              first_pass && i >= hold_from ? evict_last : evict_first);
+              first_pass && i >= held && i < still_there ? evict_last : evict_first);
   };
+  if (lane == 0)
+    for (int i = 0; i < kQuantStages && i < mine; ++i) load(i, i, true);
+  if (kTmem && warp == 0) {
+    __syncwarp();
+    tmem_alloc(smem_u32(&s_tmem), kQuantTmemCols);
+    tmem_relinquish();
+  }
+  if (kTmem) tc_fence_before();
+  __syncthreads();
+  if (kTmem) tc_fence_after();
+  const uint32_t tmem_base = kTmem ? *reinterpret_cast<volatile uint32_t*>(&s_tmem) : 0u;
+  const uint32_t my_tmem = tmem_base + (static_cast<uint32_t>(warp & 3) << 21) + static_cast<uint32_t>((warp >> 2) * 32 * kQuantTmem);
+  // What is left behind the last whole tile is the last CTA's, asked for here: after the tiles its latency would be seen (600,001
+  // elements 8.3 -> 6.2 us).
+  constexpr int kQuantRest = kQuantTile / kQuantThreads;
+  const long long rest_end = blockIdx.x == gridDim.x - 1 ? n : 0;
+  auto rest_at = [&](int k) { return static_cast<long long>(n_tiles) * kQuantTile + k * kQuantThreads + static_cast<int>(threadIdx.x); };
+  float rest[kQuantRest];
+#pragma unroll
+  for (int k = 0; k < kQuantRest; ++k) rest[k] = rest_at(k) < rest_end ? x[rest_at(k)] : 0.f;
+  volatile int* abort_flag = &s_abort;
   bool ok = true;
   uint32_t parity_bits = 0u;                   // bit s: parity of the next completion of ring slot s
   auto landed = [&](int s) {
@@ -162,8 +214,6 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
   };
 
   // ---- pass 1: the largest magnitude
-  if (lane == 0)
-    for (int i = 0; i < kQuantStages && i < mine; ++i) load(i, i, true);
   float m = 0.f;
   float4 keep[kQuantKeep][kQuantVec];
 #pragma unroll
@@ -181,19 +231,31 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
       if (lane == 0 && i + kQuantStages < mine) load(i + kQuantStages, i, true);
     }
   }
-  for (int i = kQuantKeep, s = kQuantKeep; i < mine; ++i) {
-    const float4* t = landed(s);
+  int slot = kQuantKeep;
+  auto next_slot = [&]() { if (++slot == kQuantStages) slot = 0; };
+#pragma unroll 1
+  for (int i = kQuantKeep; kTmem && i < on_chip; ++i, next_slot()) {
+    const float4* t = landed(slot);
+    float4 v[kQuantVec];
+#pragma unroll
+    for (int k = 0; k < kQuantVec; ++k) {
+      v[k] = t[lane + 32 * k];
+      m = abs_max4(m, v[k]);
+    }
+    tmem_st_tile(my_tmem + static_cast<uint32_t>((i - kQuantKeep) * 32), v);
+    __syncwarp();
+    if (lane == 0 && i + kQuantStages < mine) load(i + kQuantStages, slot, true);
+  }
+  for (int i = max(on_chip, kQuantKeep); i < mine; ++i, next_slot()) {
+    const float4* t = landed(slot);
 #pragma unroll
     for (int k = 0; k < kQuantVec; ++k) m = abs_max4(m, t[lane + 32 * k]);
     __syncwarp();
-    if (lane == 0 && i + kQuantStages < mine) load(i + kQuantStages, s, true);
-    if (++s == kQuantStages) s = 0;
+    if (lane == 0 && i + kQuantStages < mine) load(i + kQuantStages, slot, true);
   }
-  // what is left behind the last whole tile: the last CTA reads it, twice
-  const long long rest = static_cast<long long>(n_tiles) * kQuantTile;
-  const bool has_rest = blockIdx.x == gridDim.x - 1;
-  if (has_rest)
-    for (long long i = rest + threadIdx.x; i < n; i += kQuantThreads) m = fmaxf(m, fabsf(x[i]));
+  if (kTmem) tmem_wait_st();
+#pragma unroll
+  for (int k = 0; k < kQuantRest; ++k) m = fmaxf(m, fabsf(rest[k]));
 
   // ---- the largest of all CTAs.  The grid's barrier is the one of the cooperative launch, whose CTAs are all resident and all come
   // here: no wait above is longer than its limit.
@@ -206,35 +268,71 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
   if (blockIdx.x == 0 && t == 0 && amax_out) *amax_out = amax;
   const float scale = quant_scale(amax);
 
-  // ---- pass 2: quantise, from the last tile to the first
-  auto store = [&](int i, int k, const float4& v) { __stcs(reinterpret_cast<uint32_t*>(out + tile_at(i)) + lane + 32 * k, quant_four(v, scale)); };
-  auto from_ring = [&](int i, int s, const float4* t) {
+  // ---- pass 2: quantise.  First what the ring holds; every slot that gets free takes one of the tiles that are read again, DRAM's and
+  // the L2's in turn, in proportion to their numbers, so that DRAM is busy from the first to the last.
+  auto store = [&](int i, const float4 (&v)[kQuantVec]) {
+    uint32_t words[kQuantVec];
+    const bool good = quant_words(v, scale, words);
+    uint32_t* to = reinterpret_cast<uint32_t*>(out + tile_at(i)) + lane;
 #pragma unroll
-    for (int k = 0; k < kQuantVec; ++k) store(i, k, t[lane + 32 * k]);
-    __syncwarp();
-    if (lane == 0 && i - kQuantStages >= kQuantKeep) load(i - kQuantStages, s, false);
+    for (int k = 0; k < kQuantVec; ++k) __stcs(to + 32 * k, words[k]);
+    if (!good) {
+      const float4* from = reinterpret_cast<const float4*>(x + tile_at(i)) + lane;
+#pragma unroll 1
+      for (int k = 0; k < kQuantVec; ++k) to[32 * k] = quant_four(from[32 * k], scale);
+    }
   };
-  const int still_there = max(mine - kQuantStages, kQuantKeep);    // tiles [still_there, mine) are still in the ring
-  for (int i = mine - 1; i >= still_there; --i) {
-    const int s = i % kQuantStages;
-    from_ring(i, s, reinterpret_cast<const float4*>(ring + s * kQuantTile));
-  }
+  const int again = still_there - on_chip, from_dram = held - on_chip;
+  int next_l2 = still_there - 1, next_dram = held - 1, asked = 0, turn = again - 1;
+  int in_slot = 0;                             // lane s: the tile that is on its way into ring slot s
+  auto ask = [&](int s) {
+    if (!kTmem || asked == again) return;
+    ++asked;
+    turn += from_dram;
+    const bool dram = turn >= again;
+    if (dram) turn -= again;
+    const int i = dram ? next_dram-- : next_l2--;
+    if (lane == s) in_slot = i;
+    if (lane == 0) load(i, s, false);
+  };
+  auto from_ring = [&](int i, int s, const float4* t) {
+    float4 v[kQuantVec];
+#pragma unroll
+    for (int k = 0; k < kQuantVec; ++k) v[k] = t[lane + 32 * k];
+    __syncwarp();
+    ask(s);
+    store(i, v);
+  };
+  int s = mine > 0 ? (mine - 1) % kQuantStages : 0;
+  auto slot_before = [&]() { s = s == 0 ? kQuantStages - 1 : s - 1; };
+  const int first_again = s;
+  for (int i = mine - 1; i >= still_there; --i, slot_before()) from_ring(i, s, reinterpret_cast<const float4*>(ring + s * kQuantTile));
 #pragma unroll
   for (int i = 0; i < kQuantKeep; ++i)
-    if (i < mine) {
-#pragma unroll
-      for (int k = 0; k < kQuantVec; ++k) store(i, k, keep[i][k]);
-    }
-  for (int i = still_there - 1; i >= kQuantKeep; --i) {
-    const int s = i % kQuantStages;
-    from_ring(i, s, landed(s));
+    if (i < mine) store(i, keep[i]);
+#pragma unroll 1
+  for (int i = kQuantKeep; kTmem && i < on_chip; ++i) {
+    float4 v[kQuantVec];
+    tmem_ld_tile(my_tmem + static_cast<uint32_t>((i - kQuantKeep) * 32), v);
+    store(i, v);
   }
-  if (has_rest)
-    for (long long i = rest + threadIdx.x; i < n; i += kQuantThreads) out[i] = static_cast<int8_t>(quant_one(x[i], scale));
+  s = first_again;
+  for (int i = 0; kTmem && i < again; ++i, slot_before()) from_ring(__shfl_sync(0xFFFFFFFFu, in_slot, s), s, landed(s));
+#pragma unroll
+  for (int k = 0; k < kQuantRest; ++k)
+    if (rest_at(k) < rest_end) out[rest_at(k)] = static_cast<int8_t>(quant_one(rest[k], scale));
   if (!ok && lane == 0) {
     raise_status(abort_flag, status, FMHA_I8_DEV_WAIT_QUANT, blockIdx.x);
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000LL) { /* copies still in flight land before the CTA may exit */ }
+  }
+  if (kTmem) {
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+      tc_fence_after();
+      tmem_dealloc(tmem_base, kQuantTmemCols);
+    }
   }
 }
 

@@ -81,10 +81,12 @@ def torch_cuda():
 
 
 # One cluster of 1, 2, 4, 8 and 16 CTAs; then the whole chip, where a warp has 0, 1, 4 (all kept in registers), 7 and 8 (one
-# ring), 12 tiles of 1024 elements, with and without a remainder.
+# ring), 12 tiles of 1024 elements, with and without a remainder.  Up to 11 tiles a warp holds in registers and its ring; with 12 to 19
+# tensor memory holds eight as well, with 20 and 33 the rest is read again, from the L2 and, beyond what that is asked to hold, from DRAM.
 SWEEP = 148 * 8 * 1024
 @pytest.mark.parametrize("n", [1, 3, 8192, 8193, 32771, 65536, 65537, 262144, 262147, 524288, 524289, SWEEP - 1, SWEEP, 4 * SWEEP + 1,
-                               5 * SWEEP, 7 * SWEEP + 1023, 8 * SWEEP, 12 * SWEEP + 1025])
+                               5 * SWEEP, 7 * SWEEP + 1023, 8 * SWEEP, 12 * SWEEP + 1025, 11 * SWEEP, 11 * SWEEP + 1024, 19 * SWEEP - 1, 20 * SWEEP + 2047,
+                               33 * SWEEP + 5])
 def test_quantize_sizes(pkg, oracle, torch_cuda, n):
     torch = torch_cuda
     x = np.random.default_rng(n).standard_normal(n, dtype=np.float32)
@@ -98,6 +100,35 @@ def test_quantize_sizes(pkg, oracle, torch_cuda, n):
         assert np.float32(amax.item()) == np.abs(y).max()
         assert np.array_equal(host[:n], oracle.quantize(y, np.abs(y).max())), (n, at)
         assert np.all(host[n:] == 0x5A)
+    assert pkg.device_status()[0] == pkg.OK
+
+
+@pytest.mark.parametrize("n", [4099, 524289, 20 * SWEEP + 3])
+@pytest.mark.parametrize("what", ["nan", "inf", "tiny", "huge", "zero"])
+def test_quantize_values_that_are_no_ordinary_numbers(pkg, torch_cuda, n, what):
+    """Elements that are no numbers, scales that are not finite or the largest there are: floor(x * scale + 0.5) limited to +-127 step by
+    step in fp32, a NaN giving -127 (as the minimum and maximum of a number and a NaN are the number)."""
+    torch = torch_cuda
+    x = torch.randn(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    x[n // 3] = -6.5
+    if what == "nan":
+        x[::1237] = float("nan")
+    elif what == "inf":
+        x[n // 2], x[n - 1] = float("inf"), float("-inf")
+    elif what == "tiny":
+        x *= 1e-38                   # the scale is infinite
+        x[::3] = 0.0
+    elif what == "huge":
+        x *= 5e37
+    else:
+        x.zero_()
+    out, amax = torch.zeros(n, dtype=torch.int8, device="cuda"), torch.zeros(1, device="cuda")
+    pkg.quantize_f32(None, x, out, amax)
+    most = torch.nan_to_num(x, nan=0.0, posinf=float("inf"), neginf=float("-inf")).abs().max()
+    scale = torch.tensor(127.0, device="cuda") / most if most > 0 else torch.zeros((), device="cuda")
+    want = torch.nan_to_num(torch.floor(x * scale + 0.5), nan=-127.0, posinf=127.0, neginf=-127.0).clamp(-127, 127).to(torch.int8)
+    assert amax.item() == most.item()
+    assert torch.equal(out, want)
     assert pkg.device_status()[0] == pkg.OK
 
 
