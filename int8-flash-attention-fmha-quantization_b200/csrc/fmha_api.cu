@@ -126,8 +126,10 @@ int set_kernel_attributes(DeviceInfo* d) {
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>), fwd_smem_bytes<64>());
   set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>), fwd_smem_bytes<128>());
   set_decode_attributes(set);
-  set(reinterpret_cast<const void*>(&w64::fwd_kernel<false>), w64::kSmemBytes);
-  set(reinterpret_cast<const void*>(&w64::fwd_kernel<true>), w64::kSmemBytes);
+  using w64::Launch;
+  const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForward>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForwardShort>),
+                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kStats>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kPolicy>)};
+  for (const void* fn : workers) set(fn, w64::kSmemBytes);
   set(reinterpret_cast<const void*>(&quant_grid_kernel<false>), kQuantGridSmem);
   set(reinterpret_cast<const void*>(&quant_grid_kernel<true>), kQuantGridSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&quant_cluster_kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -140,20 +142,22 @@ int set_kernel_attributes(DeviceInfo* d) {
   if (e != cudaSuccess) { cudaGetLastError(); return FMHA_I8_ERR_LAUNCH; }
   // The forward kernel redistributes registers with setmaxnreg; that only terminates if the launch
   // allocation is the one the targets were sized for.
-  cudaFuncAttributes fa64{}, fa128{}, fp64{}, fp128{}, fw{}, fwp{};
+  cudaFuncAttributes fa64{}, fa128{}, fp64{}, fp128{}, fw{};
   if (cudaFuncGetAttributes(&fa64, reinterpret_cast<const void*>(&fmha_fwd_kernel<64, false>)) != cudaSuccess ||
       cudaFuncGetAttributes(&fa128, reinterpret_cast<const void*>(&fmha_fwd_kernel<128, false>)) != cudaSuccess ||
       cudaFuncGetAttributes(&fp64, reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>)) != cudaSuccess ||
       cudaFuncGetAttributes(&fp128, reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fw, reinterpret_cast<const void*>(&w64::fwd_kernel<false>)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fwp, reinterpret_cast<const void*>(&w64::fwd_kernel<true>)) != cudaSuccess ||
-      fw.numRegs != w64::kLaunchRegs || fwp.numRegs != w64::kLaunchRegs ||
       fa64.numRegs != kLaunchRegs || fa128.numRegs != kLaunchRegs || fp64.numRegs != kLaunchRegs || fp128.numRegs != kLaunchRegs) {
     cudaGetLastError();
-    std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d/%d registers per thread, expected %d, and %d, expected %d; refusing to launch\n",
-                 fa64.numRegs, fa128.numRegs, kLaunchRegs, fw.numRegs, w64::kLaunchRegs);
+    std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d/%d registers per thread, expected %d; refusing to launch\n", fa64.numRegs, fa128.numRegs, kLaunchRegs);
     return FMHA_I8_ERR_LAUNCH;
   }
+  for (const void* fn : workers)
+    if (cudaFuncGetAttributes(&fw, fn) != cudaSuccess || fw.numRegs != w64::kLaunchRegs) {
+      cudaGetLastError();
+      std::fprintf(stderr, "fmha_i8_sm100: workers' kernel built with %d registers per thread, expected %d; refusing to launch\n", fw.numRegs, w64::kLaunchRegs);
+      return FMHA_I8_ERR_LAUNCH;
+    }
   for (int i = 0; i < kClusterSizes; ++i) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
@@ -407,8 +411,12 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   const int sms = dev->sm_count - busy_sms;
   unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
   if constexpr (D == 64) {
-    if (kernel == FMHA_I8_KERNEL_WORKERS)
-      return launch_kernel(w64::fwd_kernel<kPolicy>, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
+    if (kernel == FMHA_I8_KERNEL_WORKERS) {
+      using w64::Launch;
+      auto* fn = kPolicy ? w64::fwd_kernel<Launch::kPolicy> : p.row_stats_out ? w64::fwd_kernel<Launch::kStats>
+                 : p.S <= w64::kShortTiles * kTile ? w64::fwd_kernel<Launch::kForwardShort> : w64::fwd_kernel<Launch::kForward>;
+      return launch_kernel(fn, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
+    }
   }
   if (p.parts > 1) {
     how.cluster = static_cast<unsigned>(p.parts);

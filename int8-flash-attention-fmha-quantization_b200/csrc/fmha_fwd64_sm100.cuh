@@ -7,6 +7,8 @@
 //             an SM; worker w of CTA c walks units c + grid * w, then every (4 grid)-th.
 //   driver  = one warp per worker: mask scan, TMA copies, S = Q.K^T, P.V.
 //   tensor memory: 128 columns per worker.  S of a step; then its 8-bit P over the first 32 columns and P.V over the last 64.
+//   key tiles with unmasked keys in one half only are 64 keys: S has 64 columns, the softmax threads read 64, P.V takes two of its
+//             four steps.  B256 H16 S256 (lengths 64..256) 93.5 -> 87.2 us, B64 H16 S320 61.5 -> 56.2, B64 H16 S64 13.6 -> 12.0.
 //
 // A worker's step is one serial chain -- S, maximum, exponentials, P.V, fold -- of 3600 cycles when it runs alone.  Four of them
 // on an SM hide each other's latencies; nobody waits for a stage that other threads own, which is what bounds the other kernel
@@ -22,6 +24,14 @@
 
 namespace fmha {
 namespace w64 {
+// What a launch is for: the forward pass (or its calibration); the same for units of up to kShortTiles key tiles; the statistics of
+// the rows for a whole-row P scaling policy (FwdParams::row_stats_out); the forward pass with such a policy (row_stats_in).
+// The two forward passes differ in how the maximum of a half tile branches off that of a whole one: behind the first loads, which
+// the compiler pays for with spilled values of the unit and makes a faster step of, or in front of them.  us, behind / in front: B256 H16
+// S256 (lengths 64..256) 88.4 / 87.2, B200 H12 S128 25.4 / 24.6, B64 H16 S320 57.1 / 56.2, B32 H12 S512 (256..512) 38.4 / 38.8, S576
+// (300..576) 53.4 / 54.3, B8 H32 S2048 336 / 346.
+enum class Launch { kForward, kForwardShort, kStats, kPolicy };
+constexpr int kShortTiles = 3;
 constexpr int kD = 64;
 constexpr int kWorkers = 4;          // per CTA
 // Warps: four softmax warps per worker (their number modulo 4 is their lane quarter of tensor memory), then one driver per worker.
@@ -42,13 +52,13 @@ constexpr int kWorkerBytes = 3 * kTileBytes;                   // K, V, Q
 // A worker's tensor memory: 128 columns.  S of a step; then P over its first 32 columns and P.V over its last 64.
 constexpr uint32_t kOCol = 64;
 
-// What the workers need to know about a unit.  The list of key tiles is only used by the driver that writes it.
+// What the workers need to know about a unit.
 struct UnitInfo {
   int n_live;                         // key tiles with at least one unmasked key
   int rows;                           // query rows of the unit: 128, fewer in a head's last tile
   int64_t first_row;                  // of the slice's query rows, the unit's first
   uint8_t live[kMaxTiles];            // indices of the live key tiles, ascending
-  uint8_t mixed[kMaxTiles];           // 1 = that live tile has masked keys too
+  uint8_t kind[kMaxTiles];            // their kinds (kTile...)
 };
 struct WorkerCtl {
   uint64_t q_full, k_full, v_full;    // the tiles have landed
@@ -83,9 +93,27 @@ struct UnitWalk {
   int first, step;
 };
 
+// Largest of kChunks times 16 columns (biased integers), two loads in flight.
+template <int kChunks>
+__device__ __forceinline__ int columns_max(const uint32_t taddr) {
+  int max_a = INT_MIN, max_b = INT_MIN;
+  uint32_t ra[16], rb[16];
+  tmem_ld16_issue(taddr, ra);
+  tmem_ld16_issue(taddr + 16, rb);
+#pragma unroll
+  for (int c = 0; c < kChunks; c += 2) {
+    tmem_ld_fence(ra); tmem_ld_fence(rb);
+    chunk_max<16>(ra, max_a, max_b);
+    if (c + 2 < kChunks) tmem_ld16_issue(taddr + (c + 2) * 16, ra);
+    chunk_max<16>(rb, max_a, max_b);
+    if (c + 2 < kChunks) tmem_ld16_issue(taddr + (c + 3) * 16, rb);
+  }
+  return max(max_a, max_b);
+}
+
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = one query row: its scores, probabilities, fp32 running output row, maximum and sum.
-template <bool kPolicy>
+template <Launch kLaunch>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base, const UnitWalk walk) {
   WorkerCtl* ctl = &all->w[worker];
   const int lane = threadIdx.x & 31, quad = warp_index() & 3;
@@ -93,7 +121,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   const uint32_t tS = t_lane + static_cast<uint32_t>(worker * kTile), tP = tS;
   volatile int* abort_flag = &all->abort;
-  const bool stats_only = !kPolicy && p.row_stats_out != nullptr;
+  constexpr bool kPolicy = kLaunch == Launch::kPolicy, kStats = kLaunch == Launch::kStats, kShort = kLaunch == Launch::kForwardShort;
 
   uint32_t g = 0;                               // steps so far
   auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
@@ -132,25 +160,43 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
 
 #pragma unroll 1
     for (int j = 0; j < n_live; ++j, ++g) {
+      const bool whole = (ctl->info[buf].kind[j] & kTileHalf) == 0;      // 128 columns of scores, or 64
       if (!wait_or_fail(smem_u32(&ctl->s_full), g & 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
       tc_fence_after();
       FMHA_STAMP(quad == 0 ? worker * 4 + 0 : 47, g);
       if (!kPolicy) {
         // ---- pass 1: biased integer maximum of the row (inc/fmha_i8.cuh:183-206)
-        int max_a = INT_MIN, max_b = INT_MIN;
-        uint32_t ra[16], rb[16];
-        tmem_ld16_issue(tS, ra);
-        tmem_ld16_issue(tS + 16, rb);
-#pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-          tmem_ld_fence(ra); tmem_ld_fence(rb);
-          chunk_max<16>(ra, max_a, max_b);
-          if (c < 6) tmem_ld16_issue(tS + (c + 2) * 16, ra);
-          chunk_max<16>(rb, max_a, max_b);
-          if (c < 6) tmem_ld16_issue(tS + (c + 3) * 16, rb);
+        int imax;
+        if constexpr (kShort) {
+          imax = whole ? columns_max<8>(tS) : columns_max<4>(tS);
+        } else {
+          uint32_t ra[16], rb[16];
+          int max_a = INT_MIN, max_b = INT_MIN;
+          auto two_chunks = [&]() {
+            tmem_ld_fence(ra); tmem_ld_fence(rb);
+            chunk_max<16>(ra, max_a, max_b);
+            chunk_max<16>(rb, max_a, max_b);
+          };
+          auto two_chunks_and_next = [&](int next) {
+            tmem_ld_fence(ra); tmem_ld_fence(rb);
+            chunk_max<16>(ra, max_a, max_b);
+            tmem_ld16_issue(tS + next * 16, ra);
+            chunk_max<16>(rb, max_a, max_b);
+            tmem_ld16_issue(tS + next * 16 + 16, rb);
+          };
+          tmem_ld16_issue(tS, ra);
+          tmem_ld16_issue(tS + 16, rb);
+          two_chunks_and_next(2);
+          if (whole) {
+            two_chunks_and_next(4);
+            two_chunks_and_next(6);
+            two_chunks();
+          } else {
+            two_chunks();
+          }
+          imax = max(max_a, max_b);
         }
-        const int imax = max(max_a, max_b);
-        if (stats_only) imax_run = (j == 0) ? imax : max(imax_run, imax);
+        if (kStats) imax_run = (j == 0) ? imax : max(imax_run, imax);
         k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, p.p_mul);
       }
       FMHA_STAMP(quad == 0 ? worker * 4 + 1 : 47, g);
@@ -158,21 +204,31 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       // ---- pass 2: exp, row sum, requantise (inc/fmha_i8.cuh:208-253); the bytes go over columns already consumed
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t sa[8], sb[8], packed[2];
-      tmem_ld8_issue(tS, sa);
-#pragma unroll
-      for (uint32_t c = 0; c < 16; c += 2) {
+      auto sixteen = [&](uint32_t c, auto more) {           // columns 8 c to 8 c + 15; the first eight are in flight
         tmem_ld_fence(sa);
         tmem_ld8_issue(tS + (c + 1) * 8, sb);
         chunk_exp_pack<8, kPolicy, 0>(sa, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
         tmem_st2(tP + c * 2, packed);
         tmem_ld_fence(sb);
-        if (c < 14) tmem_ld8_issue(tS + (c + 2) * 8, sa);
+        if (decltype(more)::value) tmem_ld8_issue(tS + (c + 2) * 8, sa);
         chunk_exp_pack<8, kPolicy, 1>(sb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
         tmem_st2(tP + c * 2 + 2, packed);
+      };
+      constexpr Flight<1> more;
+      constexpr Flight<0> last;
+      tmem_ld8_issue(tS, sa);
+      if (whole) {
+#pragma unroll
+        for (uint32_t c = 0; c < 14; c += 2) sixteen(c, more);
+        sixteen(14, last);
+      } else {
+#pragma unroll
+        for (uint32_t c = 0; c < 6; c += 2) sixteen(c, more);
+        sixteen(6, last);
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(smem_u32(stats_only ? &ctl->s_free : &ctl->p_ready));
+      mbar_arrive(smem_u32(kStats ? &ctl->s_free : &ctl->p_ready));
       FMHA_STAMP(quad == 0 ? worker * 4 + 2 : 47, g);
 
       // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304), while P.V is under way
@@ -184,7 +240,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
         l_run = fmaf(e_old, l_run, e_cur * (k.f * ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y))));
         m_run = m_new;
       }
-      if (stats_only) continue;                                        // no output is wanted: there is no P.V
+      if (kStats) continue;                                        // no output is wanted: there is no P.V
       const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
       const float2 e_old2 = make_float2(e_old, e_old);
 
@@ -213,7 +269,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     const int64_t out_row = output_row();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
-    if (stats_only) {
+    if (kStats) {
       // the row's maximum and exp-sum over all keys, for the policy launch that follows
       if (out_row >= 0) p.row_stats_out[out_row] = make_float2(__int_as_float(imax_run), l_run);
       continue;
@@ -263,10 +319,11 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
 // the reuse of a tile, which the driver itself has seen used.
 struct DriverStep {
   int tile;                  // key tile, -1: no more steps
-  bool mixed;                // it has masked keys
+  int kind;                  // its kind (kTile...)
   bool first;                // of its unit
   int bh, batch;
 };
+template <bool kStats>
 __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const int worker, const CUtensorMap* map_q, const CUtensorMap* map_k,
                                             const CUtensorMap* map_v, const uint32_t tmem_base, const uint32_t worker_smem, uint8_t* presets,
                                             const UnitWalk walk) {
@@ -276,12 +333,12 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   const uint32_t tS = tmem_base + static_cast<uint32_t>(worker * kTile), tO = tS + kOCol;
   const uint32_t k_smem = worker_smem, v_smem = worker_smem + kTileBytes, q_smem = worker_smem + 2 * kTileBytes;
   constexpr uint32_t idesc_s = make_idesc_i8(kTile, false);       // S = Q.K^T : N = 128 keys, both K-major
+  constexpr uint32_t idesc_half = make_idesc_i8(kTile / 2, false), idesc_preset_half = make_idesc_bf16(kTile / 2);
   constexpr uint32_t idesc_preset_s = make_idesc_bf16(kTile), idesc_preset_o = make_idesc_bf16(kD);
   constexpr uint32_t idesc_o = make_idesc_i8(kD, true, true);     // P.V : P unsigned, V an MN-major operand
   const uint32_t preset_smem = smem_u32(presets);
   const uint64_t d_a = preset_desc(preset_smem, 0), d_b = preset_desc(preset_smem, 1);
   const uint64_t dq = make_smem_desc(q_smem, kD), dk = make_smem_desc(k_smem, kD), dv = make_smem_desc(v_smem, kD);
-  const bool no_pv = p.row_stats_out != nullptr;
   const int n_tiles = (p.S + kTile - 1) / kTile;
   uint32_t fail = 0u, g = 0, units = 0;
   auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
@@ -295,17 +352,17 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   auto next_step = [&]() -> DriverStep {
     while (j >= n_live) {
       u += walk.step;
-      if (u >= p.n_units) { u = p.n_units - walk.step; n_live = 0; return DriverStep{-1, false, false, 0, 0}; }
+      if (u >= p.n_units) { u = p.n_units - walk.step; n_live = 0; return DriverStep{-1, 0, false, 0, 0}; }
       ++it;
       const int buf = it % kInfoBufs;
       if (it >= kInfoBufs && !wait(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), FMHA_I8_DEV_WAIT_INFO))
-        return DriverStep{-1, false, false, 0, 0};
+        return DriverStep{-1, 0, false, 0, 0};
       // (plain divisions: with unit_geom's multipliers this warp spills, 368 -> 371 us for B8 H32 S2048)
       bh = u / p.q_tiles;
       batch = (p.bh_begin + bh) / p.H;
       q_row0 = (u - bh * p.q_tiles) * kTile;
       UnitInfo* info = &ctl->info[buf];
-      scan_mask_warp(info, p.mask + static_cast<int64_t>(batch) * p.S, p.S, n_tiles);
+      scan_mask_warp<true>(info, p.mask + static_cast<int64_t>(batch) * p.S, p.S, n_tiles);
       if (elect_one()) {
         info->rows = min(kTile, p.Sq - q_row0);
         info->first_row = static_cast<int64_t>(bh) * p.Sq + q_row0;
@@ -316,7 +373,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
       j = 0;
     }
     const UnitInfo* info = &ctl->info[it % kInfoBufs];
-    const DriverStep s{info->live[j], info->mixed[j] != 0, j == 0, bh, batch};
+    const DriverStep s{info->live[j], info->kind[j], j == 0, bh, batch};
     ++j;
     return s;
   };
@@ -335,10 +392,12 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   DriverStep cur = next_step();
   load_k(cur);
   while (cur.tile >= 0 && fail == 0u) {
+    const bool mixed = (cur.kind & kTileMixed) != 0, whole = (cur.kind & kTileHalf) == 0;
+    const uint32_t row0 = (cur.kind & kTileUpper) != 0 ? kTile / 2 : 0u;          // first row in use of the K and V tiles
     bool masked[4] = {};
-    if (cur.mixed) {
+    if (mixed) {
       const int8_t* mask_row = p.mask + static_cast<int64_t>(cur.batch) * p.S;
-      const int key0 = cur.tile * kTile + lane;
+      const int key0 = cur.tile * kTile + static_cast<int>(row0) + lane;
 #pragma unroll
       for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || mask_row[key0 + 32 * i] != 0;
     }
@@ -348,15 +407,16 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
     tc_fence_after();
     FMHA_STAMP(16 + worker * 4 + 0, g);
     // the tile's preset operand: the common one, or this worker's own, which nothing has read since the last S
-    const uint32_t operand = cur.mixed ? 2u + static_cast<uint32_t>(worker) : 1u;
-    if (cur.mixed) fill_mask_operand(presets + operand * kPresetBytes, masked, 128);
+    const uint32_t operand = mixed ? 2u + static_cast<uint32_t>(worker) : 1u;
+    if (mixed) fill_mask_operand(presets + operand * kPresetBytes, masked, 128);
     const uint64_t d_preset = preset_desc(preset_smem, operand);
     if (elect_one()) {
-      mma_f16_ss(tS, d_a, d_preset, idesc_preset_s, 0u);      // accumulator := 0x4B400000, masked keys -2^127
+      const uint32_t idesc_preset = whole ? idesc_preset_s : idesc_preset_half, idesc = whole ? idesc_s : idesc_half;
+      mma_f16_ss(tS, d_a, d_preset, idesc_preset, 0u);        // accumulator := 0x4B400000, masked keys -2^127
 #pragma unroll
-      for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(dk, kk * 32), idesc_s, 1u);
+      for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(dk, row0 * kD + kk * 32), idesc, 1u);
       mma_commit(smem_u32(&ctl->s_full));
-      if (!no_pv) {
+      if (!kStats) {
         mbar_arrive_expect_tx(smem_u32(&ctl->v_full), kTileBytes);
         tma_load_3d(v_smem, map_v, smem_u32(&ctl->v_full), 0, cur.tile * kTile, cur.bh);
       }
@@ -365,7 +425,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
     const DriverStep next = next_step();
     if (fail != 0u || !wait(smem_u32(&ctl->s_full), g & 1u, FMHA_I8_DEV_WAIT_S_READY)) break;
     load_k(next);
-    if (!no_pv) {
+    if (!kStats) {
       if (!wait(smem_u32(&ctl->v_full), g & 1u, FMHA_I8_DEV_WAIT_V_LOAD)) break;
       if (!wait(smem_u32(&ctl->p_ready), g & 1u, FMHA_I8_DEV_WAIT_P_READY)) break;
       tc_fence_after();
@@ -373,7 +433,11 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
       if (elect_one()) {
         mma_f16_ss(tO, d_a, d_b, idesc_preset_o, 0u);
 #pragma unroll
-        for (int kk = 0; kk < kTile / 32; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);
+        for (int kk = 0; kk < kTile / 64; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, (row0 + kk * 32) * kD), idesc_o, 1u);
+        if (whole) {
+#pragma unroll
+          for (int kk = kTile / 64; kk < kTile / 32; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);
+        }
         mma_commit(smem_u32(&ctl->o_full));
       }
       FMHA_STAMP(16 + worker * 4 + 3, g);
@@ -389,9 +453,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   }
 }
 
-// kPolicy: the launch that applies a whole-row P scaling policy from row statistics (see FwdParams::row_stats_in);
-// the product default, and the statistics launch, are kPolicy = false.
-template <bool kPolicy>
+template <Launch kLaunch>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
            const FwdParams p) {
@@ -442,10 +504,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
   uint8_t* worker_smem = tiles + worker * kWorkerBytes;
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
-    w64::softmax_role<kPolicy>(p, ctl, worker, tmem_base, walk);
+    w64::softmax_role<kLaunch>(p, ctl, worker, tmem_base, walk);
   } else {
     setmaxnreg_dec<kDriverRegs>();
-    driver_role(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets, walk);
+    driver_role<kLaunch == Launch::kStats>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets, walk);
   }
   tc_fence_before();
   __syncthreads();

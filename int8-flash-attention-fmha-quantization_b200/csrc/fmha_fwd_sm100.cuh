@@ -205,13 +205,22 @@ struct FwdParams {
                         // (a policy launch sets scale_v_out to the factor that turns sum_j P8 v8 [/ l] into int8 output units)
 };
 
+// Kinds of live key tiles.  Tiles with unmasked keys in one half only -- the last one of a sequence, every other time -- are
+// processed as the 64 keys of that half by the workers of fmha_fwd64_sm100.cuh: the other half's probabilities are zero and change
+// no maximum, no sum and no product.  Here they are tiles with masked keys: a second, shorter way through the softmax threads' 64
+// registers costs the first one more than it saves (B64 H32 S192 D128 72 -> 79 us, B8 H32 S2048 D128 415 -> 434).
+constexpr uint8_t kTileMixed = 1;      // (the half in use of) the tile has masked keys too
+constexpr uint8_t kTileLower = 2;      // keys 64..127 are all masked
+constexpr uint8_t kTileUpper = 4;      // keys 0..63 are all masked
+constexpr uint8_t kTileHalf = kTileLower | kTileUpper;
+
 // What every role needs to know about one work unit's padding mask.  kInfoBufs of these live in shared
 // memory: the scanner warp fills the ones of coming units while the current unit is being processed.
 struct UnitInfo {
   int n_live;                         // key tiles with at least one unmasked key (of this CTA's part of them)
   int begin;                          // this CTA's part begins here in the lists below
   uint8_t live[kMaxTiles];            // indices of the live key tiles, ascending
-  uint8_t mixed[kMaxTiles];           // 1 = that live tile has masked keys too
+  uint8_t kind[kMaxTiles];            // their kinds
 };
 
 template <int NK, int NV> struct FwdCtl {
@@ -261,8 +270,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 // Builds one unit's view of its batch's padding mask: the list of live tiles and whether each has masked keys too.
 // Executed by ONE warp; a lane looks at 32 keys, four lanes make a tile.  kGroups: groups of eight tiles whose loads are in
-// flight together (four for long masks: 128 tiles one group after the other take 5 us).
-template <int kGroups, typename Info>
+// flight together (four for long masks: 128 tiles one group after the other take 5 us).  kHalves: tiles with one open half are told apart.
+template <int kGroups, bool kHalves, typename Info>
 __device__ __forceinline__ int scan_mask_groups(Info* info, const uint32_t* words, int S, int n_tiles) {
   const int lane = threadIdx.x & 31;
   int n = 0;
@@ -292,17 +301,21 @@ __device__ __forceinline__ int scan_mask_groups(Info* info, const uint32_t* word
       if (is_live) {
         const int pos = n + __popc(ballot & ((1u << lane) - 1u));
         info->live[pos] = static_cast<uint8_t>(base0 + 8 * q + lane);
-        info->mixed[pos] = ((any_masked >> (4 * lane)) & 0xFu) != 0u ? 1 : 0;
+        const uint32_t tile_masked = (any_masked >> (4 * lane)) & 0xFu, tile_open = (any_open >> (4 * lane)) & 0xFu;
+        // (without kHalves they count as masked keys: one request of S320 waits for this, 6.5 -> 6.8 us)
+        if (kHalves && (tile_open & 0xCu) == 0u) info->kind[pos] = kTileLower | ((tile_masked & 0x3u) != 0u ? kTileMixed : 0);
+        else if (kHalves && (tile_open & 0x3u) == 0u) info->kind[pos] = kTileUpper | ((tile_masked & 0xCu) != 0u ? kTileMixed : 0);
+        else info->kind[pos] = tile_masked != 0u ? kTileMixed : 0;
       }
       n += __popc(ballot);
     }
   }
   return n;
 }
-template <typename Info>
+template <bool kHalves, typename Info>
 __device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_row, int S, int n_tiles) {
   const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
-  const int n = n_tiles <= 32 ? scan_mask_groups<1>(info, words, S, n_tiles) : scan_mask_groups<4>(info, words, S, n_tiles);
+  const int n = n_tiles <= 32 ? scan_mask_groups<1, kHalves>(info, words, S, n_tiles) : scan_mask_groups<4, kHalves>(info, words, S, n_tiles);
   if ((threadIdx.x & 31) == 0) info->n_live = n;
   __syncwarp();
 }
@@ -939,7 +952,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       const uint32_t sb = g % SBufs<D>::n, stage = g % NK;
       const uint64_t dk = make_smem_desc(k_smem + stage * Cfg::kTileBytes, D);
       const uint32_t tS = tmem_base + sb * kTile;
-      const bool mixed = info->mixed[info->begin + j] != 0;
+      const bool mixed = info->kind[info->begin + j] != 0;
       bool masked[4] = {};
       if (mixed) {
         const int key0 = info->live[info->begin + j] * kTile + static_cast<int>(threadIdx.x & 31);
@@ -1126,7 +1139,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           if (!ok) { if (lane == 0) raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it); break; }
         }
         const UnitGeom geo = unit_geom(p, u);
-        scan_mask_warp(&ctl->info[buf], p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
+        scan_mask_warp<false>(&ctl->info[buf], p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
         if (lane == 0) {
           const int n = ctl->info[buf].n_live, parts = it < walk.own ? 1 : p.parts, rank = static_cast<int>(blockIdx.x) % parts;
           ctl->info[buf].begin = n * rank / parts;

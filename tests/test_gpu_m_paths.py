@@ -505,3 +505,43 @@ def test_outputs_on_both_sides_of_the_clamp(pkg, wl, oracle, torch_cuda, D, Sk, 
     assert np.abs(got.astype(int)).max() <= 127
     assert (np.abs(got.astype(int)) == 127).any() == (o_scale < 0.5)
     assert pkg.device_status()[0] == pkg.OK
+
+
+# Key tiles with unmasked keys in one half only, which the workers process as 64 keys.  Lengths on either side of half a tile, sequences
+# that end in half a tile, an open lower or upper half with and without masked keys in it, alone and beside whole tiles; in the workers'
+# two forms (up to three key tiles and more), the other kernels, and the launches of a whole-row policy.
+HALVES = {
+    "lengths": lambda Sk, b, rng: np.arange(Sk) >= [1, 63, 64, 65, 127, 128, 129, 192, 193, 255, Sk - 64, Sk - 1, Sk][b % 13],
+    "upper": lambda Sk, b, rng: (np.arange(Sk) % 128 < 64) | (np.arange(Sk) % 5 == b % 7),
+    "either": lambda Sk, b, rng: ((np.arange(Sk) // 64) % 4 != b % 4) & ((np.arange(Sk) // 64) % 3 != b % 3) | (rng.random(Sk) < 0.1 * (b % 2)),
+}
+@pytest.mark.parametrize("B,H,Sq,Sk,D", [(104, 16, 64, 64, 64), (104, 8, 256, 256, 64), (52, 16, 320, 320, 64), (52, 8, 130, 576, 64),
+                                         (13, 2, 320, 320, 64), (13, 2, 320, 320, 128), (13, 1, 100, 576, 64), (13, 1, 257, 576, 128), (13, 4, 1, 576, 128)])
+@pytest.mark.parametrize("how", sorted(HALVES))
+def test_half_tiles(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk, D, how):
+    torch = torch_cuda
+    q8, k8, v8, _, (qa, ka, va, _) = _tensors(wl, B, H, Sq, Sk, D, seed=Sk + D + B)
+    # A probability at a rounding boundary moves an output by s_max * v_amax / o_amax (static), at most v_amax / o_amax (the others) of
+    # its steps: with o_amax = v_amax by one, as assert_parity expects.  (With the o_amax of _tensors, v_amax / 8, by up to four.)
+    amax = (qa, ka, va, va)
+    rng = np.random.default_rng(Sk)
+    mask = np.stack([HALVES[how](Sk, b, rng) for b in range(B)]).astype(np.int8)
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    o = torch.full_like(q, 0x5A)
+    param, desc = pkg.FMHAParamI8(*amax, 0.5), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D)
+    pkg.FMHAInferI8Cross(None, param, desc, q, k, v, m, o)
+    got = o.cpu().numpy()
+    # a few heads of every batch against the oracle, all of them against the CUDA-core kernel
+    ref = torch.empty_like(o)
+    pkg.debug_simt_x(None, param, desc, q, k, v, m, ref)
+    assert_parity(got, ref.cpu().numpy(), "against the CUDA-core kernel")
+    some = slice(0, 13)
+    want = oracle.q128(q8[some, :1], k8[some, :1], v8[some, :1], mask[some], amax)
+    assert_parity(got[some, :1], want, "against the oracle")
+    if Sq > 8:
+        scratch = torch.zeros(2 * B * H * Sq, device="cuda")
+        for policy, which in ((pkg.POLICY_ROW, oracle.POLICY_ROW), (pkg.POLICY_STATIC, oracle.POLICY_STATIC)):
+            pkg.FMHAInferI8Policy(None, param, desc, q, k, v, m, o, policy, scratch)
+            want = oracle.policy(q8[some, :1], k8[some, :1], v8[some, :1], mask[some], (*amax, 0.5), which)
+            assert_parity(o.cpu().numpy()[some, :1], want, f"policy {policy}")
+    assert pkg.device_status()[0] == pkg.OK
