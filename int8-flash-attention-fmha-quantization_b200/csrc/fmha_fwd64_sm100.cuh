@@ -54,7 +54,7 @@ constexpr uint32_t kOCol = 64;
 
 // What the workers need to know about a unit.
 struct UnitInfo {
-  int n_live;                         // key tiles with at least one unmasked key
+  int n_live;                         // key tiles with at least one unmasked key, never none; -1: there are no more units
   int rows;                           // query rows of the unit: 128, fewer in a head's last tile
   int64_t first_row;                  // of the slice's query rows, the unit's first
   uint8_t live[kMaxTiles];            // indices of the live key tiles, ascending
@@ -114,7 +114,7 @@ __device__ __forceinline__ int columns_max(const uint32_t taddr) {
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = one query row: its scores, probabilities, fp32 running output row, maximum and sum.
 template <Launch kLaunch>
-__device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base, const UnitWalk walk) {
+__device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base) {
   WorkerCtl* ctl = &all->w[worker];
   const int lane = threadIdx.x & 31, quad = warp_index() & 3;
   const int row = quad * 32 + lane;
@@ -129,12 +129,12 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     raise_status(abort_flag, p.status, code, g);
     return false;
   };
-  int it = 0;
 #pragma unroll 1
-  for (int u = walk.first; u < p.n_units; u += walk.step, ++it) {
+  for (int it = 0;; ++it) {
     const int buf = it % kInfoBufs;
     if (!wait_or_fail(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO)) return;
     const int n_live = ctl->info[buf].n_live;
+    if (n_live < 0) return;
     float2 o2[kD / 2];
 #pragma unroll
     for (int i = 0; i < kD / 2; ++i) o2[i] = make_float2(0.f, 0.f);
@@ -276,7 +276,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     }
     // policy launch: the accumulated integer sum becomes the output through one factor per row: out_mul (/ l for the per-row policy)
     if (kPolicy && p.p_static_mul != 0.f) l_run = l_run > 0.f ? 1.f : 0.f;
-    if (n_live == 0) l_run = 0.f;
     const float inv = l_run > 0.f ? __frcp_rn(l_run) : 0.f;
     if (p.amax_out != nullptr) {
       // calibration: only the largest magnitude of the unquantised output is wanted (the reference takes o_amax from its
@@ -347,22 +346,46 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
     return false;
   };
 
-  int u = walk.first - walk.step, it = -1, j = 0, n_live = 0;
+  uint32_t u = static_cast<uint32_t>(walk.first) - static_cast<uint32_t>(walk.step);      // (the first beyond the last may not be an int)
+  int it = -1, j = 0, n_live = 0;
   int bh = 0, batch = 0, q_row0 = 0;          // of the unit of the step handed out last
+  // The results of rows without an unmasked key.
+  auto empty_unit = [&](int rows, int64_t first_row) {
+    if (kStats) {
+      for (int r = lane; r < rows; r += 32) p.row_stats_out[first_row + r] = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
+    } else if (p.amax_out == nullptr) {
+      uint4* dst = reinterpret_cast<uint4*>(p.o + first_row * kD);
+      for (int i = lane; i < rows * (kD / 16); i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
   auto next_step = [&]() -> DriverStep {
+    constexpr DriverStep none{-1, 0, false, 0, 0};
     while (j >= n_live) {
+      if (n_live < 0) return none;
       u += walk.step;
-      if (u >= p.n_units) { u = p.n_units - walk.step; n_live = 0; return DriverStep{-1, 0, false, 0, 0}; }
-      ++it;
-      const int buf = it % kInfoBufs;
-      if (it >= kInfoBufs && !wait(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), FMHA_I8_DEV_WAIT_INFO))
-        return DriverStep{-1, 0, false, 0, 0};
-      // (plain divisions: with unit_geom's multipliers this warp spills, 368 -> 371 us for B8 H32 S2048)
-      bh = u / p.q_tiles;
-      batch = (p.bh_begin + bh) / p.H;
-      q_row0 = (u - bh * p.q_tiles) * kTile;
+      const int buf = ++it % kInfoBufs;
+      if (it >= kInfoBufs && !wait(smem_u32(&ctl->info_empty[buf]), static_cast<uint32_t>(((it / kInfoBufs) - 1) & 1), FMHA_I8_DEV_WAIT_INFO)) return none;
       UnitInfo* info = &ctl->info[buf];
+      if (u >= static_cast<uint32_t>(p.n_units)) {
+        n_live = -1;
+        if (elect_one()) {
+          info->n_live = -1;
+          mbar_arrive(smem_u32(&ctl->info_full[buf]));
+        }
+        return none;
+      }
+      // (plain divisions: with unit_geom's multipliers this warp spills, 368 -> 371 us for B8 H32 S2048)
+      bh = static_cast<int>(u) / p.q_tiles;
+      batch = (p.bh_begin + bh) / p.H;
+      q_row0 = (static_cast<int>(u) - bh * p.q_tiles) * kTile;
       scan_mask_warp<true>(info, p.mask + static_cast<int64_t>(batch) * p.S, p.S, n_tiles);
+      if (info->n_live == 0) {
+        // Nobody else hears of a unit without keys: this warp is the one that P.V of the step before is waiting for, and may not wait
+        // until the softmax warps have got through a row of such units.
+        empty_unit(min(kTile, p.Sq - q_row0), static_cast<int64_t>(bh) * p.Sq + q_row0);
+        --it;
+        continue;
+      }
       if (elect_one()) {
         info->rows = min(kTile, p.Sq - q_row0);
         info->first_row = static_cast<int64_t>(bh) * p.Sq + q_row0;
@@ -504,7 +527,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
   uint8_t* worker_smem = tiles + worker * kWorkerBytes;
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
-    w64::softmax_role<kLaunch>(p, ctl, worker, tmem_base, walk);
+    w64::softmax_role<kLaunch>(p, ctl, worker, tmem_base);
   } else {
     setmaxnreg_dec<kDriverRegs>();
     driver_role<kLaunch == Launch::kStats>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets, walk);

@@ -545,3 +545,38 @@ def test_half_tiles(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk, D, how):
             want = oracle.policy(q8[some, :1], k8[some, :1], v8[some, :1], mask[some], (*amax, 0.5), which)
             assert_parity(o.cpu().numpy()[some, :1], want, f"policy {policy}")
     assert pkg.device_status()[0] == pkg.OK
+
+
+# Many query tiles, most of whose sequences have no unmasked key at all: behind the last open one a worker meets five to seven empty
+# ones in a row, more than it has room to announce.
+@pytest.mark.parametrize("what", ["forward", "row", "static", "amax"])
+@pytest.mark.parametrize("open_batches", [0, 1, 592, 600])
+def test_rows_of_empty_units(pkg, wl, oracle, torch_cuda, open_batches, what):
+    torch = torch_cuda
+    B, H, Sq, Sk, D = 4200, 1, 70, 64, 64
+    q8, k8, v8, _, (qa, ka, va, _) = _tensors(wl, B, H, Sq, Sk, D, seed=7)
+    mask = np.ones((B, Sk), np.int8)
+    mask[:open_batches, :50] = 0
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    o = torch.full_like(q, 0x5A)
+    param, desc = pkg.FMHAParamI8(qa, ka, va, va, 0.5), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D)
+    assert pkg.debug_plan(desc)[0] == pkg.KERNEL_WORKERS
+    n = max(1, open_batches)
+    if what == "amax":
+        most = torch.zeros(1, device="cuda")
+        pkg.calibrate_o_amax(None, param, desc, q, k, v, m, most)
+        o32, _ = oracle.fp32_attention(*(x[:n].astype(np.float32) * np.float32(a / 127) for x, a in ((q8, qa), (k8, ka), (v8, va))), mask[:n])
+        want = float(np.abs(o32).max()) if open_batches else 0.0
+        assert abs(most.item() - want) <= 0.02 * want
+    else:
+        if what == "forward":
+            pkg.FMHAInferI8Cross(None, param, desc, q, k, v, m, o)
+            want = oracle.q128(q8[:n], k8[:n], v8[:n], mask[:n], (qa, ka, va, va))
+        else:
+            policy, which = (pkg.POLICY_ROW, oracle.POLICY_ROW) if what == "row" else (pkg.POLICY_STATIC, oracle.POLICY_STATIC)
+            pkg.FMHAInferI8Policy(None, param, desc, q, k, v, m, o, policy, torch.zeros(2 * B * H * Sq, device="cuda"))
+            want = oracle.policy(q8[:n], k8[:n], v8[:n], mask[:n], (qa, ka, va, va, 0.5), which)
+        got = o.cpu().numpy()
+        assert_parity(got[:n], want, what)
+        assert not got[open_batches:].any()
+    assert pkg.device_status()[0] == pkg.OK
