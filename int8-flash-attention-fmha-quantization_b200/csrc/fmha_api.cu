@@ -400,13 +400,11 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mk, k, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mv, v, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
-  // Overlap pays where the launch latency is a visible part of the launch: up to four rounds of units (512 units of a
-  // whole-row policy 49.5 -> 46.2 us).  Far beyond that it gives nothing (B8 H32 S2048 415 and 412, B256 H16 S256 D64 with lengths 64..256
-  // 90.1 and 91.0, repeats differ by more), and CTAs then land on SMs in the order the launch before frees them, where neighbours
-  // that share a head are no longer neighbours on the chip.  (Between four and thirty rounds it would still gain: B4 H32 S1024
-  // D128, seven rounds, 61.5 -> 58.2; B64 H32 S256 D128, 28 rounds, 87 -> 83.)
+  // Overlap takes the launch latency and the set-up of a launch out of the time of calls in a row.  (us without / with, more than four
+  // rounds of units: B32 H12 S512 D64 with lengths 256..512 38.5 / 36.3, B200 H12 S128 24.5 / 22.3, B4 H32 S1024 D128 59.6 / 57.1, B64 H32
+  // S256 79.4 / 76.2, B8 H32 S2048 428 / 423, D64 335.7 / 333.7; B256 H16 S256 D64 with lengths 64..256 85.6 / 85.4.)
   LaunchHow how;
-  how.overlap = p.n_units <= 4 * dev->sm_count;
+  how.overlap = true;
   // persistent CTAs: one per SM (tensor memory is allocated whole), each walking its share of the units
   const int sms = dev->sm_count - busy_sms;
   unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
@@ -420,7 +418,6 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   }
   if (p.parts > 1) {
     how.cluster = static_cast<unsigned>(p.parts);
-    how.overlap = true;
     grid = static_cast<unsigned>(p.own_rounds > 0 ? dev->sm_count : p.n_units * p.parts);
   }
   return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);

@@ -226,6 +226,7 @@ struct UnitInfo {
 template <int NK, int NV> struct FwdCtl {
   uint64_t q_full[4], q_empty[4];      // Q ring (kQBufs used): rows have landed / the unit's last S = Q.K^T has completed
   uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV];
+  uint64_t early_full;                 // the first unit's Q rows and its likely first K tile, asked for before its mask is known
   uint64_t s_full[kSBufsMax];          // per S accumulator: S = Q.K^T has completed
   uint64_t s_free[kSBufsMax];          // per S accumulator: the merge threads have drained the partial output that lived in it
   uint64_t o_full[kSBufsMax];          // per S accumulator: P.V of the step that owns it has completed
@@ -854,25 +855,47 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
   uint32_t g = 0;            // steps loaded so far: ring position and phase continue across units
   uint32_t qn = 0;           // non-empty units so far: Q buffer and phase
   uint32_t fail = 0u, fail_tile = 0u;
-  for (int it = 0; it < walk.count && fail == 0u; ++it) {
+  // The first unit's Q rows, and the K tile that its list begins with unless the mask skips tiles, are asked for while the scanner
+  // still waits for the mask: a call of one or two rounds is a chain of latencies, and this takes one of them out.
+  int early_tile = -1;
+  if (walk.count > 0) {
+    const UnitGeom geo = unit_geom(p, walk.unit(0));
+    const int parts = walk.own > 0 ? 1 : p.parts;
+    early_tile = (p.S + kTile - 1) / kTile * (static_cast<int>(blockIdx.x) % parts) / parts;
+    if (elect_one()) {
+      const uint32_t bar = smem_u32(&ctl->early_full);
+      mbar_arrive_expect_tx(bar, static_cast<uint32_t>(2 * Cfg::kTileBytes));
+      tma_load_3d(q_smem, map_q, bar, 0, geo.q_row0, geo.bh_local);
+      tma_load_3d(k_smem, map_k, bar, 0, early_tile * kTile, geo.bh_local);
+    }
+  }
+  auto load_unit = [&](const int it, auto is_first) {
+    constexpr bool kFirst = decltype(is_first)::value != 0;
     const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
     if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
-      fail = FMHA_I8_DEV_WAIT_INFO; fail_tile = it; break;
+      fail = FMHA_I8_DEV_WAIT_INFO; fail_tile = it; return;
     }
     const UnitGeom geo = unit_geom(p, u);
     const UnitInfo* info = &ctl->info[buf];
     const int n_live = info->n_live;
+    if (kFirst && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->early_full), 0u, abort_flag))) {
+      fail = FMHA_I8_DEV_WAIT_Q_LOAD; fail_tile = it; return;
+    }
     if (n_live > 0) {
       const uint32_t qb = qn % NQ;
       // the Q buffer is free once the last S = Q.K^T of the unit that used it NQ units ago has completed
       if (qn >= NQ && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->q_empty[qb]), ((qn / NQ) - 1) & 1u, abort_flag))) {
-        fail = FMHA_I8_DEV_WAIT_K_FREE; fail_tile = it; break;
+        fail = FMHA_I8_DEV_WAIT_K_FREE; fail_tile = it; return;
       }
       if (elect_one()) {
         const uint32_t bar_q = smem_u32(&ctl->q_full[qb]);
-        mbar_arrive_expect_tx(bar_q, static_cast<uint32_t>(Cfg::kTileBytes));
-        tma_load_3d(q_smem + qb * Cfg::kTileBytes, map_q, bar_q, 0, geo.q_row0, geo.bh_local);
+        if (kFirst) {
+          mbar_arrive(bar_q);
+        } else {
+          mbar_arrive_expect_tx(bar_q, static_cast<uint32_t>(Cfg::kTileBytes));
+          tma_load_3d(q_smem + qb * Cfg::kTileBytes, map_q, bar_q, 0, geo.q_row0, geo.bh_local);
+        }
       }
       ++qn;
       for (int j = 0; j < n_live; ++j, ++g) {
@@ -882,8 +905,12 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
           fail = FMHA_I8_DEV_WAIT_K_FREE; fail_tile = g; break;
         }
         if (elect_one()) {
-          mbar_arrive_expect_tx(smem_u32(&ctl->k_full[sk]), Cfg::kTileBytes);
-          tma_load_3d(k_smem + sk * Cfg::kTileBytes, map_k, smem_u32(&ctl->k_full[sk]), 0, t * kTile, geo.bh_local);
+          if (kFirst && j == 0 && t == early_tile) {
+            mbar_arrive(smem_u32(&ctl->k_full[sk]));
+          } else {
+            mbar_arrive_expect_tx(smem_u32(&ctl->k_full[sk]), Cfg::kTileBytes);
+            tma_load_3d(k_smem + sk * Cfg::kTileBytes, map_k, smem_u32(&ctl->k_full[sk]), 0, t * kTile, geo.bh_local);
+          }
         }
         if (rv > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->v_empty[sv]), (rv - 1) & 1u, abort_flag))) {
           fail = FMHA_I8_DEV_WAIT_V_FREE; fail_tile = g; break;
@@ -896,7 +923,9 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
     }
     __syncwarp();
     if (fail == 0u && elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
-  }
+  };
+  if (walk.count > 0) load_unit(0, Flight<1>());
+  for (int it = 1; it < walk.count && fail == 0u; ++it) load_unit(it, Flight<0>());
   if (fail != 0u) {
     if (elect_one()) raise_status(abort_flag, p.status, fail, fail_tile);
     // unwinding: let copies that are still in flight land before the CTA may exit
@@ -1092,6 +1121,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_init(smem_u32(&ctl->info_full[b]), 1);
       mbar_init(smem_u32(&ctl->info_empty[b]), kInfoConsumers);
     }
+    mbar_init(smem_u32(&ctl->early_full), 1);
     mbar_init_fence();
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
