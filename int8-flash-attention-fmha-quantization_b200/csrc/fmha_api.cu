@@ -121,14 +121,15 @@ int set_kernel_attributes(DeviceInfo* d) {
   auto set = [&](const void* fn, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   };
-  set(reinterpret_cast<const void*>(&fmha_fwd_kernel<64, false>), fwd_smem_bytes<64>());
-  set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, false>), fwd_smem_bytes<128>());
-  set(reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>), fwd_smem_bytes<64>());
-  set(reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>), fwd_smem_bytes<128>());
+  const void* const general64[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kForward>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowMax>),
+                                   reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kPolicy>)};
+  const void* const general128[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kForward>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowMax>),
+                                    reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kPolicy>)};
+  for (const void* fn : general64) set(fn, fwd_smem_bytes<64>());
+  for (const void* fn : general128) set(fn, fwd_smem_bytes<128>());
   set_decode_attributes(set);
-  using w64::Launch;
   const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForward>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForwardShort>),
-                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kStats>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kPolicy>)};
+                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowMax>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowStats>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kPolicy>)};
   for (const void* fn : workers) set(fn, w64::kSmemBytes);
   set(reinterpret_cast<const void*>(&quant_grid_kernel<false>), kQuantGridSmem);
   set(reinterpret_cast<const void*>(&quant_grid_kernel<true>), kQuantGridSmem);
@@ -142,22 +143,16 @@ int set_kernel_attributes(DeviceInfo* d) {
   if (e != cudaSuccess) { cudaGetLastError(); return FMHA_I8_ERR_LAUNCH; }
   // The forward kernel redistributes registers with setmaxnreg; that only terminates if the launch
   // allocation is the one the targets were sized for.
-  cudaFuncAttributes fa64{}, fa128{}, fp64{}, fp128{}, fw{};
-  if (cudaFuncGetAttributes(&fa64, reinterpret_cast<const void*>(&fmha_fwd_kernel<64, false>)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa128, reinterpret_cast<const void*>(&fmha_fwd_kernel<128, false>)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fp64, reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fp128, reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>)) != cudaSuccess ||
-      fa64.numRegs != kLaunchRegs || fa128.numRegs != kLaunchRegs || fp64.numRegs != kLaunchRegs || fp128.numRegs != kLaunchRegs) {
+  auto check = [](const void* fn, int regs) {
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, fn) == cudaSuccess && fa.numRegs == regs) return true;
     cudaGetLastError();
-    std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d/%d registers per thread, expected %d; refusing to launch\n", fa64.numRegs, fa128.numRegs, kLaunchRegs);
-    return FMHA_I8_ERR_LAUNCH;
-  }
-  for (const void* fn : workers)
-    if (cudaFuncGetAttributes(&fw, fn) != cudaSuccess || fw.numRegs != w64::kLaunchRegs) {
-      cudaGetLastError();
-      std::fprintf(stderr, "fmha_i8_sm100: workers' kernel built with %d registers per thread, expected %d; refusing to launch\n", fw.numRegs, w64::kLaunchRegs);
-      return FMHA_I8_ERR_LAUNCH;
-    }
+    std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d registers per thread, expected %d; refusing to launch\n", fa.numRegs, regs);
+    return false;
+  };
+  for (const void* fn : general64) if (!check(fn, kLaunchRegs)) return FMHA_I8_ERR_LAUNCH;
+  for (const void* fn : general128) if (!check(fn, kLaunchRegs)) return FMHA_I8_ERR_LAUNCH;
+  for (const void* fn : workers) if (!check(fn, w64::kLaunchRegs)) return FMHA_I8_ERR_LAUNCH;
   for (int i = 0; i < kClusterSizes; ++i) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
@@ -170,9 +165,9 @@ int set_kernel_attributes(DeviceInfo* d) {
     cfg.numAttrs = 1;
     int n64 = 0, n128 = 0;
     cfg.dynamicSmemBytes = fwd_smem_bytes<64>();
-    if (cudaOccupancyMaxActiveClusters(&n64, fmha_fwd_kernel<64, false>, &cfg) != cudaSuccess) n64 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n64, fmha_fwd_kernel<64, Launch::kForward>, &cfg) != cudaSuccess) n64 = 0;
     cfg.dynamicSmemBytes = fwd_smem_bytes<128>();
-    if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128, false>, &cfg) != cudaSuccess) n128 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128, Launch::kForward>, &cfg) != cudaSuccess) n128 = 0;
     cudaGetLastError();
     d->max_clusters[i] = n64 < n128 ? n64 : n128;
   }
@@ -393,7 +388,7 @@ int plan_call(FwdParams* p, int D, bool plain, int busy_sms, const DeviceInfo* d
   return FMHA_I8_KERNEL_GENERAL;
 }
 
-template <int D, bool kPolicy = false>
+template <int D, Launch kLaunch = Launch::kForward>
 int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v, int kernel, int busy_sms) {
   CUtensorMap mq, mk, mv;
   int st;
@@ -410,9 +405,9 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
   if constexpr (D == 64) {
     if (kernel == FMHA_I8_KERNEL_WORKERS) {
-      using w64::Launch;
-      auto* fn = kPolicy ? w64::fwd_kernel<Launch::kPolicy> : p.row_stats_out ? w64::fwd_kernel<Launch::kStats>
-                 : p.S <= w64::kShortTiles * kTile ? w64::fwd_kernel<Launch::kForwardShort> : w64::fwd_kernel<Launch::kForward>;
+      auto* fn = w64::fwd_kernel<kLaunch>;
+      if constexpr (kLaunch == Launch::kForward)
+        if (p.S <= w64::kShortTiles * kTile) fn = w64::fwd_kernel<Launch::kForwardShort>;
       return launch_kernel(fn, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
     }
   }
@@ -420,7 +415,7 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
     how.cluster = static_cast<unsigned>(p.parts);
     grid = static_cast<unsigned>(p.own_rounds > 0 ? dev->sm_count : p.n_units * p.parts);
   }
-  return launch_kernel(fmha_fwd_kernel<D, kPolicy>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
+  return launch_kernel(fmha_fwd_kernel<D, kLaunch>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
 
 // The few-rows kernel.  CTAs per head: enough for two rounds of the 3 CTAs that an SM holds, so that heads of different
@@ -459,9 +454,9 @@ int launch_decode(cudaStream_t s, DeviceInfo* dev, const FwdParams& p, const voi
 // What a launch of the forward kernels is beside the plain forward pass into o.  (Calibration comes as infer_x_impl's `calib`: the
 // largest |output| goes to that device float and o, which may be null, is not touched.)
 struct LaunchMode {
-  float2* stats_out = nullptr;     // statistics launch of a whole-row policy: {row max bits, exp-sum} per query row, o untouched
+  float2* stats_out = nullptr;     // statistics launch of a whole-row policy: {row max bits, exp-sum or 0} per query row, o untouched
   const float2* stats_in = nullptr;  // policy launch: those statistics
-  int policy = 0;                  // FMHA_I8_POLICY_* of a policy launch
+  int policy = 0;                  // FMHA_I8_POLICY_* that the launch belongs to
   int busy_sms = 0;                // SMs that something else is using for longer than this launch
 };
 
@@ -534,9 +529,14 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   const bool plain = !calib && !(mode && (mode->stats_out || mode->stats_in));
   const int kernel = plan_call(&p, sh.D, plain, busy, dev);
   if (kernel == FMHA_I8_KERNEL_FEW_ROWS) return sh.D == 128 ? launch_decode<128>(s, dev, p, q, k, v) : launch_decode<64>(s, dev, p, q, k, v);
-  if (policy_launch)
-    return sh.D == 128 ? launch_fwd<128, true>(s, dev, p, q, k, v, kernel, busy) : launch_fwd<64, true>(s, dev, p, q, k, v, kernel, busy);
-  return sh.D == 128 ? launch_fwd<128>(s, dev, p, q, k, v, kernel, busy) : launch_fwd<64>(s, dev, p, q, k, v, kernel, busy);
+  auto launch = [&](auto d) {
+    constexpr int D = decltype(d)::value;
+    if (policy_launch) return launch_fwd<D, Launch::kPolicy>(s, dev, p, q, k, v, kernel, busy);
+    if (p.row_stats_out && mode->policy == FMHA_I8_POLICY_ROW) return launch_fwd<D, Launch::kRowMax>(s, dev, p, q, k, v, kernel, busy);
+    if (p.row_stats_out) return launch_fwd<D, Launch::kRowStats>(s, dev, p, q, k, v, kernel, busy);
+    return launch_fwd<D>(s, dev, p, q, k, v, kernel, busy);
+  };
+  return sh.D == 128 ? launch(std::integral_constant<int, 128>()) : launch(std::integral_constant<int, 64>());
 }
 
 int infer_slice_impl(void* stream, const float amax[5], const int desc[4], const void* q, const void* k,
@@ -702,8 +702,10 @@ int fmha_i8_sm100_infer_policy(void* stream, const float amax[5], const int desc
   if (flags & FMHA_I8_FLAG_UINT8_P) return finish(FMHA_I8_ERR_BAD_FLAGS);       // the policies bring their own P format
   if (!row_scratch || !o) return finish(FMHA_I8_ERR_NULL_POINTER);
   if (!aligned(row_scratch, 8)) return finish(FMHA_I8_ERR_MISALIGNED);
-  // launch 1: the forward pass with the reference's tile-local arithmetic, keeping only each row's maximum and exp-sum
+  // launch 1: each row's maximum over all keys, which is all that the per-row scale needs (launch 2 forms the row's sum beside the
+  // probabilities); for the static scale the exp-sum too, in the reference's tile-local arithmetic
   LaunchMode stats;
+  stats.policy = policy;
   stats.stats_out = reinterpret_cast<float2*>(row_scratch);
   int st = infer_x_impl(stream, amax, sh, q, k, v, mask, nullptr, bh_begin, bh_count, flags, nullptr, &stats);
   if (st != FMHA_I8_OK) return finish(st);

@@ -24,13 +24,10 @@
 
 namespace fmha {
 namespace w64 {
-// What a launch is for: the forward pass (or its calibration); the same for units of up to kShortTiles key tiles; the statistics of
-// the rows for a whole-row P scaling policy (FwdParams::row_stats_out); the forward pass with such a policy (row_stats_in).
-// The two forward passes differ in how the maximum of a half tile branches off that of a whole one: behind the first loads, which
+// The two forward passes, kForward and for units of up to kShortTiles key tiles kForwardShort, differ in how the maximum of a half tile branches off that of a whole one: behind the first loads, which
 // the compiler pays for with spilled values of the unit and makes a faster step of, or in front of them.  us, behind / in front: B256 H16
 // S256 (lengths 64..256) 88.4 / 87.2, B200 H12 S128 25.4 / 24.6, B64 H16 S320 57.1 / 56.2, B32 H12 S512 (256..512) 38.4 / 38.8, S576
 // (300..576) 53.4 / 54.3, B8 H32 S2048 336 / 346.
-enum class Launch { kForward, kForwardShort, kStats, kPolicy };
 constexpr int kShortTiles = 3;
 constexpr int kD = 64;
 constexpr int kWorkers = 4;          // per CTA
@@ -121,7 +118,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   const uint32_t tS = t_lane + static_cast<uint32_t>(worker * kTile), tP = tS;
   volatile int* abort_flag = &all->abort;
-  constexpr bool kPolicy = kLaunch == Launch::kPolicy, kStats = kLaunch == Launch::kStats, kShort = kLaunch == Launch::kForwardShort;
+  constexpr bool kPolicy = kLaunch == Launch::kPolicy, kStats = stats_launch(kLaunch), kShort = kLaunch == Launch::kForwardShort;
 
   uint32_t g = 0;                               // steps so far
   auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
@@ -142,7 +139,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     if (n_live < 0) continue;
     ++announced;
     float m_run = -INFINITY, l_run = 0.f;
-    int imax_run = static_cast<int>(kMagicBits);          // statistics launch: biased integer row maximum over all tiles
+    int imax_run = static_cast<int>(kMagicBits);          // statistics launches: biased integer row maximum over all tiles
     RowConsts k;                                          // (policy launch: constant over a unit)
     float p_cap = 0.f;
     // this thread's output row, -1 past the last row of the head (looked up where it is needed: nothing of it stays in registers)
@@ -153,7 +150,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       // row for the whole unit (fmha_i8_quant_deviation.py:62-121).
       float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
       if (out_row >= 0) st = __ldcg(&p.row_stats_in[out_row]);       // (through the L1, 48.1 -> 48.4 us for B4 H16 S1024)
-      l_run = st.y;
       const float l_row = st.y > 0.f ? st.y : 1.f;
       // dynamic: P8 = rn(levels * e); static: P8 = min(rn(levels * (e / l) / s_max), levels)
       const float mul = (p.p_static_mul != 0.f) ? p.p_static_mul / l_row : p.p_row_mul;
@@ -200,6 +196,11 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
           imax = max(max_a, max_b);
         }
         if (kStats) imax_run = (j == 0) ? imax : max(imax_run, imax);
+        if (kLaunch == Launch::kRowMax) {
+          tc_fence_before();
+          mbar_arrive(smem_u32(&ctl->s_free));
+          continue;
+        }
         k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, p.p_mul);
       }
       FMHA_STAMP(quad == 0 ? worker * 4 + 1 : 47, g);
@@ -235,13 +236,16 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       FMHA_STAMP(quad == 0 ? worker * 4 + 2 : 47, g);
 
       // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304), while P.V is under way
+      const float l_tile = k.f * ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y));
       float e_old = j > 0 ? 1.f : 0.f, e_cur = 1.f;                                  // policy launch: every tile of a row has the same scale
       if (!kPolicy) {
         const float m_new = fmaxf(m_run, k.m_tile);
         e_old = __expf(m_run - m_new);                                 // 0 on the first tile (m_run = -inf)
         e_cur = clear_low2(__expf(k.m_tile - m_new));                  // 22 significant bits: kMagic*e_cur is exact
-        l_run = fmaf(e_old, l_run, e_cur * (k.f * ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y))));
+        l_run = fmaf(e_old, l_run, e_cur * l_tile);
         m_run = m_new;
+      } else {
+        l_run += l_tile;
       }
       if (kStats) continue;                                        // no output is wanted: there is no P.V
       const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
@@ -560,7 +564,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     w64::softmax_role<kLaunch>(p, ctl, worker, tmem_base);
   } else {
     setmaxnreg_dec<kDriverRegs>();
-    driver_role<kLaunch == Launch::kStats>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
+    driver_role<stats_launch(kLaunch)>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
   }
   tc_fence_before();
   __syncthreads();

@@ -173,6 +173,11 @@ __device__ __forceinline__ int fast_div(int u, const FastDiv d) {
   return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(u)) * d.mul) >> d.shift);
 }
 
+// What a launch is for: the forward pass (or its calibration); the workers' form of it for units of few key tiles; one of the launches
+// of a whole-row P scaling policy (FwdParams): the rows' maxima, their maxima and sums, or the forward pass with such a policy.
+enum class Launch { kForward, kForwardShort, kRowMax, kRowStats, kPolicy };
+__host__ __device__ constexpr bool stats_launch(Launch l) { return l == Launch::kRowMax || l == Launch::kRowStats; }
+
 struct FwdParams {
   const int8_t* mask;   // [B,S] whole mask
   int8_t* o;            // first head of the slice
@@ -196,9 +201,9 @@ struct FwdParams {
   float amax_scale;     // v_amax / (127 * 128)  (127 * 255 with unsigned P)
   unsigned* status;     // eight device status words
   // Whole-row P scaling policies (the reference's accuracy study, fmha_i8_quant_deviation.py:57-121), two launches:
-  float2* row_stats_out;       // statistics launch: per query row {bits of the biased integer row maximum over ALL keys,
-                               // sum over all keys of exp(score - row maximum)} is written here, nothing to o
-  const float2* row_stats_in;  // policy launch (kernel instantiated with kPolicy): those statistics, read back
+  float2* row_stats_out;       // Launch::kRowMax, kRowStats: per query row {bits of the biased integer row maximum over ALL keys, sum over
+                               // all keys of exp(score - row maximum) (kRowMax: 0)} is written here, nothing to o
+  const float2* row_stats_in;  // Launch::kPolicy: those statistics, read back
   float p_row_mul;      // policy launch: P8 = rn(p_row_mul * exp(score - row max))                  ("dynamic", per-row scale), or
   float p_static_mul;   //                P8 = min(rn(p_static_mul * exp(score - row max) / l), levels)  ("static" scale; 0 = dynamic)
   float p_levels;       // quantisation levels of P in a policy launch (127 in the reference's study)
@@ -497,9 +502,10 @@ __device__ __forceinline__ UnitGeom unit_geom(const FwdParams& p, int u) {
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = one half (64 keys) of one query row of one chain.  Walks the CTA's step sequence and
 // handles the steps of its chain.
-template <int D, bool kPolicy>
+template <int D, Launch kLaunch>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                              const UnitWalk walk) {
+  constexpr bool kPolicy = kLaunch == Launch::kPolicy;
   const int warp = warp_index() - kWarpSoftmax0, lane = threadIdx.x & 31;
   const int chain = warp >> 3, half = (warp >> 2) & 1, quad = warp & 3;
   const int row = quad * 32 + lane;
@@ -577,7 +583,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       tmem_ld16_issue(tS + 48, rb);
       tmem_ld_fence(ra); tmem_ld_fence(rb);
       chunk_max<16>(ra, max_a, max_b);
-      tmem_ld16_issue(tS + c0 * 16, ra);                             // first chunk of pass 2, in flight during the exchange
+      if (kLaunch != Launch::kRowMax) tmem_ld16_issue(tS + c0 * 16, ra);     // first chunk of pass 2, in flight during the exchange
       chunk_max<16>(rb, max_a, max_b);
       const int mine = max(max_a, max_b);
       // ---- exchange with the thread that owns the other half of this row
@@ -585,13 +591,18 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       xrow[half * kTile] = mine;
       mbar_arrive(bar_x);
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(bar_x, n & 1u, abort_flag))) {
-        tmem_ld_fence(ra);
+        if (kLaunch != Launch::kRowMax) tmem_ld_fence(ra);
         raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_S_READY, g);
         return;
       }
       const int imax = max(mine, xrow[(half ^ 1) * kTile]);
       k = row_consts(imax, c2s, row_scale, scale_qk, p_mul);
-      if (half == 0) ctl->st_i[g & 3u][row] = imax;
+      if (stats_launch(kLaunch) && half == 0) ctl->st_i[g & 3u][row] = imax;
+      if (kLaunch == Launch::kRowMax) {
+        tc_fence_before();
+        mbar_arrive(smem_u32(&ctl->p_ready[g & 3u]));
+        continue;
+      }
       }
       if (half == 0 && quad == 0) FMHA_STAMP(chain * 4 + 1, n);
 
@@ -629,10 +640,11 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
 // ---------------------------------------------------------------------------------------------- merge role
 // One thread = one half (D/2 columns) of the fp32 running output row of one query row, plus the running
 // maximum and the running sum of that row (kept by both threads of the row).
-template <int D, bool kPolicy>
+template <int D, Launch kLaunch>
 __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base, uint8_t* tiles,
                                            const UnitWalk walk) {
   constexpr int DH = D / 2;
+  constexpr bool kPolicy = kLaunch == Launch::kPolicy;
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int quad = warp & 3, ch = (warp - kWarpMerge0) >> 2;       // ch = which half of the output columns
   const int row = quad * 32 + lane;
@@ -654,12 +666,8 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
     const int n_live = ctl->info[buf].n_live;
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));     // only the tile count is needed here
-    const UnitGeom geo = unit_geom(p, u);
-    const int q_row = geo.q_row0 + row;
-
     float m_run = -INFINITY, l_run = 0.f;
-    int imax_run = INT_MIN;                                 // statistics launch: biased integer row maximum over all tiles
-    const bool stats_only = !kPolicy && p.row_stats_out != nullptr;
+    int imax_run = INT_MIN;                                 // statistics launches: biased integer row maximum over all tiles
 
 #pragma unroll 1
     for (int j = 0; j < n_live; ++j) {
@@ -672,7 +680,10 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
       }
       // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304)
       float e_old = j > 0 ? 1.f : 0.f, e_cur = 1.f;                    // policy launch: every tile of a row has the same scale
-      if (!kPolicy) {
+      if (stats_launch(kLaunch)) imax_run = max(imax_run, ctl->st_i[slot][row]);
+      if (kPolicy) {
+        l_run += ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);      // (one scale: the tiles' sums add up)
+      } else if (kLaunch != Launch::kRowMax) {
         const float m_tile = ctl->st_m[slot][row];
         const float l_tile = ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);
         const float m_new = fmaxf(m_run, m_tile);
@@ -680,7 +691,12 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
         e_cur = clear_low2(__expf(m_tile - m_new));                    // 22 significant bits: kMagic*e_cur is exact
         l_run = fmaf(e_old, l_run, e_cur * l_tile);
         m_run = m_new;
-        imax_run = max(imax_run, ctl->st_i[slot][row]);
+      }
+      if (stats_launch(kLaunch)) {                                     // no output is wanted: there is no P.V
+        tc_fence_after();
+        tc_fence_before();
+        mbar_arrive(smem_u32(&ctl->s_free[sb]));
+        continue;
       }
       const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
       const float2 e_old2 = make_float2(e_old, e_old);
@@ -693,7 +709,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
       }
       tc_fence_after();
       if (quad == 0) FMHA_STAMP(8 + 2 * ch, g);
-      if (!stats_only) {
+      {
         // output column c of this step: tensor-memory column of 16-column chunk i of MY half
         auto chunk_col = [&](int i) -> uint32_t { return t_lane + sb * kTile + PLayout<D>::kOOff + ch * DH + i * 16; };
         // two loads in flight at a time: a round trip to tensor memory costs more than folding a chunk in
@@ -713,16 +729,17 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
           drain_chunk<16>(rb, o2 + (c + 1) * 8, e_cur2, e_bias, e_old2);
           if (c + 3 < DH / 16) tmem_ld16_issue(chunk_col(c + 3), rb);
         }
-      } else {
-        tc_fence_before();
-        mbar_arrive(smem_u32(&ctl->s_free[sb]));
       }
       if (quad == 0) FMHA_STAMP(9 + 2 * ch, g);
     }
     g0 += static_cast<uint32_t>(n_live);
 
+    // (the unit's place is worked out here and not where it begins: nothing of it stays in registers over its steps)
+    const UnitGeom geo = unit_geom(p, u);
+    const int q_row = geo.q_row0 + row;
+
     // ---- statistics launch: the row's maximum and exp-sum over all keys, for the policy launch that follows
-    if (stats_only) {
+    if (stats_launch(kLaunch)) {
       if (ch == 0 && q_row < p.Sq)
         p.row_stats_out[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row] =
             make_float2(__int_as_float(n_live > 0 ? imax_run : static_cast<int>(kMagicBits)), n_live > 0 ? l_run : 0.f);
@@ -730,9 +747,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
     }
     if (kPolicy) {
       // the accumulated integer sum becomes the output through one factor per row: out_mul (/ l for the per-row policy)
-      float l_row = 0.f;
-      if (q_row < p.Sq) l_row = p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row].y;
-      l_run = (p.p_static_mul != 0.f) ? (l_row > 0.f ? 1.f : 0.f) : l_row;
+      if (p.p_static_mul != 0.f) l_run = l_run > 0.f ? 1.f : 0.f;
     }
 
     // ---- calibration mode: only the largest magnitude of the unquantised output is wanted (the reference
@@ -843,8 +858,8 @@ __device__ __forceinline__ void merge_parts(const FwdParams& p, const uint32_t p
 // ---------------------------------------------------------------------------------------------- loader
 // One warp, run warp-wide (every lane waits and counts, one elected lane issues the copies): the Q tile of every
 // non-empty unit, then per step the K tile and the V tile, in step order.
-// (In a statistics launch, too: this kernel multiplies P and V there like anywhere else, and the merge warps drop the product.)
-template <int D>
+// (In a statistics launch no V tiles: there is no P.V.)
+template <int D, bool kStats>
 __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl,
                                             const CUtensorMap* map_q, const CUtensorMap* map_k, const CUtensorMap* map_v,
                                             const uint32_t q_smem, const uint32_t k_smem, const uint32_t v_smem,
@@ -912,6 +927,7 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
             tma_load_3d(k_smem + sk * Cfg::kTileBytes, map_k, smem_u32(&ctl->k_full[sk]), 0, t * kTile, geo.bh_local);
           }
         }
+        if (kStats) continue;
         if (rv > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->v_empty[sv]), (rv - 1) & 1u, abort_flag))) {
           fail = FMHA_I8_DEV_WAIT_V_FREE; fail_tile = g; break;
         }
@@ -1017,7 +1033,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   if (err.code != 0u && elect_one()) raise_status(abort_flag, p.status, err.code, err.tile);
 }
 
-template <int D>
+template <int D, bool kStats>
 __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                               const uint32_t v_smem, const uint32_t bias_a_smem, const uint32_t bias_b_smem,
                                               const UnitWalk walk) {
@@ -1039,7 +1055,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
     const int n_live = ctl->info[buf].n_live;
     __syncwarp();
     if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));            // only the tile count is needed here
-    for (int j = 0; j < n_live; ++j, ++g) {
+    for (int j = 0; !kStats && j < n_live; ++j, ++g) {
       const uint32_t sb = g % SBufs<D>::n, stage = g % NV;
       const uint64_t dv = make_smem_desc(v_smem + stage * Cfg::kTileBytes, D);
       const uint32_t tS = tmem_base + sb * kTile;
@@ -1067,9 +1083,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
 }
 
 // Persistent kernel: gridDim.x = min(units, SMs) CTAs; CTA b processes units b, b + gridDim.x, ...
-// kPolicy: the launch that applies a whole-row P scaling policy from row statistics (see FwdParams::row_stats_in);
-// the product default, and the statistics launch, are kPolicy = false.
-template <int D, bool kPolicy>
+template <int D, Launch kLaunch>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const FwdParams p) {
@@ -1144,19 +1158,19 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // phase of an info barrier = (it / kInfoBufs) & 1; `g` counts its steps (live key tiles) across units.
   if (warp >= kWarpSoftmax0) {
     setmaxnreg_dec<FwdRegs<D>::kSoftmax>();
-    softmax_role<D, kPolicy>(p, ctl, tmem_base, walk);
+    softmax_role<D, kLaunch>(p, ctl, tmem_base, walk);
   } else if (warp >= kWarpMerge0) {
     setmaxnreg_inc<FwdRegs<D>::kMerge>();
-    merge_role<D, kPolicy>(p, ctl, tmem_base, tiles, walk);
+    merge_role<D, kLaunch>(p, ctl, tmem_base, tiles, walk);
   } else {
     if (FwdRegs<D>::kOther < kLaunchRegs) setmaxnreg_dec<FwdRegs<D>::kOther>();
     else if (FwdRegs<D>::kOther > kLaunchRegs) setmaxnreg_inc<FwdRegs<D>::kOther>();
     if (warp == kWarpLoad) {
-      loader_role<D>(p, ctl, &map_q, &map_k, &map_v, q_smem, k_smem, v_smem, walk);
+      loader_role<D, stats_launch(kLaunch)>(p, ctl, &map_q, &map_k, &map_v, q_smem, k_smem, v_smem, walk);
     } else if (warp == kWarpMmaS) {
       s_issuer_role<D>(p, ctl, tmem_base, q_smem, k_smem, bias_a, walk);
     } else if (warp == kWarpMmaO) {
-      o_issuer_role<D>(p, ctl, tmem_base, v_smem, smem_u32(bias_a), smem_u32(bias_b), walk);
+      o_issuer_role<D, stats_launch(kLaunch)>(p, ctl, tmem_base, v_smem, smem_u32(bias_a), smem_u32(bias_b), walk);
     } else if (warp == kWarpScan) {
       // ---------------------------------------------------------------- scanner: mask information, units ahead
       bool ok = true;
