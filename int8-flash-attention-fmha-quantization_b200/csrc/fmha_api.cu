@@ -122,14 +122,15 @@ int set_kernel_attributes(DeviceInfo* d) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   };
   const void* const general64[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kForward>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowMax>),
-                                   reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kPolicy>)};
+                                   reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowPolicy>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kStaticPolicy>)};
   const void* const general128[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kForward>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowMax>),
-                                    reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kPolicy>)};
+                                    reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowPolicy>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kStaticPolicy>)};
   for (const void* fn : general64) set(fn, fwd_smem_bytes<64>());
   for (const void* fn : general128) set(fn, fwd_smem_bytes<128>());
   set_decode_attributes(set);
   const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForward>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForwardShort>),
-                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowMax>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowStats>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kPolicy>)};
+                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowMax>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowStats>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowPolicy>),
+                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kStaticPolicy>)};
   for (const void* fn : workers) set(fn, w64::kSmemBytes);
   set(reinterpret_cast<const void*>(&quant_grid_kernel<false>), kQuantGridSmem);
   set(reinterpret_cast<const void*>(&quant_grid_kernel<true>), kQuantGridSmem);
@@ -531,8 +532,10 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   if (kernel == FMHA_I8_KERNEL_FEW_ROWS) return sh.D == 128 ? launch_decode<128>(s, dev, p, q, k, v) : launch_decode<64>(s, dev, p, q, k, v);
   auto launch = [&](auto d) {
     constexpr int D = decltype(d)::value;
-    if (policy_launch) return launch_fwd<D, Launch::kPolicy>(s, dev, p, q, k, v, kernel, busy);
-    if (p.row_stats_out && mode->policy == FMHA_I8_POLICY_ROW) return launch_fwd<D, Launch::kRowMax>(s, dev, p, q, k, v, kernel, busy);
+    const bool row = mode && mode->policy == FMHA_I8_POLICY_ROW;
+    if (p.row_stats_in && row) return launch_fwd<D, Launch::kRowPolicy>(s, dev, p, q, k, v, kernel, busy);
+    if (p.row_stats_in) return launch_fwd<D, Launch::kStaticPolicy>(s, dev, p, q, k, v, kernel, busy);
+    if (p.row_stats_out && row) return launch_fwd<D, Launch::kRowMax>(s, dev, p, q, k, v, kernel, busy);
     if (p.row_stats_out) return launch_fwd<D, Launch::kRowStats>(s, dev, p, q, k, v, kernel, busy);
     return launch_fwd<D>(s, dev, p, q, k, v, kernel, busy);
   };

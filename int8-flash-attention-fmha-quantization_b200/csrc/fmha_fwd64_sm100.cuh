@@ -118,7 +118,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   const uint32_t tS = t_lane + static_cast<uint32_t>(worker * kTile), tP = tS;
   volatile int* abort_flag = &all->abort;
-  constexpr bool kPolicy = kLaunch == Launch::kPolicy, kStats = stats_launch(kLaunch), kShort = kLaunch == Launch::kForwardShort;
+  constexpr bool kPolicy = policy_launch(kLaunch), kStatic = kLaunch == Launch::kStaticPolicy, kStats = stats_launch(kLaunch), kShort = kLaunch == Launch::kForwardShort;
 
   uint32_t g = 0;                               // steps so far
   auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
@@ -150,10 +150,11 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       // row for the whole unit (fmha_i8_quant_deviation.py:62-121).
       float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
       if (out_row >= 0) st = __ldcg(&p.row_stats_in[out_row]);       // (through the L1, 48.1 -> 48.4 us for B4 H16 S1024)
-      const float l_row = st.y > 0.f ? st.y : 1.f;
-      // dynamic: P8 = rn(levels * e); static: P8 = min(rn(levels * (e / l) / s_max), levels)
-      const float mul = (p.p_static_mul != 0.f) ? p.p_static_mul / l_row : p.p_row_mul;
+      // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = min(rn(levels * (e / l) / s_max), levels)
+      const float mul = kStatic ? p.p_static_mul / (st.y > 0.f ? st.y : 1.f) : p.p_row_mul;
       k = row_consts(__float_as_int(st.x), p.c2, p.row_scale, p.scale_qk, mul);
+      // the static policy's accumulated integer sum becomes the output through one factor, the per-row policy's through that / l
+      if (kStatic) l_run = st.y > 0.f ? 1.f : 0.f;
       p_cap = p.p_levels / k.p_mul_f.x;       // an exponential above this would quantise beyond the top level
     }
 
@@ -211,11 +212,11 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       auto sixteen = [&](uint32_t c, auto more) {           // columns 8 c to 8 c + 15; the first eight are in flight
         tmem_ld_fence(sa);
         tmem_ld8_issue(tS + (c + 1) * 8, sb);
-        chunk_exp_pack<8, kPolicy, 0>(sa, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
+        chunk_exp_pack<8, kStatic, 0>(sa, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
         tmem_st2(tP + c * 2, packed);
         tmem_ld_fence(sb);
         if (decltype(more)::value) tmem_ld8_issue(tS + (c + 2) * 8, sa);
-        chunk_exp_pack<8, kPolicy, 1>(sb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
+        chunk_exp_pack<8, kStatic, 1>(sb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
         tmem_st2(tP + c * 2 + 2, packed);
       };
       constexpr Flight<1> more;
@@ -244,7 +245,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
         e_cur = clear_low2(__expf(k.m_tile - m_new));                  // 22 significant bits: kMagic*e_cur is exact
         l_run = fmaf(e_old, l_run, e_cur * l_tile);
         m_run = m_new;
-      } else {
+      } else if (!kStatic) {
         l_run += l_tile;
       }
       if (kStats) continue;                                        // no output is wanted: there is no P.V
@@ -281,8 +282,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       if (out_row >= 0) p.row_stats_out[out_row] = make_float2(__int_as_float(imax_run), l_run);
       continue;
     }
-    // policy launch: the accumulated integer sum becomes the output through one factor per row: out_mul (/ l for the per-row policy)
-    if (kPolicy && p.p_static_mul != 0.f) l_run = l_run > 0.f ? 1.f : 0.f;
     const float inv = l_run > 0.f ? __frcp_rn(l_run) : 0.f;
     if (p.amax_out != nullptr) {
       // calibration: only the largest magnitude of the unquantised output is wanted (the reference takes o_amax from its

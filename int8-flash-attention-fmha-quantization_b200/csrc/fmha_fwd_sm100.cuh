@@ -174,8 +174,10 @@ __device__ __forceinline__ int fast_div(int u, const FastDiv d) {
 }
 
 // What a launch is for: the forward pass (or its calibration); the workers' form of it for units of few key tiles; one of the launches
-// of a whole-row P scaling policy (FwdParams): the rows' maxima, their maxima and sums, or the forward pass with such a policy.
-enum class Launch { kForward, kForwardShort, kRowMax, kRowStats, kPolicy };
+// of a whole-row P scaling policy (FwdParams): for the per-row scale the rows' maxima and the forward pass, for the static scale the rows'
+// maxima and sums and the forward pass.
+enum class Launch { kForward, kForwardShort, kRowMax, kRowPolicy, kRowStats, kStaticPolicy };
+__host__ __device__ constexpr bool policy_launch(Launch l) { return l == Launch::kRowPolicy || l == Launch::kStaticPolicy; }
 __host__ __device__ constexpr bool stats_launch(Launch l) { return l == Launch::kRowMax || l == Launch::kRowStats; }
 
 struct FwdParams {
@@ -203,7 +205,7 @@ struct FwdParams {
   // Whole-row P scaling policies (the reference's accuracy study, fmha_i8_quant_deviation.py:57-121), two launches:
   float2* row_stats_out;       // Launch::kRowMax, kRowStats: per query row {bits of the biased integer row maximum over ALL keys, sum over
                                // all keys of exp(score - row maximum) (kRowMax: 0)} is written here, nothing to o
-  const float2* row_stats_in;  // Launch::kPolicy: those statistics, read back
+  const float2* row_stats_in;  // Launch::kRowPolicy, kStaticPolicy: those statistics, read back
   float p_row_mul;      // policy launch: P8 = rn(p_row_mul * exp(score - row max))                  ("dynamic", per-row scale), or
   float p_static_mul;   //                P8 = min(rn(p_static_mul * exp(score - row max) / l), levels)  ("static" scale; 0 = dynamic)
   float p_levels;       // quantisation levels of P in a policy launch (127 in the reference's study)
@@ -505,7 +507,7 @@ __device__ __forceinline__ UnitGeom unit_geom(const FwdParams& p, int u) {
 template <int D, Launch kLaunch>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                              const UnitWalk walk) {
-  constexpr bool kPolicy = kLaunch == Launch::kPolicy;
+  constexpr bool kPolicy = policy_launch(kLaunch);
   const int warp = warp_index() - kWarpSoftmax0, lane = threadIdx.x & 31;
   const int chain = warp >> 3, half = (warp >> 2) & 1, quad = warp & 3;
   const int row = quad * 32 + lane;
@@ -536,9 +538,8 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       const int q_row = geo.q_row0 + row;
       float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 1.f);
       if (q_row < p.Sq) st = p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row];
-      const float l_row = st.y > 0.f ? st.y : 1.f;
-      // dynamic: P8 = rn(levels * e); static: P8 = min(rn(levels * (e / l) / s_max), levels)
-      const float mul = (p.p_static_mul != 0.f) ? p.p_static_mul / l_row : p.p_row_mul;
+      // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = min(rn(levels * (e / l) / s_max), levels)
+      const float mul = kLaunch == Launch::kStaticPolicy ? p.p_static_mul / (st.y > 0.f ? st.y : 1.f) : p.p_row_mul;
       kp = row_consts(__float_as_int(st.x), c2s, row_scale, scale_qk, mul);
       p_cap = p.p_levels / kp.p_mul_f.x;        // an exponential above this would quantise beyond the top level
     }
@@ -610,13 +611,13 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t packed[4];
       tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + cs) * 16, rb);
-      chunk_exp_pack<16, kPolicy>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + c0 * 4, packed);
+      chunk_exp_pack<16, kLaunch == Launch::kStaticPolicy>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + c0 * 4, packed);
       tmem_ld_fence(rb); tmem_ld16_issue(tS + (c0 + 2 * cs) * 16, ra);
-      chunk_exp_pack<16, kPolicy>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + cs) * 4, packed);
+      chunk_exp_pack<16, kLaunch == Launch::kStaticPolicy>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + cs) * 4, packed);
       tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + 3 * cs) * 16, rb);
-      chunk_exp_pack<16, kPolicy>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 2 * cs) * 4, packed);
+      chunk_exp_pack<16, kLaunch == Launch::kStaticPolicy>(ra, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 2 * cs) * 4, packed);
       tmem_ld_fence(rb);
-      chunk_exp_pack<16, kPolicy>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 3 * cs) * 4, packed);
+      chunk_exp_pack<16, kLaunch == Launch::kStaticPolicy>(rb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap); tmem_st4(tP + (c0 + 3 * cs) * 4, packed);
       // ---- publish the row statistics of this step for the merge threads
       const int slot = static_cast<int>(g & 3u);
       const float part = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
@@ -644,7 +645,7 @@ template <int D, Launch kLaunch>
 __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base, uint8_t* tiles,
                                            const UnitWalk walk) {
   constexpr int DH = D / 2;
-  constexpr bool kPolicy = kLaunch == Launch::kPolicy;
+  constexpr bool kPolicy = policy_launch(kLaunch);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int quad = warp & 3, ch = (warp - kWarpMerge0) >> 2;       // ch = which half of the output columns
   const int row = quad * 32 + lane;
@@ -681,9 +682,9 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
       // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304)
       float e_old = j > 0 ? 1.f : 0.f, e_cur = 1.f;                    // policy launch: every tile of a row has the same scale
       if (stats_launch(kLaunch)) imax_run = max(imax_run, ctl->st_i[slot][row]);
-      if (kPolicy) {
+      if (kLaunch == Launch::kRowPolicy) {
         l_run += ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);      // (one scale: the tiles' sums add up)
-      } else if (kLaunch != Launch::kRowMax) {
+      } else if (!kPolicy && kLaunch != Launch::kRowMax) {
         const float m_tile = ctl->st_m[slot][row];
         const float l_tile = ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);
         const float m_new = fmaxf(m_run, m_tile);
@@ -745,10 +746,9 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
             make_float2(__int_as_float(n_live > 0 ? imax_run : static_cast<int>(kMagicBits)), n_live > 0 ? l_run : 0.f);
       continue;
     }
-    if (kPolicy) {
-      // the accumulated integer sum becomes the output through one factor per row: out_mul (/ l for the per-row policy)
-      if (p.p_static_mul != 0.f) l_run = l_run > 0.f ? 1.f : 0.f;
-    }
+    // the static policy's accumulated integer sum becomes the output through one factor, the per-row policy's through that / l
+    if (kLaunch == Launch::kStaticPolicy && q_row < p.Sq)
+      l_run = p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row].y > 0.f ? 1.f : 0.f;
 
     // ---- calibration mode: only the largest magnitude of the unquantised output is wanted (the reference
     //      takes o_amax from its fp32 CPU result, test_fmha_i8.cpp:161)
