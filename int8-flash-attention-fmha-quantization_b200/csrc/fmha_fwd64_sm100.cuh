@@ -17,17 +17,17 @@
 // SM.  An eighth of the exponentials is computed on the multiply-add pipe (all on the exponential unit: 2.5 % slower on
 // B8 H32 S2048; a quarter: 3 % slower).  Pass 2 reads eight columns at a time: with sixteen the 104 registers of a softmax
 // thread do not suffice, and the spills cost 4 to 9 %.
-// Measured against the other kernel: B32 H12 S512 (lengths 256..512) 42.1 -> 39.3 us, B256 H16 S256 (64..256) 98 -> 90,
-// B8 H32 S2048 368 -> 343, B4 H16 S1024 with the per-row policy 52.4 -> 46.2.
+// Measured against the other kernel when it was new: B32 H12 S512 (lengths 256..512) 42.1 -> 39.3 us, B256 H16 S256 (64..256) 98 -> 90,
+// B8 H32 S2048 368 -> 343, B4 H16 S1024 with the per-row policy 52.4 -> 46.2; these take 36.8, 88 to 91, 339 and 35.5 now.
 #pragma once
 #include "fmha_fwd_sm100.cuh"
 
 namespace fmha {
 namespace w64 {
-// The two forward passes, kForward and for units of up to kShortTiles key tiles kForwardShort, differ in how the maximum of a half tile branches off that of a whole one: behind the first loads, which
-// the compiler pays for with spilled values of the unit and makes a faster step of, or in front of them.  us, behind / in front: B256 H16
-// S256 (lengths 64..256) 88.4 / 87.2, B200 H12 S128 25.4 / 24.6, B64 H16 S320 57.1 / 56.2, B32 H12 S512 (256..512) 38.4 / 38.8, S576
-// (300..576) 53.4 / 54.3, B8 H32 S2048 336 / 346.
+// The two forward passes, kForward and for units of up to kShortTiles key tiles kForwardShort, differ in how the maximum of a half tile
+// branches off that of a whole one: behind the first loads, which the compiler pays for with spilled values of the unit and makes a
+// faster step of, or in front of them.  us, behind / in front: B256 H16 S256 (lengths 64..256) 88.4 / 87.2, B200 H12 S128 25.4 / 24.6,
+// B64 H16 S320 57.1 / 56.2, B32 H12 S512 (256..512) 38.4 / 38.8, S576 (300..576) 53.4 / 54.3, B8 H32 S2048 336 / 346.
 constexpr int kShortTiles = 3;
 constexpr int kD = 64;
 constexpr int kWorkers = 4;          // per CTA
