@@ -271,7 +271,7 @@ int fill_params(FwdParams* p, const float amax[5], int D, unsigned flags = 0u) {
   p->amax_scale = amax[2] / ((up ? 255.f : 128.f) * 127.f);   // O~/l counts P in 1/128 (1/255) and V in v_amax/127
   p->c2 = static_cast<float>(static_cast<double>(p->row_scale) * static_cast<double>(p->scale_qk) * 1.4426950408889634);
   if (!(p->c2 > 0.f) || !std::isfinite(p->c2 * kMagic)) return FMHA_I8_ERR_BAD_AMAX;
-  p->c2 = std::fmax(p->c2, kMinC2);
+  p->c2 = std::fmin(std::fmax(p->c2, kMinC2), kMaxC2);
   return FMHA_I8_OK;
 }
 

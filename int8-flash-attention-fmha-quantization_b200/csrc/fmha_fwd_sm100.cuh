@@ -146,6 +146,12 @@ constexpr uint32_t kMagicBits = 0x4B400000u;
 // at most 2 * 128 * 128 * head_dim = 2^22, and 2^22 * 2^-100 = 2^-78 is far below half an ulp of 1 (2^-25): the exponentials of a
 // call whose own factor is smaller are all 1, and they are with this one.
 constexpr float kMinC2 = 0x1p-100f;
+// Largest one.  Scores are whole numbers: from here on a key whose score is not the row's maximum has an exponential of 2^-64 or less, which
+// changes no sum and quantises to zero, and with this factor it has the same.  What it is for: the residue of row_consts, at most 32
+// here, grows with the factor.
+constexpr float kMaxC2 = 64.0f;
+// Up to this factor 2^-residue is 1 - residue ln 2 to 2^-22, the accuracy of the exponentials (the residue is 2^-10 at the most).
+constexpr float kLinearC2 = 0x1p-9f;
 constexpr int kBiasBytes = 4096;               // 128 rows x 16 bf16, unswizzled core-matrix layout
 template <int D> __host__ __device__ constexpr int bias_bytes() { return (2 + SBufs<D>::n) * kBiasBytes; }
 
@@ -362,7 +368,7 @@ __device__ __forceinline__ void chunk_max(const uint32_t (&r)[N], int& max_a, in
   }
 }
 
-// 2^a for two values a <= 0 on the multiply-add pipe: a = n + f with |f| <= 1/2, a degree-5 minimax polynomial for 2^f (fitted by
+// 2^a for two values a <= 32 on the multiply-add pipe: a = n + f with |f| <= 1/2, a degree-5 minimax polynomial for 2^f (fitted by
 // exchange; 2.1e-7 in fp32 arithmetic, the error bound of ex2.approx is 2^-22 = 2.4e-7), n added to the exponent.
 __device__ __forceinline__ float2 exp2_poly(float2 a) {
   const float2 magic = make_float2(kMagic, kMagic), neg_magic = make_float2(-kMagic, -kMagic);
@@ -420,13 +426,13 @@ struct RowConsts {
 };
 __device__ __forceinline__ RowConsts row_consts(const int imax, const float c2s, const float row_scale, const float scale_qk, const float p_mul) {
   // exponent argument (s - smax) * c2 = x * c2 - M * c2 with x = kMagic + s and M = kMagic + smax.
-  // M * c2 = hi + lo exactly (lo is the rounding residual); the factor 2^-lo is folded into the
-  // quantisation constant and the row sum, so nothing is lost and nothing is paid per element.
+  // M * c2 = hi + lo exactly (lo is the rounding residual, half an ulp of hi or less: 2^-14 for c2 = 1e-4, 1/2 for 1, 32 for
+  // 64); the factor 2^-lo is folded into the quantisation constant and the row sum, so nothing is lost and nothing is paid per element.
   RowConsts k;
   const float M = __uint_as_float(static_cast<uint32_t>(imax));
   const float hi = M * c2s;
   const float lo = fmaf(M, c2s, -hi);
-  k.f = fmaf(-lo, 0.6931471805599453f, 1.0f);
+  k.f = c2s < kLinearC2 ? fmaf(-lo, 0.6931471805599453f, 1.0f) : ex2_approx(-lo);
   k.c2 = make_float2(c2s, c2s);
   k.neg_hi = make_float2(-hi, -hi);
   k.p_mul_f = make_float2(p_mul * k.f, p_mul * k.f);        // 128 f (or 255 f): quantisation multiplier

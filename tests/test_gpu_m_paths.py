@@ -580,3 +580,52 @@ def test_rows_of_empty_units(pkg, wl, oracle, torch_cuda, open_batches, what):
         assert_parity(got[:n], want, what)
         assert not got[open_batches:].any()
     assert pkg.device_status()[0] == pkg.OK
+
+
+# Factors from scores to exponents at which a difference of one in the scores is anything from a few per cent to everything: 2^(-c2) per
+# unit.  (Not chosen at a boundary of the rounding of 128, 255 or 127 times 2^(-c2 * n): every key of a row has one of a few scores.)
+LARGE_SCALES = [0.0031, 0.077, 0.317, 0.931, 2.37, 3.13, 10.7, 49.3, 71.9, 1.3e4, 1.1e15, 1.7e31]
+LARGE_SCALE_CALLS = {  # B, H, Sq, Sk, D -> the kernel that runs it
+    (2, 3, 1, 704, 128): "KERNEL_FEW_ROWS", (2, 3, 3, 704, 64): "KERNEL_FEW_ROWS", (1, 3, 200, 1024, 128): "KERNEL_GENERAL",
+    (8, 20, 256, 512, 128): "KERNEL_GENERAL", (2, 3, 70, 448, 64): "KERNEL_GENERAL", (26, 12, 256, 320, 64): "KERNEL_WORKERS",
+    (18, 16, 256, 640, 64): "KERNEL_WORKERS"}
+
+
+@pytest.mark.parametrize("c2", LARGE_SCALES)
+@pytest.mark.parametrize("B,H,Sq,Sk,D", sorted(LARGE_SCALE_CALLS))
+def test_large_score_scales(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk, D, c2):
+    """Scores that are small whole numbers, so that a row's keys share their maximum with others of the same tile and of other tiles at
+    every scale, up to the largest that a call takes."""
+    torch = torch_cuda
+    rng = np.random.default_rng(Sk + D)
+    q8 = np.zeros((B, H, Sq, D), np.int8)
+    at = rng.integers(0, D, (B, H, Sq, 4))
+    np.put_along_axis(q8, at, rng.choice(np.array([-1, 1], np.int8), at.shape), -1)
+    k8 = rng.choice(np.array([-1, 0, 0, 0, 1], np.int8), (B, H, Sk, D))
+    v8 = np.clip(np.rint(rng.standard_normal((B, H, Sk, D)) * 40), -127, 127).astype(np.int8)
+    mask = (np.arange(Sk)[None, :] >= rng.integers(Sk // 2, Sk + 1, B)[:, None]).astype(np.int8)
+    each = float(np.sqrt(c2 * np.sqrt(D) * 127.0 ** 2 / np.log2(np.e)))          # q_amax and k_amax for that factor
+    # o_amax: where a level lies at a rounding boundary, all of a row's equal keys, 20 at the most here, move by one.  With the static
+    # scale that is v_amax / o_amax * s_max / 127 times the sum of their values (standard deviation 40 sqrt(20) = 180): 1.3 v_amax / o_amax for the
+    # largest s_max, three times that in the worst of some thousand rows; 2 with this o_amax.
+    amax = (each, each, 3.0, 6.0)
+    # s_max: nine tenths of the largest probability.  (With all of it, rows of two equal keys would have 127 / 2 to round.)
+    score = np.einsum("bid,bjd->bij", q8[:, 0].astype(np.float32), k8[:, 0].astype(np.float32)).astype(np.float64)
+    score[np.broadcast_to(mask[:, None, :] != 0, score.shape)] = -np.inf
+    s_max = 0.9 / float(np.exp2(c2 * (score - score.max(-1, keepdims=True))).sum(-1).min())
+    q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    o, ref = torch.full_like(q, 0x5A), torch.empty_like(q)
+    param, desc = pkg.FMHAParamI8(*amax, s_max), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D)
+    assert pkg.debug_plan(desc)[0] == getattr(pkg, LARGE_SCALE_CALLS[(B, H, Sq, Sk, D)])
+    pkg.FMHAInferI8Cross(None, param, desc, q, k, v, m, o)
+    got = o.cpu().numpy()
+    assert_parity(got[:, :1], oracle.q128(q8[:, :1], k8[:, :1], v8[:, :1], mask, amax), "against the oracle")
+    pkg.debug_simt_x(None, param, desc, q, k, v, m, ref)
+    assert_parity(got, ref.cpu().numpy(), "against the CUDA-core kernel")
+    pkg.FMHAInferI8Cross(None, param, desc, q, k, v, m, o, uint8_p=True)
+    assert_parity(o.cpu().numpy()[:, :1], oracle.q128(q8[:, :1], k8[:, :1], v8[:, :1], mask, amax, p_levels=255), "255 levels")
+    scratch = torch.zeros(2 * B * H * Sq, device="cuda")
+    for policy, which in ((pkg.POLICY_ROW, oracle.POLICY_ROW), (pkg.POLICY_STATIC, oracle.POLICY_STATIC)):
+        pkg.FMHAInferI8Policy(None, param, desc, q, k, v, m, o, policy, scratch)
+        assert_parity(o.cpu().numpy()[:, :1], oracle.policy(q8[:, :1], k8[:, :1], v8[:, :1], mask, (*amax, s_max), which), f"policy {policy}")
+    assert pkg.device_status()[0] == pkg.OK
