@@ -253,7 +253,10 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
     __syncwarp();
     if (lane == 0 && i + kQuantStages < mine) load(i + kQuantStages, slot, true);
   }
-  if (kTmem) tmem_wait_st();
+  if (kTmem) {
+    __syncwarp();
+    tmem_wait_st();
+  }
 #pragma unroll
   for (int k = 0; k < kQuantRest; ++k) m = fmaxf(m, fabsf(rest[k]));
 

@@ -271,8 +271,11 @@ __device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&r)[4])
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
                : "memory");
 }
-// Warp-collective load (complete on return) and store of 32 consecutive 32-bit columns per lane, as eight float4.
+// Warp-collective load (complete on return) and store of 32 consecutive 32-bit columns per lane, as eight float4.  The instructions ask for
+// lanes that run together, and the lanes of those who call these may have parted: in copies that one of them asks for, in values that
+// only some of them have to look at again.
 __device__ __forceinline__ void tmem_ld_tile(uint32_t taddr, float4 (&v)[8]) {
+  __syncwarp();
   uint32_t r[32];
   tmem_ld32(taddr, r);
 #pragma unroll
@@ -280,6 +283,7 @@ __device__ __forceinline__ void tmem_ld_tile(uint32_t taddr, float4 (&v)[8]) {
     v[i] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
 }
 __device__ __forceinline__ void tmem_st_tile(uint32_t taddr, const float4 (&v)[8]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "

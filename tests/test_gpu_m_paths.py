@@ -104,7 +104,7 @@ def test_quantize_sizes(pkg, oracle, torch_cuda, n):
 
 
 @pytest.mark.parametrize("n", [4099, 524289, 20 * SWEEP + 3])
-@pytest.mark.parametrize("what", ["nan", "inf", "tiny", "huge", "zero"])
+@pytest.mark.parametrize("what", ["nan", "one_lane", "inf", "tiny", "huge", "zero"])
 def test_quantize_values_that_are_no_ordinary_numbers(pkg, torch_cuda, n, what):
     """Elements that are no numbers, scales that are not finite or the largest there are: floor(x * scale + 0.5) limited to +-127 step by
     step in fp32, a NaN giving -127 (as the minimum and maximum of a number and a NaN are the number)."""
@@ -113,6 +113,9 @@ def test_quantize_values_that_are_no_ordinary_numbers(pkg, torch_cuda, n, what):
     x[n // 3] = -6.5
     if what == "nan":
         x[::1237] = float("nan")
+    elif what == "one_lane":         # one of the 32 lanes that share a tile of 1024 elements, another one in every tile
+        tiles = torch.arange(n // 1024, device="cuda")
+        x[1024 * tiles + 128 * (tiles % 8) + 4 * (tiles % 31)] = float("nan")
     elif what == "inf":
         x[n // 2], x[n - 1] = float("inf"), float("-inf")
     elif what == "tiny":

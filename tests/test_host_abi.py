@@ -142,3 +142,16 @@ def test_kernels_that_may_start_early_use_ordinary_loads():
                 seen += 1
                 assert "__restrict__" not in kernel[:kernel.index("{")], (name, kernel[:120])
     assert seen == 4                                    # the general, the head_dim-64 and the few-rows kernel, the quantiser's cluster
+
+
+def test_tensor_memory_instructions_of_the_quantiser_follow_a_convergence():
+    """Tensor-memory instructions are for warps whose lanes run together (.sync.aligned).  In the quantiser lanes part before them: one
+    asks for the next copy, and those with values that are no ordinary numbers quantise theirs again."""
+    csrc = os.path.join(ROOT, "int8-flash-attention-fmha-quantization_b200", "csrc")
+    ptx = open(os.path.join(csrc, "ptx.cuh")).read()
+    for name in ("tmem_ld_tile", "tmem_st_tile"):
+        body = ptx[ptx.index("void %s(" % name):]
+        assert body[body.index("{"):].split()[1] == "__syncwarp();", name
+    quant = open(os.path.join(csrc, "fmha_quant_sm100.cuh")).read()
+    others = re.findall(r"(\S+)\s+(tmem_(?!alloc|dealloc|relinquish|ld_tile|st_tile)\w+\()", quant)
+    assert others == [("__syncwarp();", "tmem_wait_st(")]
