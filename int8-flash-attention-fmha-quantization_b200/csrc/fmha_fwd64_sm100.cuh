@@ -52,6 +52,7 @@ constexpr uint32_t kOCol = 64;
 // What the workers need to know about a unit.
 struct UnitInfo {
   int n_live;                         // key tiles with at least one unmasked key, never none; -1: there are no more units
+  int last;                           // 1: no unit follows, of which the softmax warps then need not hear separately
   int rows;                           // query rows of the unit: 128, fewer in a head's last tile
   int64_t first_row;                  // of the slice's query rows, the unit's first
   uint8_t live[kMaxTiles];            // indices of the live key tiles, ascending
@@ -137,7 +138,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     if (!wait_or_fail(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO)) return;
     const int n_live = ctl->info[buf].n_live;
     if (n_live < 0) continue;
-    ++announced;
+    announced += 1 - ctl->info[buf].last;
     float m_run = -INFINITY, l_run = 0.f;
     int imax_run = static_cast<int>(kMagicBits);          // statistics launches: biased integer row maximum over all tiles
     RowConsts k;                                          // (policy launch: constant over a unit)
@@ -353,6 +354,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   };
 
   int taken = worker;                         // number of the unit to begin with; -1: ask for one
+  bool last = false;                          // the unit handed out last is known to be the last
   int it = -1, j = 0, n_live = 0;
   uint32_t u = 0u;                            // the unit of the step handed out last
   int bh = 0, batch = 0, q_row0 = 0;          // its head, sequence and first query row
@@ -368,7 +370,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   auto next_step = [&]() -> DriverStep {
     constexpr DriverStep none{-1, 0, false, 0, 0};
     while (j >= n_live) {
-      if (n_live < 0) return none;
+      if (n_live < 0 || last) return none;
       // The workers of a CTA take its units as they finish: with a fixed stride all wait for the one with the most tiles (B32 H12 S1024,
       // lengths 300..1024, 100.7 against 107.6 us; B256 H16 S256, 64..256, 91.8 against 94.8).
       if (taken < 0) {
@@ -400,7 +402,12 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
         --it;
         continue;
       }
+      // All units are taken when the counter says so.  A call of one round of workers knows it from the beginning, and need not ask for
+      // another unit nor announce that there is none while P.V of its last step waits: B8 H16 S512 18.4 -> 18.3 us, B4 H16 S1024
+      // 30.4 -> 30.3, B256 H16 S256 (64..256) 90.1 -> 89.4.
+      last = uniform(cta_unit(*reinterpret_cast<volatile int*>(&all->next)) >= static_cast<uint32_t>(p.n_units));
       if (elect_one()) {
+        info->last = last ? 1 : 0;
         info->rows = min(kTile, p.Sq - q_row0);
         info->first_row = static_cast<int64_t>(bh) * p.Sq + q_row0;
       }
