@@ -330,7 +330,7 @@ struct DriverStep {
   bool first;                // of its unit
   int bh, batch;
 };
-template <bool kStats>
+template <bool kStats, bool kEarlyK>
 __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const int worker, const CUtensorMap* map_q, const CUtensorMap* map_k,
                                             const CUtensorMap* map_v, const uint32_t tmem_base, const uint32_t worker_smem, uint8_t* presets) {
   WorkerCtl* ctl = &all->w[worker];
@@ -433,21 +433,28 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
     __syncwarp();
   };
 
-  // The first unit's Q rows and first K tile are asked for while its mask is still on the way (B32 H12 S512 38.0 -> 37.0 us).
+  // The first unit's Q rows, and with few key tiles to a unit its first K tile, are asked for while its mask is still on the way.  Both
+  // with many key tiles: B8 H16 S512 18.1 -> 18.3 us, the static policy there 31.7 -> 32.0.  Neither: B32 H12 S512 (256..512) 36.7 -> 37.4.
+  // Only Q with few: B200 H12 S128 22.6 -> 22.8.
   const uint32_t first = cta_unit(worker);
   const bool early = first < static_cast<uint32_t>(p.n_units);
   if (early && elect_one()) {
     const int head = static_cast<int>(first) / p.q_tiles;
-    mbar_arrive_expect_tx(smem_u32(&ctl->early_full), 2 * kTileBytes);
+    mbar_arrive_expect_tx(smem_u32(&ctl->early_full), kEarlyK ? 2 * kTileBytes : kTileBytes);
     tma_load_3d(q_smem, map_q, smem_u32(&ctl->early_full), 0, (static_cast<int>(first) - head * p.q_tiles) * kTile, head);
-    tma_load_3d(k_smem, map_k, smem_u32(&ctl->early_full), 0, 0, head);
+    if (kEarlyK) tma_load_3d(k_smem, map_k, smem_u32(&ctl->early_full), 0, 0, head);
   }
   __syncwarp();
   DriverStep cur = next_step();
   if (early) wait(smem_u32(&ctl->early_full), 0u, FMHA_I8_DEV_WAIT_Q_LOAD);
-  if (cur.tile == 0 && u == first) {
+  if (cur.tile >= 0 && u == first && (!kEarlyK || cur.tile == 0)) {
     if (elect_one()) {
-      mbar_arrive(smem_u32(&ctl->k_full));
+      if (kEarlyK) {
+        mbar_arrive(smem_u32(&ctl->k_full));
+      } else {
+        mbar_arrive_expect_tx(smem_u32(&ctl->k_full), kTileBytes);
+        tma_load_3d(k_smem, map_k, smem_u32(&ctl->k_full), 0, cur.tile * kTile, bh);
+      }
       mbar_arrive(smem_u32(&ctl->q_full));
     }
     __syncwarp();
@@ -571,7 +578,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     w64::softmax_role<kLaunch>(p, ctl, worker, tmem_base);
   } else {
     setmaxnreg_dec<kDriverRegs>();
-    driver_role<stats_launch(kLaunch)>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
+    driver_role<stats_launch(kLaunch), kLaunch == Launch::kForwardShort>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
   }
   tc_fence_before();
   __syncthreads();
