@@ -43,12 +43,40 @@ def test_back_to_back_calls_see_each_others_output(pkg, wl, torch_cuda, S, D):
     assert pkg.device_status()[0] == pkg.OK
 
 
-@pytest.mark.parametrize("what", ["few_rows", "policy", "policy_many"])
+# More query tiles than a round of the workers (592) holds, for each kernel and each form of the workers: launches of any length overlap.
+@pytest.mark.parametrize("B,H,S,D,kernel", [(40, 16, 128, 64, "KERNEL_WORKERS"), (21, 16, 320, 64, "KERNEL_WORKERS"), (9, 16, 1024, 64, "KERNEL_WORKERS"),
+                                            (40, 16, 128, 128, "KERNEL_GENERAL"), (14, 16, 384, 128, "KERNEL_GENERAL")])
+def test_long_launches_see_each_others_output(pkg, wl, torch_cuda, B, H, S, D, kernel):
+    """A chain of calls, each with the output of the one before as its queries and keys, gives what the same calls give with a
+    synchronisation between them."""
+    torch = torch_cuda
+    q8, _, v8, mask, amax = _tensors(wl, B, H, S, S, D, seed=S, valid=np.random.default_rng(S).integers(1, S + 1, B))
+    param, desc = pkg.FMHAParamI8(*amax[:3], amax[2] / 4, 1.0), pkg.AttnDataDescriptor(B, S, H, D)
+    plan = pkg.debug_plan(pkg.AttnDataDescriptorX(B, S, S, H, D))
+    assert plan[0] == getattr(pkg, kernel) and B * H * -(-S // 128) > 592
+    q, v, m = (torch.from_numpy(x).cuda() for x in (q8, v8, mask))
+    results = []
+    for wait in (True, False):
+        x, bufs = q, [torch.zeros_like(q) for _ in range(12)]
+        torch.cuda.synchronize()
+        for o in bufs:
+            pkg.FMHAInferI8(None, param, desc, x, x, v, m, o)
+            x = o
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        results.append(bufs)
+    for i, (a, b) in enumerate(zip(*results)):
+        assert a.any() and torch.equal(a, b), f"call {i} of the chain read its input too early"
+    assert pkg.device_status()[0] == pkg.OK
+
+
+@pytest.mark.parametrize("what", ["few_rows", "policy", "policy_many", "policy_rounds"])
 def test_buffers_rewritten_between_overlapping_launches(pkg, wl, torch_cuda, what):
     """One set of buffers, filled anew by every step's launches while the launches of the step before may still drain: the quantised
     query of a decoding step, the row statistics of a policy.  The outputs are those of steps with a synchronisation between them."""
     torch = torch_cuda
-    B, H, Sq, Sk, D = {"few_rows": (3, 5, 1, 704, 128), "policy": (1, 5, 100, 320, 64), "policy_many": (30, 13, 100, 192, 64)}[what]
+    B, H, Sq, Sk, D = {"few_rows": (3, 5, 1, 704, 128), "policy": (1, 5, 100, 320, 64), "policy_many": (30, 13, 100, 192, 64), "policy_rounds": (70, 13, 100, 192, 64)}[what]
     _, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, D, seed=Sq, valid=np.random.default_rng(B).integers(1, Sk, B))
     k, v, m = (torch.from_numpy(x).cuda() for x in (k8, v8, mask))
     desc, param = pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), pkg.FMHAParamI8(*amax, 1.0)
