@@ -358,9 +358,12 @@ void plan_parts(FwdParams* p, int D, const DeviceInfo* dev) {
 
 // Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  Cycles per key tile, measured: a CTA of
 // fmha_fwd_sm100.cuh works on one unit at a time, 1600 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5850 per
-// tile for all four, 4900 / 4350 / 3400 with three, two or one left in the last round.  (us, fmha_fwd_sm100.cuh / fmha_fwd64_sm100.cuh: B64 H16 S64
-// 14.9 / 12.5; B12 H12 S256 8.1 / 8.5, the estimate's worst error among these; B6 H12 S512 11.6 / 13.0; B16 H12 S512 28.8 / 27.8; B3 H12
-// S1024 18.4 / 22.0; B8 H12 S1024 44.3 / 47.7; B1 H24 S2048 45.5 / 45.2; B1 H40 S2048 67.2 / 82.1; B8 H32 S2048 368 / 343.)
+// tile for all four, 4900 / 4350 / 3400 with three, two or one left in the last round.  (The constants are from before the workers took
+// half tiles as such and units as they finish.  us, fmha_fwd_sm100.cuh / fmha_fwd64_sm100.cuh, measured since: B64 H16 S64 12.4 / 9.4, B64 H12 S128 11.3 / 11.5,
+// B200 H12 S128 23.9 / 22.4, B12 H12 S256 8.2 / 9.0 (the estimate's worst error among 32 shapes: it takes the workers there), B40 H12 S256 17.4 / 18.2,
+// B64 H16 S320 60.2 / 55.4, B6 H12 S512 11.5 / 13.0, B8 H16 S512 18.2 / 18.1, B16 H12 S512 25.0 / 26.1, B3 H12 S1024 18.1 / 21.2, B8 H12 S1024 43.9 / 45.7,
+// B16 H12 S1024 77.4 / 74.2, B1 H24 S2048 44.7 / 45.5, B1 H40 S2048 67.1 / 79.6, B8 H32 S2048 374 / 337; all but the first S256 within 5 % of the better one.
+// The launches of a policy go by the same line: B4 H16 S1024 (512..1024 keys) per-row 37.0 / 35.3, static 50.3 / 45.8; B3 H12 S1024 25.4 / 29.3, 34.4 / 37.5.)
 bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
   const long long sms = dev->sm_count, tiles = (p.S + kTile - 1) / kTile, round = sms * w64::kWorkers;
   const long long last[w64::kWorkers + 1] = {0, 3400, 4350, 4900, 5850};
@@ -396,9 +399,11 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mk, k, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mv, v, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
-  // Overlap takes the launch latency and the set-up of a launch out of the time of calls in a row.  (us without / with, more than four
-  // rounds of units: B32 H12 S512 D64 with lengths 256..512 38.5 / 36.3, B200 H12 S128 24.5 / 22.3, B4 H32 S1024 D128 59.6 / 57.1, B64 H32
-  // S256 79.4 / 76.2, B8 H32 S2048 428 / 423, D64 335.7 / 333.7; B256 H16 S256 D64 with lengths 64..256 85.6 / 85.4.)
+  // Overlap takes the launch latency and the set-up of a launch out of the time of calls in a row; a call that nothing precedes gains
+  // nothing.  (Per cent of the time with more than four rounds of units: B32 H12 S512 D64 with lengths 256..512 -6, B200 H12 S128 -9, B4 H32
+  // S1024 D128 -4, B64 H32 S256 -4, B8 H32 S2048 and B256 H16 S256 D64 with lengths 64..256 -1 to 0.)  Its price: the CTAs of the next launch
+  // take an SM as soon as this one leaves it, and wait there for the last of this one; a kernel of another stream that would have run
+  // on such SMs meanwhile comes after them.
   LaunchHow how;
   how.overlap = true;
   // persistent CTAs: one per SM (tensor memory is allocated whole), each walking its share of the units

@@ -8,26 +8,26 @@
 //   driver  = one warp per worker: mask scan, TMA copies, S = Q.K^T, P.V.
 //   tensor memory: 128 columns per worker.  S of a step; then its 8-bit P over the first 32 columns and P.V over the last 64.
 //   key tiles with unmasked keys in one half only are 64 keys: S has 64 columns, the softmax threads read 64, P.V takes two of its
-//             four steps.  B256 H16 S256 (lengths 64..256) 93.5 -> 87.2 us, B64 H16 S320 61.5 -> 56.2, B64 H16 S64 13.6 -> 12.0.
+//             four steps.  B256 H16 S256 (lengths 64..256) -7 %, B64 H16 S320 -9 %, B64 H16 S64 -12 %.
 //
 // A worker's step is one serial chain -- S, maximum, exponentials, P.V, fold -- of 3600 cycles when it runs alone.  Four of them
 // on an SM hide each other's latencies; nobody waits for a stage that other threads own, which is what bounds the other kernel
 // on short sequences (its merge warps need 4500 cycles per unit of two steps whatever the other warps do).  What bounds this
-// one: issue slots and the exponential unit, 61 % and 66 % busy on long sequences, where a step takes 5520 cycles, i.e. 1380 per
+// one: issue slots and the exponential unit, 62 % and 68 % busy on long sequences, where a step takes 5400 cycles, i.e. 1350 per
 // SM.  An eighth of the exponentials is computed on the multiply-add pipe (all on the exponential unit: 2.5 % slower on
 // B8 H32 S2048; a quarter: 3 % slower).  Pass 2 reads eight columns at a time: with sixteen the 104 registers of a softmax
 // thread do not suffice, and the spills cost 4 to 9 %.
-// Measured against the other kernel when it was new: B32 H12 S512 (lengths 256..512) 42.1 -> 39.3 us, B256 H16 S256 (64..256) 98 -> 90,
-// B8 H32 S2048 368 -> 343, B4 H16 S1024 with the per-row policy 52.4 -> 46.2; these take 36.8, 88 to 91, 339 and 35.5 now.
+// Measured against the other kernel: see use_workers().
 #pragma once
 #include "fmha_fwd_sm100.cuh"
 
 namespace fmha {
 namespace w64 {
 // The two forward passes, kForward and for units of up to kShortTiles key tiles kForwardShort, differ in how the maximum of a half tile
-// branches off that of a whole one: behind the first loads, which the compiler pays for with spilled values of the unit and makes a
-// faster step of, or in front of them.  us, behind / in front: B256 H16 S256 (lengths 64..256) 88.4 / 87.2, B200 H12 S128 25.4 / 24.6,
-// B64 H16 S320 57.1 / 56.2, B32 H12 S512 (256..512) 38.4 / 38.8, S576 (300..576) 53.4 / 54.3, B8 H32 S2048 336 / 346.
+// branches off that of a whole one: behind the first loads or in front of them.  Behind, the step is faster, and the compiler spills
+// values of the unit (-Xptxas -v: 72 bytes stored, 100 loaded, none in front), which short units pay for.  Behind against in front, in
+// per cent of the time: B256 H16 S256 (lengths 64..256) +1.4, B200 H12 S128 +3, B64 H16 S320 +1.6; B8 H16 S512 -2.3, B32 H12 S512 (256..512)
+// -2.6, S576 (300..576) -2.8, B1 H32 S2048 -4, B8 H32 S2048 -3.  (What is spilled is the compiler's choice: to be measured again when the step changes.)
 constexpr int kShortTiles = 3;
 constexpr int kD = 64;
 constexpr int kWorkers = 4;          // per CTA
@@ -297,8 +297,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     }
     // normalise, requantise, store (inc/fmha_i8.cuh:318-332)
     const float scale = p.scale_v_out * inv;
-    // (the clamp only where a warp has an output beyond 127: B256 H16 S256 with lengths 64..256 93.6 -> 92.0 us, B200 H12 S128
-    // 25.7 -> 24.8)
+    // (the clamp only where a warp has an output beyond 127: B256 H16 S256 with lengths 64..256 -1.7 %, B200 H12 S128 -3.5 %)
     const bool clamp = __any_sync(0xFFFFFFFFu, needs_clamp<kD / 2>(o2, scale));
     if (out_row >= 0) {
       int8_t* dst = p.o + out_row * kD;
@@ -372,7 +371,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
     while (j >= n_live) {
       if (n_live < 0 || last) return none;
       // The workers of a CTA take its units as they finish: with a fixed stride all wait for the one with the most tiles (B32 H12 S1024,
-      // lengths 300..1024, 100.7 against 107.6 us; B256 H16 S256, 64..256, 91.8 against 94.8).
+      // lengths 300..1024, -6 %; B256 H16 S256, 64..256, -3 %).
       if (taken < 0) {
         if (lane == 0) taken = atomicAdd(&all->next, 1);
         taken = uniform(taken);
@@ -403,8 +402,8 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
         continue;
       }
       // All units are taken when the counter says so.  A call of one round of workers knows it from the beginning, and need not ask for
-      // another unit nor announce that there is none while P.V of its last step waits: B8 H16 S512 18.4 -> 18.3 us, B4 H16 S1024
-      // 30.4 -> 30.3, B256 H16 S256 (64..256) 90.1 -> 89.4.
+      // another unit nor announce that there is none while P.V of its last step waits: -0.3 to -1 % for calls of one round, B256 H16 S256
+      // (64..256) -1 %.
       last = uniform(cta_unit(*reinterpret_cast<volatile int*>(&all->next)) >= static_cast<uint32_t>(p.n_units));
       if (elect_one()) {
         info->last = last ? 1 : 0;

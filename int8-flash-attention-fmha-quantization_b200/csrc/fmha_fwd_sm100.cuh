@@ -41,8 +41,8 @@
 //                and leaves it in [112,128)).
 //                These threads hold no output row, so they are light (64 registers).
 //
-// What bounds it: issue slots (64 % busy; 4300 warp instructions for a step of 128 x 128 scores at head_dim 128, 2700 of them
-// arithmetic) and the exponential unit (63 %), on a chain of hand-offs that the sets of buffers overlap; in units of one or two
+// What bounds it: issue slots (62 % busy; 4180 warp instructions for a step of 128 x 128 scores at head_dim 128, 2450 of them
+// arithmetic) and the exponential unit (64 %), on a chain of hand-offs that the sets of buffers overlap; in units of one or two
 // steps the merge warps, which spend more on a unit's epilogue than on a step.  B8 H32 S2048 D128: 405 us while the chip is cool enough
 // for 1965 MHz, 430 to 440 back to back, where the power limit holds it at 1820 to 1860.
 //
@@ -55,7 +55,7 @@
 // The padding mask goes the same way: where a key tile has masked keys, the issuer of S presets their columns to -2^127
 // instead (a second product, 2^100 * -2^27, that swallows the first).  The scores added to that bit pattern leave a float
 // of the same size (-2^126 at the least), below every real score as an integer and as a float.  Its exponential is zero,
-// or 2^-126 where the workers of fmha_fwd64_sm100.cuh compute it on the multiply-add pipe: nothing beside the row maximum's 1, and
+// or 2^-126 where the workers of fmha_fwd64_sm100.cuh compute it on the multiply-add pipe: nothing beside the row maximum's, which is 2^-32 at the least, and
 // quantised to zero.  (As long as 2^126 * c2 is large: kMinC2.)  The softmax threads treat every tile alike.  Before, they tested a mask bit per score in a loop that was not pipelined: B256 H16 S256
 // D64 with lengths 64..256 took 132 us instead of 115, B24 H16 S576 D64 with lengths 300..576 66 instead of 59, and the
 // smaller code makes unmasked head_dim-64 calls faster too (B8 H32 S2048: 430 -> 400 us).
@@ -215,7 +215,7 @@ struct FwdParams {
                                // all keys of exp(score - row maximum) (kRowMax: 0)} is written here, nothing to o
   const float2* row_stats_in;  // Launch::kRowPolicy, kStaticPolicy: those statistics, read back
   float p_row_mul;      // policy launch: P8 = rn(p_row_mul * exp(score - row max))                  ("dynamic", per-row scale), or
-  float p_static_mul;   //                P8 = min(rn(p_static_mul * exp(score - row max) / l), levels)  ("static" scale; 0 = dynamic)
+  float p_static_mul;   //                P8 = min(rn(p_static_mul * exp(score - row max) / l), levels)  ("static" scale)
   float p_levels;       // quantisation levels of P in a policy launch (127 in the reference's study)
                         // (a policy launch sets scale_v_out to the factor that turns sum_j P8 v8 [/ l] into int8 output units)
 };
@@ -390,8 +390,8 @@ __device__ __forceinline__ float2 exp2_poly(float2 a) {
 // A word's bytes are put together in pairs by the arithmetic that rounds them: kMagic + n1, times 256 and less 255 kMagic, is
 // kMagic + 256 n1, all exact, and adding 128 p0 to that rounds to kMagic + 256 n1 + n0, where 128 p0 alone would round (256 n1 is
 // even).  The two low bytes are the pair, as long as no byte is negative.  One byte permutation then makes a word of two pairs:
-// four instructions per word against two multiply-adds and three permutations, which run at half rate.  (B1 H32 S16384 D128 3248 -> 3166
-// us, B8 H32 S2048 441 -> 435 in one run, not more than the power limit's noise in others; B256 H16 S256 D64, 64..256 keys, 98.1 -> 97.3.)
+// four instructions per word against two multiply-adds and three permutations, which run at half rate.  (Long head_dim-128 sequences -1.4 to
+// -2.6 % in one run, within the power limit's noise in others; B256 H16 S256 D64, 64..256 keys, -0.8 %.)
 // kCap: p is limited to p_cap before it is quantised (the static policy clips at its top level, fmha_i8_quant_deviation.py:38-43).
 // kPolyPairs: that many pairs of values per eight are computed by exp2_poly.  kPack = false: only the sums are wanted.
 template <int N, bool kCap = false, int kPolyPairs = 0, bool kPack = true>
@@ -717,7 +717,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
       const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
       const float2 e_old2 = make_float2(e_old, e_old);
 
-      // ---- drain my half of O~ = bias -/+ (P8 . V) into the fp32 running row.  The partial output of step g lives in
+      // ---- drain my half of O~ = bias + P8 . V into the fp32 running row.  The partial output of step g lives in
       //      the accumulator S(g) came from: all of it at head_dim 128, columns [16,80) at head_dim 64.
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->o_full[sb]), (g / SBufs<D>::n) & 1u, abort_flag))) {
         raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_O_READY, g);

@@ -8,8 +8,8 @@
 //                         ring of bulk copies.  At the end of pass 1 the ring still holds each warp's last tiles, its
 //                         registers the first ones and its part of tensor memory the next (92 MB over the chip); pass 2
 //                         takes those from there and reads the others again, as far as it can from the L2.
-// 255,749 elements take 4.2 us, 67,108,864 take 78.4: DRAM, since pass 1 reads all 268 MB from there and pass 2 what neither the SMs
-// (92 MB) nor the L2 (50) kept.  Without tensor memory the latter take 84.2 us, and 33,554,432 elements 37.7 instead of 35.6.
+// 255,749 elements take 4.1 us, 67,108,864 take 74 to 78: DRAM, since pass 1 reads all 268 MB from there and pass 2 what neither the SMs
+// (92 MB) nor the L2 (some 50) kept, 126 MB.  Without tensor memory the latter take 7 % longer, 33,554,432 elements 6 %.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -158,7 +158,7 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
   uint64_t* bar = bars[warp];
 
   // warp w of CTA c takes tiles w * CTAs + c, then every (warps * CTAs)-th: the whole chip reads one stretch of memory
-  // at a time, and the last stretch is the one that pass 2 begins with
+  // at a time
   const int n_tiles = static_cast<int>(n / kQuantTile);
   const int stride = static_cast<int>(gridDim.x) * kQuantWarps, first = warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
   const int mine = first < n_tiles ? (n_tiles - first + stride - 1) / stride : 0;

@@ -56,8 +56,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 
 
-// About one second at boost clock.  No legitimate wait in these kernels is longer than the time
-// one CTA needs for one key tile (microseconds).
+// About one second at boost clock.  Most waits are for one key tile of one CTA (microseconds).  The longest are the softmax warps' of a
+// worker (fmha_fwd64_sm100.cuh) while its driver goes through a row of units without keys, of which they do not hear: 1.1 us a unit with
+// 64 keys, 8.8 with 32,768, measured, shared by the CTA's four workers.  As many such units as outputs fit into 180 GB (11 million of 8 KB with long
+// masks, 43 million of one row with short ones) are 0.2 s or less of it.
 constexpr long long kWaitLimitCycles = 2000000000LL;
 // A wait only gives up after this many probes as well: the cycle counter keeps running while the context is
 // switched out on a shared GPU, probes do not, so a long time slice elsewhere cannot by itself end a wait.
