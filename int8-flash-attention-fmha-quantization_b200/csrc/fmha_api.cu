@@ -3,6 +3,7 @@
 // (src/fmha_i8.cu:31-173): one runtime-shaped kernel instead of a table of compile-time shapes.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -356,20 +357,28 @@ void plan_parts(FwdParams* p, int D, const DeviceInfo* dev) {
   }
 }
 
-// Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  Cycles per key tile, measured: a CTA of
-// fmha_fwd_sm100.cuh works on one unit at a time, 1600 per tile and 1200 per unit; one of fmha_fwd64_sm100.cuh on four, 5850 per
-// tile for all four, 4900 / 4350 / 3400 with three, two or one left in the last round.  (The constants are from before the workers took
-// half tiles as such and units as they finish.  us, fmha_fwd_sm100.cuh / fmha_fwd64_sm100.cuh, measured since: B64 H16 S64 12.4 / 9.4, B64 H12 S128 11.3 / 11.5,
-// B200 H12 S128 23.9 / 22.4, B12 H12 S256 8.2 / 9.0 (the estimate's worst error among 32 shapes: it takes the workers there), B40 H12 S256 17.4 / 18.2,
-// B64 H16 S320 60.2 / 55.4, B6 H12 S512 11.5 / 13.0, B8 H16 S512 18.2 / 18.1, B16 H12 S512 25.0 / 26.1, B3 H12 S1024 18.1 / 21.2, B8 H12 S1024 43.9 / 45.7,
-// B16 H12 S1024 77.4 / 74.2, B1 H24 S2048 44.7 / 45.5, B1 H40 S2048 67.1 / 79.6, B8 H32 S2048 374 / 337; all but the first S256 within 5 % of the better one.
-// The launches of a policy go by the same line: B4 H16 S1024 (512..1024 keys) per-row 37.0 / 35.3, static 50.3 / 45.8; B3 H12 S1024 25.4 / 29.3, 34.4 / 37.5.)
-bool use_workers(const FwdParams& p, const DeviceInfo* dev) {
+// Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  In cycles, fitted to 221 shapes of 100 to 3500 query
+// tiles of 64 to 2048 keys: a CTA of fmha_fwd_sm100.cuh works on one unit at a time, 1530 per key tile and 650 per unit, 2900 at least (pairs that
+// share the last round: 980 and 3700); one of fmha_fwd64_sm100.cuh on four, 5350 per tile and 2500 for a round of four, 3100 / 3700 / 4700 /
+// 5850 and 2000 (one tile: 1200) for a last round of one to four, 600 for the call; the half tile of an odd multiple of 64 keys is six tenths there.  The kernel chosen is
+// 0.2 % slower than the better one on average, 3 % at the most, but for the smallest (100 units of 64 keys 5.45 / 5.1).  us, fmha_fwd_sm100.cuh /
+// fmha_fwd64_sm100.cuh, 160 units of 64 keys 6.2 / 5.25; 444 of 128 8.2 / 7.5; 296, 592, 740, 1184 of 256 8.3 / 9.0, 12.1 / 12.4, 14.05 / 16.0,
+// 19.7 / 19.6; 444 and 664 of 512 14.8 / 15.6, 21.3 / 24.3; 592 and 888 of 1024 31.2 / 30.2, 44.8 / 46.25; 592 and 1184 of 2048 58.1 / 54.6, 110.5 / 102.6.
+//
+// The launches of a policy and of a calibration have a line of their own (1600 and 1200; 5850, 4900 / 4350 / 3400 per tile): the general kernel gains
+// less from a statistics launch.  Both launches, per-row and static, us: B4 H16 S1024 (512..1024 keys) 37.0 / 35.3, 50.3 / 45.8; B8 H16 S512 27.1 / 25.0,
+// 35.9 / 32.3; B1 H32 S2048 75.0 / 70.8, 108.9 / 97.3; B3 H12 S1024 25.4 / 29.3, 34.4 / 37.5.
+bool use_workers(const FwdParams& p, bool plain, const DeviceInfo* dev) {
   const long long sms = dev->sm_count, tiles = (p.S + kTile - 1) / kTile, round = sms * w64::kWorkers;
-  const long long last[w64::kWorkers + 1] = {0, 3400, 4350, 4900, 5850};
-  const long long workers = p.n_units / round * 5850 + last[(p.n_units % round + sms - 1) / sms];
-  const long long own = p.n_units / sms, more = p.n_units % sms != 0, unit = 1600 * tiles + 1200;
-  return workers * tiles < own * unit + more * (pairs_share_last_round(p, dev) ? unit / 2 + 4500 : unit);
+  const long long own = p.n_units / sms, more = p.n_units % sms != 0, full = p.n_units / round, last = (p.n_units % round + sms - 1) / sms;
+  if (plain) {
+    const long long per_tile[w64::kWorkers + 1] = {0, 3100, 3700, 4700, 5850};
+    const long long tenths = 10 * tiles - (p.S % kTile != 0 ? 4 : 0), unit = std::max(1530 * tiles + 650, 2900LL);
+    const long long workers = 600 + full * (535 * tenths + 2500) + (last > 0 ? per_tile[last] * tenths / 10 + (tiles > 1 ? 2000 : 1200) : 0);
+    return workers < own * unit + more * (pairs_share_last_round(p, dev) ? 980 * tiles + 3700 : unit);
+  }
+  const long long per_tile[w64::kWorkers + 1] = {0, 3400, 4350, 4900, 5850}, unit = 1600 * tiles + 1200;
+  return (full * 5850 + per_tile[last]) * tiles < own * unit + more * (pairs_share_last_round(p, dev) ? unit / 2 + 4500 : unit);
 }
 
 // Few query rows run the few-rows kernel.  Up to four rows it is bound by reading K and V; from five on (computed as eight) its integer dot
@@ -387,7 +396,7 @@ bool few_rows(int Sq, int S, int D) { return Sq <= 4 || (D == 64 && Sq <= kDecod
 int plan_call(FwdParams* p, int D, bool plain, int busy_sms, const DeviceInfo* dev) {
   p->parts = 1;
   if (plain && few_rows(p->Sq, p->S, D)) return FMHA_I8_KERNEL_FEW_ROWS;
-  if (D == 64 && use_workers(*p, dev)) return FMHA_I8_KERNEL_WORKERS;
+  if (D == 64 && use_workers(*p, plain, dev)) return FMHA_I8_KERNEL_WORKERS;
   if (plain && busy_sms == 0) plan_parts(p, D, dev);
   return FMHA_I8_KERNEL_GENERAL;
 }

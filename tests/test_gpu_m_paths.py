@@ -44,7 +44,7 @@ def test_back_to_back_calls_see_each_others_output(pkg, wl, torch_cuda, S, D):
 
 
 # More query tiles than a round of the workers (592) holds, for each kernel and each form of the workers: launches of any length overlap.
-@pytest.mark.parametrize("B,H,S,D,kernel", [(40, 16, 128, 64, "KERNEL_WORKERS"), (21, 16, 320, 64, "KERNEL_WORKERS"), (9, 16, 1024, 64, "KERNEL_WORKERS"),
+@pytest.mark.parametrize("B,H,S,D,kernel", [(60, 16, 128, 64, "KERNEL_WORKERS"), (21, 16, 320, 64, "KERNEL_WORKERS"), (9, 16, 1024, 64, "KERNEL_WORKERS"),
                                             (40, 16, 128, 128, "KERNEL_GENERAL"), (14, 16, 384, 128, "KERNEL_GENERAL")])
 def test_long_launches_see_each_others_output(pkg, wl, torch_cuda, B, H, S, D, kernel):
     """A chain of calls, each with the output of the one before as its queries and keys, gives what the same calls give with a
@@ -618,7 +618,7 @@ def test_rows_of_empty_units(pkg, wl, oracle, torch_cuda, open_batches, what):
 LARGE_SCALES = [0.0031, 0.077, 0.317, 0.931, 2.37, 3.13, 10.7, 49.3, 71.9, 1.3e4, 1.1e15, 1.7e31]
 LARGE_SCALE_CALLS = {  # B, H, Sq, Sk, D -> the kernel that runs it
     (2, 3, 1, 704, 128): "KERNEL_FEW_ROWS", (2, 3, 3, 704, 64): "KERNEL_FEW_ROWS", (1, 3, 200, 1024, 128): "KERNEL_GENERAL",
-    (8, 20, 256, 512, 128): "KERNEL_GENERAL", (2, 3, 70, 448, 64): "KERNEL_GENERAL", (26, 12, 256, 320, 64): "KERNEL_WORKERS",
+    (8, 20, 256, 512, 128): "KERNEL_GENERAL", (2, 3, 70, 448, 64): "KERNEL_GENERAL", (40, 12, 256, 320, 64): "KERNEL_WORKERS",
     (18, 16, 256, 640, 64): "KERNEL_WORKERS"}
 
 
