@@ -361,7 +361,7 @@ void plan_parts(FwdParams* p, int D, const DeviceInfo* dev) {
 // tiles of 64 to 2048 keys: a CTA of fmha_fwd_sm100.cuh works on one unit at a time, 1530 per key tile and 650 per unit, 2900 at least (pairs that
 // share the last round: 980 and 3700); one of fmha_fwd64_sm100.cuh on four, 5350 per tile and 2500 for a round of four, 3100 / 3700 / 4700 /
 // 5850 and 2000 (one tile: 1200) for a last round of one to four, 600 for the call; the half tile of an odd multiple of 64 keys is six tenths there.  The kernel chosen is
-// 0.2 % slower than the better one on average, 3 % at the most, but for the smallest (100 units of 64 keys 5.45 / 5.1).  us, fmha_fwd_sm100.cuh /
+// 0.2 % slower than the better one on average, 4 % at the most, but for the smallest (100 units of 64 keys 5.45 / 5.1).  us, fmha_fwd_sm100.cuh /
 // fmha_fwd64_sm100.cuh, 160 units of 64 keys 6.2 / 5.25; 444 of 128 8.2 / 7.5; 296, 592, 740, 1184 of 256 8.3 / 9.0, 12.1 / 12.4, 14.05 / 16.0,
 // 19.7 / 19.6; 444 and 664 of 512 14.8 / 15.6, 21.3 / 24.3; 592 and 888 of 1024 31.2 / 30.2, 44.8 / 46.25; 592 and 1184 of 2048 58.1 / 54.6, 110.5 / 102.6.
 //

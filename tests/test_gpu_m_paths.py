@@ -660,3 +660,16 @@ def test_large_score_scales(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk, D, c2):
         pkg.FMHAInferI8Policy(None, param, desc, q, k, v, m, o, policy, scratch)
         assert_parity(o.cpu().numpy()[:, :1], oracle.policy(q8[:, :1], k8[:, :1], v8[:, :1], mask, (*amax, s_max), which), f"policy {policy}")
     assert pkg.device_status()[0] == pkg.OK
+
+
+# Query tiles of S keys on either side of the line between the two head_dim-64 kernels (on 148 SMs), and the policies' own line.
+@pytest.mark.parametrize("units,S,forward,policy", [
+    (100, 64, "GENERAL", "GENERAL"), (296, 128, "WORKERS", "WORKERS"), (296, 256, "GENERAL", "WORKERS"), (520, 256, "WORKERS", "WORKERS"),
+    (740, 256, "GENERAL", "WORKERS"), (1184, 256, "WORKERS", "WORKERS"), (444, 512, "GENERAL", "WORKERS"), (592, 1024, "WORKERS", "WORKERS"),
+    (288, 1024, "GENERAL", "GENERAL"), (1184, 2048, "WORKERS", "WORKERS")])
+def test_line_between_the_kernels_of_head_dim_64(pkg, torch_cuda, units, S, forward, policy):
+    if torch_cuda.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line lies elsewhere on another number of SMs")
+    desc = pkg.AttnDataDescriptorX(units * 128 // max(S, 128), S, S, 1, 64)
+    assert pkg.debug_plan(desc)[0] == getattr(pkg, "KERNEL_" + forward)
+    assert pkg.debug_plan(desc, pkg.POLICY_ROW)[0] == getattr(pkg, "KERNEL_" + policy)
