@@ -346,6 +346,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   const uint64_t d_a = preset_desc(preset_smem, 0), d_b = preset_desc(preset_smem, 1);
   const uint64_t dq = make_smem_desc(q_smem, kD), dk = make_smem_desc(k_smem, kD), dv = make_smem_desc(v_smem, kD);
   const int n_tiles = (p.S + kTile - 1) / kTile;
+  const bool lead = elect_one();
   uint32_t fail = 0u, g = 0, units = 0;
   auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
     if (warp_wait(bar, parity, abort_flag)) return true;
@@ -471,20 +472,24 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
 #pragma unroll
       for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || mask_row[key0 + 32 * i] != 0;
     }
+    // What the MMAs need is formed and kept in registers before the waits that they follow (the compiler would form it where it is used): 120 of the
+    // 290 cycles from S's buffer being free to its last instruction.  B8 H32 S2048 334.7 -> 332.6 us, B256 H16 S256 (64..256) 86.7 -> 85.7, B32 H12 S512
+    // (256..512) 36.3 -> 36.0.  (The instructions under a predicate instead of a branch: +2 %.)
+    // The tile's preset operand: the common one, or this worker's own, which nothing has read since the last S.
+    const uint32_t operand = mixed ? 2u + static_cast<uint32_t>(worker) : 1u;
+    if (mixed) fill_mask_operand(presets + operand * kPresetBytes, masked, 128);
+    uint64_t d_preset = preset_desc(preset_smem, operand), d_k = desc_advance(dk, row0 * kD), d_v = desc_advance(dv, row0 * kD);
+    uint32_t idesc_preset = whole ? idesc_preset_s : idesc_preset_half, idesc = whole ? idesc_s : idesc_half;
+    asm volatile("" : "+l"(d_preset), "+l"(d_k), "+l"(d_v), "+r"(idesc_preset), "+r"(idesc));
     if (cur.first && !wait(smem_u32(&ctl->q_full), units++ & 1u, FMHA_I8_DEV_WAIT_Q_LOAD)) break;
     if (!wait(smem_u32(&ctl->k_full), g & 1u, FMHA_I8_DEV_WAIT_K_LOAD)) break;
     if (g > 0u && !wait(smem_u32(&ctl->s_free), (g - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
     tc_fence_after();
     FMHA_STAMP(16 + worker * 4 + 0, g);
-    // the tile's preset operand: the common one, or this worker's own, which nothing has read since the last S
-    const uint32_t operand = mixed ? 2u + static_cast<uint32_t>(worker) : 1u;
-    if (mixed) fill_mask_operand(presets + operand * kPresetBytes, masked, 128);
-    const uint64_t d_preset = preset_desc(preset_smem, operand);
-    if (elect_one()) {
-      const uint32_t idesc_preset = whole ? idesc_preset_s : idesc_preset_half, idesc = whole ? idesc_s : idesc_half;
+    if (lead) {
       mma_f16_ss(tS, d_a, d_preset, idesc_preset, 0u);        // accumulator := 0x4B400000, masked keys -2^127
 #pragma unroll
-      for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(dk, row0 * kD + kk * 32), idesc, 1u);
+      for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(d_k, kk * 32), idesc, 1u);
       mma_commit(smem_u32(&ctl->s_full));
       if (!kStats) {
         mbar_arrive_expect_tx(smem_u32(&ctl->v_full), kTileBytes);
@@ -500,10 +505,10 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
       if (!wait(smem_u32(&ctl->p_ready), g & 1u, FMHA_I8_DEV_WAIT_P_READY)) break;
       tc_fence_after();
       FMHA_STAMP(16 + worker * 4 + 2, g);
-      if (elect_one()) {
+      if (lead) {
         mma_f16_ss(tO, d_a, d_b, idesc_preset_o, 0u);
 #pragma unroll
-        for (int kk = 0; kk < kTile / 64; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, (row0 + kk * 32) * kD), idesc_o, 1u);
+        for (int kk = 0; kk < kTile / 64; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(d_v, kk * 32 * kD), idesc_o, 1u);
         if (whole) {
 #pragma unroll
           for (int kk = kTile / 64; kk < kTile / 32; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);

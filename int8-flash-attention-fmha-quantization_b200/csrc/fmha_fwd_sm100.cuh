@@ -991,6 +991,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   constexpr uint32_t idesc_s = make_idesc_i8(kTile, false);   // S = Q.K^T : N = 128 keys, both K-major
   constexpr uint32_t idesc_bias_s = make_idesc_bf16(kTile);
   const uint64_t d_bias_a = make_smem_desc_noswizzle(smem_u32(bias_a), 128, 256);
+  const bool lead = elect_one();
   IssuerErr err;
   uint32_t g = 0, qn = 0;
   bool ok = true;
@@ -1011,8 +1012,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
     const int8_t* mask_row = p.mask + static_cast<int64_t>(unit_geom(p, u).batch) * p.S;
     for (int j = 0; j < n_live; ++j, ++g) {
       const uint32_t sb = g % SBufs<D>::n, stage = g % NK;
-      const uint64_t dk = make_smem_desc(k_smem + stage * Cfg::kTileBytes, D);
-      const uint32_t tS = tmem_base + sb * kTile;
+      uint32_t tS = tmem_base + sb * kTile;
       const bool mixed = info->kind[info->begin + j] != 0;
       bool masked[4] = {};
       if (mixed) {
@@ -1023,21 +1023,29 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       // K first (it has normally been there for a while), then the accumulator: it still holds the partial output of
       // step g - n until the merge warps have drained it, and that hand-off is on the step-to-step critical path
       if (!issuer_wait(err, smem_u32(&ctl->k_full[stage]), (g / NK) & 1u, FMHA_I8_DEV_WAIT_K_LOAD, g, abort_flag)) { ok = false; break; }
+      // What the MMAs need is formed and kept in registers before the wait that they follow; the compiler would form it where it is used, a
+      // hundred cycles on the step-to-step path (here and for P.V, head_dim 128: B8 H32 S2048 425 -> 417 us, B4 H32 S1024 59.1 -> 58.1, B2 H16 Sq200 Sk1984
+      // 15.7 -> 15.4).
+      // The tile's preset operand: the common one, or this accumulator's own, which nothing has read since S of step g - n; that has completed,
+      // or K of this step would not be there
+      static_assert(Cfg::kStagesK <= SBufs<D>::n, "K of a step may land before S of step g - n has completed");
+      const uint32_t b_index = mixed ? 1 + sb : 0u;
+      if (mixed) fill_mask_operand(bias_a + (1 + b_index) * kBiasBytes, masked);
+      uint64_t d_bias_b = make_smem_desc_noswizzle(smem_u32(bias_a) + (1 + b_index) * kBiasBytes, 128, 256);
+      uint64_t dk = make_smem_desc(k_smem + stage * Cfg::kTileBytes, D);
+      uint32_t bar_s = smem_u32(&ctl->s_full[sb]), bar_k = smem_u32(&ctl->k_empty[stage]), bar_q = j == n_live - 1 ? smem_u32(&ctl->q_empty[qb]) : 0u;
+      asm volatile("" : "+l"(d_bias_b), "+l"(dk), "+r"(tS), "+r"(bar_s), "+r"(bar_k), "+r"(bar_q));
       if (g >= SBufs<D>::n && !issuer_wait(err, smem_u32(&ctl->s_free[sb]), ((g / SBufs<D>::n) - 1) & 1u, FMHA_I8_DEV_WAIT_O_FREE, g, abort_flag)) { ok = false; break; }
       FMHA_STAMP(15, g);
       tc_fence_after();
-      // the tile's preset operand: the common one, or this accumulator's own, which nothing has read since step g - n
-      const uint32_t b_index = mixed ? 1 + sb : 0u;
-      if (mixed) fill_mask_operand(bias_a + (1 + b_index) * kBiasBytes, masked);
-      const uint64_t d_bias_b = make_smem_desc_noswizzle(smem_u32(bias_a) + (1 + b_index) * kBiasBytes, 128, 256);
-      if (elect_one()) {
+      if (lead) {
         mma_f16_ss(tS, d_bias_a, d_bias_b, idesc_bias_s, 0u);      // accumulator := 0x4B400000, masked keys -2^127
 #pragma unroll
         for (int kk = 0; kk < D / 32; ++kk)
           mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(dk, kk * 32), idesc_s, 1u);
-        mma_commit(smem_u32(&ctl->s_full[sb]));
-        mma_commit(smem_u32(&ctl->k_empty[stage]));
-        if (j == n_live - 1) mma_commit(smem_u32(&ctl->q_empty[qb]));                   // that was the unit's last use of its Q rows
+        mma_commit(bar_s);
+        mma_commit(bar_k);
+        if (bar_q != 0u) mma_commit(bar_q);                   // that was the unit's last use of its Q rows
       }
       FMHA_STAMP(12, g);
     }
@@ -1061,6 +1069,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   constexpr uint32_t idesc_bias = make_idesc_bf16(D);
   const uint64_t d_bias_a = make_smem_desc_noswizzle(bias_a_smem, 128, 256);
   const uint64_t d_bias_b = make_smem_desc_noswizzle(bias_b_smem, 128, 256);
+  const bool lead = elect_one();
   IssuerErr err;
   uint32_t g = 0;
   bool ok = true;
@@ -1073,10 +1082,12 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
     if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));            // only the tile count is needed here
     for (int j = 0; !kStats && j < n_live; ++j, ++g) {
       const uint32_t sb = g % SBufs<D>::n, stage = g % NV;
-      const uint64_t dv = make_smem_desc(v_smem + stage * Cfg::kTileBytes, D);
+      uint64_t dv = make_smem_desc(v_smem + stage * Cfg::kTileBytes, D);
       const uint32_t tS = tmem_base + sb * kTile;
-      const uint32_t tP = PLayout<D>::kAnnex ? tmem_base + SBufs<D>::n * kTile + sb * PLayout<D>::kAnnexCols : tS;
-      const uint32_t tO = tS + PLayout<D>::kOOff;
+      uint32_t bar_o = smem_u32(&ctl->o_full[sb]), bar_v = smem_u32(&ctl->v_empty[stage]);
+      uint32_t tP = PLayout<D>::kAnnex ? tmem_base + SBufs<D>::n * kTile + sb * PLayout<D>::kAnnexCols : tS;
+      uint32_t tO = tS + PLayout<D>::kOOff;
+      asm volatile("" : "+l"(dv), "+r"(tP), "+r"(tO), "+r"(bar_o), "+r"(bar_v));
       // V first (loaded steps ago), then P: the MMAs go out as soon as the last softmax warp has arrived
       if (!issuer_wait(err, smem_u32(&ctl->v_full[stage]), (g / NV) & 1u, FMHA_I8_DEV_WAIT_V_LOAD, g, abort_flag)) { ok = false; break; }
       if (!issuer_wait(err, smem_u32(&ctl->p_ready[g & 3u]), (g >> 2) & 1u, FMHA_I8_DEV_WAIT_P_READY, g, abort_flag)) { ok = false; break; }
@@ -1084,13 +1095,13 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       tc_fence_after();
       // The accumulator of this step is S(g)'s own buffer (free since the softmax threads have read S(g)), minus the
       // columns that hold P bytes at head_dim 64.
-      if (elect_one()) {
+      if (lead) {
         mma_f16_ss(tO, d_bias_a, d_bias_b, idesc_bias, 0u);      // accumulator := 0x4B400000
 #pragma unroll
         for (int kk = 0; kk < kTile / 32; ++kk)
           mma_i8_ts(tO, tP + PLayout<D>::p_col(kk), desc_advance(dv, kk * 32 * D), idesc_o, 1u);
-        mma_commit(smem_u32(&ctl->o_full[sb]));
-        mma_commit(smem_u32(&ctl->v_empty[stage]));
+        mma_commit(bar_o);
+        mma_commit(bar_v);
       }
       FMHA_STAMP(14, g);
     }

@@ -56,42 +56,52 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 
 
-// About one second at boost clock.  Most waits are for one key tile of one CTA (microseconds).  The longest are the softmax warps' of a
+// The limits of a wait: about one second at boost clock, and probes that take one and a half, since one that finds the phase incomplete
+// blocks for 2911 cycles, measured.  (The kernels' waits are counted and not timed: while the context is switched out on a shared GPU no probes
+// are made, so a long time slice elsewhere cannot end a wait.)  Most waits are for one key tile of one CTA (microseconds).  The longest are the softmax warps' of a
 // worker (fmha_fwd64_sm100.cuh) while its driver goes through a row of units without keys, of which they do not hear: 1.1 us a unit with
 // 64 keys, 8.8 with 32,768, measured, shared by the CTA's four workers.  As many such units as outputs fit into 180 GB (11 million of 8 KB with long
-// masks, 43 million of one row with short ones) are 0.2 s or less of it.
+// masks, 43 million of one row with short ones) are 0.2 s or less.
 constexpr long long kWaitLimitCycles = 2000000000LL;
-// A wait only gives up after this many probes as well: the cycle counter keeps running while the context is
-// switched out on a shared GPU, probes do not, so a long time slice elsewhere cannot by itself end a wait.
-constexpr uint32_t kMinProbes = 4096u;
+constexpr uint32_t kWaitProbes = 1u << 20;
 
-// Waits for the phase with the given parity to complete.  Gives up when the cycle limit is reached (and at
-// least min_probes probes were made) or when another thread of the CTA has already raised *abort_flag.
-// The loop is deliberately not tight: mbarrier.try_wait returns after a short, hardware-defined time when the phase is not
-// complete, and measured on B200 a waiting warp that probes as fast as it can (three instructions per probe) slows the working warps
-// of its SM down more than this one does, while nanosleep between probes costs more latency on the hand-offs than it saves
-// (any argument up to 80 ns sleeps equally long).
-__device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, const volatile int* abort_flag, long long limit_cycles,
-                                                  uint32_t min_probes = 0u) {
+// Waits for the phase with the given parity to complete.  Gives up when the cycle limit is reached or when another thread of the CTA has
+// already raised *abort_flag.
+__device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, const volatile int* abort_flag, long long limit_cycles) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 31u) == 0u) {
       if (*abort_flag) return false;
-      if (it >= min_probes && clock64() - t0 > limit_cycles) return false;
+      if (clock64() - t0 > limit_cycles) return false;
     }
   }
 }
+// The same with kWaitProbes for the limit, in as few instructions as can be: the kernels have some twenty waits each, and how far their code
+// is spread costs them time (with the cycle counter read and a first probe in front of the loop, as above, B64 H32 S256 D128 took 82.9 us instead of
+// 77.8, B256 H16 S256 D64, 64..256 keys, 88.6 instead of 86.0, B8 H32 S2048 D128 424 instead of 419.5; the loop left to the compiler 78.6, 87.1 and 421.7).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
-  return mbar_wait_limited(bar, parity, abort_flag, kWaitLimitCycles, kMinProbes);
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 left, flag;\n\t"
+      "mov.u32 left, %4;\n"
+      "WAIT_%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra DONE_%=;\n\t"
+      "ld.volatile.shared.u32 flag, [%3];\n\t"
+      "sub.u32 left, left, 1;\n\t"
+      "setp.eq.u32 q, flag, 0;\n\t"
+      "setp.ne.and.u32 q, left, 0, q;\n\t"
+      "@q bra WAIT_%=;\n"
+      "DONE_%=:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kWaitProbes)
+      : "memory");
+  return ok != 0u;
 }
-
-// Warp-wide wait of the head_dim-64 workers: most of their waits find the phase complete, and without the loop around the
-// first probe that costs three instructions (B8 H32 S2048: 345 -> 342 us).  Not for the other kernel: at head_dim 128 it is as
-// fast for long sequences, but its short units get 3 % slower.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
-  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag));
 }
 
