@@ -105,10 +105,10 @@ int fmha_i8_sm100_infer_cross(void* stream, const float amax[5], const int desc5
  *   FMHA_I8_POLICY_STATIC  "static quantization": P8 = min(rn(127 p / s_max), 127) with ONE calibrated scale for
  *                          every row: amax[4] = s_max, the FMHAParamI8 field the reference fills
  *                          (test_fmha_i8.cpp:152) and never reads (README.md:27; :82-102 of the script)
- * P is unsigned with 127 levels as in the study.  A row's scale is only known when all its keys have been seen, so
- * the call makes two launches on `stream`: the first computes every row's maximum (for the static scale its
- * exp-sum too), the second quantises and multiplies.  row_scratch: caller-owned device memory, 2 floats per query row of the slice
- * (8 * bh_count * seq_len_q bytes, 8-byte aligned); nothing is allocated.  Other arguments as in
+ * P is unsigned with 127 levels as in the study.  A row's scale is only known when all its keys have been seen: one
+ * launch goes over them twice.  row_scratch: caller-owned device memory, 2 floats per query row of the slice
+ * (8 * bh_count * seq_len_q bytes, 8-byte aligned), for the rows' statistics; its contents after the call are not specified (the
+ * present kernel keeps the statistics on the chip and leaves it as it is).  Nothing is allocated.  Other arguments as in
  * fmha_i8_sm100_infer_cross; FMHA_I8_FLAG_UINT8_P is not accepted. */
 #define FMHA_I8_POLICY_TILE 0
 #define FMHA_I8_POLICY_ROW 1
@@ -148,7 +148,9 @@ int fmha_i8_sm100_infer_host_slice(const float amax[5], const int desc[4],
 
 /* Debug: how a call on this device would run, without running it: plan[0] = the kernel, plan[1] = CTAs that share the key tiles of a
  * query tile (1: none do), plan[2] = whole rounds of query tiles, one per SM, in front of the shared ones.  desc5 as in
- * fmha_i8_sm100_infer_cross (all heads), policy as in fmha_i8_sm100_infer_policy. */
+ * fmha_i8_sm100_infer_cross (all heads), policy as in fmha_i8_sm100_infer_policy: the plan of FMHA_I8_POLICY_TILE is that of the forward pass,
+ * that of the others the calibration's (fmha_i8_sm100_calibrate_o_amax); the whole-row policies themselves have one kernel without
+ * variants, csrc/fmha_policy_sm100.cuh. */
 #define FMHA_I8_KERNEL_FEW_ROWS 0   /* csrc/fmha_decode_sm100.cuh */
 #define FMHA_I8_KERNEL_GENERAL 1    /* csrc/fmha_fwd_sm100.cuh */
 #define FMHA_I8_KERNEL_WORKERS 2    /* csrc/fmha_fwd64_sm100.cuh */

@@ -14,7 +14,7 @@ LIB = os.path.join(HERE, "libfmha_i8_sm100.so")
 BINDING = os.path.join(HERE, "_fmha_i8_py.so")
 BINDING_SOURCE = os.path.join(CSRC, "py_binding.cpp")
 SOURCES = ["fmha_api.cu"]
-HEADERS = ["ptx.cuh", "fmha_fwd_sm100.cuh", "fmha_debug_sm100.cuh", "fmha_quant_sm100.cuh", "fmha_decode_sm100.cuh", "fmha_fwd64_sm100.cuh", "fmha_host_sm100.cuh",
+HEADERS = ["ptx.cuh", "fmha_fwd_sm100.cuh", "fmha_debug_sm100.cuh", "fmha_quant_sm100.cuh", "fmha_decode_sm100.cuh", "fmha_fwd64_sm100.cuh", "fmha_policy_sm100.cuh", "fmha_host_sm100.cuh",
            os.path.join("..", "..", "include", "fmha_i8_c.h"),
            os.path.join("..", "..", "include", "fmha_i8.h"),
            os.path.join("..", "..", "include", "fmha_param_i8.h")]

@@ -18,6 +18,7 @@
 #include "fmha_fwd64_sm100.cuh"
 #include "fmha_fwd_sm100.cuh"
 #include "fmha_host_sm100.cuh"
+#include "fmha_policy_sm100.cuh"
 #include "fmha_quant_sm100.cuh"
 
 namespace {
@@ -114,6 +115,17 @@ template <typename Set> void set_decode_attributes(Set set) {
   one(std::integral_constant<int, 64>(), std::integral_constant<int, 8>());
 }
 
+// Calls use(kernel, bytes of shared memory, registers per thread at launch) for every instance of the whole-row policies' kernel.
+template <typename Use> void for_policy_kernels(Use use) {
+  auto one = [&](auto d) {
+    constexpr int D = decltype(d)::value;
+    use(reinterpret_cast<const void*>(&wholerow::policy_kernel<D, false>), wholerow::smem_bytes<D>(), wholerow::kLaunchRegs);
+    use(reinterpret_cast<const void*>(&wholerow::policy_kernel<D, true>), wholerow::smem_bytes<D>(), wholerow::kLaunchRegs);
+  };
+  one(std::integral_constant<int, 64>());
+  one(std::integral_constant<int, 128>());
+}
+
 int set_kernel_attributes(DeviceInfo* d) {
   if (d->attr_set.load(std::memory_order_acquire)) return FMHA_I8_OK;
   std::lock_guard<std::mutex> lock(g_dev_mutex);
@@ -122,17 +134,13 @@ int set_kernel_attributes(DeviceInfo* d) {
   auto set = [&](const void* fn, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   };
-  const void* const general64[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kForward>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowMax>),
-                                   reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kRowPolicy>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, Launch::kStaticPolicy>)};
-  const void* const general128[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kForward>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowMax>),
-                                    reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowStats>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kRowPolicy>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, Launch::kStaticPolicy>)};
-  for (const void* fn : general64) set(fn, fwd_smem_bytes<64>());
-  for (const void* fn : general128) set(fn, fwd_smem_bytes<128>());
+  const void* const general64 = reinterpret_cast<const void*>(&fmha_fwd_kernel<64>), * const general128 = reinterpret_cast<const void*>(&fmha_fwd_kernel<128>);
+  set(general64, fwd_smem_bytes<64>());
+  set(general128, fwd_smem_bytes<128>());
   set_decode_attributes(set);
-  const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForward>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kForwardShort>),
-                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowMax>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowStats>), reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kRowPolicy>),
-                                 reinterpret_cast<const void*>(&w64::fwd_kernel<Launch::kStaticPolicy>)};
+  const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<true>), reinterpret_cast<const void*>(&w64::fwd_kernel<false>)};
   for (const void* fn : workers) set(fn, w64::kSmemBytes);
+  for_policy_kernels([&](const void* fn, size_t bytes, int) { set(fn, bytes); });
   set(reinterpret_cast<const void*>(&quant_grid_kernel<false>), kQuantGridSmem);
   set(reinterpret_cast<const void*>(&quant_grid_kernel<true>), kQuantGridSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&quant_cluster_kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -152,9 +160,10 @@ int set_kernel_attributes(DeviceInfo* d) {
     std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d registers per thread, expected %d; refusing to launch\n", fa.numRegs, regs);
     return false;
   };
-  for (const void* fn : general64) if (!check(fn, kLaunchRegs)) return FMHA_I8_ERR_LAUNCH;
-  for (const void* fn : general128) if (!check(fn, kLaunchRegs)) return FMHA_I8_ERR_LAUNCH;
-  for (const void* fn : workers) if (!check(fn, w64::kLaunchRegs)) return FMHA_I8_ERR_LAUNCH;
+  bool as_built = check(general64, kLaunchRegs) && check(general128, kLaunchRegs);
+  for (const void* fn : workers) as_built = as_built && check(fn, w64::kLaunchRegs);
+  for_policy_kernels([&](const void* fn, size_t, int regs) { as_built = as_built && check(fn, regs); });
+  if (!as_built) return FMHA_I8_ERR_LAUNCH;
   for (int i = 0; i < kClusterSizes; ++i) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
@@ -167,9 +176,9 @@ int set_kernel_attributes(DeviceInfo* d) {
     cfg.numAttrs = 1;
     int n64 = 0, n128 = 0;
     cfg.dynamicSmemBytes = fwd_smem_bytes<64>();
-    if (cudaOccupancyMaxActiveClusters(&n64, fmha_fwd_kernel<64, Launch::kForward>, &cfg) != cudaSuccess) n64 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n64, fmha_fwd_kernel<64>, &cfg) != cudaSuccess) n64 = 0;
     cfg.dynamicSmemBytes = fwd_smem_bytes<128>();
-    if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128, Launch::kForward>, &cfg) != cudaSuccess) n128 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128>, &cfg) != cudaSuccess) n128 = 0;
     cudaGetLastError();
     d->max_clusters[i] = n64 < n128 ? n64 : n128;
   }
@@ -213,12 +222,12 @@ PointerAttributeFn pointer_attribute_fn() {
 
 // int8 tensor [n_heads, S, D] seen as a 3-D map (D innermost) with boxes of 128 rows of one head.
 // Rows past S are zero-filled by the copy engine instead of running into the next head.
-int make_map(CUtensorMap* map, const void* base, int n_heads, int S, int D) {
+int make_map(CUtensorMap* map, const void* base, int n_heads, int S, int D, int rows = kTile) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return FMHA_I8_ERR_DRIVER;
   const cuuint64_t dims[3] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(n_heads)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(S) * D};
-  const cuuint32_t box[3] = {static_cast<cuuint32_t>(D), static_cast<cuuint32_t>(kTile), 1u};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(D), static_cast<cuuint32_t>(rows), 1u};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   const CUtensorMapSwizzle sw = (D == 128) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
@@ -365,9 +374,7 @@ void plan_parts(FwdParams* p, int D, const DeviceInfo* dev) {
 // fmha_fwd64_sm100.cuh, 160 units of 64 keys 6.2 / 5.25; 444 of 128 8.2 / 7.5; 296, 592, 740, 1184 of 256 8.3 / 9.0, 12.1 / 12.4, 14.05 / 16.0,
 // 19.7 / 19.6; 444 and 664 of 512 14.8 / 15.6, 21.3 / 24.3; 592 and 888 of 1024 31.2 / 30.2, 44.8 / 46.25; 592 and 1184 of 2048 58.1 / 54.6, 110.5 / 102.6.
 //
-// The launches of a policy and of a calibration have a line of their own (1600 and 1200; 5850, 4900 / 4350 / 3400 per tile): the general kernel gains
-// less from a statistics launch.  Both launches, per-row and static, us: B4 H16 S1024 (512..1024 keys) 37.0 / 35.3, 50.3 / 45.8; B8 H16 S512 27.1 / 25.0,
-// 35.9 / 32.3; B1 H32 S2048 75.0 / 70.8, 108.9 / 97.3; B3 H12 S1024 25.4 / 29.3, 34.4 / 37.5.
+// Calibrations have a line of their own (1600 and 1200; 5850, 4900 / 4350 / 3400 per tile), drawn before.
 bool use_workers(const FwdParams& p, bool plain, const DeviceInfo* dev) {
   const long long sms = dev->sm_count, tiles = (p.S + kTile - 1) / kTile, round = sms * w64::kWorkers;
   const long long own = p.n_units / sms, more = p.n_units % sms != 0, full = p.n_units / round, last = (p.n_units % round + sms - 1) / sms;
@@ -391,8 +398,7 @@ bool use_workers(const FwdParams& p, bool plain, const DeviceInfo* dev) {
 //   D64, 4 rows   B128 H32 S128 42.6 / 32.9, S256 and beyond the few-rows one or within a few per cent
 bool few_rows(int Sq, int S, int D) { return Sq <= 4 || (D == 64 && Sq <= kDecodeMaxRows && S > kTile); }
 
-// Chooses the kernel of a call and how its units are divided: fills p->parts and p->own_rounds.  `plain`: neither calibration nor a
-// launch of a whole-row policy; `busy_sms`: SMs that something else is using.
+// Chooses the kernel of a call and how its units are divided: fills p->parts and p->own_rounds.  `plain`: no calibration; `busy_sms`: SMs that something else is using.
 int plan_call(FwdParams* p, int D, bool plain, int busy_sms, const DeviceInfo* dev) {
   p->parts = 1;
   if (plain && few_rows(p->Sq, p->S, D)) return FMHA_I8_KERNEL_FEW_ROWS;
@@ -401,7 +407,20 @@ int plan_call(FwdParams* p, int D, bool plain, int busy_sms, const DeviceInfo* d
   return FMHA_I8_KERNEL_GENERAL;
 }
 
-template <int D, Launch kLaunch = Launch::kForward>
+template <int D, bool kStatic>
+int launch_policy(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v) {
+  CUtensorMap mq, mk, mv;
+  int st;
+  if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
+  if ((st = make_map(&mk, k, p.bh_count, p.S, D, wholerow::kKeys)) != FMHA_I8_OK) return st;
+  if ((st = make_map(&mv, v, p.bh_count, p.S, D, wholerow::kKeys)) != FMHA_I8_OK) return st;
+  LaunchHow how;
+  how.overlap = true;
+  const unsigned grid = static_cast<unsigned>(p.n_units < dev->sm_count ? p.n_units : dev->sm_count);
+  return launch_kernel(wholerow::policy_kernel<D, kStatic>, dim3(grid), dim3(wholerow::kThreads), wholerow::smem_bytes<D>(), stream, how, mq, mk, mv, p);
+}
+
+template <int D>
 int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v, int kernel, int busy_sms) {
   CUtensorMap mq, mk, mv;
   int st;
@@ -420,9 +439,7 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
   if constexpr (D == 64) {
     if (kernel == FMHA_I8_KERNEL_WORKERS) {
-      auto* fn = w64::fwd_kernel<kLaunch>;
-      if constexpr (kLaunch == Launch::kForward)
-        if (p.S <= w64::kShortTiles * kTile) fn = w64::fwd_kernel<Launch::kForwardShort>;
+      auto* fn = p.S <= w64::kShortTiles * kTile ? w64::fwd_kernel<true> : w64::fwd_kernel<false>;
       return launch_kernel(fn, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
     }
   }
@@ -430,7 +447,7 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
     how.cluster = static_cast<unsigned>(p.parts);
     grid = static_cast<unsigned>(p.own_rounds > 0 ? dev->sm_count : p.n_units * p.parts);
   }
-  return launch_kernel(fmha_fwd_kernel<D, kLaunch>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
+  return launch_kernel(fmha_fwd_kernel<D>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
 
 // The few-rows kernel.  CTAs per head: enough for two rounds of the 3 CTAs that an SM holds, so that heads of different
@@ -466,15 +483,6 @@ int launch_decode(cudaStream_t s, DeviceInfo* dev, const FwdParams& p, const voi
   return launch_decode_rows<D, 4>(s, dev, p, q, k, v);
 }
 
-// What a launch of the forward kernels is beside the plain forward pass into o.  (Calibration comes as infer_x_impl's `calib`: the
-// largest |output| goes to that device float and o, which may be null, is not touched.)
-struct LaunchMode {
-  float2* stats_out = nullptr;     // statistics launch of a whole-row policy: {row max bits, exp-sum or 0} per query row, o untouched
-  const float2* stats_in = nullptr;  // policy launch: those statistics
-  int policy = 0;                  // FMHA_I8_POLICY_* that the launch belongs to
-  int busy_sms = 0;                // SMs that something else is using for longer than this launch
-};
-
 int fill_units(FwdParams* p, const Shape& sh, int bh_count) {
   p->S = sh.Sk;
   p->Sq = sh.Sq;
@@ -491,9 +499,8 @@ int fill_units(FwdParams* p, const Shape& sh, int bh_count) {
 
 int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void* q, const void* k,
                  const void* v, const void* mask, void* o, int bh_begin, int bh_count, unsigned flags,
-                 float* calib = nullptr, const LaunchMode* mode = nullptr) {
-  const bool no_output = calib || (mode && mode->stats_out);
-  if (!amax || !q || !k || !v || !mask || (!o && !no_output)) return FMHA_I8_ERR_NULL_POINTER;
+                 float* calib = nullptr, int policy = FMHA_I8_POLICY_TILE, int busy_sms = 0) {
+  if (!amax || !q || !k || !v || !mask || (!o && !calib)) return FMHA_I8_ERR_NULL_POINTER;
   if (!(flags & FMHA_I8_FLAG_USE_TCU)) return FMHA_I8_ERR_NO_CUDA_CORE_PATH;
   if (flags & ~(FMHA_I8_FLAG_USE_TCU | FMHA_I8_FLAG_UINT8_P)) return FMHA_I8_ERR_BAD_FLAGS;
   int st = check_shape_x(sh);
@@ -505,23 +512,16 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   FwdParams p{};
   if ((st = fill_params(&p, amax, sh.D, flags)) != FMHA_I8_OK) return st;
   p.amax_out = calib;
-  const bool policy_launch = mode && mode->stats_in;
-  if (mode) {
-    p.row_stats_out = mode->stats_out;
-    p.row_stats_in = mode->stats_in;
-    if (policy_launch) {
-      // fmha_i8_quant_deviation.py:7,38-43: 127 levels, unsigned, P8 = clip(rn(p * 127 / p_amax), 0, 127).
-      // Per-row ("dynamic", :104-118): p_amax = the row's largest probability = 1/l, so P8 = rn(127 e) and the output
-      // is (sum P8 v8) / (127 l) * v_amax/127.  Static (:82-98): p_amax = s_max for every row, so
-      // P8 = min(rn(127 e / (l s_max)), 127) and the output is (sum P8 v8) * s_max/127 * v_amax/127.
-      const float levels = 127.f;
-      if (mode->policy == FMHA_I8_POLICY_STATIC && (!(amax[4] > 0.f) || !std::isfinite(amax[4]))) return FMHA_I8_ERR_BAD_AMAX;
-      p.p_levels = levels;
-      p.p_row_mul = levels;
-      p.p_static_mul = (mode->policy == FMHA_I8_POLICY_STATIC) ? levels / amax[4] : 0.f;
-      p.p_mul = levels;
-      p.scale_v_out = (mode->policy == FMHA_I8_POLICY_STATIC) ? amax[4] * amax[2] / (levels * amax[3]) : amax[2] / (levels * amax[3]);
-    }
+  const bool is_static = policy == FMHA_I8_POLICY_STATIC;
+  if (policy != FMHA_I8_POLICY_TILE) {
+    // fmha_i8_quant_deviation.py:7,38-43: 127 levels, unsigned, P8 = clip(rn(p * 127 / p_amax), 0, 127).
+    // Per-row ("dynamic", :104-118): p_amax = the row's largest probability = 1/l, so P8 = rn(127 e) and the output
+    // is (sum P8 v8) / (127 l) * v_amax/127.  Static (:82-98): p_amax = s_max for every row, so
+    // P8 = min(rn(127 e / (l s_max)), 127) and the output is (sum P8 v8) * s_max/127 * v_amax/127.
+    const float levels = wholerow::kLevels;
+    if (is_static && (!(amax[4] > 0.f) || !std::isfinite(amax[4]))) return FMHA_I8_ERR_BAD_AMAX;
+    p.p_mul = is_static ? levels / amax[4] : levels;
+    p.scale_v_out = is_static ? amax[4] * amax[2] / (levels * amax[3]) : amax[2] / (levels * amax[3]);
   }
   int err = FMHA_I8_OK;
   DeviceInfo* dev = current_device(&err);
@@ -540,27 +540,21 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   if ((st = fill_units(&p, sh, bh_count)) != FMHA_I8_OK) return st;
   p.status = dev->status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int busy = mode ? mode->busy_sms : 0;
-  const bool plain = !calib && !(mode && (mode->stats_out || mode->stats_in));
-  const int kernel = plan_call(&p, sh.D, plain, busy, dev);
-  if (kernel == FMHA_I8_KERNEL_FEW_ROWS) return sh.D == 128 ? launch_decode<128>(s, dev, p, q, k, v) : launch_decode<64>(s, dev, p, q, k, v);
+  const int kernel = plan_call(&p, sh.D, !calib && policy == FMHA_I8_POLICY_TILE, busy_sms, dev);
   auto launch = [&](auto d) {
     constexpr int D = decltype(d)::value;
-    const bool row = mode && mode->policy == FMHA_I8_POLICY_ROW;
-    if (p.row_stats_in && row) return launch_fwd<D, Launch::kRowPolicy>(s, dev, p, q, k, v, kernel, busy);
-    if (p.row_stats_in) return launch_fwd<D, Launch::kStaticPolicy>(s, dev, p, q, k, v, kernel, busy);
-    if (p.row_stats_out && row) return launch_fwd<D, Launch::kRowMax>(s, dev, p, q, k, v, kernel, busy);
-    if (p.row_stats_out) return launch_fwd<D, Launch::kRowStats>(s, dev, p, q, k, v, kernel, busy);
-    return launch_fwd<D>(s, dev, p, q, k, v, kernel, busy);
+    if (policy != FMHA_I8_POLICY_TILE) return is_static ? launch_policy<D, true>(s, dev, p, q, k, v) : launch_policy<D, false>(s, dev, p, q, k, v);
+    if (kernel == FMHA_I8_KERNEL_FEW_ROWS) return launch_decode<D>(s, dev, p, q, k, v);
+    return launch_fwd<D>(s, dev, p, q, k, v, kernel, busy_sms);
   };
   return sh.D == 128 ? launch(std::integral_constant<int, 128>()) : launch(std::integral_constant<int, 64>());
 }
 
 int infer_slice_impl(void* stream, const float amax[5], const int desc[4], const void* q, const void* k,
-                     const void* v, const void* mask, void* o, int bh_begin, int bh_count, unsigned flags, const LaunchMode* mode = nullptr) {
+                     const void* v, const void* mask, void* o, int bh_begin, int bh_count, unsigned flags, int busy_sms = 0) {
   if (!desc) return FMHA_I8_ERR_NULL_POINTER;
   const Shape sh{desc[0], desc[1], desc[1], desc[2], desc[3]};
-  return infer_x_impl(stream, amax, sh, q, k, v, mask, o, bh_begin, bh_count, flags, nullptr, mode);
+  return infer_x_impl(stream, amax, sh, q, k, v, mask, o, bh_begin, bh_count, flags, nullptr, FMHA_I8_POLICY_TILE, busy_sms);
 }
 
 // Device staging buffers of fmha_i8_sm100_infer_host, one set per device, grown on demand, plus the
@@ -719,18 +713,7 @@ int fmha_i8_sm100_infer_policy(void* stream, const float amax[5], const int desc
   if (flags & FMHA_I8_FLAG_UINT8_P) return finish(FMHA_I8_ERR_BAD_FLAGS);       // the policies bring their own P format
   if (!row_scratch || !o) return finish(FMHA_I8_ERR_NULL_POINTER);
   if (!aligned(row_scratch, 8)) return finish(FMHA_I8_ERR_MISALIGNED);
-  // launch 1: each row's maximum over all keys, which is all that the per-row scale needs (launch 2 forms the row's sum beside the
-  // probabilities); for the static scale the exp-sum too, in the reference's tile-local arithmetic
-  LaunchMode stats;
-  stats.policy = policy;
-  stats.stats_out = reinterpret_cast<float2*>(row_scratch);
-  int st = infer_x_impl(stream, amax, sh, q, k, v, mask, nullptr, bh_begin, bh_count, flags, nullptr, &stats);
-  if (st != FMHA_I8_OK) return finish(st);
-  // launch 2 (same stream, so ordered behind launch 1): every tile of a row quantised with the row's one scale
-  LaunchMode apply;
-  apply.stats_in = reinterpret_cast<const float2*>(row_scratch);
-  apply.policy = policy;
-  return finish(infer_x_impl(stream, amax, sh, q, k, v, mask, o, bh_begin, bh_count, flags, nullptr, &apply));
+  return finish(infer_x_impl(stream, amax, sh, q, k, v, mask, o, bh_begin, bh_count, flags, nullptr, policy));
 }
 
 int fmha_i8_sm100_calibrate_o_amax(void* stream, const float amax[5], const int desc5[5], const void* q, const void* k,
@@ -797,8 +780,7 @@ static int infer_host_slice_impl(const float amax[5], const int desc[4], const v
   int bounds[kHostChunks + 1];
   const int n_chunks = cut_heads(desc, bh_count, bounds);
   const FetchPlan plan = plan_fetch(desc, host_q, host_k, host_v, static_cast<const int8_t*>(host_mask), bh_begin, bh_count, n_chunks);
-  LaunchMode mode;
-  mode.busy_sms = plan.by_kernel ? kFetchCtas : 0;
+  const int busy_sms = plan.by_kernel ? kFetchCtas : 0;
   cudaError_t e = cudaMemcpyAsync(s.mask, host_mask, mask_bytes, cudaMemcpyHostToDevice, s.s_in);
   for (int i = 0; i < n_chunks && e == cudaSuccess; ++i) {
     const int begin = bounds[i];
@@ -823,7 +805,7 @@ static int infer_host_slice_impl(const float amax[5], const int desc[4], const v
     if (e == cudaSuccess) e = cudaEventRecord(s.landed[i], s.s_in);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s.s_run, s.landed[i], 0);
     if (e != cudaSuccess) break;
-    st = infer_slice_impl(s.s_run, amax, desc, dq, dk, dv, s.mask, dout, bh_begin + begin, end - begin, flags, &mode);
+    st = infer_slice_impl(s.s_run, amax, desc, dq, dk, dv, s.mask, dout, bh_begin + begin, end - begin, flags, busy_sms);
     if (st != FMHA_I8_OK) break;
     e = cudaEventRecord(s.computed[i], s.s_run);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s.s_out, s.computed[i], 0);

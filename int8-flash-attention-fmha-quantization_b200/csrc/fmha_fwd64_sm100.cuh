@@ -23,7 +23,7 @@
 
 namespace fmha {
 namespace w64 {
-// The two forward passes, kForward and for units of up to kShortTiles key tiles kForwardShort, differ in how the maximum of a half tile
+// There are two instances, one of them (kShort) for units of up to kShortTiles key tiles.  They differ in how the maximum of a half tile
 // branches off that of a whole one: behind the first loads or in front of them.  Behind, the step is faster, and the compiler spills
 // values of the unit (-Xptxas -v: 72 bytes stored, 100 loaded, none in front), which short units pay for.  Behind against in front, in
 // per cent of the time: B256 H16 S256 (lengths 64..256) +2, B200 H12 S128 +1, B64 H16 S256 -1.5; B64 H16 S320 -2, B16 H12 S384 -3, B64 H16
@@ -112,7 +112,7 @@ __device__ __forceinline__ int columns_max(const uint32_t taddr) {
 
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = one query row: its scores, probabilities, fp32 running output row, maximum and sum.
-template <Launch kLaunch>
+template <bool kShort>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base) {
   WorkerCtl* ctl = &all->w[worker];
   const int lane = threadIdx.x & 31, quad = warp_index() & 3;
@@ -120,8 +120,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   const uint32_t tS = t_lane + static_cast<uint32_t>(worker * kTile), tP = tS;
   volatile int* abort_flag = &all->abort;
-  constexpr bool kPolicy = policy_launch(kLaunch), kStatic = kLaunch == Launch::kStaticPolicy, kStats = stats_launch(kLaunch), kShort = kLaunch == Launch::kForwardShort;
-
   uint32_t g = 0;                               // steps so far
   auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
     if (warp_wait(bar, parity, abort_flag)) return true;
@@ -141,24 +139,8 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     if (n_live < 0) continue;
     announced += 1 - ctl->info[buf].last;
     float m_run = -INFINITY, l_run = 0.f;
-    int imax_run = static_cast<int>(kMagicBits);          // statistics launches: biased integer row maximum over all tiles
-    RowConsts k;                                          // (policy launch: constant over a unit)
-    float p_cap = 0.f;
     // this thread's output row, -1 past the last row of the head (looked up where it is needed: nothing of it stays in registers)
     auto output_row = [&]() -> int64_t { return row < ctl->info[buf].rows ? ctl->info[buf].first_row + row : -1; };
-    if (kPolicy) {
-      const int64_t out_row = output_row();
-      // Policy launch: the row's maximum over ALL keys and its exp-sum come from the statistics launch; one scale per
-      // row for the whole unit (fmha_i8_quant_deviation.py:62-121).
-      float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
-      if (out_row >= 0) st = __ldcg(&p.row_stats_in[out_row]);       // (through the L1, 48.1 -> 48.4 us for B4 H16 S1024)
-      // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = min(rn(levels * (e / l) / s_max), levels)
-      const float mul = kStatic ? p.p_static_mul / (st.y > 0.f ? st.y : 1.f) : p.p_row_mul;
-      k = row_consts(__float_as_int(st.x), p.c2, p.row_scale, p.scale_qk, mul);
-      // the static policy's accumulated integer sum becomes the output through one factor, the per-row policy's through that / l
-      if (kStatic) l_run = st.y > 0.f ? 1.f : 0.f;
-      p_cap = p.p_levels / k.p_mul_f.x;       // an exponential above this would quantise beyond the top level
-    }
 
 #pragma unroll 1
     for (int j = 0; j < n_live; ++j, ++g) {
@@ -166,61 +148,52 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       if (!wait_or_fail(smem_u32(&ctl->s_full), g & 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
       tc_fence_after();
       FMHA_STAMP(quad == 0 ? worker * 4 + 0 : 47, g);
-      if (!kPolicy) {
-        // ---- pass 1: biased integer maximum of the row (inc/fmha_i8.cuh:183-206)
-        int imax;
-        if constexpr (kShort) {
-          imax = whole ? columns_max<8>(tS) : columns_max<4>(tS);
+      // ---- pass 1: biased integer maximum of the row (inc/fmha_i8.cuh:183-206)
+      int imax;
+      if constexpr (kShort) {
+        imax = whole ? columns_max<8>(tS) : columns_max<4>(tS);
+      } else {
+        uint32_t ra[16], rb[16];
+        int max_a = INT_MIN, max_b = INT_MIN;
+        auto two_chunks = [&]() {
+          tmem_ld_fence(ra); tmem_ld_fence(rb);
+          chunk_max<16>(ra, max_a, max_b);
+          chunk_max<16>(rb, max_a, max_b);
+        };
+        auto two_chunks_and_next = [&](int next) {
+          tmem_ld_fence(ra); tmem_ld_fence(rb);
+          chunk_max<16>(ra, max_a, max_b);
+          tmem_ld16_issue(tS + next * 16, ra);
+          chunk_max<16>(rb, max_a, max_b);
+          tmem_ld16_issue(tS + next * 16 + 16, rb);
+        };
+        tmem_ld16_issue(tS, ra);
+        tmem_ld16_issue(tS + 16, rb);
+        two_chunks_and_next(2);
+        if (whole) {
+          two_chunks_and_next(4);
+          two_chunks_and_next(6);
+          two_chunks();
         } else {
-          uint32_t ra[16], rb[16];
-          int max_a = INT_MIN, max_b = INT_MIN;
-          auto two_chunks = [&]() {
-            tmem_ld_fence(ra); tmem_ld_fence(rb);
-            chunk_max<16>(ra, max_a, max_b);
-            chunk_max<16>(rb, max_a, max_b);
-          };
-          auto two_chunks_and_next = [&](int next) {
-            tmem_ld_fence(ra); tmem_ld_fence(rb);
-            chunk_max<16>(ra, max_a, max_b);
-            tmem_ld16_issue(tS + next * 16, ra);
-            chunk_max<16>(rb, max_a, max_b);
-            tmem_ld16_issue(tS + next * 16 + 16, rb);
-          };
-          tmem_ld16_issue(tS, ra);
-          tmem_ld16_issue(tS + 16, rb);
-          two_chunks_and_next(2);
-          if (whole) {
-            two_chunks_and_next(4);
-            two_chunks_and_next(6);
-            two_chunks();
-          } else {
-            two_chunks();
-          }
-          imax = max(max_a, max_b);
+          two_chunks();
         }
-        if (kStats) imax_run = (j == 0) ? imax : max(imax_run, imax);
-        if (kLaunch == Launch::kRowMax) {
-          tc_fence_before();
-          mbar_arrive(smem_u32(&ctl->s_free));
-          continue;
-        }
-        k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, p.p_mul);
+        imax = max(max_a, max_b);
       }
+      const RowConsts k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, p.p_mul);
       FMHA_STAMP(quad == 0 ? worker * 4 + 1 : 47, g);
 
       // ---- pass 2: exp, row sum, requantise (inc/fmha_i8.cuh:208-253); the bytes go over columns already consumed
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t sa[8], sb[8], packed[2];
-      // (a statistics launch stores no P: the static policy, B4 H16 S1024, 53.7 -> 53.1 us)
       auto sixteen = [&](uint32_t c, auto more) {           // columns 8 c to 8 c + 15; the first eight are in flight
         tmem_ld_fence(sa);
         tmem_ld8_issue(tS + (c + 1) * 8, sb);
-        chunk_exp_pack<8, kStatic, 0, !kStats>(sa, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
-        if (!kStats) tmem_st2(tP + c * 2, packed);
+        chunk_exp_pack<8>(sa, k.c2, k.neg_hi, k.p_mul_f, sum, packed);
+        tmem_st2(tP + c * 2, packed);
         tmem_ld_fence(sb);
         if (decltype(more)::value) tmem_ld8_issue(tS + (c + 2) * 8, sa);
-        chunk_exp_pack<8, kStatic, 1, !kStats>(sb, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
-        if (!kStats) tmem_st2(tP + c * 2 + 2, packed);
+        chunk_exp_pack<8, false, 1>(sb, k.c2, k.neg_hi, k.p_mul_f, sum, packed);
+        tmem_st2(tP + c * 2 + 2, packed);
       };
       constexpr Flight<1> more;
       constexpr Flight<0> last;
@@ -234,24 +207,18 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
         for (uint32_t c = 0; c < 6; c += 2) sixteen(c, more);
         sixteen(6, last);
       }
-      if (!kStats) tmem_wait_st();
+      tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(smem_u32(kStats ? &ctl->s_free : &ctl->p_ready));
+      mbar_arrive(smem_u32(&ctl->p_ready));
       FMHA_STAMP(quad == 0 ? worker * 4 + 2 : 47, g);
 
       // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304), while P.V is under way
       const float l_tile = k.f * ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y));
-      float e_old = j > 0 ? 1.f : 0.f, e_cur = 1.f;                                  // policy launch: every tile of a row has the same scale
-      if (!kPolicy) {
-        const float m_new = fmaxf(m_run, k.m_tile);
-        e_old = __expf(m_run - m_new);                                 // 0 on the first tile (m_run = -inf)
-        e_cur = clear_low2(__expf(k.m_tile - m_new));                  // 22 significant bits: kMagic*e_cur is exact
-        l_run = fmaf(e_old, l_run, e_cur * l_tile);
-        m_run = m_new;
-      } else if (!kStatic) {
-        l_run += l_tile;
-      }
-      if (kStats) continue;                                        // no output is wanted: there is no P.V
+      const float m_new = fmaxf(m_run, k.m_tile);
+      const float e_old = __expf(m_run - m_new);                       // 0 on the first tile (m_run = -inf)
+      const float e_cur = clear_low2(__expf(k.m_tile - m_new));        // 22 significant bits: kMagic*e_cur is exact
+      l_run = fmaf(e_old, l_run, e_cur * l_tile);
+      m_run = m_new;
       const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
       const float2 e_old2 = make_float2(e_old, e_old);
 
@@ -280,11 +247,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     const int64_t out_row = output_row();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
-    if (kStats) {
-      // the row's maximum and exp-sum over all keys, for the policy launch that follows
-      if (out_row >= 0) p.row_stats_out[out_row] = make_float2(__int_as_float(imax_run), l_run);
-      continue;
-    }
     const float inv = l_run > 0.f ? __frcp_rn(l_run) : 0.f;
     if (p.amax_out != nullptr) {
       // calibration: only the largest magnitude of the unquantised output is wanted (the reference takes o_amax from its
@@ -330,7 +292,7 @@ struct DriverStep {
   bool first;                // of its unit
   int bh, batch;
 };
-template <bool kStats, bool kEarlyK>
+template <bool kEarlyK>
 __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const int worker, const CUtensorMap* map_q, const CUtensorMap* map_k,
                                             const CUtensorMap* map_v, const uint32_t tmem_base, const uint32_t worker_smem, uint8_t* presets) {
   WorkerCtl* ctl = &all->w[worker];
@@ -361,9 +323,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   int bh = 0, batch = 0, q_row0 = 0;          // its head, sequence and first query row
   // The results of rows without an unmasked key.
   auto empty_unit = [&](int rows, int64_t first_row) {
-    if (kStats) {
-      for (int r = lane; r < rows; r += 32) p.row_stats_out[first_row + r] = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 0.f);
-    } else if (p.amax_out == nullptr) {
+    if (p.amax_out == nullptr) {
       uint4* dst = reinterpret_cast<uint4*>(p.o + first_row * kD);
       for (int i = lane; i < rows * (kD / 16); i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
     }
@@ -435,7 +395,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   };
 
   // The first unit's Q rows, and with few key tiles to a unit its first K tile, are asked for while its mask is still on the way.  Both
-  // with many key tiles: B8 H16 S512 18.1 -> 18.3 us, the static policy there 31.7 -> 32.0.  Neither: B32 H12 S512 (256..512) 36.7 -> 37.4.
+  // with many key tiles: B8 H16 S512 18.1 -> 18.3 us.  Neither: B32 H12 S512 (256..512) 36.7 -> 37.4.
   // Only Q with few: B200 H12 S128 22.6 -> 22.8.
   const uint32_t first = cta_unit(worker);
   const bool early = first < static_cast<uint32_t>(p.n_units);
@@ -491,32 +451,28 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
 #pragma unroll
       for (int kk = 0; kk < kD / 32; ++kk) mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(d_k, kk * 32), idesc, 1u);
       mma_commit(smem_u32(&ctl->s_full));
-      if (!kStats) {
-        mbar_arrive_expect_tx(smem_u32(&ctl->v_full), kTileBytes);
-        tma_load_3d(v_smem, map_v, smem_u32(&ctl->v_full), 0, cur.tile * kTile, cur.bh);
-      }
+      mbar_arrive_expect_tx(smem_u32(&ctl->v_full), kTileBytes);
+      tma_load_3d(v_smem, map_v, smem_u32(&ctl->v_full), 0, cur.tile * kTile, cur.bh);
     }
     FMHA_STAMP(16 + worker * 4 + 1, g);
     const DriverStep next = next_step();
     if (fail != 0u || !wait(smem_u32(&ctl->s_full), g & 1u, FMHA_I8_DEV_WAIT_S_READY)) break;
     load_k(next);
-    if (!kStats) {
-      if (!wait(smem_u32(&ctl->v_full), g & 1u, FMHA_I8_DEV_WAIT_V_LOAD)) break;
-      if (!wait(smem_u32(&ctl->p_ready), g & 1u, FMHA_I8_DEV_WAIT_P_READY)) break;
-      tc_fence_after();
-      FMHA_STAMP(16 + worker * 4 + 2, g);
-      if (lead) {
-        mma_f16_ss(tO, d_a, d_b, idesc_preset_o, 0u);
+    if (!wait(smem_u32(&ctl->v_full), g & 1u, FMHA_I8_DEV_WAIT_V_LOAD)) break;
+    if (!wait(smem_u32(&ctl->p_ready), g & 1u, FMHA_I8_DEV_WAIT_P_READY)) break;
+    tc_fence_after();
+    FMHA_STAMP(16 + worker * 4 + 2, g);
+    if (lead) {
+      mma_f16_ss(tO, d_a, d_b, idesc_preset_o, 0u);
 #pragma unroll
-        for (int kk = 0; kk < kTile / 64; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(d_v, kk * 32 * kD), idesc_o, 1u);
-        if (whole) {
+      for (int kk = 0; kk < kTile / 64; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(d_v, kk * 32 * kD), idesc_o, 1u);
+      if (whole) {
 #pragma unroll
-          for (int kk = kTile / 64; kk < kTile / 32; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);
-        }
-        mma_commit(smem_u32(&ctl->o_full));
+        for (int kk = kTile / 64; kk < kTile / 32; ++kk) mma_i8_ts(tO, tS + kk * 8, desc_advance(dv, kk * 32 * kD), idesc_o, 1u);
       }
-      FMHA_STAMP(16 + worker * 4 + 3, g);
+      mma_commit(smem_u32(&ctl->o_full));
     }
+    FMHA_STAMP(16 + worker * 4 + 3, g);
     cur = next;
     ++g;
   }
@@ -528,7 +484,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   }
 }
 
-template <Launch kLaunch>
+template <bool kShort>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
            const FwdParams p) {
@@ -580,10 +536,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
   uint8_t* worker_smem = tiles + worker * kWorkerBytes;
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
-    w64::softmax_role<kLaunch>(p, ctl, worker, tmem_base);
+    w64::softmax_role<kShort>(p, ctl, worker, tmem_base);
   } else {
     setmaxnreg_dec<kDriverRegs>();
-    driver_role<stats_launch(kLaunch), kLaunch == Launch::kForwardShort>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
+    driver_role<kShort>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
   }
   tc_fence_before();
   __syncthreads();

@@ -179,15 +179,6 @@ __device__ __forceinline__ int fast_div(int u, const FastDiv d) {
   return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(u)) * d.mul) >> d.shift);
 }
 
-// What a launch is for: the forward pass (or its calibration); the workers' form of it for units of few key tiles; one of the launches
-// of a whole-row P scaling policy (FwdParams): for the per-row scale the rows' maxima and the forward pass, for the static scale the rows'
-// maxima and sums and the forward pass.
-// (One kernel that asked at run time, with P.V or the exponentials formed in the statistics launch too: B4 H16 S1024 D64 per-row 46.0 us
-// instead of 35.5, B8 H16 S512 D128 per-row 38.8 instead of 31.1.)
-enum class Launch { kForward, kForwardShort, kRowMax, kRowPolicy, kRowStats, kStaticPolicy };
-__host__ __device__ constexpr bool policy_launch(Launch l) { return l == Launch::kRowPolicy || l == Launch::kStaticPolicy; }
-__host__ __device__ constexpr bool stats_launch(Launch l) { return l == Launch::kRowMax || l == Launch::kRowStats; }
-
 struct FwdParams {
   const int8_t* mask;   // [B,S] whole mask
   int8_t* o;            // first head of the slice
@@ -210,15 +201,15 @@ struct FwdParams {
                         // in real units, max |O~ / l| * amax_scale, is folded into this device float
   float amax_scale;     // v_amax / (127 * 128)  (127 * 255 with unsigned P)
   unsigned* status;     // eight device status words
-  // Whole-row P scaling policies (the reference's accuracy study, fmha_i8_quant_deviation.py:57-121), two launches:
-  float2* row_stats_out;       // Launch::kRowMax, kRowStats: per query row {bits of the biased integer row maximum over ALL keys, sum over
-                               // all keys of exp(score - row maximum) (kRowMax: 0)} is written here, nothing to o
-  const float2* row_stats_in;  // Launch::kRowPolicy, kStaticPolicy: those statistics, read back
-  float p_row_mul;      // policy launch: P8 = rn(p_row_mul * exp(score - row max))                  ("dynamic", per-row scale), or
-  float p_static_mul;   //                P8 = min(rn(p_static_mul * exp(score - row max) / l), levels)  ("static" scale)
-  float p_levels;       // quantisation levels of P in a policy launch (127 in the reference's study)
-                        // (a policy launch sets scale_v_out to the factor that turns sum_j P8 v8 [/ l] into int8 output units)
+  // (Whole-row P scaling policies, fmha_policy_sm100.cuh: P8 = rn(p_mul * exp(score - row max)), or with the static scale
+  // rn(p_mul * exp(score - row max) / l); scale_v_out is the factor that turns sum_j P8 v8 [/ l] into int8 output units.)
+  unsigned char unused[32];            // see kParamBytes
 };
+
+// What a launch costs the host depends on the bytes of its parameters, in steps of 64 (as commands they go to the GPU in lines of that size): B1 H2 S64
+// D64 takes 4.1 to 4.4 us a call with 536 or 600 of them, 24 modulo 64, and 4.4 to 4.8 with 504, 520, 528, 552, 568 or 760.
+constexpr size_t kParamBytes = 3 * sizeof(CUtensorMap) + sizeof(FwdParams);
+static_assert(kParamBytes % 64 == 24, "a launch's parameters have a size that is slow to hand over");
 
 // Kinds of live key tiles.  Tiles with unmasked keys in one half only -- the last one of a sequence, every other time -- are
 // processed as the 64 keys of that half by the workers of fmha_fwd64_sm100.cuh: the other half's probabilities are zero and change
@@ -252,7 +243,6 @@ template <int NK, int NV> struct FwdCtl {
   int abort;
   // row statistics of a step, written by the softmax threads and read by the merge threads (slot = g & 3)
   float st_m[4][kTile], st_f[4][kTile], st_s0[4][kTile], st_s1[4][kTile];
-  int st_i[4][kTile];                  // biased integer row maximum of the step's tile (for the statistics launch)
   int xmax[2][2][2][kTile];            // [chain][step parity][half][row]: biased integer maximum of that half row
   float2 part[kTile];                  // row maximum and sum of a partial result (a unit shared by a cluster)
   UnitInfo info[kInfoBufs];
@@ -514,10 +504,9 @@ __device__ __forceinline__ UnitGeom unit_geom(const FwdParams& p, int u) {
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = one half (64 keys) of one query row of one chain.  Walks the CTA's step sequence and
 // handles the steps of its chain.
-template <int D, Launch kLaunch>
+template <int D>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                              const UnitWalk walk) {
-  constexpr bool kPolicy = policy_launch(kLaunch);
   const int warp = warp_index() - kWarpSoftmax0, lane = threadIdx.x & 31;
   const int chain = warp >> 3, half = (warp >> 2) & 1, quad = warp & 3;
   const int row = quad * 32 + lane;
@@ -530,7 +519,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
   uint32_t n = 0;     // steps this chain has processed so far (phase of xch)
   uint32_t g0 = 0;    // global index of the current unit's first step
   for (int it = 0; it < walk.count; ++it) {
-    const int u = walk.unit(it);
     const int buf = it % kInfoBufs;
     if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag))) {
       raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it);
@@ -539,20 +527,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
     const int n_live = ctl->info[buf].n_live;
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));     // only the tile count is needed here
-    // Policy launch: the row's maximum over ALL keys and its exp-sum come from the statistics launch; one scale per
-    // row for the whole unit, no tile maximum, no exchange (fmha_i8_quant_deviation.py:62-121).
-    RowConsts kp;
-    float p_cap = 0.f;
-    if (kPolicy) {
-      const UnitGeom geo = unit_geom(p, u);
-      const int q_row = geo.q_row0 + row;
-      float2 st = make_float2(__int_as_float(static_cast<int>(kMagicBits)), 1.f);
-      if (q_row < p.Sq) st = p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row];
-      // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = min(rn(levels * (e / l) / s_max), levels)
-      const float mul = kLaunch == Launch::kStaticPolicy ? p.p_static_mul / (st.y > 0.f ? st.y : 1.f) : p.p_row_mul;
-      kp = row_consts(__float_as_int(st.x), c2s, row_scale, scale_qk, mul);
-      p_cap = p.p_levels / kp.p_mul_f.x;        // an exponential above this would quantise beyond the top level
-    }
 #pragma unroll 1
     for (int j = (chain ^ static_cast<int>(g0)) & 1; j < n_live; j += 2, ++n) {
       const uint32_t g = g0 + static_cast<uint32_t>(j);
@@ -575,11 +549,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
           : tS + (half ? 48u : 0u);
 
       uint32_t ra[16], rb[16];
-      RowConsts k;
-      if (kPolicy) {
-        k = kp;
-        tmem_ld16_issue(tS + c0 * 16, ra);
-      } else {
       // ---- pass 1: biased integer maximum of my 64 columns (inc/fmha_i8.cuh:183-206)
       int max_a = INT_MIN, max_b = INT_MIN;
       // two tensor-memory round trips (a round trip costs about as much as the whole arithmetic of this pass), two
@@ -594,7 +563,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       tmem_ld16_issue(tS + 48, rb);
       tmem_ld_fence(ra); tmem_ld_fence(rb);
       chunk_max<16>(ra, max_a, max_b);
-      if (kLaunch != Launch::kRowMax) tmem_ld16_issue(tS + c0 * 16, ra);     // first chunk of pass 2, in flight during the exchange
+      tmem_ld16_issue(tS + c0 * 16, ra);     // first chunk of pass 2, in flight during the exchange
       chunk_max<16>(rb, max_a, max_b);
       const int mine = max(max_a, max_b);
       // ---- exchange with the thread that owns the other half of this row
@@ -602,28 +571,20 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       xrow[half * kTile] = mine;
       mbar_arrive(bar_x);
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(bar_x, n & 1u, abort_flag))) {
-        if (kLaunch != Launch::kRowMax) tmem_ld_fence(ra);
+        tmem_ld_fence(ra);
         raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_S_READY, g);
         return;
       }
       const int imax = max(mine, xrow[(half ^ 1) * kTile]);
-      k = row_consts(imax, c2s, row_scale, scale_qk, p_mul);
-      if (stats_launch(kLaunch) && half == 0) ctl->st_i[g & 3u][row] = imax;
-      if (kLaunch == Launch::kRowMax) {
-        tc_fence_before();
-        mbar_arrive(smem_u32(&ctl->p_ready[g & 3u]));
-        continue;
-      }
-      }
+      const RowConsts k = row_consts(imax, c2s, row_scale, scale_qk, p_mul);
       if (half == 0 && quad == 0) FMHA_STAMP(chain * 4 + 1, n);
 
       // ---- pass 2: exp, row sum, requantise, P over columns already consumed (inc/fmha_i8.cuh:208-253)
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t packed[4];
-      // (a statistics launch stores no P: the static policy, B8 H16 S512 D128, 36.8 -> 35.9 us, B2 H32 S2048 187.5 -> 182.4)
       auto sixteen = [&](const uint32_t (&r)[16], int c) {
-        chunk_exp_pack<16, kLaunch == Launch::kStaticPolicy, 0, !stats_launch(kLaunch)>(r, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
-        if (!stats_launch(kLaunch)) tmem_st4(tP + (c0 + c * cs) * 4, packed);
+        chunk_exp_pack<16>(r, k.c2, k.neg_hi, k.p_mul_f, sum, packed);
+        tmem_st4(tP + (c0 + c * cs) * 4, packed);
       };
       tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + cs) * 16, rb);
       sixteen(ra, 0);
@@ -643,7 +604,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       } else {
         ctl->st_s1[slot][row] = part;
       }
-      if (!stats_launch(kLaunch)) tmem_wait_st();
+      tmem_wait_st();
       tc_fence_before();
       mbar_arrive(smem_u32(&ctl->p_ready[slot]));
       if (half == 0 && quad == 0) FMHA_STAMP(chain * 4 + 2, n);
@@ -656,11 +617,10 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
 // ---------------------------------------------------------------------------------------------- merge role
 // One thread = one half (D/2 columns) of the fp32 running output row of one query row, plus the running
 // maximum and the running sum of that row (kept by both threads of the row).
-template <int D, Launch kLaunch>
+template <int D>
 __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base, uint8_t* tiles,
                                            const UnitWalk walk) {
   constexpr int DH = D / 2;
-  constexpr bool kPolicy = policy_launch(kLaunch);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int quad = warp & 3, ch = (warp - kWarpMerge0) >> 2;       // ch = which half of the output columns
   const int row = quad * 32 + lane;
@@ -683,7 +643,6 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));     // only the tile count is needed here
     float m_run = -INFINITY, l_run = 0.f;
-    int imax_run = INT_MIN;                                 // statistics launches: biased integer row maximum over all tiles
 
 #pragma unroll 1
     for (int j = 0; j < n_live; ++j) {
@@ -695,25 +654,13 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
         return;
       }
       // ---- merge of tile statistics (inc/fmha_i8.cuh:301-304)
-      float e_old = j > 0 ? 1.f : 0.f, e_cur = 1.f;                    // policy launch: every tile of a row has the same scale
-      if (stats_launch(kLaunch)) imax_run = max(imax_run, ctl->st_i[slot][row]);
-      if (kLaunch == Launch::kRowPolicy) {
-        l_run += ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);      // (one scale: the tiles' sums add up)
-      } else if (!kPolicy && kLaunch != Launch::kRowMax) {
-        const float m_tile = ctl->st_m[slot][row];
-        const float l_tile = ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);
-        const float m_new = fmaxf(m_run, m_tile);
-        e_old = __expf(m_run - m_new);                                 // 0 on the first tile (m_run = -inf)
-        e_cur = clear_low2(__expf(m_tile - m_new));                    // 22 significant bits: kMagic*e_cur is exact
-        l_run = fmaf(e_old, l_run, e_cur * l_tile);
-        m_run = m_new;
-      }
-      if (stats_launch(kLaunch)) {                                     // no output is wanted: there is no P.V
-        tc_fence_after();
-        tc_fence_before();
-        mbar_arrive(smem_u32(&ctl->s_free[sb]));
-        continue;
-      }
+      const float m_tile = ctl->st_m[slot][row];
+      const float l_tile = ctl->st_f[slot][row] * (ctl->st_s0[slot][row] + ctl->st_s1[slot][row]);
+      const float m_new = fmaxf(m_run, m_tile);
+      const float e_old = __expf(m_run - m_new);                       // 0 on the first tile (m_run = -inf)
+      const float e_cur = clear_low2(__expf(m_tile - m_new));          // 22 significant bits: kMagic*e_cur is exact
+      l_run = fmaf(e_old, l_run, e_cur * l_tile);
+      m_run = m_new;
       const float2 e_cur2 = make_float2(e_cur, e_cur), e_bias = make_float2(-e_cur * kMagic, -e_cur * kMagic);
       const float2 e_old2 = make_float2(e_old, e_old);
 
@@ -754,17 +701,6 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
     const UnitGeom geo = unit_geom(p, u);
     const int q_row = geo.q_row0 + row;
 
-    // ---- statistics launch: the row's maximum and exp-sum over all keys, for the policy launch that follows
-    if (stats_launch(kLaunch)) {
-      if (ch == 0 && q_row < p.Sq)
-        p.row_stats_out[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row] =
-            make_float2(__int_as_float(n_live > 0 ? imax_run : static_cast<int>(kMagicBits)), n_live > 0 ? l_run : 0.f);
-      continue;
-    }
-    // the static policy's accumulated integer sum becomes the output through one factor, the per-row policy's through that / l
-    if (kLaunch == Launch::kStaticPolicy && q_row < p.Sq)
-      l_run = p.row_stats_in[static_cast<int64_t>(geo.bh_local) * p.Sq + q_row].y > 0.f ? 1.f : 0.f;
-
     // ---- calibration mode: only the largest magnitude of the unquantised output is wanted (the reference
     //      takes o_amax from its fp32 CPU result, test_fmha_i8.cpp:161)
     if (p.amax_out != nullptr) {
@@ -782,7 +718,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
 
     // ---- a partial result: fp32 half row into the tiles, which nothing uses any more (16-byte chunk c of row r at chunk
     //      c ^ (r & 15): neither these stores nor the merge's loads meet in a bank), maximum and sum beside it
-    if (!kPolicy && it >= walk.own) {
+    if (it >= walk.own) {
       float4* dst = reinterpret_cast<float4*>(tiles) + row * (D / 4);
 #pragma unroll
       for (int c = 0; c < DH / 4; ++c) dst[(ch * (DH / 4) + c) ^ (row & 15)] = make_float4(o2[2 * c].x, o2[2 * c].y, o2[2 * c + 1].x, o2[2 * c + 1].y);
@@ -873,8 +809,7 @@ __device__ __forceinline__ void merge_parts(const FwdParams& p, const uint32_t p
 // ---------------------------------------------------------------------------------------------- loader
 // One warp, run warp-wide (every lane waits and counts, one elected lane issues the copies): the Q tile of every
 // non-empty unit, then per step the K tile and the V tile, in step order.
-// (In a statistics launch no V tiles: there is no P.V.)
-template <int D, bool kStats>
+template <int D>
 __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl,
                                             const CUtensorMap* map_q, const CUtensorMap* map_k, const CUtensorMap* map_v,
                                             const uint32_t q_smem, const uint32_t k_smem, const uint32_t v_smem,
@@ -943,7 +878,6 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, FwdCtl<FwdCfg<D>
             tma_load_3d(k_smem + sk * Cfg::kTileBytes, map_k, smem_u32(&ctl->k_full[sk]), 0, t * kTile, geo.bh_local);
           }
         }
-        if (kStats) continue;
         if (rv > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&ctl->v_empty[sv]), (rv - 1) & 1u, abort_flag))) {
           fail = FMHA_I8_DEV_WAIT_V_FREE; fail_tile = g; break;
         }
@@ -1057,7 +991,7 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   if (err.code != 0u && elect_one()) raise_status(abort_flag, p.status, err.code, err.tile);
 }
 
-template <int D, bool kStats>
+template <int D>
 __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base,
                                               const uint32_t v_smem, const uint32_t bias_a_smem, const uint32_t bias_b_smem,
                                               const UnitWalk walk) {
@@ -1080,7 +1014,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
     const int n_live = ctl->info[buf].n_live;
     __syncwarp();
     if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));            // only the tile count is needed here
-    for (int j = 0; !kStats && j < n_live; ++j, ++g) {
+    for (int j = 0; j < n_live; ++j, ++g) {
       const uint32_t sb = g % SBufs<D>::n, stage = g % NV;
       uint64_t dv = make_smem_desc(v_smem + stage * Cfg::kTileBytes, D);
       const uint32_t tS = tmem_base + sb * kTile;
@@ -1110,7 +1044,7 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
 }
 
 // Persistent kernel: gridDim.x = min(units, SMs) CTAs; CTA b processes units b, b + gridDim.x, ...
-template <int D, Launch kLaunch>
+template <int D>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const FwdParams p) {
@@ -1185,19 +1119,19 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // phase of an info barrier = (it / kInfoBufs) & 1; `g` counts its steps (live key tiles) across units.
   if (warp >= kWarpSoftmax0) {
     setmaxnreg_dec<FwdRegs<D>::kSoftmax>();
-    softmax_role<D, kLaunch>(p, ctl, tmem_base, walk);
+    softmax_role<D>(p, ctl, tmem_base, walk);
   } else if (warp >= kWarpMerge0) {
     setmaxnreg_inc<FwdRegs<D>::kMerge>();
-    merge_role<D, kLaunch>(p, ctl, tmem_base, tiles, walk);
+    merge_role<D>(p, ctl, tmem_base, tiles, walk);
   } else {
     if (FwdRegs<D>::kOther < kLaunchRegs) setmaxnreg_dec<FwdRegs<D>::kOther>();
     else if (FwdRegs<D>::kOther > kLaunchRegs) setmaxnreg_inc<FwdRegs<D>::kOther>();
     if (warp == kWarpLoad) {
-      loader_role<D, stats_launch(kLaunch)>(p, ctl, &map_q, &map_k, &map_v, q_smem, k_smem, v_smem, walk);
+      loader_role<D>(p, ctl, &map_q, &map_k, &map_v, q_smem, k_smem, v_smem, walk);
     } else if (warp == kWarpMmaS) {
       s_issuer_role<D>(p, ctl, tmem_base, q_smem, k_smem, bias_a, walk);
     } else if (warp == kWarpMmaO) {
-      o_issuer_role<D, stats_launch(kLaunch)>(p, ctl, tmem_base, v_smem, smem_u32(bias_a), smem_u32(bias_b), walk);
+      o_issuer_role<D>(p, ctl, tmem_base, v_smem, smem_u32(bias_a), smem_u32(bias_b), walk);
     } else if (warp == kWarpScan) {
       // ---------------------------------------------------------------- scanner: mask information, units ahead
       bool ok = true;

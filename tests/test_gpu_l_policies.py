@@ -100,3 +100,39 @@ def test_policy_arguments_are_checked_on_the_host(pkg):
     bad = pkg.FMHAParamI8(1, 1, 1, 1, 0.0)
     sc = torch.zeros(128, dtype=torch.float32, device="cuda")
     assert pkg.FMHAInferI8Policy(None, bad, desc, t, t, t, mk, t, pkg.POLICY_STATIC, sc, check=False) == pkg.ERR_BAD_AMAX
+
+
+# The policies' kernel where its parts meet: one to seven groups of 64 keys with an unmasked one (three and two of them have scores under way
+# at once, eight and four places of two hold K and V), alone or beside masked ones, groups that do not follow each other, units of one
+# row and of 128, fewer units than an SM takes at once and several for every place.
+GROUPS = {
+    "lengths": lambda Sk, b: np.arange(Sk) >= min(Sk, (1, 64, 65, 128, 129, 192, 256, 257, 320, 384, 385, 448)[b % 12]),
+    "holes": lambda Sk, b: (np.arange(Sk) // 64 % 3 == b % 3) | (np.arange(Sk) % 64 >= 64 - 7 * (b % 4)) | (np.arange(Sk) // 64 == b % 9),
+}
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,D", [(12, 2, 1, 448, 64), (12, 2, 130, 448, 128), (24, 28, 65, 320, 64), (24, 14, 129, 256, 128), (12, 1, 128, 1088, 64)])
+@pytest.mark.parametrize("how", sorted(GROUPS))
+@pytest.mark.parametrize("policy", ["row", "static"])
+def test_policy_kernel_at_the_edges_of_its_rings(pkg, wl, oracle, B, H, Sq, Sk, D, how, policy):
+    import torch
+    torch.cuda.set_device(0)
+    rng = np.random.Generator(np.random.Philox(key=Sk + D))
+    q8, qa = wl.quantize_np(rng.standard_normal((B, H, Sq, D), dtype=np.float32))
+    k8, ka = wl.quantize_np(rng.standard_normal((B, H, Sk, D), dtype=np.float32))
+    v8, va = wl.quantize_np(rng.standard_normal((B, H, Sk, D), dtype=np.float32))
+    mask = np.stack([GROUPS[how](Sk, b) for b in range(B)]).astype(np.int8)
+    # o_amax = v_amax: a probability at a rounding boundary moves an output by one at the most
+    amax = (qa, ka, va, va, 0.5)
+    tq, tk, tv, tm = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    to = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    pkg.FMHAInferI8Policy(None, pkg.FMHAParamI8(*amax), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), tq, tk, tv, tm, to[128:-128],
+                          pkg.POLICY_ROW if policy == "row" else pkg.POLICY_STATIC, torch.zeros(B * H * Sq * 2, device="cuda"))
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    got = to.cpu().numpy()
+    assert (got[:128] == 0x5A).all() and (got[-128:] == 0x5A).all()
+    got = got[128:-128].reshape(q8.shape)
+    heads = slice(0, None, 13)                      # of every batch
+    want = oracle.policy(q8[:, heads], k8[:, heads], v8[:, heads], mask, amax, oracle.POLICY_ROW if policy == "row" else oracle.POLICY_STATIC)
+    assert_parity(got[:, heads], want, f"{policy} {how}")

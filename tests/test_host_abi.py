@@ -155,3 +155,10 @@ def test_tensor_memory_instructions_of_the_quantiser_follow_a_convergence():
     quant = open(os.path.join(csrc, "fmha_quant_sm100.cuh")).read()
     others = re.findall(r"(\S+)\s+(tmem_(?!alloc|dealloc|relinquish|ld_tile|st_tile)\w+\()", quant)
     assert others == [("__syncwarp();", "tmem_wait_st(")]
+
+
+def test_the_policies_kernel_uses_ordinary_loads():
+    """The same for the kernel of the whole-row policies, which waits in a function of its own."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "int8-flash-attention-fmha-quantization_b200", "csrc", "fmha_policy_sm100.cuh")).read())
+    assert text.count("grid_dependency_wait();") == 1 and text.count("__global__") == 1
+    assert "__restrict__" not in text and "__ldg" not in text
