@@ -134,9 +134,10 @@ int set_kernel_attributes(DeviceInfo* d) {
   auto set = [&](const void* fn, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   };
-  const void* const general64 = reinterpret_cast<const void*>(&fmha_fwd_kernel<64>), * const general128 = reinterpret_cast<const void*>(&fmha_fwd_kernel<128>);
-  set(general64, fwd_smem_bytes<64>());
-  set(general128, fwd_smem_bytes<128>());
+  const void* const general64[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<64, true>), reinterpret_cast<const void*>(&fmha_fwd_kernel<64, false>)};
+  const void* const general128[] = {reinterpret_cast<const void*>(&fmha_fwd_kernel<128, true>), reinterpret_cast<const void*>(&fmha_fwd_kernel<128, false>)};
+  for (const void* fn : general64) set(fn, fwd_smem_bytes<64>());
+  for (const void* fn : general128) set(fn, fwd_smem_bytes<128>());
   set_decode_attributes(set);
   const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<true>), reinterpret_cast<const void*>(&w64::fwd_kernel<false>)};
   for (const void* fn : workers) set(fn, w64::kSmemBytes);
@@ -160,7 +161,9 @@ int set_kernel_attributes(DeviceInfo* d) {
     std::fprintf(stderr, "fmha_i8_sm100: forward kernel built with %d registers per thread, expected %d; refusing to launch\n", fa.numRegs, regs);
     return false;
   };
-  bool as_built = check(general64, kLaunchRegs) && check(general128, kLaunchRegs);
+  bool as_built = true;
+  for (const void* fn : general64) as_built = as_built && check(fn, kLaunchRegs);
+  for (const void* fn : general128) as_built = as_built && check(fn, kLaunchRegs);
   for (const void* fn : workers) as_built = as_built && check(fn, w64::kLaunchRegs);
   for_policy_kernels([&](const void* fn, size_t, int regs) { as_built = as_built && check(fn, regs); });
   if (!as_built) return FMHA_I8_ERR_LAUNCH;
@@ -176,9 +179,9 @@ int set_kernel_attributes(DeviceInfo* d) {
     cfg.numAttrs = 1;
     int n64 = 0, n128 = 0;
     cfg.dynamicSmemBytes = fwd_smem_bytes<64>();
-    if (cudaOccupancyMaxActiveClusters(&n64, fmha_fwd_kernel<64>, &cfg) != cudaSuccess) n64 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n64, fmha_fwd_kernel<64, true>, &cfg) != cudaSuccess) n64 = 0;
     cfg.dynamicSmemBytes = fwd_smem_bytes<128>();
-    if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128>, &cfg) != cudaSuccess) n128 = 0;
+    if (cudaOccupancyMaxActiveClusters(&n128, fmha_fwd_kernel<128, true>, &cfg) != cudaSuccess) n128 = 0;
     cudaGetLastError();
     d->max_clusters[i] = n64 < n128 ? n64 : n128;
   }
@@ -447,7 +450,8 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
     how.cluster = static_cast<unsigned>(p.parts);
     grid = static_cast<unsigned>(p.own_rounds > 0 ? dev->sm_count : p.n_units * p.parts);
   }
-  return launch_kernel(fmha_fwd_kernel<D>, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
+  auto* fn = p.parts > 1 || p.amax_out != nullptr ? fmha_fwd_kernel<D, true> : fmha_fwd_kernel<D, false>;
+  return launch_kernel(fn, dim3(grid), dim3(kFwdThreads), fwd_smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
 
 // The few-rows kernel.  CTAs per head: enough for two rounds of the 3 CTAs that an SM holds, so that heads of different

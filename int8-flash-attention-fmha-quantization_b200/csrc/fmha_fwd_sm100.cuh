@@ -475,10 +475,11 @@ struct UnitWalk {
   int own, count, shared;
   __device__ __forceinline__ int unit(int it) const { return it < own ? static_cast<int>(blockIdx.x + it * gridDim.x) : shared; }
 };
+template <bool kFull>
 __device__ __forceinline__ UnitWalk unit_walk(const FwdParams& p) {
   const int b = static_cast<int>(blockIdx.x), ctas = static_cast<int>(gridDim.x);
   UnitWalk w;
-  if (p.parts == 1) {
+  if (!kFull || p.parts == 1) {
     w.own = w.count = (p.n_units - b + ctas - 1) / ctas;
     w.shared = 0;
   } else {
@@ -617,7 +618,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
 // ---------------------------------------------------------------------------------------------- merge role
 // One thread = one half (D/2 columns) of the fp32 running output row of one query row, plus the running
 // maximum and the running sum of that row (kept by both threads of the row).
-template <int D>
+template <int D, bool kFull>
 __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>::kStagesK, FwdCfg<D>::kStagesV>* ctl, const uint32_t tmem_base, uint8_t* tiles,
                                            const UnitWalk walk) {
   constexpr int DH = D / 2;
@@ -703,7 +704,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
 
     // ---- calibration mode: only the largest magnitude of the unquantised output is wanted (the reference
     //      takes o_amax from its fp32 CPU result, test_fmha_i8.cpp:161)
-    if (p.amax_out != nullptr) {
+    if (kFull && p.amax_out != nullptr) {
       float mx = 0.f;
       if (q_row < p.Sq && n_live > 0 && l_run > 0.f) {
         const float inv = 1.0f / l_run;
@@ -718,7 +719,7 @@ __device__ __forceinline__ void merge_role(const FwdParams& p, FwdCtl<FwdCfg<D>:
 
     // ---- a partial result: fp32 half row into the tiles, which nothing uses any more (16-byte chunk c of row r at chunk
     //      c ^ (r & 15): neither these stores nor the merge's loads meet in a bank), maximum and sum beside it
-    if (it >= walk.own) {
+    if (kFull && it >= walk.own) {
       float4* dst = reinterpret_cast<float4*>(tiles) + row * (D / 4);
 #pragma unroll
       for (int c = 0; c < DH / 4; ++c) dst[(ch * (DH / 4) + c) ^ (row & 15)] = make_float4(o2[2 * c].x, o2[2 * c].y, o2[2 * c + 1].x, o2[2 * c + 1].y);
@@ -1043,8 +1044,11 @@ __device__ __forceinline__ void o_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
   if (err.code != 0u && elect_one()) raise_status(abort_flag, p.status, err.code, err.tile);
 }
 
-// Persistent kernel: gridDim.x = min(units, SMs) CTAs; CTA b processes units b, b + gridDim.x, ...
-template <int D>
+// Persistent kernel: gridDim.x = min(units, SMs) CTAs; CTA b processes units b, b + gridDim.x, ...  kFull: units shared by clusters and
+// calibration too; without them the code is 47 KB instead of 60 (head_dim 128), which all but the longest calls feel, and the merge
+// warps spill nothing.  us, with -> without: B64 H32 S256 D128 75.6 -> 71.7, B128 H16 S128 D128 29.5 -> 27.3, B4 H32 S1024 D128 58.4 -> 57.2, B1 H12 S320 D128
+// 6.88 -> 6.35 and D64 6.23 -> 5.85, B6 H12 S512 D64 11.0 -> 10.5; B8 H32 S2048 D128 as before.
+template <int D, bool kFull>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const FwdParams p) {
@@ -1068,7 +1072,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   grid_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = (p.S + kTile - 1) / kTile;
-  const UnitWalk walk = unit_walk(p);
+  const UnitWalk walk = unit_walk<kFull>(p);
 
   if (threadIdx.x == 0) {
     ctl->abort = 0;
@@ -1122,7 +1126,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     softmax_role<D>(p, ctl, tmem_base, walk);
   } else if (warp >= kWarpMerge0) {
     setmaxnreg_inc<FwdRegs<D>::kMerge>();
-    merge_role<D>(p, ctl, tmem_base, tiles, walk);
+    merge_role<D, kFull>(p, ctl, tmem_base, tiles, walk);
   } else {
     if (FwdRegs<D>::kOther < kLaunchRegs) setmaxnreg_dec<FwdRegs<D>::kOther>();
     else if (FwdRegs<D>::kOther > kLaunchRegs) setmaxnreg_inc<FwdRegs<D>::kOther>();
@@ -1157,7 +1161,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   // every unit of this CTA has been computed and stored by the time the merge warps leave their loop
   tc_fence_before();
-  if (walk.count == walk.own) {      // (the same for all CTAs of a cluster)
+  if (!kFull || walk.count == walk.own) {      // (the same for all CTAs of a cluster)
     __syncthreads();
   } else {
     __syncwarp();
