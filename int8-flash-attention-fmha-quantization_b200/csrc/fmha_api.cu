@@ -139,7 +139,7 @@ int set_kernel_attributes(DeviceInfo* d) {
   for (const void* fn : general64) set(fn, fwd_smem_bytes<64>());
   for (const void* fn : general128) set(fn, fwd_smem_bytes<128>());
   set_decode_attributes(set);
-  const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<true>), reinterpret_cast<const void*>(&w64::fwd_kernel<false>)};
+  const void* const workers[] = {reinterpret_cast<const void*>(&w64::fwd_kernel<true, false>), reinterpret_cast<const void*>(&w64::fwd_kernel<false, false>), reinterpret_cast<const void*>(&w64::fwd_kernel<true, true>), reinterpret_cast<const void*>(&w64::fwd_kernel<false, true>)};
   for (const void* fn : workers) set(fn, w64::kSmemBytes);
   for_policy_kernels([&](const void* fn, size_t bytes, int) { set(fn, bytes); });
   set(reinterpret_cast<const void*>(&quant_grid_kernel<false>), kQuantGridSmem);
@@ -442,7 +442,8 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   unsigned grid = static_cast<unsigned>(p.n_units < sms ? p.n_units : sms);
   if constexpr (D == 64) {
     if (kernel == FMHA_I8_KERNEL_WORKERS) {
-      auto* fn = p.S <= w64::kShortTiles * kTile ? w64::fwd_kernel<true> : w64::fwd_kernel<false>;
+      const bool few = p.S <= w64::kShortTiles * kTile;
+      auto* fn = p.amax_out != nullptr ? (few ? w64::fwd_kernel<true, true> : w64::fwd_kernel<false, true>) : few ? w64::fwd_kernel<true, false> : w64::fwd_kernel<false, false>;
       return launch_kernel(fn, dim3(grid), dim3(w64::kThreads), w64::kSmemBytes, stream, how, mq, mk, mv, p);
     }
   }

@@ -23,12 +23,16 @@
 
 namespace fmha {
 namespace w64 {
-// There are two instances, one of them (kShort) for units of up to kShortTiles key tiles.  They differ in how the maximum of a half tile
+// Two instances of each kind, one of them (kShort) for units of up to kShortTiles key tiles.  They differ in how the maximum of a half tile
 // branches off that of a whole one: behind the first loads or in front of them.  Behind, the step is faster, and the compiler spills
 // values of the unit (-Xptxas -v: 72 bytes stored, 100 loaded, none in front), which short units pay for.  Behind against in front, in
 // per cent of the time: B256 H16 S256 (lengths 64..256) +2, B200 H12 S128 +1, B64 H16 S256 -1.5; B64 H16 S320 -2, B16 H12 S384 -3, B64 H16
 // S384 (130..384) -1.4, B8 H16 S512 -2.3, B32 H12 S512 (256..512) -2.6, S576 (300..576) -2.8, B8 H32 S2048 -3.  (What is spilled is the compiler's
 // choice: to be measured again when the step changes.)
+// The two kinds: without and with calibration (kCalib).  The smaller the code the faster short units are -- it is 54 and 62 KB without calibration, 25 of it
+// the drivers', and was 74: long masks scanned in smaller steps, not at all where there are none, calibration apart, units taken apart by
+// multiplications.  Together: B256 H16 S256 (64..256) 88.7 -> 85.1 us, B32 H12 S512 (256..512) 36.2 -> 35.4, B200 H12 S128 22.1 -> 21.5, B64 H16 S320 53.6 -> 52.5, B8 H32
+// S2048 335 -> 330.  (One copy of the driver per worker, 226 KB: 540.)
 constexpr int kShortTiles = 2;
 constexpr int kD = 64;
 constexpr int kWorkers = 4;          // per CTA
@@ -112,7 +116,7 @@ __device__ __forceinline__ int columns_max(const uint32_t taddr) {
 
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = one query row: its scores, probabilities, fp32 running output row, maximum and sum.
-template <bool kShort>
+template <bool kShort, bool kCalib>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base) {
   WorkerCtl* ctl = &all->w[worker];
   const int lane = threadIdx.x & 31, quad = warp_index() & 3;
@@ -248,7 +252,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
     const float inv = l_run > 0.f ? __frcp_rn(l_run) : 0.f;
-    if (p.amax_out != nullptr) {
+    if (kCalib) {
       // calibration: only the largest magnitude of the unquantised output is wanted (the reference takes o_amax from its
       // fp32 CPU result, test_fmha_i8.cpp:161); non-negative floats order like their bit patterns
       float mx = 0.f;
@@ -292,7 +296,7 @@ struct DriverStep {
   bool first;                // of its unit
   int bh, batch;
 };
-template <bool kEarlyK>
+template <bool kEarlyK, bool kCalib>
 __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const int worker, const CUtensorMap* map_q, const CUtensorMap* map_k,
                                             const CUtensorMap* map_v, const uint32_t tmem_base, const uint32_t worker_smem, uint8_t* presets) {
   WorkerCtl* ctl = &all->w[worker];
@@ -321,10 +325,11 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   int it = -1, j = 0, n_live = 0;
   uint32_t u = 0u;                            // the unit of the step handed out last
   int bh = 0, batch = 0, q_row0 = 0;          // its head, sequence and first query row
-  // The results of rows without an unmasked key.
+  // The results of rows without an unmasked key.  (Not unrolled: 1 KB of code.)
   auto empty_unit = [&](int rows, int64_t first_row) {
-    if (p.amax_out == nullptr) {
+    if (!kCalib) {
       uint4* dst = reinterpret_cast<uint4*>(p.o + first_row * kD);
+#pragma unroll 1
       for (int i = lane; i < rows * (kD / 16); i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
     }
   };
@@ -351,11 +356,10 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
         }
         return none;
       }
-      // (plain divisions: with unit_geom's multipliers this warp spills, 368 -> 371 us for B8 H32 S2048)
-      bh = static_cast<int>(u) / p.q_tiles;
-      batch = (p.bh_begin + bh) / p.H;
+      bh = fast_div(static_cast<int>(u), p.by_q_tiles);
+      batch = fast_div(p.bh_begin + bh, p.by_heads);
       q_row0 = (static_cast<int>(u) - bh * p.q_tiles) * kTile;
-      scan_mask_warp<true>(info, p.mask + static_cast<int64_t>(batch) * p.S, p.S, n_tiles);
+      scan_mask_warp<true, kEarlyK ? 1 : 2>(info, p.mask + static_cast<int64_t>(batch) * p.S, p.S, n_tiles);
       if (info->n_live == 0) {
         // Nobody else hears of a unit without keys: this warp is the one that P.V of the step before is waiting for, and may not wait
         // until the softmax warps have got through a row of such units.
@@ -400,7 +404,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   const uint32_t first = cta_unit(worker);
   const bool early = first < static_cast<uint32_t>(p.n_units);
   if (early && elect_one()) {
-    const int head = static_cast<int>(first) / p.q_tiles;
+    const int head = fast_div(static_cast<int>(first), p.by_q_tiles);
     mbar_arrive_expect_tx(smem_u32(&ctl->early_full), kEarlyK ? 2 * kTileBytes : kTileBytes);
     tma_load_3d(q_smem, map_q, smem_u32(&ctl->early_full), 0, (static_cast<int>(first) - head * p.q_tiles) * kTile, head);
     if (kEarlyK) tma_load_3d(k_smem, map_k, smem_u32(&ctl->early_full), 0, 0, head);
@@ -484,7 +488,7 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
   }
 }
 
-template <bool kShort>
+template <bool kShort, bool kCalib>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
            const FwdParams p) {
@@ -536,10 +540,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
   uint8_t* worker_smem = tiles + worker * kWorkerBytes;
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
-    w64::softmax_role<kShort>(p, ctl, worker, tmem_base);
+    w64::softmax_role<kShort, kCalib>(p, ctl, worker, tmem_base);
   } else {
     setmaxnreg_dec<kDriverRegs>();
-    driver_role<kShort>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
+    driver_role<kShort, kCalib>(p, ctl, worker, &map_q, &map_k, &map_v, tmem_base, smem_u32(worker_smem), presets);
   }
   tc_fence_before();
   __syncthreads();

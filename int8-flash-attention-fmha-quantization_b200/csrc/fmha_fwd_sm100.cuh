@@ -276,7 +276,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 // Builds one unit's view of its batch's padding mask: the list of live tiles and whether each has masked keys too.
 // Executed by ONE warp; a lane looks at 32 keys, four lanes make a tile.  kGroups: groups of eight tiles whose loads are in
-// flight together (four for long masks: 128 tiles one group after the other take 5 us).  kHalves: tiles with one open half are told apart.
+// flight together (for masks of more than 32 tiles, kLong: 128 tiles one group after the other take 5 us; in the workers, which feel the 7 KB of
+// code that four take, two: B1 H16 S8192 348 -> 338 us, one 347).  kHalves: tiles with one open half are told apart.
 template <int kGroups, bool kHalves, typename Info>
 __device__ __forceinline__ int scan_mask_groups(Info* info, const uint32_t* words, int S, int n_tiles) {
   const int lane = threadIdx.x & 31;
@@ -318,10 +319,10 @@ __device__ __forceinline__ int scan_mask_groups(Info* info, const uint32_t* word
   }
   return n;
 }
-template <bool kHalves, typename Info>
+template <bool kHalves, int kLong, typename Info>
 __device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_row, int S, int n_tiles) {
   const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
-  const int n = n_tiles <= 32 ? scan_mask_groups<1, kHalves>(info, words, S, n_tiles) : scan_mask_groups<4, kHalves>(info, words, S, n_tiles);
+  const int n = kLong == 1 || n_tiles <= 32 ? scan_mask_groups<1, kHalves>(info, words, S, n_tiles) : scan_mask_groups<kLong, kHalves>(info, words, S, n_tiles);
   if ((threadIdx.x & 31) == 0) info->n_live = n;
   __syncwarp();
 }
@@ -1148,7 +1149,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           if (!ok) { if (lane == 0) raise_status(abort_flag, p.status, FMHA_I8_DEV_WAIT_INFO, it); break; }
         }
         const UnitGeom geo = unit_geom(p, u);
-        scan_mask_warp<false>(&ctl->info[buf], p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
+        scan_mask_warp<false, 4>(&ctl->info[buf], p.mask + static_cast<int64_t>(geo.batch) * p.S, p.S, n_tiles);
         if (lane == 0) {
           const int n = ctl->info[buf].n_live, parts = it < walk.own ? 1 : p.parts, rank = static_cast<int>(blockIdx.x) % parts;
           ctl->info[buf].begin = n * rank / parts;
