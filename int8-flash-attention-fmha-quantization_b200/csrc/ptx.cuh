@@ -101,8 +101,30 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const v
       : "memory");
   return ok != 0u;
 }
+// For a warp whose lanes run together, with one answer for all of them: the vote in the loop makes its branches uniform, and nothing follows it
+// (a vote on the lanes' answers behind the loop above: B256 H16 S256 D64, 64..256 keys, 87.8 us instead of 85.6, B200 H12 S128 22.4 instead of 21.9, B64 H16 S64
+// 8.87 instead of 8.69; the general kernel's waits, of 32 lanes too, measure the same either way).
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
-  return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag));
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q, r;\n\t.reg .u32 left, flag;\n\t"
+      "mov.u32 left, %4;\n"
+      "WAIT_%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+      "@q bra.uni DONE_%=;\n\t"
+      "ld.volatile.shared.u32 flag, [%3];\n\t"
+      "sub.u32 left, left, 1;\n\t"
+      "setp.eq.u32 r, flag, 0;\n\t"
+      "setp.ne.and.u32 r, left, 0, r;\n\t"
+      "vote.sync.all.pred r, r, 0xffffffff;\n\t"
+      "@r bra.uni WAIT_%=;\n"
+      "DONE_%=:\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kWaitProbes)
+      : "memory");
+  return ok != 0u;
 }
 
 // One lane of a converged warp (the same one every time).  The single-thread roles of the forward kernel run
