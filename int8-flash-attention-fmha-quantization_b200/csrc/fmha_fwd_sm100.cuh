@@ -213,8 +213,9 @@ static_assert(kParamBytes % 64 == 24, "a launch's parameters have a size that is
 
 // Kinds of live key tiles.  Tiles with unmasked keys in one half only -- the last one of a sequence, every other time -- are
 // processed as the 64 keys of that half by the workers of fmha_fwd64_sm100.cuh: the other half's probabilities are zero and change
-// no maximum, no sum and no product.  Here they are tiles with masked keys: a second, shorter way through the softmax threads' 64
-// registers costs the first one more than it saves (B64 H32 S192 D128 72 -> 79 us, B8 H32 S2048 D128 415 -> 434).
+// no maximum, no sum and no product.  Here they are tiles with masked keys, of which the threads of a half without an unmasked one skip the
+// exponentials: a second, shorter way through the whole step with the softmax threads' 64 registers costs the first one more than it saves (B64 H32
+// S192 D128 72 -> 79 us, B8 H32 S2048 D128 415 -> 434).
 constexpr uint8_t kTileMixed = 1;      // (the half in use of) the tile has masked keys too
 constexpr uint8_t kTileLower = 2;      // keys 64..127 are all masked
 constexpr uint8_t kTileUpper = 4;      // keys 0..63 are all masked
@@ -580,6 +581,10 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       const int imax = max(mine, xrow[(half ^ 1) * kTile]);
       const RowConsts k = row_consts(imax, c2s, row_scale, scale_qk, p_mul);
       if (half == 0 && quad == 0) FMHA_STAMP(chain * 4 + 1, n);
+      // Half a tile without an unmasked key (the last one of a sequence, every other time): no exponentials, all P are zero.  (The mask is the same
+      // for all rows, and scores of unmasked keys are positive as biased integers.  B128 H16 S192 D128 66.7 -> 64.2 us, B128 H16 S64 23.2 -> 21.9, one
+      // request of S320 5.77 -> 5.60 and at head_dim 128 6.36 -> 6.11; long sequences without such halves up to +0.3 %.)
+      const bool none = __all_sync(0xFFFFFFFFu, mine < 0);
 
       // ---- pass 2: exp, row sum, requantise, P over columns already consumed (inc/fmha_i8.cuh:208-253)
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -588,6 +593,13 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
         chunk_exp_pack<16>(r, k.c2, k.neg_hi, k.p_mul_f, sum, packed);
         tmem_st4(tP + (c0 + c * cs) * 4, packed);
       };
+      if (none) {
+        tmem_ld_fence(ra);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) packed[c] = 0u;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_st4(tP + c * 4, packed);
+      } else {
       tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + cs) * 16, rb);
       sixteen(ra, 0);
       tmem_ld_fence(rb); tmem_ld16_issue(tS + (c0 + 2 * cs) * 16, ra);
@@ -596,6 +608,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
       sixteen(ra, 2);
       tmem_ld_fence(rb);
       sixteen(rb, 3);
+      }
       // ---- publish the row statistics of this step for the merge threads
       const int slot = static_cast<int>(g & 3u);
       const float part = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
@@ -943,7 +956,6 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
       if (elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
       continue;
     }
-    if (!issuer_wait(err, smem_u32(&ctl->q_full[qb]), (qn / NQ) & 1u, FMHA_I8_DEV_WAIT_Q_LOAD, g, abort_flag)) break;
     const uint64_t dq = make_smem_desc(q_smem + qb * Cfg::kTileBytes, D);
     const int8_t* mask_row = p.mask + static_cast<int64_t>(unit_geom(p, u).batch) * p.S;
     for (int j = 0; j < n_live; ++j, ++g) {
@@ -956,6 +968,8 @@ __device__ __forceinline__ void s_issuer_role(const FwdParams& p, FwdCtl<FwdCfg<
 #pragma unroll
         for (int i = 0; i < 4; ++i) masked[i] = key0 + 32 * i >= p.S || mask_row[key0 + 32 * i] != 0;
       }
+      // (behind the loads of mask bytes: one request of S320 5.60 -> 5.50 us)
+      if (j == 0 && !issuer_wait(err, smem_u32(&ctl->q_full[qb]), (qn / NQ) & 1u, FMHA_I8_DEV_WAIT_Q_LOAD, g, abort_flag)) { ok = false; break; }
       // K first (it has normally been there for a while), then the accumulator: it still holds the partial output of
       // step g - n until the merge warps have drained it, and that hand-off is on the step-to-step critical path
       if (!issuer_wait(err, smem_u32(&ctl->k_full[stage]), (g / NK) & 1u, FMHA_I8_DEV_WAIT_K_LOAD, g, abort_flag)) { ok = false; break; }
