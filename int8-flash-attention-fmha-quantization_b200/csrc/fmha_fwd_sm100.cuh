@@ -206,10 +206,12 @@ struct FwdParams {
   unsigned char unused[32];            // see kParamBytes
 };
 
-// What a launch costs the host depends on the bytes of its parameters, in steps of 64 (as commands they go to the GPU in lines of that size): B1 H2 S64
-// D64 takes 4.1 to 4.4 us a call with 536 or 600 of them, 24 modulo 64, and 4.4 to 4.8 with 504, 520, 528, 552, 568 or 760.
+// The size of a launch's parameters matters beyond what it holds, for reasons that were not found: B1 H2 S64 D64 takes 4.1 to 4.4 us a call with 536 or
+// 600 bytes (24 modulo 64) and 4.4 to 4.8 with 504, 520, 528, 552, 568 or 760, in calls in a row, where the host is what they wait for; at head_dim
+// 128 it makes no difference to short calls, but B8 H32 S2048 takes 405 us with 520 or more and 415 with 504 or 512 (what the compiler keeps in registers
+// changes).
 constexpr size_t kParamBytes = 3 * sizeof(CUtensorMap) + sizeof(FwdParams);
-static_assert(kParamBytes % 64 == 24, "a launch's parameters have a size that is slow to hand over");
+static_assert(kParamBytes == 536, "another size: measure the smallest and the long calls again");
 
 // Kinds of live key tiles.  Tiles with unmasked keys in one half only -- the last one of a sequence, every other time -- are
 // processed as the 64 keys of that half by the workers of fmha_fwd64_sm100.cuh: the other half's probabilities are zero and change
