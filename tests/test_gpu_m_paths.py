@@ -673,3 +673,13 @@ def test_line_between_the_kernels_of_head_dim_64(pkg, torch_cuda, units, S, forw
     desc = pkg.AttnDataDescriptorX(units * 128 // max(S, 128), S, S, 1, 64)
     assert pkg.debug_plan(desc)[0] == getattr(pkg, "KERNEL_" + forward)
     assert pkg.debug_plan(desc, pkg.POLICY_ROW)[0] == getattr(pkg, "KERNEL_" + policy)
+
+
+# Single key tiles in less than two rounds of SMs, and query tiles too many for clusters of four: either side of the lines (on 148 SMs).
+@pytest.mark.parametrize("H,Sq,Sk,D,kernel,parts", [
+    (160, 128, 128, 64, "GENERAL", 1), (295, 128, 128, 64, "GENERAL", 1), (160, 128, 64, 64, "WORKERS", 1), (32, 128, 768, 64, "GENERAL", 4), (37, 128, 896, 64, "GENERAL", 1),
+    (37, 128, 1024, 64, "GENERAL", 2), (72, 128, 896, 64, "GENERAL", 1), (60, 128, 1152, 128, "GENERAL", 1), (60, 128, 1280, 128, "GENERAL", 2)])
+def test_lines_of_single_tiles_and_of_pairs(pkg, torch_cuda, H, Sq, Sk, D, kernel, parts):
+    if torch_cuda.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines lie elsewhere on another number of SMs")
+    assert pkg.debug_plan(pkg.AttnDataDescriptorX(1, Sq, Sk, H, D))[:2] == (getattr(pkg, "KERNEL_" + kernel), parts)
