@@ -208,7 +208,7 @@ quant_grid_kernel(const float* __restrict__ x, long long n, int8_t* __restrict__
   bool ok = true;
   uint32_t parity_bits = 0u;                   // bit s: parity of the next completion of ring slot s
   auto landed = [&](int s) {
-    ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&bar[s]), (parity_bits >> s) & 1u, abort_flag));
+    ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait_timed(smem_u32(&bar[s]), (parity_bits >> s) & 1u, abort_flag));
     parity_bits ^= 1u << s;
     return reinterpret_cast<const float4*>(ring + s * kQuantTile);
   };
