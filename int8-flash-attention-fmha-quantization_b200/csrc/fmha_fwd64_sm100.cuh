@@ -285,33 +285,6 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   }
 }
 
-// scan_mask_warp for up to two key tiles: a lane looks at four keys of each.  A driver that has just issued S of a unit's last step goes through this
-// before it gets to that step's P.V and to the next unit's first copies, 2300 cycles with the general form, which P.V of a half tile
-// waits for.  B256 H16 S256 (64..256 keys) 85.5 -> 84.3 us, B200 H12 S128 21.2 -> 21.0, B64 H16 S64 8.75 -> 8.56.
-__device__ __forceinline__ void scan_two_tiles(UnitInfo* info, const int8_t* mask_row, int S) {
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
-  const int lane = threadIdx.x & 31;
-  uint32_t w[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) w[t] = t * kTile + lane * 4 < S ? words[t * 32 + lane] : 0xFFFFFFFFu;
-  int n = 0;
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const uint32_t open = __ballot_sync(0xFFFFFFFFu, __vcmpeq4(w[t], 0u) != 0u), masked = __ballot_sync(0xFFFFFFFFu, w[t] != 0u);
-    const bool no_upper = (open >> 16) == 0u, no_lower = (open & 0xFFFFu) == 0u;
-    const uint32_t in_use = no_upper ? masked & 0xFFFFu : no_lower ? masked >> 16 : masked;
-    if (open != 0u) {
-      if (lane == 0) {
-        info->live[n] = static_cast<uint8_t>(t);
-        info->kind[n] = static_cast<uint8_t>((no_upper ? kTileLower : no_lower ? kTileUpper : 0) | (in_use != 0u ? kTileMixed : 0));
-      }
-      ++n;
-    }
-  }
-  if (lane == 0) info->n_live = n;
-  __syncwarp();
-}
-
 // ---------------------------------------------------------------------------------------------- driver
 // One warp per worker, run warp-wide (every lane waits and counts, one elected lane issues).  Per step: S, then -- while the
 // softmax warps work -- V of the step, the mask scan and, S having completed, K (and Q) of the step after it, then P.V.  A
@@ -387,7 +360,8 @@ __device__ __forceinline__ void driver_role(const FwdParams& p, Ctl* all, const 
       batch = fast_div(p.bh_begin + bh, p.by_heads);
       q_row0 = (static_cast<int>(u) - bh * p.q_tiles) * kTile;
       const int8_t* mask_row = p.mask + static_cast<int64_t>(batch) * p.S;
-      if (kEarlyK) scan_two_tiles(info, mask_row, p.S);
+      if (kEarlyK) scan_few_tiles<2, true>(info, mask_row, p.S);
+      else if (n_tiles <= 4) scan_few_tiles<4, true>(info, mask_row, p.S);
       else scan_mask_warp<true, 2>(info, mask_row, p.S, n_tiles);
       if (info->n_live == 0) {
         // Nobody else hears of a unit without keys: this warp is the one that P.V of the step before is waiting for, and may not wait
