@@ -158,7 +158,7 @@ fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdP
     const uint32_t masked = key0 < p.S ? ~__vcmpeq4(mask4[key0 >> 2], 0u) : 0xFFFFFFFFu;    // byte = 0xFF: masked
 
     // ---- scores of my four keys (inc/fmha_i8.cuh:120-172)
-    if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar_k, n & 1u, abort_flag)))) break;
+    if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait_timed(bar_k, n & 1u, abort_flag)))) break;
     int s[R][4];
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -229,7 +229,7 @@ fmha_decode_kernel(const int8_t* q, const int8_t* k, const int8_t* v, const FwdP
 
     // ---- P.V of my four output columns (inc/fmha_i8.cuh:255-296); at head_dim 64 the two halves of the warp take one half
     //      of the keys each and are added up at the end
-    if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar_v, n & 1u, abort_flag)))) break;
+    if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait_timed(bar_v, n & 1u, abort_flag)))) break;
     constexpr int kWords = D / 4, kGroups = 32 * kWords / 32;       // words per row; groups of four keys per lane
     const int col = lane & (kWords - 1), group0 = (D == 64) ? (lane >> 4) * kGroups : 0;
     const uint32_t* vw = reinterpret_cast<const uint32_t*>(v_tile) + 4 * group0 * kWords + col;

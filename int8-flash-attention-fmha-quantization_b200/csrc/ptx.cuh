@@ -78,7 +78,8 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
     }
   }
 }
-// For waits that are short if not satisfied at once, where the first probe apart is 0.4 % of the time (the quantiser, 67,108,864 elements 75.8 us, with mbar_wait 76.1).
+// For kernels that stream through memory and have few waits, where the first probe apart is 0.3 to 0.4 % of the time (the quantiser, 67,108,864 elements
+// 75.8 us, with mbar_wait 76.1; decoding, B16 H32 Sq1 Sk4096 (1025..4096) 57.29, with mbar_wait 57.45).
 __device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
   return mbar_wait_limited(bar, parity, abort_flag, kWaitLimitCycles, 4096u);
 }
