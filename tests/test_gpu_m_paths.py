@@ -109,8 +109,8 @@ def torch_cuda():
 
 
 # One cluster of 1, 2, 4, 8 and 16 CTAs; then the whole chip, where a warp has 0, 1, 4 (all kept in registers), 7 and 8 (one
-# ring), 12 tiles of 1024 elements, with and without a remainder.  Up to 11 tiles a warp holds in registers and its ring; with 12 to 19
-# tensor memory holds eight as well, with 20 and 33 the rest is read again, from the L2 and, beyond what that is asked to hold, from DRAM.
+# ring), 12 tiles of 1024 elements, with and without a remainder.  Up to 12 tiles a warp holds in registers and its ring; with 13 to 20
+# tensor memory holds eight as well, with 21 and 33 the rest is read again, from the L2 and, beyond what that is asked to hold, from DRAM.
 SWEEP = 148 * 8 * 1024
 @pytest.mark.parametrize("n", [1, 3, 8192, 8193, 32771, 65536, 65537, 262144, 262147, 524288, 524289, SWEEP - 1, SWEEP, 4 * SWEEP + 1,
                                5 * SWEEP, 7 * SWEEP + 1023, 8 * SWEEP, 12 * SWEEP + 1025, 11 * SWEEP, 11 * SWEEP + 1024, 19 * SWEEP - 1, 20 * SWEEP + 2047,
@@ -129,6 +129,12 @@ def test_quantize_sizes(pkg, oracle, torch_cuda, n):
         assert np.array_equal(host[:n], oracle.quantize(y, np.abs(y).max())), (n, at)
         assert np.all(host[n:] == 0x5A)
     assert pkg.device_status()[0] == pkg.OK
+
+
+@pytest.mark.parametrize("n", [5 * SWEEP + 1024, 6 * SWEEP + 3, 12 * SWEEP, 12 * SWEEP + 1024, 20 * SWEEP, 20 * SWEEP + 1024, 21 * SWEEP + 1, 27 * SWEEP + 7])
+def test_quantize_sizes_around_what_a_warp_holds(pkg, oracle, torch_cuda, n):
+    """Five tiles of a warp in registers, seven in its ring, eight in tensor memory: on and beyond each sum of them."""
+    test_quantize_sizes(pkg, oracle, torch_cuda, n)
 
 
 @pytest.mark.parametrize("n", [4099, 524289, 20 * SWEEP + 3])
