@@ -207,6 +207,7 @@ int set_kernel_attributes(DeviceInfo* d) {
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+using ReplaceAddressFn = CUresult (*)(CUtensorMap*, void*);
 using PointerAttributeFn = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
 template <typename Fn> Fn driver_fn(const char* name) {
   void* f = nullptr;
@@ -216,6 +217,10 @@ template <typename Fn> Fn driver_fn(const char* name) {
 }
 EncodeTiledFn encode_fn() {
   static EncodeTiledFn fn = driver_fn<EncodeTiledFn>("cuTensorMapEncodeTiled");
+  return fn;
+}
+ReplaceAddressFn replace_address_fn() {
+  static ReplaceAddressFn fn = driver_fn<ReplaceAddressFn>("cuTensorMapReplaceAddress");
   return fn;
 }
 PointerAttributeFn pointer_attribute_fn() {
@@ -237,6 +242,15 @@ int make_map(CUtensorMap* map, const void* base, int n_heads, int S, int D, int 
                         CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? FMHA_I8_OK : FMHA_I8_ERR_DRIVER;
+}
+
+// The map of another tensor of the same form, in 9 ns instead of the 46 of a new one: two of a call's three where queries and keys are as many, one
+// otherwise.  B1 H2 S64 D64, whose time is the host's: 3.66 -> 3.59 us.
+int same_map(CUtensorMap* map, const CUtensorMap& of, const void* base) {
+  ReplaceAddressFn fn = replace_address_fn();
+  if (!fn) return FMHA_I8_ERR_DRIVER;
+  *map = of;
+  return fn(map, const_cast<void*>(base)) == CUDA_SUCCESS ? FMHA_I8_OK : FMHA_I8_ERR_DRIVER;
 }
 
 bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
@@ -420,7 +434,7 @@ int launch_policy(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, cons
   int st;
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
   if ((st = make_map(&mk, k, p.bh_count, p.S, D, wholerow::kKeys)) != FMHA_I8_OK) return st;
-  if ((st = make_map(&mv, v, p.bh_count, p.S, D, wholerow::kKeys)) != FMHA_I8_OK) return st;
+  if ((st = same_map(&mv, mk, v)) != FMHA_I8_OK) return st;
   LaunchHow how;
   how.overlap = true;
   const unsigned grid = static_cast<unsigned>(p.n_units < dev->sm_count ? p.n_units : dev->sm_count);
@@ -432,8 +446,8 @@ int launch_fwd(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const v
   CUtensorMap mq, mk, mv;
   int st;
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
-  if ((st = make_map(&mk, k, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
-  if ((st = make_map(&mv, v, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
+  if ((st = p.S == p.Sq ? same_map(&mk, mq, k) : make_map(&mk, k, p.bh_count, p.S, D)) != FMHA_I8_OK) return st;
+  if ((st = same_map(&mv, mk, v)) != FMHA_I8_OK) return st;
   // Overlap takes the launch latency and the set-up of a launch out of the time of calls in a row; a call that nothing precedes gains
   // nothing.  (Per cent of the time with more than four rounds of units: B32 H12 S512 D64 with lengths 256..512 -6, B200 H12 S128 -9, B4 H32
   // S1024 D128 -4, B64 H32 S256 -4, B8 H32 S2048 and B256 H16 S256 D64 with lengths 64..256 -1 to 0.)  Its price: the CTAs of the next launch
