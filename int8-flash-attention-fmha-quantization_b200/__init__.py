@@ -37,7 +37,7 @@ FLAG_UINT8_P = 2     # P quantised as unsigned 8 bit, 255 levels (the reference 
 EXPORTS = (
     "fmha_i8_sm100_infer", "fmha_i8_sm100_infer_slice", "fmha_i8_sm100_infer_cross", "fmha_i8_sm100_calibrate_o_amax", "fmha_i8_sm100_infer_host",
     "fmha_i8_sm100_infer_host_slice", "fmha_i8_sm100_infer_policy",
-    "fmha_i8_sm100_debug_plan", "fmha_i8_sm100_debug_host_fetch", "fmha_i8_sm100_debug_qk", "fmha_i8_sm100_debug_pv", "fmha_i8_sm100_debug_simt", "fmha_i8_sm100_debug_simt_x", "fmha_i8_sm100_debug_wait_probe",
+    "fmha_i8_sm100_debug_plan", "fmha_i8_sm100_debug_host_fetch", "fmha_i8_sm100_debug_qk", "fmha_i8_sm100_debug_pv", "fmha_i8_sm100_debug_simt", "fmha_i8_sm100_debug_simt_x", "fmha_i8_sm100_debug_wait_probe", "fmha_i8_sm100_debug_wait_loops",
     "fmha_i8_sm100_quantize_f32", "fmha_i8_sm100_quantize_f32_noalloc", "fmha_i8_sm100_debug_quantize_whole_chip", "fmha_i8_sm100_device_status", "fmha_i8_sm100_last_status", "fmha_i8_sm100_status_string",
     "fmha_i8_sm100_launch_count", "fmha_i8_sm100_version",
 )
@@ -113,6 +113,7 @@ def lib():
         L.fmha_i8_sm100_debug_simt.argtypes = [vp, fp, ip, vp, vp, vp, vp, vp]
         L.fmha_i8_sm100_debug_simt_x.argtypes = [vp, fp, ip, vp, vp, vp, vp, vp, u]
         L.fmha_i8_sm100_debug_wait_probe.argtypes = [vp, ctypes.c_longlong]
+        L.fmha_i8_sm100_debug_wait_loops.argtypes = [vp, ctypes.c_longlong, vp]
         L.fmha_i8_sm100_quantize_f32.argtypes = [vp, vp, ctypes.c_longlong, vp, vp]
         L.fmha_i8_sm100_quantize_f32_noalloc.argtypes = [vp, vp, ctypes.c_longlong, vp, vp]
         L.fmha_i8_sm100_debug_quantize_whole_chip.argtypes = [vp, vp, ctypes.c_longlong, vp, vp]
@@ -313,6 +314,13 @@ def debug_wait_probe(stream, limit_cycles):
     st = lib().fmha_i8_sm100_debug_wait_probe(_stream_handle(stream), int(limit_cycles))
     if st != OK:
         raise FmhaError(st, "debug_wait_probe")
+
+
+def debug_wait_loops(stream, limit_cycles, out):
+    """Runs the kernels' wait loops with short limits; `out`: 15 int32 words on the device (see the C header)."""
+    st = lib().fmha_i8_sm100_debug_wait_loops(_stream_handle(stream), int(limit_cycles), _ptr(out))
+    if st != OK:
+        raise FmhaError(st, "debug_wait_loops")
 
 
 def quantize_f32(stream, x, out, amax_out=None, n=None, entry="fmha_i8_sm100_quantize_f32"):

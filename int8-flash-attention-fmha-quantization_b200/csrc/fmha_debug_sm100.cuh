@@ -207,6 +207,48 @@ __global__ void __launch_bounds__(32) wait_probe_kernel(unsigned* status, long l
   if (!done && threadIdx.x == 0) raise_status(&abort_word, status, FMHA_I8_DEV_WAIT_DEBUG, 4);
 }
 
+// The loops that the kernels wait in, each with a few probes only, by one warp: which == 0 mbar_wait (general kernel), 1 warp_wait (workers,
+// policies), 2 mbar_wait_limited (decoding, quantiser).  out[5 * which + ...] = {a wait for a phase that has completed says so, a wait
+// for one that never does says that it gave up, the cycles which that took, the same two for a wait that finds the abort flag raised}.
+__global__ void __launch_bounds__(32) wait_loops_kernel(unsigned* out, long long limit_cycles) {
+  constexpr uint32_t kFew = 64u;
+  __shared__ uint64_t bars[2];
+  __shared__ volatile int abort_word;
+  const uint32_t done = smem_u32(&bars[0]), never = smem_u32(&bars[1]);
+  if (threadIdx.x == 0) {
+    abort_word = 0;
+    mbar_init(done, 1);
+    mbar_init(never, 1);
+    mbar_init_fence();
+    mbar_arrive(done);
+  }
+  __syncwarp();
+  auto wait = [&](int which, uint32_t bar) -> bool {
+    if (which == 0) return mbar_wait<kFew>(bar, 0u, &abort_word);
+    if (which == 1) return warp_wait<kFew>(bar, 0u, &abort_word);
+    return mbar_wait_limited(bar, 0u, &abort_word, limit_cycles);
+  };
+  for (int which = 0; which < 3; ++which) {
+    unsigned* o = out + 5 * which;
+    const bool passed = __all_sync(0xFFFFFFFFu, wait(which, done));
+    if (threadIdx.x == 0) o[0] = passed ? 1u : 0u;
+    for (int raised = 0; raised < 2; ++raised) {
+      __syncwarp();
+      if (threadIdx.x == 0) abort_word = raised;
+      __syncwarp();
+      const long long t0 = clock64();
+      const bool gave_up = __all_sync(0xFFFFFFFFu, !wait(which, never));
+      if (threadIdx.x == 0) {
+        o[1 + 2 * raised] = gave_up ? 1u : 0u;
+        o[2 + 2 * raised] = static_cast<unsigned>(clock64() - t0);
+      }
+    }
+    __syncwarp();
+    if (threadIdx.x == 0) abort_word = 0;
+    __syncwarp();
+  }
+}
+
 // The whole forward pass on CUDA cores, one thread per query row, in the operation order of the
 // reference kernel's arithmetic (inc/fmha_i8.cuh:183-253,298-332): expf, per-tile renormalised
 // running output, no fused multiply-add in the merge.  grid (query tiles, heads), 128 threads.

@@ -86,6 +86,8 @@ __device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity, c
 // The same with kWaitProbes for the limit, in as few instructions as can be: the kernels have some twenty waits each, and how far their code
 // is spread costs them time (with the cycle counter read and a first probe in front of the loop, as above, B64 H32 S256 D128 took 82.9 us instead of
 // 77.8, B256 H16 S256 D64, 64..256 keys, 88.6 instead of 86.0, B8 H32 S2048 D128 424 instead of 419.5; the loop left to the compiler 78.6, 87.1 and 421.7).
+// (kProbes: for tests.)
+template <uint32_t kProbes = kWaitProbes>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
   uint32_t ok;
   asm volatile(
@@ -102,13 +104,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const v
       "DONE_%=:\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kWaitProbes)
+      : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kProbes)
       : "memory");
   return ok != 0u;
 }
 // For a warp whose lanes run together, with one answer for all of them: the vote in the loop makes its branches uniform, and nothing follows it
 // (a vote on the lanes' answers behind the loop above: B256 H16 S256 D64, 64..256 keys, 87.8 us instead of 85.6, B200 H12 S128 22.4 instead of 21.9, B64 H16 S64
 // 8.87 instead of 8.69; the general kernel's waits, of 32 lanes too, measure the same either way).
+template <uint32_t kProbes = kWaitProbes>
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
   uint32_t ok;
   asm volatile(
@@ -127,7 +130,7 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const v
       "DONE_%=:\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kWaitProbes)
+      : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kProbes)
       : "memory");
   return ok != 0u;
 }

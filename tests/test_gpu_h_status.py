@@ -30,9 +30,12 @@ def test_wait_that_runs_out_is_reported_and_the_context_survives(pkg, wl, oracle
     tq, tk, tv, tm = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, m))
     prm, desc = pkg.FMHAParamI8(*amax, 1.0), pkg.AttnDataDescriptor(B, S, H, D)
 
+    # (what a process does for the first time takes longer than the wait below: the forward call, the fill)
+    to = torch.full_like(tq, 0x5A)
+    pkg.FMHAInferI8(None, prm, desc, tq, tk, tv, tm, torch.empty_like(tq), True)
+    torch.cuda.synchronize()
     pkg.debug_wait_probe(None, 4_000_000)                 # about two milliseconds of SM cycles
     # a forward pass enqueued behind it, before the failure is visible on the host, runs normally
-    to = torch.full_like(tq, 0x5A)
     pkg.FMHAInferI8(None, prm, desc, tq, tk, tv, tm, to, True)
     torch.cuda.synchronize()
     d = np.abs(to.cpu().numpy().astype(np.int32) - want.astype(np.int32))
@@ -63,6 +66,22 @@ def test_wait_that_runs_out_is_reported_and_the_context_survives(pkg, wl, oracle
     pkg.FMHAInferI8(None, prm, desc, tq, tk, tv, tm, to, True)
     st, words = pkg.device_status()
     assert st == pkg.OK, words
+
+
+@pytest.mark.parametrize("loop", [0, 1, 2])
+def test_the_loops_that_the_kernels_wait_in_end(pkg, loop):
+    """mbar_wait, warp_wait and mbar_wait_limited themselves, on a barrier that never completes: they say so and return, they give up at once when
+    the abort flag is up, and a completed phase is seen."""
+    import torch
+    torch.cuda.set_device(0)
+    out = torch.full((3, 5), 77, dtype=torch.int32, device="cuda")
+    limit = 4_000_000
+    pkg.debug_wait_loops(None, limit, out)
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    passed, ran_out, cycles, cut_short, cut_cycles = out.cpu().tolist()[loop]
+    assert (passed, ran_out, cut_short) == (1, 1, 1)
+    assert 0 < cycles < 4 * limit and 0 < cut_cycles < limit // 2
 
 
 def test_probe_limit_is_checked_on_the_host(pkg):
