@@ -191,11 +191,12 @@ int fmha_i8_sm100_debug_simt_x(void* stream, const float amax[5], const int desc
  * is launched); fmha_i8_sm100_device_status() reports the words and clears them.  No counterpart in the
  * reference, which checks nothing. */
 int fmha_i8_sm100_debug_wait_probe(void* stream, long long limit_cycles);
-/* Debug: the three loops that the kernels wait in (0: the general forward kernel's, 1: the head_dim-64 workers' and the policies', 2: decoding's and
- * the quantiser's), each with a few probes, or with limit_cycles for its limit, on a barrier that never completes; one warp, which
- * returns normally and raises no status.  out15: device memory, 15 words, for each loop {1 if a wait for a completed phase says so, 1 if one that runs out
- * says so, the cycles it took, 1 if one that finds the abort flag raised gives up, the cycles that took}. */
-int fmha_i8_sm100_debug_wait_loops(void* stream, long long limit_cycles, unsigned* out15);
+/* Debug: the four loops that the kernels wait in (0: the general forward kernel's, 1: the head_dim-64 workers' and the policies', 2: theirs
+ * where a wait may be long, 3: decoding's and the quantiser's) with 64 probes, 2 and 3 with limit_cycles for their limit, on a barrier that never
+ * completes; one warp, which returns normally and raises no status.  out20: device memory, 20 words, for each loop {1 if a wait for a
+ * completed phase (2: one that completes after a quarter of the limit) says so, 1 if one that runs out says so, the cycles it took, 1 if one
+ * that finds the abort flag raised gives up, the cycles that took}. */
+int fmha_i8_sm100_debug_wait_loops(void* stream, long long limit_cycles, unsigned* out20);
 
 /* Per-tensor symmetric quantisation on the device, the producer step in front of the attention call:
  * amax = max|x| (abs_max, inc/utils.hpp:31-39) and q[i] = clamp(floor(x[i]*127/amax + 0.5), -127, 127)

@@ -317,7 +317,7 @@ def debug_wait_probe(stream, limit_cycles):
 
 
 def debug_wait_loops(stream, limit_cycles, out):
-    """Runs the kernels' wait loops with short limits; `out`: 15 int32 words on the device (see the C header)."""
+    """Runs the kernels' wait loops with short limits; `out`: 20 int32 words on the device (see the C header)."""
     st = lib().fmha_i8_sm100_debug_wait_loops(_stream_handle(stream), int(limit_cycles), _ptr(out))
     if st != OK:
         raise FmhaError(st, "debug_wait_loops")

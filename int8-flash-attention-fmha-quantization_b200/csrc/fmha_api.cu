@@ -982,13 +982,13 @@ int fmha_i8_sm100_debug_wait_probe(void* stream, long long limit_cycles) {
   return finish(cudaGetLastError() == cudaSuccess ? FMHA_I8_OK : FMHA_I8_ERR_LAUNCH);
 }
 
-int fmha_i8_sm100_debug_wait_loops(void* stream, long long limit_cycles, unsigned* out15) {
-  if (!out15) return finish(FMHA_I8_ERR_NULL_POINTER);
+int fmha_i8_sm100_debug_wait_loops(void* stream, long long limit_cycles, unsigned* out20) {
+  if (!out20) return finish(FMHA_I8_ERR_NULL_POINTER);
   if (limit_cycles < 1000 || limit_cycles > kWaitLimitCycles) return finish(FMHA_I8_ERR_TOO_LARGE);
-  if (!aligned(out15, 4)) return finish(FMHA_I8_ERR_MISALIGNED);
+  if (!aligned(out20, 4)) return finish(FMHA_I8_ERR_MISALIGNED);
   int err = FMHA_I8_OK;
   if (!current_device(&err)) return finish(err);
-  wait_loops_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(out15, limit_cycles);
+  wait_loops_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(out20, limit_cycles);
   g_launch_count.fetch_add(1, std::memory_order_relaxed);
   return finish(cudaGetLastError() == cudaSuccess ? FMHA_I8_OK : FMHA_I8_ERR_LAUNCH);
 }

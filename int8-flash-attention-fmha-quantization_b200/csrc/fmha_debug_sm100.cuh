@@ -203,34 +203,44 @@ __global__ void __launch_bounds__(32) wait_probe_kernel(unsigned* status, long l
     mbar_init_fence();
   }
   __syncwarp();
-  const bool done = __all_sync(0xFFFFFFFFu, mbar_wait_limited(smem_u32(&never), 0u, &abort_word, limit_cycles));
+  const bool done = warp_wait_long<16>(smem_u32(&never), 0u, &abort_word, static_cast<uint32_t>(limit_cycles));
   if (!done && threadIdx.x == 0) raise_status(&abort_word, status, FMHA_I8_DEV_WAIT_DEBUG, 4);
 }
 
-// The loops that the kernels wait in, each with a few probes only, by one warp: which == 0 mbar_wait (general kernel), 1 warp_wait (workers,
-// policies), 2 mbar_wait_limited (decoding, quantiser).  out[5 * which + ...] = {a wait for a phase that has completed says so, a wait
-// for one that never does says that it gave up, the cycles which that took, the same two for a wait that finds the abort flag raised}.
-__global__ void __launch_bounds__(32) wait_loops_kernel(unsigned* out, long long limit_cycles) {
+// The loops that the kernels wait in, each with kFew probes, by one warp: which == 0 mbar_wait (general kernel), 1 warp_wait, 2 warp_wait_long
+// (workers, policies), 3 mbar_wait_limited (decoding, quantiser).  out[5 * which + ...] = {a wait for a phase that has completed says so, a
+// wait for one that never does says that it gave up, the cycles which that took, the same two for a wait that finds the abort flag
+// raised}.  The phase of warp_wait_long completes while it waits, a quarter of its limit after the beginning.
+__global__ void __launch_bounds__(64) wait_loops_kernel(unsigned* out, long long limit_cycles) {
   constexpr uint32_t kFew = 64u;
-  __shared__ uint64_t bars[2];
+  __shared__ uint64_t bars[3];
   __shared__ volatile int abort_word;
-  const uint32_t done = smem_u32(&bars[0]), never = smem_u32(&bars[1]);
+  const uint32_t done = smem_u32(&bars[0]), never = smem_u32(&bars[1]), late = smem_u32(&bars[2]);
   if (threadIdx.x == 0) {
     abort_word = 0;
     mbar_init(done, 1);
     mbar_init(never, 1);
+    mbar_init(late, 1);
     mbar_init_fence();
     mbar_arrive(done);
   }
-  __syncwarp();
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    const long long begin = clock64();
+    while (clock64() - begin < limit_cycles / 4) { /* waiting for the time to come */ }
+    if (threadIdx.x == 32) mbar_arrive(late);
+    return;
+  }
   auto wait = [&](int which, uint32_t bar) -> bool {
     if (which == 0) return mbar_wait<kFew>(bar, 0u, &abort_word);
     if (which == 1) return warp_wait<kFew>(bar, 0u, &abort_word);
+    if (which == 2) return warp_wait_long<kFew>(bar, 0u, &abort_word, static_cast<uint32_t>(limit_cycles));
     return mbar_wait_limited(bar, 0u, &abort_word, limit_cycles);
   };
-  for (int which = 0; which < 3; ++which) {
+  for (int i = 2; i < 6; ++i) {            // warp_wait_long first: nothing has taken time yet
+    const int which = i % 4;
     unsigned* o = out + 5 * which;
-    const bool passed = __all_sync(0xFFFFFFFFu, wait(which, done));
+    const bool passed = __all_sync(0xFFFFFFFFu, wait(which, which == 2 ? late : done));
     if (threadIdx.x == 0) o[0] = passed ? 1u : 0u;
     for (int raised = 0; raised < 2; ++raised) {
       __syncwarp();

@@ -125,10 +125,9 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   const uint32_t tS = t_lane + static_cast<uint32_t>(worker * kTile), tP = tS;
   volatile int* abort_flag = &all->abort;
   uint32_t g = 0;                               // steps so far
-  auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
-    if (warp_wait(bar, parity, abort_flag)) return true;
-    raise_status(abort_flag, p.status, code, g);
-    return false;
+  auto or_fail = [&](bool waited, unsigned code) -> bool {
+    if (!waited) raise_status(abort_flag, p.status, code, g);
+    return waited;
   };
   int announced = 1;
   // The running row is never cleared: the first tile of a unit multiplies what the unit before has left by zero.
@@ -138,7 +137,8 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
 #pragma unroll 1
   for (int it = 0; it < announced; ++it) {
     const int buf = it % kInfoBufs;
-    if (!wait_or_fail(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO)) return;
+    // (this wait and P.V's are long while the driver goes through units without keys)
+    if (!or_fail(warp_wait_long(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag), FMHA_I8_DEV_WAIT_INFO)) return;
     const int n_live = ctl->info[buf].n_live;
     if (n_live < 0) continue;
     announced += 1 - ctl->info[buf].last;
@@ -149,7 +149,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
 #pragma unroll 1
     for (int j = 0; j < n_live; ++j, ++g) {
       const bool whole = (ctl->info[buf].kind[j] & kTileHalf) == 0;      // 128 columns of scores, or 64
-      if (!wait_or_fail(smem_u32(&ctl->s_full), g & 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
+      if (!or_fail(warp_wait(smem_u32(&ctl->s_full), g & 1u, abort_flag), FMHA_I8_DEV_WAIT_S_READY)) return;
       tc_fence_after();
       FMHA_STAMP(quad == 0 ? worker * 4 + 0 : 47, g);
       // ---- pass 1: biased integer maximum of the row (inc/fmha_i8.cuh:183-206)
@@ -227,7 +227,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       const float2 e_old2 = make_float2(e_old, e_old);
 
       // ---- P.V of this step into the running row (inc/fmha_i8.cuh:306-310)
-      if (!wait_or_fail(smem_u32(&ctl->o_full), g & 1u, FMHA_I8_DEV_WAIT_O_READY)) return;
+      if (!or_fail(warp_wait_long(smem_u32(&ctl->o_full), g & 1u, abort_flag), FMHA_I8_DEV_WAIT_O_READY)) return;
       tc_fence_after();
       FMHA_STAMP(quad == 0 ? worker * 4 + 3 : 47, g);
       // (two loads in flight: a round trip to tensor memory costs more than folding a chunk in)

@@ -123,16 +123,17 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   volatile int* abort_flag = &all->abort;
   uint32_t uses0 = 0, uses1 = 0;                // phase 1: uses of each buffer
   Ring<C::kBufs> unit_begin;                    // buffer of the unit's first group in phase 2
-  auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool {
-    if (warp_wait(bar, parity, abort_flag)) return true;
-    raise_status(abort_flag, p.status, code, uses0);
-    return false;
+  auto or_fail = [&](bool waited, unsigned code) -> bool {
+    if (!waited) raise_status(abort_flag, p.status, code, uses0);
+    return waited;
   };
+  auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool { return or_fail(warp_wait(bar, parity, abort_flag), code); };
 #pragma unroll 1
   for (int it = 0;; ++it) {
     const int buf = it % kInfoBufs;
     const uint32_t parity = static_cast<uint32_t>(it & 1);
-    if (!wait_or_fail(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO)) return;
+    // (long, as the issuer's, while the loader goes through units without keys)
+    if (!or_fail(warp_wait_long(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag), FMHA_I8_DEV_WAIT_INFO)) return;
     const UnitInfo* info = &ctl->info[buf];
     const int n = info->n;
     if (n < 0) return;
@@ -429,7 +430,10 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
   };
   for (int it = 0; fail == 0u; ++it) {
     const int buf = it % kInfoBufs;
-    if (!wait(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), FMHA_I8_DEV_WAIT_INFO)) break;
+    if (!warp_wait_long(smem_u32(&ctl->info_full[buf]), static_cast<uint32_t>((it / kInfoBufs) & 1), abort_flag)) {
+      fail = FMHA_I8_DEV_WAIT_INFO;
+      break;
+    }
     const UnitInfo* info = &ctl->info[buf];
     const int n = info->n;
     if (n < 0) break;

@@ -56,12 +56,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 
 
-// The limits of a wait: about one second at boost clock, and probes that take one and a half, since one that finds the phase incomplete
-// blocks for 2911 cycles, measured.  (The kernels' waits are counted and not timed: while the context is switched out on a shared GPU no probes
-// are made, so a long time slice elsewhere cannot end a wait.)  Most waits are for one key tile of one CTA (microseconds).  The longest are the softmax warps' of a
-// worker (fmha_fwd64_sm100.cuh) while its driver goes through a row of units without keys, of which they do not hear: 1.1 us a unit with
-// 64 keys, 8.8 with 32,768, measured, shared by the CTA's four workers.  As many such units as outputs fit into 180 GB (11 million of 8 KB with long
-// masks, 43 million of one row with short ones) are 0.2 s or less.
+// The limits of a wait.  Most are for one key tile of one CTA, microseconds, and are counted, kWaitProbes: a time slice of another context on a
+// shared GPU, in which no probes are made, cannot end such a wait.  How long a probe blocks that finds the phase incomplete is the system's
+// choice: 2911 cycles here, so that all of them take one and a half seconds (tests/test_gpu_h_status.py measures it); if they did not block at
+// all their instructions would still take some 20 ms.
+// That is not enough for waits which may be long for a good reason: those of a warp that does not hear of units without keys while another
+// one goes through a row of them (warp_wait_long).  1.1 us a unit with 64 keys, 8.8 with 32,768, measured in the workers, shared by the CTA's
+// four: as many as outputs fit into 180 GB (11 million of 8 KB with long masks, 43 million of one row with short ones) are 0.2 s or less.  Such
+// a wait ends when kWaitLimitCycles, about one second at boost clock, have passed as well.
 constexpr long long kWaitLimitCycles = 2000000000LL;
 constexpr uint32_t kWaitProbes = 1u << 20;
 
@@ -131,6 +133,38 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const v
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(ok)
       : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kProbes)
+      : "memory");
+  return ok != 0u;
+}
+
+// The same where the wait may be long (see kWaitLimitCycles), four instructions more: it ends when the probes are used up and the cycles have
+// passed.  (The low half of the cycle counter is enough: a probe takes microseconds, so the first that comes too late sees it.)  With all
+// waits like this, B64 H32 S256 D128 74.0 -> 74.7 us, B128 H16 S128 D128 28.3 -> 28.6, B64 H16 S64 D64 8.50 -> 8.64, B32 H12 S512 D64 (256..512)
+// 34.9 -> 35.1.
+template <uint32_t kProbes = kWaitProbes>
+__device__ __forceinline__ bool warp_wait_long(uint32_t bar, uint32_t parity, const volatile int* abort_flag, uint32_t limit_cycles = kWaitLimitCycles) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q, r;\n\t.reg .s32 left;\n\t.reg .u32 flag, start, t;\n\t"
+      "mov.u32 start, %%clock;\n\t"
+      "mov.s32 left, %4;\n"
+      "WAIT_%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+      "@q bra.uni DONE_%=;\n\t"
+      "ld.volatile.shared.u32 flag, [%3];\n\t"
+      "sub.s32 left, left, 1;\n\t"
+      "mov.u32 t, %%clock;\n\t"
+      "sub.u32 t, t, start;\n\t"
+      "setp.gt.s32 r, left, 0;\n\t"
+      "setp.lt.or.u32 r, t, %5, r;\n\t"
+      "setp.eq.and.u32 r, flag, 0, r;\n\t"
+      "vote.sync.all.pred r, r, 0xffffffff;\n\t"
+      "@r bra.uni WAIT_%=;\n"
+      "DONE_%=:\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(kProbes), "r"(limit_cycles)
       : "memory");
   return ok != 0u;
 }

@@ -162,3 +162,13 @@ def test_the_policies_kernel_uses_ordinary_loads():
     text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "int8-flash-attention-fmha-quantization_b200", "csrc", "fmha_policy_sm100.cuh")).read())
     assert text.count("grid_dependency_wait();") == 1 and text.count("__global__") == 1
     assert "__restrict__" not in text and "__ldg" not in text
+
+
+def test_waits_that_units_without_keys_can_make_long_are_timed():
+    """The workers' drivers and the policies' loaders go through units without keys alone: a wait for the next unit, and the workers' for the P.V that the
+    driver issues behind its search for one, may take a fifth of a second and must not end with its probes."""
+    csrc = os.path.join(ROOT, "int8-flash-attention-fmha-quantization_b200", "csrc")
+    for name, bars, sites in (("fmha_fwd64_sm100.cuh", "info_full|o_full", 2), ("fmha_policy_sm100.cuh", "info_full", 2)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        waits = re.findall(r"(\w+)\(smem_u32\(&ctl->(?:%s)\b[^)]*\), (?!1\))" % bars, text)
+        assert waits == ["warp_wait_long"] * sites, (name, waits)
