@@ -136,3 +136,33 @@ def test_policy_kernel_at_the_edges_of_its_rings(pkg, wl, oracle, B, H, Sq, Sk, 
     heads = slice(0, None, 13)                      # of every batch
     want = oracle.policy(q8[:, heads], k8[:, heads], v8[:, heads], mask, amax, oracle.POLICY_ROW if policy == "row" else oracle.POLICY_STATIC)
     assert_parity(got[:, heads], want, f"{policy} {how}")
+
+
+# Rows of 32,768 keys whose probabilities are equal but for the largest: fp32 sums of equal values err the most, always in one direction.  A
+# row's sum may be added up in 256 steps a thread, each of 64 keys (relative error 4e-6 for these values, restated on the CPU), not in 4096
+# steps of one (4e-5 to 5e-5).  The output is put beside a rounding boundary, 100.5 (1 +- 1.5e-5), so that the second falls on the wrong
+# side; beside the sum's, the exponential's two ulps and the requantisation's are 5e-7.
+@pytest.mark.parametrize("x", [0.05, 0.277, 0.504, 0.731])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("side", [1, -1])
+def test_row_sums_of_long_rows(pkg, oracle, x, D, side):
+    import torch
+    torch.cuda.set_device(0)
+    S, Sq = 32768, 128
+    q8, k8, v8 = np.zeros((1, 1, Sq, D), np.int8), np.zeros((1, 1, S, D), np.int8), np.full((1, 1, S, D), 100, np.int8)
+    q8[..., 0], k8[0, 0, 0, 0] = 64, 127
+    row_scale = float(oracle.row_scale(D))
+    k_amax = np.float32(x * 127 * 127 / (64 * 127 * row_scale))              # q_amax = 1: the other keys' scores lie x below the first one's
+    e = np.exp(-float(np.float32(k_amax / np.float32(127 * 127))) * 64 * 127 * row_scale)
+    level = np.rint(127 * e)
+    assert abs(127 * e - level) < 0.49
+    mean = 100 * (127 + level * (S - 1)) / (127 * (1 + e * (S - 1)))         # of the products, in units of v_amax / 127
+    o_amax = np.float32(mean / (100.5 * (1 + side * 1.5e-5)))
+    assert abs(mean / float(o_amax) / 100.5 - 1 - side * 1.5e-5) < 2e-7
+    tq, tk, tv = (torch.from_numpy(t).cuda() for t in (q8, k8, v8))
+    to = torch.full_like(tq, 0x5A)
+    pkg.FMHAInferI8Policy(None, pkg.FMHAParamI8(1.0, float(k_amax), 1.0, float(o_amax), 1.0), pkg.AttnDataDescriptorX(1, Sq, S, 1, D), tq, tk, tv,
+                          torch.zeros((1, S), dtype=torch.int8, device="cuda"), to, pkg.POLICY_ROW, torch.zeros(2 * Sq, device="cuda"))
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    assert (to == (101 if side > 0 else 100)).all(), to.unique().tolist()
