@@ -166,3 +166,31 @@ def test_row_sums_of_long_rows(pkg, oracle, x, D, side):
     st, words = pkg.device_status()
     assert st == pkg.OK, words
     assert (to == (101 if side > 0 else 100)).all(), to.unique().tolist()
+
+
+# The longest rows that a call may have, and near them: 512 groups to a list, rings gone round hundreds of times, sums of 2^29.
+@pytest.mark.parametrize("Sk", [8256, 32768])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("how", ["all", "holes", "one_group", "ragged"])
+@pytest.mark.parametrize("policy", ["row", "static"])
+def test_policies_of_long_rows(pkg, wl, oracle, Sk, D, how, policy):
+    import torch
+    torch.cuda.set_device(0)
+    B, H, Sq = 2, 2, 130
+    rng = np.random.Generator(np.random.Philox(key=Sk + D))
+    q8, qa = wl.quantize_np(rng.standard_normal((B, H, Sq, D), dtype=np.float32))
+    k8, ka = wl.quantize_np(rng.standard_normal((B, H, Sk, D), dtype=np.float32))
+    v8 = np.full((B, H, Sk, D), 127, np.int8) if how == "all" else wl.quantize_np(rng.standard_normal((B, H, Sk, D), dtype=np.float32))[0]
+    j = np.arange(Sk)
+    mask = np.stack([{"all": j < 0, "holes": (j // 64 % 3 == b) | (j % 64 >= 64 - 5 * b), "one_group": (j // 64 != Sk // 64 - 1 - b) & (j // 64 != 5),
+                      "ragged": j >= Sk - 64 * b - 17}[how] for b in range(B)]).astype(np.int8)
+    # o_amax: v_amax where all values are 127, else what averages of that many values reach; s_max: that of a few rows is exceeded
+    amax = (qa, ka, 1.0, 1.0 if how == "all" else 0.25, 4.0 / Sk)
+    tq, tk, tv, tm = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    to = torch.full_like(tq, 0x5A)
+    pkg.FMHAInferI8Policy(None, pkg.FMHAParamI8(*amax), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), tq, tk, tv, tm, to,
+                          pkg.POLICY_ROW if policy == "row" else pkg.POLICY_STATIC, torch.zeros(B * H * Sq * 2, device="cuda"))
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    want = oracle.policy(q8, k8, v8, mask, amax, oracle.POLICY_ROW if policy == "row" else oracle.POLICY_STATIC)
+    assert_parity(to.cpu().numpy(), want, f"{policy} {how}")
