@@ -17,9 +17,11 @@
 // the multiply-add pipe, 4 to 8 % of the time at both head_dims), the chain of one issuer per worker in phase 1.  An issuer's instructions
 // follow one another, so what it takes together shares a barrier (a wait for K and one for V: 25.6 us instead of 19.5 with one unit to an SM, B1 H4
 // S2048).
-// us, as two launches of the forward kernels -> here: per-row B4 H16 S1024 D64 (512..1024 keys)
-// 35.2 -> 25.0, B64 H16 S256 46.0 -> 32.6, B1 H32 S2048 70.9 -> 54.0, B1 H2 S64 7.2 -> 4.5, D128 B8 H16 S512 31.1 -> 20.7, B2 H32 S2048 155 -> 110; static
-// 45.1 -> 37.5 and D128 B8 H16 S512 36.0 -> 29.4; one unit to an SM and 8192 keys 75.7 -> 68.5 (static 107 -> 105).
+// us, as two launches of the forward kernels -> here: per-row B4 H16 S1024 D64 (512..1024 keys) 35.1 -> 24.6, B64 H16 S256 46.0 -> 33.1, B1 H32
+// S2048 70.8 -> 53.2, B1 H2 S64 7.2 -> 4.5, D128 B8 H16 S512 31.6 -> 20.8, B2 H32 S2048 155 -> 117; static the first 45.4 -> 36.0, D128 B8 H16 S512
+// 36.0 -> 28.6; one unit to an SM, static, B1 H2 S8192 D64 107.2 -> 100.6, D128 109.2 -> 108.7, eight units of 16,384 keys at head_dim 128 208.0 -> 211.2.
+// (The static policy's sum with constants of its own for each group, and a quarter of its exponentials on the multiply-add pipe in two of four
+// chunks instead of in all: 37.3 for the first, B1 H2 Sq1 Sk32768 D64 399.9 instead of 383.3, D128 424.5 instead of 403.1; two launches 384.4 and 406.1.)
 // (Four workers of one thread per row with one buffer of 64 columns each: 28.6 for the first, 2650 cycles of which 900 go by between the last
 // exponential of a group and the first of the next.)
 #pragma once
@@ -122,6 +124,8 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
   const uint32_t tO = t_worker + static_cast<uint32_t>(C::kOutCol + chain * C::kOutCols);
   volatile int* abort_flag = &all->abort;
   uint32_t uses0 = 0, uses1 = 0;                // phase 1: uses of each buffer
+  // static, phase 1: scores that much above the sum's reference are exponentials of up to two
+  const int slack = kStatic ? static_cast<int>(fminf(1.f / p.c2, 4194304.f)) : 0;
   Ring<C::kBufs> unit_begin;                    // buffer of the unit's first group in phase 2
   auto or_fail = [&](bool waited, unsigned code) -> bool {
     if (!waited) raise_status(abort_flag, p.status, code, uses0);
@@ -138,9 +142,11 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     const int n = info->n;
     if (n < 0) return;
 
-    // ---- phase 1: the row's maximum over all keys, as a biased integer (static: and the exp-sum in terms of the running maximum)
+    // ---- phase 1: the row's maximum over all keys, as a biased integer (static: and the exp-sum in terms of exp(m_run))
     int imax = INT_MIN;
     float m_run = -INFINITY, l_run = 0.f;
+    RowConsts base = {};
+    int limit = INT_MIN;
 #pragma unroll 1
     for (int a = 0; a * kChains < n; ++a) {
       const int b = a & 1, i = a * kChains + chain;
@@ -166,17 +172,22 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
           // (only groups with masked keys are preset)
           imax = max(imax, (info->group[i] & kMixed) != 0 ? mine : mine + static_cast<int>(kMagicBits));
         } else {
+          // The sum is kept in terms of a maximum that is renewed when a row of the warp has gone beyond it by more than a factor of two, which few groups do
+          // after the first: a group adds to the sum and forms no constants.
           imax = max(imax, mine);
-          const RowConsts k = row_consts(mine, p.c2, p.row_scale, p.scale_qk, 1.f);
+          if (__any_sync(0xFFFFFFFFu, mine > limit)) {
+            base = row_consts(imax, p.c2, p.row_scale, p.scale_qk, 1.f);
+            l_run *= __expf(m_run - base.m_tile);
+            m_run = base.m_tile;
+            limit = imax + slack;
+          }
           float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
           uint32_t none[4];
-          chunk_exp_pack<16, false, 0, false>(r0, k.c2, k.neg_hi, k.p_mul_f, sum, none);
-          chunk_exp_pack<16, false, 1, false>(r1, k.c2, k.neg_hi, k.p_mul_f, sum, none);
-          chunk_exp_pack<16, false, 0, false>(r2, k.c2, k.neg_hi, k.p_mul_f, sum, none);
-          chunk_exp_pack<16, false, 1, false>(r3, k.c2, k.neg_hi, k.p_mul_f, sum, none);
-          const float l = k.f * ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y)), m_new = fmaxf(m_run, k.m_tile);
-          l_run = fmaf(__expf(m_run - m_new), l_run, __expf(k.m_tile - m_new) * l);
-          m_run = m_new;
+          chunk_exp_pack<16, false, 1, false>(r0, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+          chunk_exp_pack<16, false, 1, false>(r1, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+          chunk_exp_pack<16, false, 1, false>(r2, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+          chunk_exp_pack<16, false, 1, false>(r3, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+          l_run = fmaf(base.f, (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y), l_run);
         }
       } else {
         mbar_arrive(smem_u32(&ctl->max_free[b]));
@@ -190,9 +201,9 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     const float2 other = ctl->stat[parity][chain ^ 1][row];
     imax = max(imax, __float_as_int(other.x));
     if (kStatic) {
-      const float m_other = ctl->sum[parity][chain ^ 1][row], m_new = fmaxf(m_run, m_other);
+      const float m_other = ctl->sum[parity][chain ^ 1][row], m = row_consts(imax, p.c2, p.row_scale, p.scale_qk, 1.f).m_tile;
       // (a thread without a group has 0 and -inf; the other one has some)
-      l_run = fmaf(__expf(m_run - m_new), l_run, __expf(m_other - m_new) * other.y);
+      l_run = fmaf(__expf(m_run - m), l_run, __expf(m_other - m) * other.y);
     }
     // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = min(rn(levels * (e / l) / s_max), levels)
     const RowConsts k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, kStatic ? p.p_mul / (l_run > 0.f ? l_run : 1.f) : p.p_mul);

@@ -194,3 +194,31 @@ def test_policies_of_long_rows(pkg, wl, oracle, Sk, D, how, policy):
     assert st == pkg.OK, words
     want = oracle.policy(q8, k8, v8, mask, amax, oracle.POLICY_ROW if policy == "row" else oracle.POLICY_STATIC)
     assert_parity(to.cpu().numpy(), want, f"{policy} {how}")
+
+
+# The static policy's sum is kept in terms of a maximum that is renewed only when a row has gone beyond it by more than a factor of two:
+# scores that rise from group to group by less and by more than that, that fall, that jump in the last group, alike in all rows or not, at
+# scales from where the limit is beyond all scores to where it is the maximum itself.
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("scale", [1e-6, 0.003, 0.02, 0.3, 30.0])
+@pytest.mark.parametrize("how", ["rising", "falling", "last", "first"])
+def test_static_policy_whose_maxima_move(pkg, oracle, D, scale, how):
+    import torch
+    torch.cuda.set_device(0)
+    Sk, Sq = 1088, 128
+    rng = np.random.default_rng(D)
+    q8 = np.zeros((1, 1, Sq, D), np.int8)
+    q8[0, 0, :, 0] = np.arange(Sq) - 20                      # the rows' scores rise at different rates, a few fall
+    k8 = rng.integers(-2, 3, (1, 1, Sk, D)).astype(np.int8)
+    g = np.arange(Sk) // 64
+    k8[0, 0, :, 0] = {"rising": 7 * g, "falling": 7 * (16 - g), "last": 120 * (g == 16), "first": 120 * (g == 0)}[how]
+    v8 = rng.integers(-127, 128, (1, 1, Sk, D)).astype(np.int8)
+    mask = (rng.random((1, Sk)) < 0.1).astype(np.int8)
+    amax = (127.0, 127.0 * scale, 1.0, 1.0, 0.05)            # (a score of 1 counts scale / sqrt(D))
+    tq, tk, tv, tm = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    to = torch.full_like(tq, 0x5A)
+    pkg.FMHAInferI8Policy(None, pkg.FMHAParamI8(*amax), pkg.AttnDataDescriptorX(1, Sq, Sk, 1, D), tq, tk, tv, tm, to, pkg.POLICY_STATIC,
+                          torch.zeros(2 * Sq, device="cuda"))
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    assert_parity(to.cpu().numpy(), oracle.policy(q8, k8, v8, mask, amax, oracle.POLICY_STATIC), f"{how} {scale}")
