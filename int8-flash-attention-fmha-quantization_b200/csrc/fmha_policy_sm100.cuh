@@ -18,10 +18,10 @@
 // follow one another, so what it takes together shares a barrier (a wait for K and one for V: 25.6 us instead of 19.5 with one unit to an SM, B1 H4
 // S2048).
 // us, as two launches of the forward kernels -> here: per-row B4 H16 S1024 D64 (512..1024 keys) 35.1 -> 24.6, B64 H16 S256 46.0 -> 33.1, B1 H32
-// S2048 70.8 -> 53.2, B1 H2 S64 7.2 -> 4.5, D128 B8 H16 S512 31.6 -> 20.8, B2 H32 S2048 155 -> 117; static the first 45.4 -> 36.0, D128 B8 H16 S512
-// 36.0 -> 28.6; one unit to an SM, static, B1 H2 S8192 D64 107.2 -> 100.6, D128 109.2 -> 108.7, eight units of 16,384 keys at head_dim 128 208.0 -> 211.2.
+// S2048 70.8 -> 53.2, B1 H2 S64 7.2 -> 4.5, D128 B8 H16 S512 31.6 -> 20.8, B2 H32 S2048 155 -> 117; static the first 45.4 -> 35.7, D128 B8 H16 S512
+// 35.9 -> 28.3; one unit to an SM, static, B1 H2 S8192 D64 107.0 -> 99.8, D128 109.1 both, eight units of 16,384 keys at head_dim 128 207.8 -> 210.6.
 // (The static policy's sum with constants of its own for each group, and a quarter of its exponentials on the multiply-add pipe in two of four
-// chunks instead of in all: 37.3 for the first, B1 H2 Sq1 Sk32768 D64 399.9 instead of 383.3, D128 424.5 instead of 403.1; two launches 384.4 and 406.1.)
+// chunks instead of in all: 37.3 for the first, B1 H2 Sq1 Sk32768 D64 399.9 instead of 375.8, D128 424.5 instead of 401.3; two launches 383.5 and 405.3.)
 // (Four workers of one thread per row with one buffer of 64 columns each: 28.6 for the first, 2650 cycles of which 900 go by between the last
 // exponential of a group and the first of the next.)
 #pragma once
@@ -142,11 +142,14 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     const int n = info->n;
     if (n < 0) return;
 
-    // ---- phase 1: the row's maximum over all keys, as a biased integer (static: and the exp-sum in terms of exp(m_run))
+    // ---- phase 1: the row's maximum over all keys, as a biased integer (static: and the exp-sum, in terms of that of `ref`)
     int imax = INT_MIN;
-    float m_run = -INFINITY, l_run = 0.f;
+    float l_run = 0.f;
     RowConsts base = {};
-    int limit = INT_MIN;
+    int ref = 0, limit = INT_MIN;               // (biased integers of unmasked keys are positive)
+    // What a sum in terms of `from` is worth in terms of the larger `to`.  (Of whole numbers: a difference of two scaled maxima would have to
+    // be of two rounded products, and the compiler may form one of one product and a fused multiply-add.)
+    auto rescale = [&](int from, int to) { return ex2_approx(__int2float_rn(from - to) * p.c2); };
 #pragma unroll 1
     for (int a = 0; a * kChains < n; ++a) {
       const int b = a & 1, i = a * kChains + chain;
@@ -177,8 +180,8 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
           imax = max(imax, mine);
           if (__any_sync(0xFFFFFFFFu, mine > limit)) {
             base = row_consts(imax, p.c2, p.row_scale, p.scale_qk, 1.f);
-            l_run *= __expf(m_run - base.m_tile);
-            m_run = base.m_tile;
+            l_run *= rescale(ref, imax);
+            ref = imax;
             limit = imax + slack;
           }
           float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -194,16 +197,15 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       }
     }
     ctl->stat[parity][chain][row] = make_float2(__int_as_float(imax), l_run);
-    if (kStatic) ctl->sum[parity][chain][row] = m_run;
+    if (kStatic) ctl->sum[parity][chain][row] = __int_as_float(ref);
     mbar_arrive(smem_u32(&ctl->xch[quad]));
     // (with the row policy a unit has two exchanges, with the static one)
     if (!wait_or_fail(smem_u32(&ctl->xch[quad]), kStatic ? parity : 0u, FMHA_I8_DEV_WAIT_S_READY)) return;
     const float2 other = ctl->stat[parity][chain ^ 1][row];
     imax = max(imax, __float_as_int(other.x));
     if (kStatic) {
-      const float m_other = ctl->sum[parity][chain ^ 1][row], m = row_consts(imax, p.c2, p.row_scale, p.scale_qk, 1.f).m_tile;
-      // (a thread without a group has 0 and -inf; the other one has some)
-      l_run = fmaf(__expf(m_run - m), l_run, __expf(m_other - m) * other.y);
+      // (a thread without a group has a sum of zero; the other one has some)
+      l_run = fmaf(rescale(ref, imax), l_run, rescale(__float_as_int(ctl->sum[parity][chain ^ 1][row]), imax) * other.y);
     }
     // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = min(rn(levels * (e / l) / s_max), levels)
     const RowConsts k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, kStatic ? p.p_mul / (l_run > 0.f ? l_run : 1.f) : p.p_mul);

@@ -198,9 +198,9 @@ def test_policies_of_long_rows(pkg, wl, oracle, Sk, D, how, policy):
 
 # The static policy's sum is kept in terms of a maximum that is renewed only when a row has gone beyond it by more than a factor of two:
 # scores that rise from group to group by less and by more than that, that fall, that jump in the last group, alike in all rows or not, at
-# scales from where the limit is beyond all scores to where it is the maximum itself.
+# scales from where the limit is beyond all scores to where it is the maximum itself, and to where exponents of scaled maxima would not be exact.
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("scale", [1e-6, 0.003, 0.02, 0.3, 30.0])
+@pytest.mark.parametrize("scale", [1e-6, 0.003, 0.02, 0.3, 30.0, 1e14])
 @pytest.mark.parametrize("how", ["rising", "falling", "last", "first"])
 def test_static_policy_whose_maxima_move(pkg, oracle, D, scale, how):
     import torch
