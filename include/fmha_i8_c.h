@@ -148,12 +148,13 @@ int fmha_i8_sm100_infer_host_slice(const float amax[5], const int desc[4],
 
 /* Debug: how a call on this device would run, without running it: plan[0] = the kernel, plan[1] = CTAs that share the key tiles of a
  * query tile (1: none do), plan[2] = whole rounds of query tiles, one per SM, in front of the shared ones.  desc5 as in
- * fmha_i8_sm100_infer_cross (all heads), policy as in fmha_i8_sm100_infer_policy: the plan of FMHA_I8_POLICY_TILE is that of the forward pass,
- * that of the others the calibration's (fmha_i8_sm100_calibrate_o_amax); the whole-row policies themselves have one kernel without
- * variants, csrc/fmha_policy_sm100.cuh. */
+ * fmha_i8_sm100_infer_cross (all heads), policy as in fmha_i8_sm100_infer_policy (FMHA_I8_POLICY_TILE: the forward pass), or
+ * FMHA_I8_PLAN_CALIBRATION for fmha_i8_sm100_calibrate_o_amax. */
+#define FMHA_I8_PLAN_CALIBRATION 3
 #define FMHA_I8_KERNEL_FEW_ROWS 0   /* csrc/fmha_decode_sm100.cuh */
 #define FMHA_I8_KERNEL_GENERAL 1    /* csrc/fmha_fwd_sm100.cuh */
 #define FMHA_I8_KERNEL_WORKERS 2    /* csrc/fmha_fwd64_sm100.cuh */
+#define FMHA_I8_KERNEL_POLICY 3     /* csrc/fmha_policy_sm100.cuh */
 int fmha_i8_sm100_debug_plan(const int desc5[5], int policy, int plan[3]);
 
 /* Debug: how fmha_i8_sm100_infer_host would bring these inputs in, without doing it: 1 = a kernel reads the host buffers (all of q, k

@@ -263,7 +263,8 @@ def FMHAInferI8HostSlice(fmha_param, attn_desc, host_q, host_k, host_v, host_mas
     return st
 
 
-KERNEL_FEW_ROWS, KERNEL_GENERAL, KERNEL_WORKERS = 0, 1, 2
+KERNEL_FEW_ROWS, KERNEL_GENERAL, KERNEL_WORKERS, KERNEL_POLICY = 0, 1, 2, 3
+PLAN_CALIBRATION = 3      # debug_plan's `policy` for calibrate_o_amax
 
 
 def debug_plan(attn_desc_x, policy=POLICY_TILE):

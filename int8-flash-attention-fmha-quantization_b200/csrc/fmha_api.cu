@@ -419,9 +419,11 @@ bool use_workers(const FwdParams& p, bool plain, const DeviceInfo* dev) {
 //   D64, 4 rows   B128 H32 S128 42.6 / 32.9, S256 and beyond the few-rows one or within a few per cent
 bool few_rows(int Sq, int S, int D) { return Sq <= 4 || (D == 64 && Sq <= kDecodeMaxRows && S > kTile); }
 
-// Chooses the kernel of a call and how its units are divided: fills p->parts and p->own_rounds.  `plain`: no calibration; `busy_sms`: SMs that something else is using.
-int plan_call(FwdParams* p, int D, bool plain, int busy_sms, const DeviceInfo* dev) {
+// Chooses the kernel of a call and how its units are divided: fills p->parts and p->own_rounds.  `plain`: no calibration; `busy_sms`: SMs that
+// something else is using.
+int plan_call(FwdParams* p, int D, int policy, bool plain, int busy_sms, const DeviceInfo* dev) {
   p->parts = 1;
+  if (policy != FMHA_I8_POLICY_TILE) return FMHA_I8_KERNEL_POLICY;
   if (plain && few_rows(p->Sq, p->S, D)) return FMHA_I8_KERNEL_FEW_ROWS;
   if (D == 64 && use_workers(*p, plain, dev)) return FMHA_I8_KERNEL_WORKERS;
   if (plain && busy_sms == 0) plan_parts(p, D, dev);
@@ -563,10 +565,10 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   if ((st = fill_units(&p, sh, bh_count)) != FMHA_I8_OK) return st;
   p.status = dev->status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int kernel = plan_call(&p, sh.D, !calib && policy == FMHA_I8_POLICY_TILE, busy_sms, dev);
+  const int kernel = plan_call(&p, sh.D, policy, !calib, busy_sms, dev);
   auto launch = [&](auto d) {
     constexpr int D = decltype(d)::value;
-    if (policy != FMHA_I8_POLICY_TILE) return is_static ? launch_policy<D, true>(s, dev, p, q, k, v) : launch_policy<D, false>(s, dev, p, q, k, v);
+    if (kernel == FMHA_I8_KERNEL_POLICY) return is_static ? launch_policy<D, true>(s, dev, p, q, k, v) : launch_policy<D, false>(s, dev, p, q, k, v);
     if (kernel == FMHA_I8_KERNEL_FEW_ROWS) return launch_decode<D>(s, dev, p, q, k, v);
     return launch_fwd<D>(s, dev, p, q, k, v, kernel, busy_sms);
   };
@@ -860,14 +862,15 @@ int fmha_i8_sm100_debug_plan(const int desc5[5], int policy, int plan[3]) {
   const Shape sh{desc5[0], desc5[1], desc5[2], desc5[3], desc5[4]};
   int st = check_shape_x(sh);
   if (st != FMHA_I8_OK) return finish(st);
-  if (policy < FMHA_I8_POLICY_TILE || policy > FMHA_I8_POLICY_STATIC) return finish(FMHA_I8_ERR_BAD_FLAGS);
+  if (policy < FMHA_I8_POLICY_TILE || policy > FMHA_I8_PLAN_CALIBRATION) return finish(FMHA_I8_ERR_BAD_FLAGS);
+  const bool calibration = policy == FMHA_I8_PLAN_CALIBRATION;
   int err = FMHA_I8_OK;
   DeviceInfo* dev = current_device(&err);
   if (!dev) return finish(err);
   if ((st = set_kernel_attributes(dev)) != FMHA_I8_OK) return finish(st);
   FwdParams p{};
   if ((st = fill_units(&p, sh, sh.B * sh.H)) != FMHA_I8_OK) return finish(st);
-  plan[0] = plan_call(&p, sh.D, policy == FMHA_I8_POLICY_TILE, 0, dev);
+  plan[0] = plan_call(&p, sh.D, calibration ? FMHA_I8_POLICY_TILE : policy, !calibration, 0, dev);
   plan[1] = p.parts;
   plan[2] = p.parts > 1 ? p.own_rounds : 0;
   return finish(FMHA_I8_OK);

@@ -277,7 +277,8 @@ def test_the_line_of_the_few_rows_kernel(pkg, torch_cuda):
         for B, H in ((1, 1), (16, 32)):
             desc = pkg.AttnDataDescriptorX(B, Sq, Sk, H, D)
             assert (pkg.debug_plan(desc)[0] == pkg.KERNEL_FEW_ROWS) == few, (D, Sq, Sk)
-            assert pkg.debug_plan(desc, pkg.POLICY_ROW)[0] != pkg.KERNEL_FEW_ROWS
+            assert pkg.debug_plan(desc, pkg.PLAN_CALIBRATION)[0] in (pkg.KERNEL_GENERAL, pkg.KERNEL_WORKERS)
+            assert all(pkg.debug_plan(desc, policy) == (pkg.KERNEL_POLICY, 1, 0) for policy in (pkg.POLICY_ROW, pkg.POLICY_STATIC))
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -363,7 +364,7 @@ def test_many_query_tiles_head_dim_64(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk,
     q8, k8, v8, mask, amax = _tensors(wl, B, H, Sq, Sk, 64, seed=B + Sk, mask_p=mask_p, valid=valid)
     q, k, v, m = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
     desc, param = pkg.AttnDataDescriptorX(B, Sq, Sk, H, 64), pkg.FMHAParamI8(*amax, 0.25)
-    assert pkg.debug_plan(desc)[0] == pkg.KERNEL_WORKERS and pkg.debug_plan(desc, pkg.POLICY_ROW)[0] == pkg.KERNEL_WORKERS
+    assert pkg.debug_plan(desc)[0] == pkg.KERNEL_WORKERS and pkg.debug_plan(desc, pkg.PLAN_CALIBRATION)[0] == pkg.KERNEL_WORKERS
     o = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
     scratch = torch.zeros(2 * B * H * Sq, device="cuda")
     if what == "amax":
@@ -668,17 +669,17 @@ def test_large_score_scales(pkg, wl, oracle, torch_cuda, B, H, Sq, Sk, D, c2):
     assert pkg.device_status()[0] == pkg.OK
 
 
-# Query tiles of S keys on either side of the line between the two head_dim-64 kernels (on 148 SMs), and the policies' own line.
-@pytest.mark.parametrize("units,S,forward,policy", [
+# Query tiles of S keys on either side of the line between the two head_dim-64 kernels (on 148 SMs), and calibration's own line.
+@pytest.mark.parametrize("units,S,forward,calibration", [
     (100, 64, "GENERAL", "GENERAL"), (296, 128, "WORKERS", "WORKERS"), (296, 256, "GENERAL", "WORKERS"), (520, 256, "WORKERS", "WORKERS"),
     (740, 256, "GENERAL", "WORKERS"), (1184, 256, "WORKERS", "WORKERS"), (444, 512, "GENERAL", "WORKERS"), (592, 1024, "WORKERS", "WORKERS"),
     (288, 1024, "GENERAL", "GENERAL"), (1184, 2048, "WORKERS", "WORKERS")])
-def test_line_between_the_kernels_of_head_dim_64(pkg, torch_cuda, units, S, forward, policy):
+def test_line_between_the_kernels_of_head_dim_64(pkg, torch_cuda, units, S, forward, calibration):
     if torch_cuda.cuda.get_device_properties(0).multi_processor_count != 148:
         pytest.skip("the line lies elsewhere on another number of SMs")
     desc = pkg.AttnDataDescriptorX(units * 128 // max(S, 128), S, S, 1, 64)
     assert pkg.debug_plan(desc)[0] == getattr(pkg, "KERNEL_" + forward)
-    assert pkg.debug_plan(desc, pkg.POLICY_ROW)[0] == getattr(pkg, "KERNEL_" + policy)
+    assert pkg.debug_plan(desc, pkg.PLAN_CALIBRATION)[0] == getattr(pkg, "KERNEL_" + calibration)
 
 
 # Single key tiles in less than two rounds of SMs, and query tiles too many for clusters of four: either side of the lines (on 148 SMs).
