@@ -460,8 +460,9 @@ __device__ __forceinline__ RowConsts row_consts(const int imax, const float c2s,
   k.c2 = make_float2(c2s, c2s);
   k.neg_hi = make_float2(-hi, -hi);
   k.p_mul_f = make_float2(p_mul * k.f, p_mul * k.f);        // 128 f (or 255 f): quantisation multiplier
-  // the value the reference computes for the maximal element (inc/fmha_i8.cuh:196)
-  k.m_tile = (row_scale * static_cast<float>(imax - static_cast<int>(kMagicBits))) * scale_qk;
+  // the value the reference computes for the maximal element (inc/fmha_i8.cuh:196); rounded by itself, since what is wanted of it are
+  // differences, and one of a rounded product and a fused multiply-add is not zero where the maxima are equal
+  k.m_tile = __fmul_rn(row_scale * static_cast<float>(imax - static_cast<int>(kMagicBits)), scale_qk);
   return k;
 }
 
