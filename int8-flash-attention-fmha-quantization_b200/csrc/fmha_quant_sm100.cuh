@@ -134,7 +134,7 @@ constexpr int kQuantStages = 7;                // ring of 7 x 4 KB per warp: all
 // elements 16.1 -> 15.7, 24,000,000 25.3 -> 25.0, 50,000,001 51.6 -> 51.1, 67,108,864 75.0 -> 74.2, 33,554,432 32.7 both; 6: 50.3 and 73.9,
 // but 33,554,432 take 34.8.
 constexpr int kQuantKeep = 5;
-static_assert(kQuantKeep <= kQuantStages, "the first tiles are taken from the slots of their first loads");
+static_assert(kQuantKeep < kQuantStages, "the first tiles are taken from the slots of their first loads, and the next one from the slot behind");
 constexpr int kQuantTmem = 8;                  // tiles a warp keeps in tensor memory, 32 columns each: the next
 constexpr uint32_t kQuantTmemCols = 32 * kQuantTmem * kQuantWarps / 4;      // two warps to a lane quarter
 static_assert(kQuantTmemCols <= 512, "tensor memory has 512 columns");

@@ -172,3 +172,11 @@ def test_waits_that_units_without_keys_can_make_long_are_timed():
         text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
         waits = re.findall(r"(\w+)\(smem_u32\(&ctl->(?:%s)\b[^)]*\), (?!1\))" % bars, text)
         assert waits == ["warp_wait_long"] * sites, (name, waits)
+
+
+def test_the_quantiser_keeps_fewer_tiles_than_its_ring_has_slots():
+    """Slot kQuantKeep is read behind the tiles that stay in registers: it has to exist, and the build has to refuse a number where it does not."""
+    quant = open(os.path.join(ROOT, "int8-flash-attention-fmha-quantization_b200", "csrc", "fmha_quant_sm100.cuh")).read()
+    keep, stages = (int(re.search(r"constexpr int %s = (\d+);" % name, quant).group(1)) for name in ("kQuantKeep", "kQuantStages"))
+    assert keep < stages and "int slot = kQuantKeep;" in quant
+    assert "static_assert(kQuantKeep < kQuantStages," in quant
