@@ -423,6 +423,14 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, Ctl* all, const 
 
 // ---------------------------------------------------------------------------------------------- issuer
 // One warp per worker, run warp-wide (every lane waits and counts, one elected lane issues): the MMAs of both phases.
+//
+// The order it relies on: MMAs of one thread run in the order of their issue, so S may go over the columns of P bytes right behind the P.V
+// that reads them, in phase 2 and at the beginning of the next unit.  PTX promises the order of two tcgen05.mma with one accumulator and one
+// shape, which these are not; that an earlier one has read its operand in tensor memory before a later one writes there is what published
+// kernels for this chip rely on too (FlashAttention's forward pass for sm_100 and CUTLASS's example 77_blackwell_fmha: P over S, the next
+// S issued behind P.V).  With a wait for P.V's completion in between, in both places, 80 forms of calls gave the same outputs to the last
+// bit, 30 % later and more, since the wait joins the issuer's chain: B4 H16 S1024 D64 (512..1024 keys) per-row 24.6 -> 31.8 us, B1 H32 S2048 D128
+// 57.2 -> 92.4, one unit to an SM B1 H2 S8192 D128 79.8 -> 168.  (The forward kernels need no such order: there the drain of P.V comes first.)
 template <int D, bool kStatic>
 __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base, const uint32_t worker_smem,
                                             uint8_t* presets) {
@@ -500,7 +508,8 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
       const uint32_t before = b ? uses1++ : uses0++;
       if (!landed()) break;
       if (before > 0u && !wait(smem_u32(&ctl->max_free[b]), (before - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
-      // the second half of the columns is where the sums of the unit before were
+      // (The first half of the columns may still hold P bytes of the unit before, whose P.V was issued in front: see the order above.)  The second
+      // half is where its sums were.
       if (a == 1 && it > 0 && !wait(smem_u32(&ctl->o_free), static_cast<uint32_t>((it - 1) & 1), FMHA_I8_DEV_WAIT_O_FREE)) break;
       tc_fence_after();
       if (whole) {
@@ -561,7 +570,7 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
 #pragma unroll
         for (int kk = 0; kk < kKeys / 32; ++kk) mma_i8_ts(tO, tP + kk * 8, desc_advance(dv, kk * 32 * D), idesc_o, i > 0 || kk > 0 ? 1u : 0u);
         if (ahead < n) {
-          // (behind P.V in the order of the tensor core, which has read the P bytes by then)
+          // (over the P bytes, behind the P.V that reads them: see the issuer's order above)
           issue_s(tS, d_preset, desc_advance(dv, C::kGroupBytes), true);
           mma_commit(bar_s);
           if (ahead == n - 1) mma_commit(smem_u32(&ctl->q_empty[qb]));
