@@ -545,7 +545,7 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
     // P8 = min(rn(127 e / (l s_max)), 127) and the output is (sum P8 v8) * s_max/127 * v_amax/127.
     const float levels = wholerow::kLevels;
     if (is_static && (!(amax[4] > 0.f) || !std::isfinite(amax[4]))) return FMHA_I8_ERR_BAD_AMAX;
-    p.p_mul = is_static ? levels / amax[4] : levels;
+    p.p_mul = is_static ? 1.f / amax[4] : levels;
     p.scale_v_out = is_static ? amax[4] * amax[2] / (levels * amax[3]) : amax[2] / (levels * amax[3]);
   }
   int err = FMHA_I8_OK;

@@ -202,7 +202,7 @@ struct FwdParams {
   float amax_scale;     // v_amax / (127 * 128)  (127 * 255 with unsigned P)
   unsigned* status;     // eight device status words
   // (Whole-row P scaling policies, fmha_policy_sm100.cuh: P8 = rn(p_mul * exp(score - row max)), or with the static scale
-  // rn(p_mul * exp(score - row max) / l); scale_v_out is the factor that turns sum_j P8 v8 [/ l] into int8 output units.)
+  // rn(127 min(p_mul * exp(score - row max) / l, 1)); scale_v_out is the factor that turns sum_j P8 v8 [/ l] into int8 output units.)
   unsigned char unused[32];            // see kParamBytes
 };
 
@@ -415,11 +415,12 @@ __device__ __forceinline__ float2 exp2_poly(float2 a) {
 // even).  The two low bytes are the pair, as long as no byte is negative.  One byte permutation then makes a word of two pairs:
 // four instructions per word against two multiply-adds and three permutations, which run at half rate.  (Long head_dim-128 sequences -1.4 to
 // -2.6 % in one run, within the power limit's noise in others; B256 H16 S256 D64, 64..256 keys, -0.8 %.)
-// kCap: p is limited to p_cap before it is quantised (the static policy clips at its top level, fmha_i8_quant_deviation.py:38-43).
+// kCap: p is multiplied by `share` and limited to one before it is quantised (the static policy clips at its top level,
+// fmha_i8_quant_deviation.py:38-43): multiplications that saturate, where a minimum has half their rate.
 // kPolyPairs: that many pairs of values per eight are computed by exp2_poly.  kPack = false: only the sums are wanted.
 template <int N, bool kCap = false, int kPolyPairs = 0, bool kPack = true>
 __device__ __forceinline__ void chunk_exp_pack(const uint32_t (&r)[N], const float2 c2, const float2 neg_hi,
-                                               const float2 p_mul_f, float2 (&sum)[2], uint32_t (&packed)[N / 4], const float p_cap = 0.f) {
+                                               const float2 p_mul_f, float2 (&sum)[2], uint32_t (&packed)[N / 4], const float share = 0.f) {
   const float2 magic2 = make_float2(kMagic, kMagic);
 #pragma unroll
   for (int g = 0; g < N / 4; ++g) {
@@ -430,8 +431,8 @@ __device__ __forceinline__ void chunk_exp_pack(const uint32_t (&r)[N], const flo
     float2 p01 = make_float2(ex2_approx(a01.x), ex2_approx(a01.y));
     float2 p23 = (g & 1) < kPolyPairs ? exp2_poly(a23) : make_float2(ex2_approx(a23.x), ex2_approx(a23.y));
     if (kCap) {
-      p01.x = fminf(p01.x, p_cap); p01.y = fminf(p01.y, p_cap);
-      p23.x = fminf(p23.x, p_cap); p23.y = fminf(p23.y, p_cap);
+      p01.x = __saturatef(p01.x * share); p01.y = __saturatef(p01.y * share);
+      p23.x = __saturatef(p23.x * share); p23.y = __saturatef(p23.y * share);
     }
     const float2 even = make_float2(p01.x, p23.x), odd = make_float2(p01.y, p23.y);
     sum[0] = __fadd2_rn(sum[0], even);

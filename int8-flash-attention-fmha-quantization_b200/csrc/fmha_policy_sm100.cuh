@@ -18,10 +18,11 @@
 // follow one another, so what it takes together shares a barrier (a wait for K and one for V: 25.6 us instead of 19.5 with one unit to an SM, B1 H4
 // S2048).
 // us, as two launches of the forward kernels -> here: per-row B4 H16 S1024 D64 (512..1024 keys) 35.1 -> 24.6, B64 H16 S256 46.0 -> 33.1, B1 H32
-// S2048 70.8 -> 53.2, B1 H2 S64 7.2 -> 4.5, D128 B8 H16 S512 31.6 -> 20.8, B2 H32 S2048 155 -> 117; static the first 45.4 -> 35.7, D128 B8 H16 S512
-// 35.9 -> 28.3; one unit to an SM, static, B1 H2 S8192 D64 107.0 -> 99.8, D128 109.1 both, eight units of 16,384 keys at head_dim 128 207.8 -> 210.6.
+// S2048 70.8 -> 53.2, B1 H2 S64 7.2 -> 4.5, D128 B8 H16 S512 31.6 -> 20.8, B2 H32 S2048 155 -> 117; static the first 45.1 -> 35.6, D128 B8 H16 S512
+// 35.9 -> 28.2; one unit to an SM, static, B1 H2 S8192 D64 107.0 -> 98.7, D128 108.9 -> 108.1, eight units of 16,384 keys at head_dim 128 207.8 -> 206.5.
 // (The static policy's sum with constants of its own for each group, and a quarter of its exponentials on the multiply-add pipe in two of four
-// chunks instead of in all: 37.3 for the first, B1 H2 Sq1 Sk32768 D64 399.9 instead of 375.8, D128 424.5 instead of 401.3; two launches 383.5 and 405.3.)
+// chunks instead of in all: 37.3 for the first, B1 H2 Sq1 Sk32768 D64 399.9 instead of 375.8, D128 424.5 instead of 401.3; its clip by minima instead
+// of by multiplications that saturate: 35.8, 375.5 instead of 364.9, 401.3 instead of 394.9; two launches 384 and 404.)
 // (Four workers of one thread per row with one buffer of 64 columns each: 28.6 for the first, 2650 cycles of which 900 go by between the last
 // exponential of a group and the first of the next.)
 #pragma once
@@ -207,9 +208,9 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       // (a thread without a group has a sum of zero; the other one has some)
       l_run = fmaf(rescale(ref, imax), l_run, rescale(__float_as_int(ctl->sum[parity][chain ^ 1][row]), imax) * other.y);
     }
-    // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = min(rn(levels * (e / l) / s_max), levels)
+    // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = rn(levels * min(e / (l s_max), 1))
     const RowConsts k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, kStatic ? p.p_mul / (l_run > 0.f ? l_run : 1.f) : p.p_mul);
-    const float p_cap = kLevels / k.p_mul_f.x;            // an exponential above this would quantise beyond the top level
+    const float2 p_mul = kStatic ? make_float2(kLevels, kLevels) : k.p_mul_f;
 
     // ---- phase 2: exp, row sum, requantise; the bytes go over columns already read
     float l_sum = 0.f;
@@ -224,7 +225,7 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
       uint32_t ra[16], rb[16], packed[4];
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       auto sixteen = [&](const uint32_t (&r)[16], uint32_t c, auto poly) {
-        chunk_exp_pack<16, kStatic, decltype(poly)::value>(r, k.c2, k.neg_hi, k.p_mul_f, sum, packed, p_cap);
+        chunk_exp_pack<16, kStatic, decltype(poly)::value>(r, k.c2, k.neg_hi, p_mul, sum, packed, k.p_mul_f.x);
         tmem_st4(tS + c * 4, packed);
       };
       constexpr Flight<0> mufu;
