@@ -119,8 +119,9 @@ template <typename Set> void set_decode_attributes(Set set) {
 template <typename Use> void for_policy_kernels(Use use) {
   auto one = [&](auto d) {
     constexpr int D = decltype(d)::value;
-    use(reinterpret_cast<const void*>(&wholerow::policy_kernel<D, false>), wholerow::smem_bytes<D>(), wholerow::kLaunchRegs);
-    use(reinterpret_cast<const void*>(&wholerow::policy_kernel<D, true>), wholerow::smem_bytes<D>(), wholerow::kLaunchRegs);
+    use(reinterpret_cast<const void*>(&wholerow::policy_kernel<D, false, false>), wholerow::smem_bytes<D>(), wholerow::kLaunchRegs);
+    use(reinterpret_cast<const void*>(&wholerow::policy_kernel<D, true, false>), wholerow::smem_bytes<D>(), wholerow::kLaunchRegs);
+    use(reinterpret_cast<const void*>(&wholerow::policy_kernel<D, true, true>), wholerow::smem_bytes<D>(), wholerow::kLaunchRegs);
   };
   one(std::integral_constant<int, 64>());
   one(std::integral_constant<int, 128>());
@@ -430,8 +431,8 @@ int plan_call(FwdParams* p, int D, int policy, bool plain, int busy_sms, const D
   return FMHA_I8_KERNEL_GENERAL;
 }
 
-template <int D, bool kStatic>
-int launch_policy(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v) {
+template <int D>
+int launch_policy(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, const void* q, const void* k, const void* v, bool is_static) {
   CUtensorMap mq, mk, mv;
   int st;
   if ((st = make_map(&mq, q, p.bh_count, p.Sq, D)) != FMHA_I8_OK) return st;
@@ -440,7 +441,8 @@ int launch_policy(cudaStream_t stream, DeviceInfo* dev, const FwdParams& p, cons
   LaunchHow how;
   how.overlap = true;
   const unsigned grid = static_cast<unsigned>(p.n_units < dev->sm_count ? p.n_units : dev->sm_count);
-  return launch_kernel(wholerow::policy_kernel<D, kStatic>, dim3(grid), dim3(wholerow::kThreads), wholerow::smem_bytes<D>(), stream, how, mq, mk, mv, p);
+  auto* fn = !is_static ? wholerow::policy_kernel<D, false, false> : p.S <= wholerow::kStep1 ? wholerow::policy_kernel<D, true, true> : wholerow::policy_kernel<D, true, false>;
+  return launch_kernel(fn, dim3(grid), dim3(wholerow::kThreads), wholerow::smem_bytes<D>(), stream, how, mq, mk, mv, p);
 }
 
 template <int D>
@@ -568,7 +570,7 @@ int infer_x_impl(void* stream, const float amax[5], const Shape& sh, const void*
   const int kernel = plan_call(&p, sh.D, policy, !calib, busy_sms, dev);
   auto launch = [&](auto d) {
     constexpr int D = decltype(d)::value;
-    if (kernel == FMHA_I8_KERNEL_POLICY) return is_static ? launch_policy<D, true>(s, dev, p, q, k, v) : launch_policy<D, false>(s, dev, p, q, k, v);
+    if (kernel == FMHA_I8_KERNEL_POLICY) return launch_policy<D>(s, dev, p, q, k, v, is_static);
     if (kernel == FMHA_I8_KERNEL_FEW_ROWS) return launch_decode<D>(s, dev, p, q, k, v);
     return launch_fwd<D>(s, dev, p, q, k, v, kernel, busy_sms);
   };

@@ -83,6 +83,7 @@ struct WorkerCtl {
   uint64_t full[kMaxStages], empty[kMaxStages];                          // a place of the ring has landed / has been multiplied
   uint64_t max_full[2], max_free[2];                                     // phase 1: scores are there / have been read
   uint64_t s_full[3], p_ready[3];                                        // phase 2, per buffer: scores are there / P is, and the scores have been read
+  uint64_t p_brief[kChains];                                             // kBrief, per group: P is there
   uint64_t o_full, o_free;                                               // the sums are complete / have been read
   uint64_t xch[4];                                                       // per lane quarter: both threads of a row have left their values
   uint64_t info_full[kInfoBufs], info_empty[kInfoBufs];
@@ -114,9 +115,45 @@ constexpr uint32_t kCommonB = kABytes, kOwnB = kABytes + kOperandBytes;
 
 template <int D> constexpr size_t smem_bytes() { return 1024 + kWorkers * Cfg<D>::kWorkerBytes + kPresetBytes + sizeof(Ctl); }
 
+// kBrief: the static policy's calls of no more groups than chains.  A thread has one group at the most, forms its exponentials once, in terms of
+// the group's own maximum, keeps them, and makes them bytes when the exchange has told it what they are worth: no second S, no second pass
+// over the keys.  In two phases such units are bound by their chain of dependent steps, and an SM has two units only: with many of them two
+// launches of the forward kernels were faster.  us, those -> two phases -> this, B512 H16 S128 D64 110.5 -> 113.7 -> 84.0, with 64..128 keys 110.6
+// -> 116.8 -> 87.4, 16 query rows 102.9 -> 111.6 -> 82.1, 16384 units of S64 with one row 137.8 -> 147.0 -> 113.1, B512 H16 S128 D128 190 -> 139 -> 109.
+// (The exponentials left in tensor memory meanwhile, which spills nothing instead of 24 bytes: 92.4 for the first.  Both forms in one
+// instance: the longer units lose 4 to 8 %.)
+// Sixteen scores to their exponentials, in place, and into the sums; a quarter of them on the multiply-add pipe.
+__device__ __forceinline__ void exps_in_place(uint32_t (&r)[16], const RowConsts& k, float2 (&sum)[2]) {
+#pragma unroll
+  for (int g = 0; g < 16; g += 4) {
+    const float2 a01 = __ffma2_rn(make_float2(__uint_as_float(r[g]), __uint_as_float(r[g + 1])), k.c2, k.neg_hi);
+    const float2 a23 = __ffma2_rn(make_float2(__uint_as_float(r[g + 2]), __uint_as_float(r[g + 3])), k.c2, k.neg_hi);
+    const float2 p01 = make_float2(ex2_approx(a01.x), ex2_approx(a01.y));
+    const float2 p23 = (g & 4) == 0 ? exp2_poly(a23) : make_float2(ex2_approx(a23.x), ex2_approx(a23.y));
+    sum[0] = __fadd2_rn(sum[0], make_float2(p01.x, p23.x));
+    sum[1] = __fadd2_rn(sum[1], make_float2(p01.y, p23.y));
+    r[g] = __float_as_uint(p01.x);
+    r[g + 1] = __float_as_uint(p01.y);
+    r[g + 2] = __float_as_uint(p23.x);
+    r[g + 3] = __float_as_uint(p23.y);
+  }
+}
+// Those to bytes, as in chunk_exp_pack.
+__device__ __forceinline__ void pack_shares(const uint32_t (&r)[16], const float share, uint32_t (&packed)[4]) {
+  const float2 levels = make_float2(kLevels, kLevels);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    auto p = [&](int i) { return __saturatef(__uint_as_float(r[4 * g + i]) * share); };
+    const float2 high = __ffma2_rn(__ffma2_rn(make_float2(p(1), p(3)), levels, make_float2(kMagic, kMagic)), make_float2(256.f, 256.f),
+                                   make_float2(-255.f * kMagic, -255.f * kMagic));
+    const float2 y = __ffma2_rn(make_float2(p(0), p(2)), levels, high);
+    packed[g] = __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x5410);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------- softmax role
 // One thread = every kChains-th group of 64 keys of one query row, and D / kChains columns of its output.
-template <int D, bool kStatic>
+template <int D, bool kStatic, bool kBrief>
 __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const int worker, const int chain, const uint32_t tmem_base) {
   using C = Cfg<D>;
   WorkerCtl* ctl = &all->w[worker];
@@ -133,6 +170,9 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     return waited;
   };
   auto wait_or_fail = [&](uint32_t bar, uint32_t parity, unsigned code) -> bool { return or_fail(warp_wait(bar, parity, abort_flag), code); };
+  // What a sum in terms of `from` is worth in terms of the larger `to`.  (Of whole numbers: a difference of two scaled maxima would have to be
+  // of two rounded products, and the compiler may form one of one product and a fused multiply-add.)
+  auto rescale = [&](int from, int to) { return ex2_approx(__int2float_rn(from - to) * p.c2); };
 #pragma unroll 1
   for (int it = 0;; ++it) {
     const int buf = it % kInfoBufs;
@@ -143,116 +183,164 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
     const int n = info->n;
     if (n < 0) return;
 
-    // ---- phase 1: the row's maximum over all keys, as a biased integer (static: and the exp-sum, in terms of that of `ref`)
-    int imax = INT_MIN;
-    float l_run = 0.f;
-    RowConsts base = {};
-    int ref = 0, limit = INT_MIN;               // (biased integers of unmasked keys are positive)
-    // What a sum in terms of `from` is worth in terms of the larger `to`.  (Of whole numbers: a difference of two scaled maxima would have to
-    // be of two rounded products, and the compiler may form one of one product and a fused multiply-add.)
-    auto rescale = [&](int from, int to) { return ex2_approx(__int2float_rn(from - to) * p.c2); };
-#pragma unroll 1
-    for (int a = 0; a * kChains < n; ++a) {
-      const int b = a & 1, i = a * kChains + chain;
-      if (!wait_or_fail(smem_u32(&ctl->max_full[b]), (b ? uses1++ : uses0++) & 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
-      if (i < n) {
+    float l = 1.f;                            // static: the integer sum becomes the output through one factor, else through that / l
+    if constexpr (kBrief) {
+      int imax = INT_MIN, ref = 0;
+      float l_run = 0.f;
+      RowConsts base = {};
+      const uint32_t tS = t_worker + static_cast<uint32_t>(chain * kKeys);
+      uint32_t r0[16], r1[16], r2[16], r3[16];
+      if (!wait_or_fail(smem_u32(&ctl->max_full[0]), uses0++ & 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
+      if (chain < n) {
         tc_fence_after();
-        const uint32_t from = t_worker + static_cast<uint32_t>(b * kStep1 + chain * kKeys);
-        uint32_t r0[16], r1[16], r2[16], r3[16];
-        tmem_ld16_issue(from, r0);
-        tmem_ld16_issue(from + 16, r1);
-        tmem_ld16_issue(from + 32, r2);
-        tmem_ld16_issue(from + 48, r3);
+        tmem_ld16_issue(tS, r0);
+        tmem_ld16_issue(tS + 16, r1);
+        tmem_ld16_issue(tS + 32, r2);
+        tmem_ld16_issue(tS + 48, r3);
         tmem_ld_fence(r0); tmem_ld_fence(r1); tmem_ld_fence(r2); tmem_ld_fence(r3);
-        tc_fence_before();
-        mbar_arrive(smem_u32(&ctl->max_free[b]));
         int max_a = INT_MIN, max_b = INT_MIN;
         chunk_max<16>(r0, max_a, max_b);
         chunk_max<16>(r1, max_a, max_b);
         chunk_max<16>(r2, max_a, max_b);
         chunk_max<16>(r3, max_a, max_b);
-        const int mine = max(max_a, max_b);
-        if (!kStatic) {
-          // (only groups with masked keys are preset)
-          imax = max(imax, (info->group[i] & kMixed) != 0 ? mine : mine + static_cast<int>(kMagicBits));
-        } else {
-          // The sum is kept in terms of a maximum that is renewed when a row of the warp has gone beyond it by more than a factor of two, which few groups do
-          // after the first: a group adds to the sum and forms no constants.
-          imax = max(imax, mine);
-          if (__any_sync(0xFFFFFFFFu, mine > limit)) {
-            base = row_consts(imax, p.c2, p.row_scale, p.scale_qk, 1.f);
-            l_run *= rescale(ref, imax);
-            ref = imax;
-            limit = imax + slack;
-          }
-          float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-          uint32_t none[4];
-          chunk_exp_pack<16, false, 1, false>(r0, base.c2, base.neg_hi, base.p_mul_f, sum, none);
-          chunk_exp_pack<16, false, 1, false>(r1, base.c2, base.neg_hi, base.p_mul_f, sum, none);
-          chunk_exp_pack<16, false, 1, false>(r2, base.c2, base.neg_hi, base.p_mul_f, sum, none);
-          chunk_exp_pack<16, false, 1, false>(r3, base.c2, base.neg_hi, base.p_mul_f, sum, none);
-          l_run = fmaf(base.f, (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y), l_run);
-        }
-      } else {
-        mbar_arrive(smem_u32(&ctl->max_free[b]));
+        imax = ref = max(max_a, max_b);
+        base = row_consts(imax, p.c2, p.row_scale, p.scale_qk, 1.f);
+        float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        exps_in_place(r0, base, sum);
+        exps_in_place(r1, base, sum);
+        exps_in_place(r2, base, sum);
+        exps_in_place(r3, base, sum);
+        l_run = base.f * ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y));
       }
-    }
-    ctl->stat[parity][chain][row] = make_float2(__int_as_float(imax), l_run);
-    if (kStatic) ctl->sum[parity][chain][row] = __int_as_float(ref);
-    mbar_arrive(smem_u32(&ctl->xch[quad]));
-    // (with the row policy a unit has two exchanges, with the static one)
-    if (!wait_or_fail(smem_u32(&ctl->xch[quad]), kStatic ? parity : 0u, FMHA_I8_DEV_WAIT_S_READY)) return;
-    const float2 other = ctl->stat[parity][chain ^ 1][row];
-    imax = max(imax, __float_as_int(other.x));
-    if (kStatic) {
-      // (a thread without a group has a sum of zero; the other one has some)
-      l_run = fmaf(rescale(ref, imax), l_run, rescale(__float_as_int(ctl->sum[parity][chain ^ 1][row]), imax) * other.y);
-    }
-    // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = rn(levels * min(e / (l s_max), 1))
-    const RowConsts k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, kStatic ? p.p_mul / (l_run > 0.f ? l_run : 1.f) : p.p_mul);
-    const float2 p_mul = kStatic ? make_float2(kLevels, kLevels) : k.p_mul_f;
-
-    // ---- phase 2: exp, row sum, requantise; the bytes go over columns already read
-    float l_sum = 0.f;
-    Ring<C::kBufs> set = unit_begin;
-    if (chain == 1) set.advance();
-    unit_begin.skip(static_cast<uint32_t>(n));
-#pragma unroll 1
-    for (int i = chain; i < n; i += kChains, set.template advance<kChains>()) {
-      const uint32_t tS = t_worker + set.at * kKeys;
-      if (!wait_or_fail(smem_u32(&ctl->s_full[set.at]), set.parity, FMHA_I8_DEV_WAIT_S_READY)) return;
-      tc_fence_after();
-      uint32_t ra[16], rb[16], packed[4];
-      float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      auto sixteen = [&](const uint32_t (&r)[16], uint32_t c, auto poly) {
-        chunk_exp_pack<16, kStatic, decltype(poly)::value>(r, k.c2, k.neg_hi, p_mul, sum, packed, k.p_mul_f.x);
-        tmem_st4(tS + c * 4, packed);
-      };
-      constexpr Flight<0> mufu;
-      constexpr Flight<1> some_poly;          // a quarter of them on the multiply-add pipe
-      tmem_ld16_issue(tS, ra);
-      tmem_ld16_issue(tS + 16, rb);
-      tmem_ld_fence(ra); tmem_ld_fence(rb);
-      sixteen(ra, 0, mufu);
-      tmem_ld16_issue(tS + 32, ra);
-      sixteen(rb, 1, some_poly);
-      tmem_ld16_issue(tS + 48, rb);
-      tmem_ld_fence(ra); tmem_ld_fence(rb);
-      sixteen(ra, 2, mufu);
-      sixteen(rb, 3, some_poly);
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(smem_u32(&ctl->p_ready[set.at]));
-      // (a sum for each group: over all groups of 32,768 keys in one, equal probabilities lost 5e-5 of it instead of 4e-6)
-      l_sum += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
-    }
-    float l = 1.f;                            // static: the integer sum becomes the output through one factor, else through that / l
-    if (!kStatic) {
-      l = k.f * l_sum;
-      ctl->sum[parity][chain][row] = l;
+      ctl->stat[parity][chain][row] = make_float2(__int_as_float(imax), l_run);
+      ctl->sum[parity][chain][row] = __int_as_float(ref);
       mbar_arrive(smem_u32(&ctl->xch[quad]));
-      if (!wait_or_fail(smem_u32(&ctl->xch[quad]), 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
-      l += ctl->sum[parity][chain ^ 1][row];
+      if (!wait_or_fail(smem_u32(&ctl->xch[quad]), parity, FMHA_I8_DEV_WAIT_S_READY)) return;
+      const float2 other = ctl->stat[parity][chain ^ 1][row];
+      imax = max(imax, __float_as_int(other.x));
+      const float mine = rescale(ref, imax);
+      // (a thread without a group has a sum of zero; the other one has one)
+      l_run = fmaf(mine, l_run, rescale(__float_as_int(ctl->sum[parity][chain ^ 1][row]), imax) * other.y);
+      // P8 = rn(levels * min(e / (l s_max), 1))
+      if (chain < n) {
+        const float share = p.p_mul / (l_run > 0.f ? l_run : 1.f) * (base.f * mine);
+        uint32_t packed[4];
+        pack_shares(r0, share, packed); tmem_st4(tS, packed);
+        pack_shares(r1, share, packed); tmem_st4(tS + 4, packed);
+        pack_shares(r2, share, packed); tmem_st4(tS + 8, packed);
+        pack_shares(r3, share, packed); tmem_st4(tS + 12, packed);
+        tmem_wait_st();
+        tc_fence_before();
+      }
+      if (chain < n) mbar_arrive(smem_u32(&ctl->p_brief[chain]));
+    } else {
+      // ---- phase 1: the row's maximum over all keys, as a biased integer (static: and the exp-sum, in terms of that of `ref`)
+      int imax = INT_MIN;
+      float l_run = 0.f;
+      RowConsts base = {};
+      int ref = 0, limit = INT_MIN;               // (biased integers of unmasked keys are positive)
+#pragma unroll 1
+      for (int a = 0; a * kChains < n; ++a) {
+        const int b = a & 1, i = a * kChains + chain;
+        if (!wait_or_fail(smem_u32(&ctl->max_full[b]), (b ? uses1++ : uses0++) & 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
+        if (i < n) {
+          tc_fence_after();
+          const uint32_t from = t_worker + static_cast<uint32_t>(b * kStep1 + chain * kKeys);
+          uint32_t r0[16], r1[16], r2[16], r3[16];
+          tmem_ld16_issue(from, r0);
+          tmem_ld16_issue(from + 16, r1);
+          tmem_ld16_issue(from + 32, r2);
+          tmem_ld16_issue(from + 48, r3);
+          tmem_ld_fence(r0); tmem_ld_fence(r1); tmem_ld_fence(r2); tmem_ld_fence(r3);
+          tc_fence_before();
+          mbar_arrive(smem_u32(&ctl->max_free[b]));
+          int max_a = INT_MIN, max_b = INT_MIN;
+          chunk_max<16>(r0, max_a, max_b);
+          chunk_max<16>(r1, max_a, max_b);
+          chunk_max<16>(r2, max_a, max_b);
+          chunk_max<16>(r3, max_a, max_b);
+          const int mine = max(max_a, max_b);
+          if (!kStatic) {
+            // (only groups with masked keys are preset)
+            imax = max(imax, (info->group[i] & kMixed) != 0 ? mine : mine + static_cast<int>(kMagicBits));
+          } else {
+            // The sum is kept in terms of a maximum that is renewed when a row of the warp has gone beyond it by more than a factor of two, which few groups do
+            // after the first: a group adds to the sum and forms no constants.
+            imax = max(imax, mine);
+            if (__any_sync(0xFFFFFFFFu, mine > limit)) {
+              base = row_consts(imax, p.c2, p.row_scale, p.scale_qk, 1.f);
+              l_run *= rescale(ref, imax);
+              ref = imax;
+              limit = imax + slack;
+            }
+            float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            uint32_t none[4];
+            chunk_exp_pack<16, false, 1, false>(r0, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+            chunk_exp_pack<16, false, 1, false>(r1, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+            chunk_exp_pack<16, false, 1, false>(r2, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+            chunk_exp_pack<16, false, 1, false>(r3, base.c2, base.neg_hi, base.p_mul_f, sum, none);
+            l_run = fmaf(base.f, (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y), l_run);
+          }
+        } else {
+          mbar_arrive(smem_u32(&ctl->max_free[b]));
+        }
+      }
+      ctl->stat[parity][chain][row] = make_float2(__int_as_float(imax), l_run);
+      if (kStatic) ctl->sum[parity][chain][row] = __int_as_float(ref);
+      mbar_arrive(smem_u32(&ctl->xch[quad]));
+      // (with the row policy a unit has two exchanges, with the static one)
+      if (!wait_or_fail(smem_u32(&ctl->xch[quad]), kStatic ? parity : 0u, FMHA_I8_DEV_WAIT_S_READY)) return;
+      const float2 other = ctl->stat[parity][chain ^ 1][row];
+      imax = max(imax, __float_as_int(other.x));
+      if (kStatic) {
+        // (a thread without a group has a sum of zero; the other one has some)
+        l_run = fmaf(rescale(ref, imax), l_run, rescale(__float_as_int(ctl->sum[parity][chain ^ 1][row]), imax) * other.y);
+      }
+      // dynamic: P8 = rn(levels * e), e <= 1; static: P8 = rn(levels * min(e / (l s_max), 1))
+      const RowConsts k = row_consts(imax, p.c2, p.row_scale, p.scale_qk, kStatic ? p.p_mul / (l_run > 0.f ? l_run : 1.f) : p.p_mul);
+      const float2 p_mul = kStatic ? make_float2(kLevels, kLevels) : k.p_mul_f;
+
+      // ---- phase 2: exp, row sum, requantise; the bytes go over columns already read
+      float l_sum = 0.f;
+      Ring<C::kBufs> set = unit_begin;
+      if (chain == 1) set.advance();
+      unit_begin.skip(static_cast<uint32_t>(n));
+#pragma unroll 1
+      for (int i = chain; i < n; i += kChains, set.template advance<kChains>()) {
+        const uint32_t tS = t_worker + set.at * kKeys;
+        if (!wait_or_fail(smem_u32(&ctl->s_full[set.at]), set.parity, FMHA_I8_DEV_WAIT_S_READY)) return;
+        tc_fence_after();
+        uint32_t ra[16], rb[16], packed[4];
+        float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        auto sixteen = [&](const uint32_t (&r)[16], uint32_t c, auto poly) {
+          chunk_exp_pack<16, kStatic, decltype(poly)::value>(r, k.c2, k.neg_hi, p_mul, sum, packed, k.p_mul_f.x);
+          tmem_st4(tS + c * 4, packed);
+        };
+        constexpr Flight<0> mufu;
+        constexpr Flight<1> some_poly;          // a quarter of them on the multiply-add pipe
+        tmem_ld16_issue(tS, ra);
+        tmem_ld16_issue(tS + 16, rb);
+        tmem_ld_fence(ra); tmem_ld_fence(rb);
+        sixteen(ra, 0, mufu);
+        tmem_ld16_issue(tS + 32, ra);
+        sixteen(rb, 1, some_poly);
+        tmem_ld16_issue(tS + 48, rb);
+        tmem_ld_fence(ra); tmem_ld_fence(rb);
+        sixteen(ra, 2, mufu);
+        sixteen(rb, 3, some_poly);
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(smem_u32(&ctl->p_ready[set.at]));
+        // (a sum for each group: over all groups of 32,768 keys in one, equal probabilities lost 5e-5 of it instead of 4e-6)
+        l_sum += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+      }
+      if (!kStatic) {
+        l = k.f * l_sum;
+        ctl->sum[parity][chain][row] = l;
+        mbar_arrive(smem_u32(&ctl->xch[quad]));
+        if (!wait_or_fail(smem_u32(&ctl->xch[quad]), 1u, FMHA_I8_DEV_WAIT_S_READY)) return;
+        l += ctl->sum[parity][chain ^ 1][row];
+      }
     }
     const float scale = p.scale_v_out * (kStatic ? 1.f : l > 0.f ? __frcp_rn(l) : 0.f);
 
@@ -329,7 +417,7 @@ __device__ __forceinline__ int scan_groups(uint16_t* list, const int8_t* mask_ro
   return n;
 }
 
-template <int D>
+template <int D, bool kBrief>
 __device__ __forceinline__ void loader_role(const FwdParams& p, Ctl* all, const int worker, const CUtensorMap* map_q, const CUtensorMap* map_k,
                                             const CUtensorMap* map_v, const uint32_t worker_smem) {
   using C = Cfg<D>;
@@ -404,7 +492,7 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, Ctl* all, const 
     };
     constexpr int kAhead = static_cast<int>(C::kBufs);
     // phase 1, then what phase 2 begins with
-    const int pairs = (n + 1) / 2, first = (min(n, kAhead) + 1) / 2;
+    const int pairs = (n + 1) / 2, first = kBrief ? 0 : (min(n, kAhead) + 1) / 2;
 #pragma unroll 1
     for (int a = 0; a < pairs + first; ++a) {
       const int i = 2 * (a < pairs ? a : a - pairs);
@@ -432,7 +520,7 @@ __device__ __forceinline__ void loader_role(const FwdParams& p, Ctl* all, const 
 // S issued behind P.V).  With a wait for P.V's completion in between, in both places, 80 forms of calls gave the same outputs to the last
 // bit, 30 % later and more, since the wait joins the issuer's chain: B4 H16 S1024 D64 (512..1024 keys) per-row 24.6 -> 31.8 us, B1 H32 S2048 D128
 // 57.2 -> 92.4, one unit to an SM B1 H2 S8192 D128 79.8 -> 168.  (The forward kernels need no such order: there the drain of P.V comes first.)
-template <int D, bool kStatic>
+template <int D, bool kStatic, bool kBrief>
 __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const int worker, const uint32_t tmem_base, const uint32_t worker_smem,
                                             uint8_t* presets) {
   using C = Cfg<D>;
@@ -448,6 +536,7 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
   const bool lead = elect_one();
   uint32_t fail = 0u, used = 0, groups = 0, uses0 = 0, uses1 = 0;      // places of the ring, and S, so far
   Ring<C::kBufs> s_set, p_set;
+  uint32_t briefs[kChains] = {};                                        // kBrief: units that had such a group
   auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
     if (warp_wait(bar, parity, abort_flag)) return true;
     fail = code;
@@ -493,6 +582,10 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
 #pragma unroll
       for (int kk = 0; kk < D / 32; ++kk) mma_i8_ss(tS, desc_advance(dq, kk * 32), desc_advance(dk, kk * 32), idesc_s, preset || kk > 0 ? 1u : 0u);
     };
+    auto issue_pv = [&](uint32_t tP, uint64_t dv, bool first) {
+#pragma unroll
+      for (int kk = 0; kk < kKeys / 32; ++kk) mma_i8_ts(tO, tP + kk * 8, desc_advance(dv, kk * 32 * D), idesc_o, !first || kk > 0 ? 1u : 0u);
+    };
 
     // ---- phase 1: two groups a step
     // (Which groups are preset is looked up only from the first of them on: the issuer's instructions are what a step here waits for, 750 cycles of which
@@ -508,7 +601,8 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
       asm volatile("" : "+r"(tS), "+l"(dk), "+r"(bar_full), "+r"(bar_empty));
       const uint32_t before = b ? uses1++ : uses0++;
       if (!landed()) break;
-      if (before > 0u && !wait(smem_u32(&ctl->max_free[b]), (before - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
+      // (kBrief: the P.V of the unit before has waited for everything that is read)
+      if (!kBrief && before > 0u && !wait(smem_u32(&ctl->max_free[b]), (before - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
       // (The first half of the columns may still hold P bytes of the unit before, whose P.V was issued in front: see the order above.)  The second
       // half is where its sums were.
       if (a == 1 && it > 0 && !wait(smem_u32(&ctl->o_free), static_cast<uint32_t>((it - 1) & 1), FMHA_I8_DEV_WAIT_O_FREE)) break;
@@ -528,64 +622,84 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
           if (two) issue_s(tS + kKeys, d_preset1, desc_advance(dk, C::kGroupBytes), preset1);
           mma_commit(bar_full);
           mma_commit(bar_empty);
+          if (kBrief) mma_commit(smem_u32(&ctl->q_empty[qb]));
         }
       }
       __syncwarp();
       ++used;
       groups += two ? 2u : 1u;
     }
-    // all scores of phase 1 have been read (and with them the sums of the unit before)
-    if (fail != 0u || !wait(smem_u32(&ctl->max_free[0]), (uses0 - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
-    if (uses1 > 0u && !wait(smem_u32(&ctl->max_free[1]), (uses1 - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
-    tc_fence_after();
-
-    // ---- phase 2: S runs kBufs groups ahead of P.V
-    constexpr int kAhead = static_cast<int>(C::kBufs);
-#pragma unroll 1
-    for (int i = 0; i < kAhead && i < n; ++i) {
-      if (!landed()) break;
-      const uint64_t d_preset = preset_of(i, groups), dk = place_desc() + static_cast<uint64_t>((i & 1) * C::kGroupBytes >> 4);
-      const bool last_of_place = (i & 1) != 0 || i + 1 == kAhead || i + 1 == n;
-      if (lead) {
-        issue_s(t_worker + s_set.at * kKeys, d_preset, dk, true);
-        mma_commit(smem_u32(&ctl->s_full[s_set.at]));
-        if (last_of_place) mma_commit(smem_u32(&ctl->empty[used % C::kStages]));
-        if (i == n - 1) mma_commit(smem_u32(&ctl->q_empty[qb]));
-      }
-      __syncwarp();
-      if (last_of_place) ++used;
-      ++groups;
-      s_set.advance();
-    }
-#pragma unroll 1
-    for (int i = 0; i < n && fail == 0u; ++i) {
-      const int ahead = i + kAhead;
-      if (!landed()) break;
-      uint64_t d_preset = ahead < n ? preset_of(ahead, groups) : 0u, dv = place_desc();
-      uint32_t tP = t_worker + p_set.at * kKeys, tS = t_worker + s_set.at * kKeys;
-      uint32_t bar_s = smem_u32(&ctl->s_full[s_set.at]), bar_empty = smem_u32(&ctl->empty[used % C::kStages]);
-      asm volatile("" : "+l"(d_preset), "+l"(dv), "+r"(tP), "+r"(tS), "+r"(bar_s), "+r"(bar_empty));          // formed here, not behind the wait
-      if (!wait(smem_u32(&ctl->p_ready[p_set.at]), p_set.parity, FMHA_I8_DEV_WAIT_P_READY)) break;
-      tc_fence_after();
-      if (lead) {
+    if constexpr (kBrief) {
+      // the P bytes are over the columns of the scores
 #pragma unroll
-        for (int kk = 0; kk < kKeys / 32; ++kk) mma_i8_ts(tO, tP + kk * 8, desc_advance(dv, kk * 32 * D), idesc_o, i > 0 || kk > 0 ? 1u : 0u);
-        if (ahead < n) {
-          // (over the P bytes, behind the P.V that reads them: see the issuer's order above)
-          issue_s(tS, d_preset, desc_advance(dv, C::kGroupBytes), true);
-          mma_commit(bar_s);
-          if (ahead == n - 1) mma_commit(smem_u32(&ctl->q_empty[qb]));
-        } else if (i == n - 1) {
-          mma_commit(smem_u32(&ctl->o_full));
+      for (int i = 0; i < kChains; ++i) {
+        if (i >= n || !landed()) break;
+        uint64_t dv = place_desc();
+        uint32_t tP = t_worker + static_cast<uint32_t>(i * kKeys), bar_empty = smem_u32(&ctl->empty[used % C::kStages]);
+        asm volatile("" : "+l"(dv), "+r"(tP), "+r"(bar_empty));
+        if (!wait(smem_u32(&ctl->p_brief[i]), briefs[i]++ & 1u, FMHA_I8_DEV_WAIT_P_READY)) break;
+        tc_fence_after();
+        if (lead) {
+          issue_pv(tP, dv, i == 0);
+          if (i == n - 1) mma_commit(smem_u32(&ctl->o_full));
+          mma_commit(bar_empty);
         }
-        mma_commit(bar_empty);
+        __syncwarp();
+        ++used;
       }
-      __syncwarp();
-      p_set.advance();
-      ++used;
-      if (ahead < n) {
+    } else {
+      // all scores of phase 1 have been read (and with them the sums of the unit before)
+      if (fail != 0u || !wait(smem_u32(&ctl->max_free[0]), (uses0 - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
+      if (uses1 > 0u && !wait(smem_u32(&ctl->max_free[1]), (uses1 - 1u) & 1u, FMHA_I8_DEV_WAIT_O_FREE)) break;
+      tc_fence_after();
+
+      // ---- phase 2: S runs kBufs groups ahead of P.V
+      constexpr int kAhead = static_cast<int>(C::kBufs);
+#pragma unroll 1
+      for (int i = 0; i < kAhead && i < n; ++i) {
+        if (!landed()) break;
+        const uint64_t d_preset = preset_of(i, groups), dk = place_desc() + static_cast<uint64_t>((i & 1) * C::kGroupBytes >> 4);
+        const bool last_of_place = (i & 1) != 0 || i + 1 == kAhead || i + 1 == n;
+        if (lead) {
+          issue_s(t_worker + s_set.at * kKeys, d_preset, dk, true);
+          mma_commit(smem_u32(&ctl->s_full[s_set.at]));
+          if (last_of_place) mma_commit(smem_u32(&ctl->empty[used % C::kStages]));
+          if (i == n - 1) mma_commit(smem_u32(&ctl->q_empty[qb]));
+        }
+        __syncwarp();
+        if (last_of_place) ++used;
         ++groups;
         s_set.advance();
+      }
+#pragma unroll 1
+      for (int i = 0; i < n && fail == 0u; ++i) {
+        const int ahead = i + kAhead;
+        if (!landed()) break;
+        uint64_t d_preset = ahead < n ? preset_of(ahead, groups) : 0u, dv = place_desc();
+        uint32_t tP = t_worker + p_set.at * kKeys, tS = t_worker + s_set.at * kKeys;
+        uint32_t bar_s = smem_u32(&ctl->s_full[s_set.at]), bar_empty = smem_u32(&ctl->empty[used % C::kStages]);
+        asm volatile("" : "+l"(d_preset), "+l"(dv), "+r"(tP), "+r"(tS), "+r"(bar_s), "+r"(bar_empty));          // formed here, not behind the wait
+        if (!wait(smem_u32(&ctl->p_ready[p_set.at]), p_set.parity, FMHA_I8_DEV_WAIT_P_READY)) break;
+        tc_fence_after();
+        if (lead) {
+          issue_pv(tP, dv, i == 0);
+          if (ahead < n) {
+            // (over the P bytes, behind the P.V that reads them: see the issuer's order above)
+            issue_s(tS, d_preset, desc_advance(dv, C::kGroupBytes), true);
+            mma_commit(bar_s);
+            if (ahead == n - 1) mma_commit(smem_u32(&ctl->q_empty[qb]));
+          } else if (i == n - 1) {
+            mma_commit(smem_u32(&ctl->o_full));
+          }
+          mma_commit(bar_empty);
+        }
+        __syncwarp();
+        p_set.advance();
+        ++used;
+        if (ahead < n) {
+          ++groups;
+          s_set.advance();
+        }
       }
     }
     if (fail == 0u && elect_one()) mbar_arrive(smem_u32(&ctl->info_empty[buf]));
@@ -606,6 +720,7 @@ __device__ __forceinline__ uint32_t set_up(Ctl* ctl, uint8_t* presets, const CUt
       for (int i = 0; i < kMaxStages; ++i) { mbar_init(smem_u32(&w.full[i]), 1); mbar_init(smem_u32(&w.empty[i]), 1); }
       for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&w.max_full[i]), 1); mbar_init(smem_u32(&w.max_free[i]), kChains * kTile); }
       for (int i = 0; i < 3; ++i) { mbar_init(smem_u32(&w.s_full[i]), 1); mbar_init(smem_u32(&w.p_ready[i]), kTile); }
+      for (int i = 0; i < kChains; ++i) mbar_init(smem_u32(&w.p_brief[i]), kTile);
       mbar_init(smem_u32(&w.o_full), 1);
       mbar_init(smem_u32(&w.o_free), kChains * kTile);
       for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&w.xch[i]), 64);
@@ -630,7 +745,7 @@ __device__ __forceinline__ uint32_t set_up(Ctl* ctl, uint8_t* presets, const CUt
   return tmem_base;
 }
 
-template <int D, bool kStatic>
+template <int D, bool kStatic, bool kBrief>
 __global__ void __launch_bounds__(kThreads, 1)
 policy_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
               const FwdParams p) {
@@ -646,13 +761,13 @@ policy_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   // warps: 4 kChains softmax warps per worker (their number modulo 4 is their lane quarter), the issuers, the loaders
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
-    softmax_role<D, kStatic>(p, ctl, warp / (4 * kChains), (warp >> 2) % kChains, tmem_base);
+    softmax_role<D, kStatic, kBrief>(p, ctl, warp / (4 * kChains), (warp >> 2) % kChains, tmem_base);
   } else {
     setmaxnreg_dec<kOtherRegs>();
     const int worker = (warp - kSoftmaxWarps) % kWorkers;
     const uint32_t worker_smem = smem_u32(tiles + worker * C::kWorkerBytes);
-    if (warp < kSoftmaxWarps + kWorkers) issuer_role<D, kStatic>(p, ctl, worker, tmem_base, worker_smem, presets);
-    else loader_role<D>(p, ctl, worker, &map_q, &map_k, &map_v, worker_smem);
+    if (warp < kSoftmaxWarps + kWorkers) issuer_role<D, kStatic, kBrief>(p, ctl, worker, tmem_base, worker_smem, presets);
+    else loader_role<D, kBrief>(p, ctl, worker, &map_q, &map_k, &map_v, worker_smem);
   }
   tc_fence_before();
   __syncthreads();

@@ -222,3 +222,32 @@ def test_static_policy_whose_maxima_move(pkg, oracle, D, scale, how):
     st, words = pkg.device_status()
     assert st == pkg.OK, words
     assert_parity(to.cpu().numpy(), oracle.policy(q8, k8, v8, mask, amax, oracle.POLICY_STATIC), f"{how} {scale}")
+
+
+# The static policy's calls of one and two groups of 64 keys, in one phase: either group alone or both, masked keys in either, sequences
+# without a key, fewer units than an SM takes at once and many for every place, the last rows of a head, groups of very different maxima.
+@pytest.mark.parametrize("B,H,Sq,Sk,D", [(12, 2, 1, 128, 64), (12, 2, 130, 128, 128), (48, 28, 65, 128, 64), (48, 20, 128, 128, 64), (48, 20, 100, 64, 128),
+                                         (48, 28, 129, 64, 64)])
+@pytest.mark.parametrize("scale", [1.0, 40.0])
+def test_static_policy_of_one_or_two_groups(pkg, wl, oracle, B, H, Sq, Sk, D, scale):
+    import torch
+    torch.cuda.set_device(0)
+    rng = np.random.Generator(np.random.Philox(key=Sk + D + Sq))
+    q8, qa = wl.quantize_np(rng.standard_normal((B, H, Sq, D), dtype=np.float32))
+    k8, ka = wl.quantize_np(rng.standard_normal((B, H, Sk, D), dtype=np.float32))
+    v8, va = wl.quantize_np(rng.standard_normal((B, H, Sk, D), dtype=np.float32))
+    j = np.arange(Sk)
+    masks = [j < 0, j < 64, j >= 64, j % 64 >= 40, (j % 3 == 0) & (j < 64), j >= 100, j >= 0, j != Sk - 1, j != 0, (j < 64) & (j != 5), j >= 1, j % 2 == 0]
+    mask = np.stack([masks[b % 12] for b in range(B)]).astype(np.int8)
+    amax = (qa, ka * scale, va, va, 0.1 if scale == 1.0 else 0.5)
+    tq, tk, tv, tm = (torch.from_numpy(x).cuda() for x in (q8, k8, v8, mask))
+    to = torch.full((q8.size + 256,), 0x5A, dtype=torch.int8, device="cuda")
+    pkg.FMHAInferI8Policy(None, pkg.FMHAParamI8(*amax), pkg.AttnDataDescriptorX(B, Sq, Sk, H, D), tq, tk, tv, tm, to[128:-128], pkg.POLICY_STATIC,
+                          torch.zeros(B * H * Sq * 2, device="cuda"))
+    st, words = pkg.device_status()
+    assert st == pkg.OK, words
+    got = to.cpu().numpy()
+    assert (got[:128] == 0x5A).all() and (got[-128:] == 0x5A).all()
+    heads = slice(0, None, 7)
+    want = oracle.policy(q8[:, heads], k8[:, heads], v8[:, heads], mask, amax, oracle.POLICY_STATIC)
+    assert_parity(got[128:-128].reshape(q8.shape)[:, heads], want, f"scale {scale}")

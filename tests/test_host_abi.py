@@ -185,8 +185,8 @@ def test_the_quantiser_keeps_fewer_tiles_than_its_ring_has_slots():
 def test_the_policies_issue_s_behind_p_v_from_one_lane():
     """S of a later group goes over the columns of P that P.V reads: one lane issues both, P.V first, without anything that could let another in."""
     text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "int8-flash-attention-fmha-quantization_b200", "csrc", "fmha_policy_sm100.cuh")).read())
-    assert text.count("mma_i8_ts(") == 1 and text.count("const bool lead = elect_one();") == 1
-    at = text.index("mma_i8_ts(")
+    assert text.count("mma_i8_ts(") == 1 and text.count("issue_s(tS, d_preset, desc_advance(dv") == 1 and text.count("const bool lead = elect_one();") == 1
+    at = text.index("issue_s(tS, d_preset, desc_advance(dv")
     block = text[text.rindex("if (lead) {", 0, at):]
     block = block[:block.index("__syncwarp();")]
-    assert block.index("mma_i8_ts(tO") < block.index("issue_s(tS") and "wait" not in block and block.count("if (lead)") == 1
+    assert block.index("issue_pv(tP") < block.index("issue_s(tS") and "wait" not in block and block.count("if (lead)") == 1
