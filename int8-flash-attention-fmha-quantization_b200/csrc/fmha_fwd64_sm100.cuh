@@ -25,7 +25,7 @@ namespace fmha {
 namespace w64 {
 // Two instances of each kind, one of them (kShort) for units of up to kShortTiles key tiles.  They differ in how the maximum of a half tile
 // branches off that of a whole one: behind the first loads or in front of them.  Behind, the step is faster, and the compiler spills
-// values of the unit (-Xptxas -v: 72 bytes stored, 100 loaded, none in front), which short units pay for.  Behind against in front, in
+// values of the unit (-Xptxas -v: 72 bytes stored, 68 loaded, none in front), which short units pay for.  Behind against in front, in
 // per cent of the time: B256 H16 S256 (lengths 64..256) +2, B200 H12 S128 +1, B64 H16 S256 -1.5; B64 H16 S320 -2, B16 H12 S384 -3, B64 H16
 // S384 (130..384) -1.4, B8 H16 S512 -2.3, B32 H12 S512 (256..512) -2.6, S576 (300..576) -2.8, B8 H32 S2048 -3.  (What is spilled is the compiler's
 // choice: to be measured again when the step changes.)

@@ -325,7 +325,7 @@ __device__ __forceinline__ int scan_mask_groups(Info* info, const uint32_t* word
 template <bool kHalves, int kLong, typename Info>
 __device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_row, int S, int n_tiles) {
   const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);
-  const int n = kLong == 1 || n_tiles <= 32 ? scan_mask_groups<1, kHalves>(info, words, S, n_tiles) : scan_mask_groups<kLong, kHalves>(info, words, S, n_tiles);
+  const int n = n_tiles <= 32 ? scan_mask_groups<1, kHalves>(info, words, S, n_tiles) : scan_mask_groups<kLong, kHalves>(info, words, S, n_tiles);
   if ((threadIdx.x & 31) == 0) info->n_live = n;
   __syncwarp();
 }
@@ -633,14 +633,14 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, FwdCtl<FwdCfg<D
 #pragma unroll
         for (int c = 0; c < 4; ++c) tmem_st4(tP + c * 4, packed);
       } else {
-      tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + cs) * 16, rb);
-      sixteen(ra, 0);
-      tmem_ld_fence(rb); tmem_ld16_issue(tS + (c0 + 2 * cs) * 16, ra);
-      sixteen(rb, 1);
-      tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + 3 * cs) * 16, rb);
-      sixteen(ra, 2);
-      tmem_ld_fence(rb);
-      sixteen(rb, 3);
+        tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + cs) * 16, rb);
+        sixteen(ra, 0);
+        tmem_ld_fence(rb); tmem_ld16_issue(tS + (c0 + 2 * cs) * 16, ra);
+        sixteen(rb, 1);
+        tmem_ld_fence(ra); tmem_ld16_issue(tS + (c0 + 3 * cs) * 16, rb);
+        sixteen(ra, 2);
+        tmem_ld_fence(rb);
+        sixteen(rb, 3);
       }
       // ---- publish the row statistics of this step for the merge threads
       const int slot = static_cast<int>(g & 3u);
