@@ -346,18 +346,16 @@ int launch_kernel(void (*fn)(Params...), dim3 grid, dim3 block, size_t smem, cud
 // shared memory, with 2, 4 and 8 CTAs, kShareNs for up to 64 rows at head_dim 128 or 128 at 64, kShareMoreNs more for twice as many:
 constexpr int kTileNs = 860;
 constexpr int kShareNs[kClusterSizes] = {3300, 2900, 4300}, kShareMoreNs[kClusterSizes] = {700, 1900, 1700};
-// us without -> with.  Head_dim 64: B1 H8 S1024 Sq256 10.9 -> 8.7, B1 H4 S2048 Sq200 17.6 -> 10.2, B1 H2 S4096 32.1 -> 21.3, B1 H8 S8192
-// Sq64 57.9 -> 16.9; head_dim 128: B2 H16 S1984 Sq200 19.1 -> 15.6, B1 H2 S16384 Sq128 114 -> 27.  Where the line lies, 12 units, 1 / 2 / 4
-// CTAs each: head_dim 64, 128 rows, 5 tiles 8.3 / 8.9 / 8.5, 6 tiles 9.1 / 8.9 / 8.6; head_dim 128, 33 rows, 5 tiles 9.0 / 8.9 / 9.4,
-// 6 tiles 9.8 / 9.0 / 9.5; 96 rows, 6 tiles 9.8 / 9.7 / 10.2, 7 tiles 10.7 / 10.6 / 10.3; 128 rows, 7 tiles 10.7 / 11.0 / 11.2, 8 tiles 11.6 / 11.2 / 11.2, 12 tiles 15.1 / 13.1 / 12.1.
-//
-// (Pairs are for so many units that larger clusters do not fit, and more CTAs make the merge longer: 72 units of 6 tiles at head_dim 64, one CTA
-// each / pairs, 8.2 / 9.15 us, 70 units of 8 tiles 9.8 / 9.85 and at head_dim 128 11.9 / 12.9; with 12 units pairs would cost 2700.)
+// us without -> with: head_dim 64 B1 H8 S1024 Sq256 10.9 -> 8.7, B1 H8 S8192 Sq64 57.9 -> 16.9; head_dim 128 B2 H16 S1984 Sq200 19.1 -> 15.6, B1 H2
+// S16384 Sq128 114 -> 27.  Where the line lies, 12 units of 128 rows with 1 / 2 / 4 CTAs each: head_dim 64, 5 tiles 8.3 / 8.9 / 8.5, 6 tiles 9.1 / 8.9 /
+// 8.6; head_dim 128, 7 tiles 10.7 / 11.0 / 11.2, 8 tiles 11.6 / 11.2 / 11.2, 12 tiles 15.1 / 13.1 / 12.1.
+// Pairs are for so many units that larger clusters do not fit, and more CTAs make the merge longer: 72 units of 6 tiles at head_dim 64, one CTA
+// each / pairs, 8.2 / 9.15, 70 units of 8 tiles 9.8 / 9.85 and at head_dim 128 11.9 / 12.9 (with 12 units pairs would cost 2700).
 //
 // With more units than SMs the same is done for those of the last round: where they are half as many as the SMs or fewer, a pair
-// of CTAs shares each.  (Head_dim 128: B1 H16 S1280 23.1 -> 21.8, B1 H5 S4096 60.9 -> 50.2, B1 H32 S2048 61.7 -> 58.0; 208 units of
-// 6 tiles 16.3 -> 16.5, of 8 tiles 19.8 -> 19.4; 1072 units of 6 tiles 53.5 -> 50.7, with what overlapping launches give, see
-// launch_fwd.  Head_dim 64: 208 units of 5 tiles 13.1 -> 13.8, of 6 tiles 14.9 -> 14.7.)
+// of CTAs shares each.  Head_dim 128: B1 H16 S1280 23.1 -> 21.8 us, B1 H5 S4096 60.9 -> 50.2, B1 H32 S2048 61.7 -> 58.0; where the line lies, 208
+// units of 6 tiles 16.3 -> 16.5, of 8 tiles 19.8 -> 19.4; head_dim 64, of 5 tiles 13.1 -> 13.8, of 6 tiles 14.9 -> 14.7.  (kTileNs, kPairNs and the figures of
+// this paragraph are of kernels 4 % slower than the present ones.)
 constexpr int kPairNs = 2400;
 bool pairs_share_last_round(const FwdParams& p, const DeviceInfo* dev) {
   const int last = p.n_units % dev->sm_count, tiles = (p.S + kTile - 1) / kTile;
@@ -387,16 +385,16 @@ void plan_parts(FwdParams* p, int D, const DeviceInfo* dev) {
   }
 }
 
-// Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller.  In cycles, fitted to 221 shapes of 100 to 3500 query
-// tiles of 64 to 2048 keys: a CTA of fmha_fwd_sm100.cuh works on one unit at a time, 1530 per key tile and 650 per unit, 2900 at least (2400 for a
-// last round of single tiles that leaves SMs idle: 160 and 222 units of 128 keys, general / workers, 5.1 / 5.5 and 5.4 / 5.9 us; pairs that share the last round:
-// 980 and 3700); one of fmha_fwd64_sm100.cuh on four, 5350 per tile and 2500 for a round of four, 3100 / 3700 / 4700 /
-// 5850 and 2000 (one tile: 1200) for a last round of one to four, 600 for the call; the half tile of an odd multiple of 64 keys is six tenths there.  Both kernels have
-// become 4 to 9 % faster since; over 61 of the shapes, 160 to 2368 units of 64 to 512 keys, the kernel chosen is 0.6 % slower than the better one on average, 4.4 % at the
-// most (888 units of 320 keys).  us, fmha_fwd_sm100.cuh / fmha_fwd64_sm100.cuh, 160 units of 64 keys 5.0 / 4.7; 444 of 128 7.3 / 6.95; 296, 592, 740, 1184 of
-// 256 7.4 / 8.4, 11.3 / 11.6, 13.1 / 14.8, 18.7 / 18.4; 444 of 512 14.0 / 14.8; before, 592 and 888 of 1024 31.2 / 30.2, 44.8 / 46.25; 592 and 1184 of 2048 58.1 / 54.6, 110.5 / 102.6.
+// Which of the two kernels a call at head_dim 64 runs: the one whose estimate is smaller, in cycles.  A CTA of fmha_fwd_sm100.cuh works on one
+// unit at a time: 1530 per key tile and 650 per unit, 2900 at least (2400 in a last round of single tiles that leaves SMs idle); pairs that share the
+// last round 980 and 3700.  One of fmha_fwd64_sm100.cuh works on four: 5350 per tile and 2500 for a round of four; 3100 / 3700 / 4700 / 5850 per tile
+// and 2000 (one tile: 1200) for a last round of one to four; 600 for the call.  The half tile of an odd multiple of 64 keys is six tenths there.
+// Fitted to 221 shapes of 100 to 3500 query tiles of 64 to 2048 keys, when the kernels were 4 to 9 % slower; since, over 61 of them (160 to 2368 units
+// of 64 to 512 keys), the kernel chosen is 0.6 % slower than the better one on average and 4.4 % at the most (888 units of 320 keys).
+// us, fmha_fwd_sm100.cuh / fmha_fwd64_sm100.cuh: 160 units of 64 keys 5.0 / 4.7; 160, 222, 444 of 128 5.1 / 5.5, 5.4 / 5.9, 7.3 / 6.95; 296, 592, 740, 1184
+// of 256 7.4 / 8.4, 11.3 / 11.6, 13.1 / 14.8, 18.7 / 18.4; 444 of 512 14.0 / 14.8; of the slower kernels 592 and 888 of 1024 31.2 / 30.2, 44.8 / 46.25.
 //
-// Calibrations have a line of their own (1600 and 1200; 5850, 4900 / 4350 / 3400 per tile), drawn before.
+// Calibrations have a line of their own (1600 and 1200; 5850, 4900 / 4350 / 3400 per tile), of the slower kernels too.
 bool use_workers(const FwdParams& p, bool plain, const DeviceInfo* dev) {
   const long long sms = dev->sm_count, tiles = (p.S + kTile - 1) / kTile, round = sms * w64::kWorkers;
   const long long own = p.n_units / sms, more = p.n_units % sms != 0, full = p.n_units / round, last = (p.n_units % round + sms - 1) / sms;

@@ -13,7 +13,7 @@
 // A worker's step is one serial chain -- S, maximum, exponentials, P.V, fold -- of 3600 cycles when it runs alone.  Four of them
 // on an SM hide each other's latencies; nobody waits for a stage that other threads own, which is what bounds the other kernel
 // on short sequences (its merge warps need 4500 cycles per unit of two steps whatever the other warps do).  What bounds this
-// one: issue slots and the exponential unit, 62 % and 68 % busy on long sequences, where a step takes 5400 cycles, i.e. 1350 per
+// one: issue slots and the exponential unit, 64 % and 69 % busy on long sequences, where a step takes 5300 cycles, i.e. 1330 per
 // SM.  An eighth of the exponentials is computed on the multiply-add pipe (all on the exponential unit: 2.5 % slower on
 // B8 H32 S2048; a quarter: 3 % slower).  Pass 2 reads eight columns at a time: with sixteen the 104 registers of a softmax
 // thread do not suffice, and the spills cost 4 to 9 %.
@@ -23,16 +23,14 @@
 
 namespace fmha {
 namespace w64 {
-// Two instances of each kind, one of them (kShort) for units of up to kShortTiles key tiles.  They differ in how the maximum of a half tile
-// branches off that of a whole one: behind the first loads or in front of them.  Behind, the step is faster, and the compiler spills
-// values of the unit (-Xptxas -v: 72 bytes stored, 68 loaded, none in front), which short units pay for.  Behind against in front, in
-// per cent of the time: B256 H16 S256 (lengths 64..256) +2, B200 H12 S128 +1, B64 H16 S256 -1.5; B64 H16 S320 -2, B16 H12 S384 -3, B64 H16
-// S384 (130..384) -1.4, B8 H16 S512 -2.3, B32 H12 S512 (256..512) -2.6, S576 (300..576) -2.8, B8 H32 S2048 -3.  (What is spilled is the compiler's
-// choice: to be measured again when the step changes.)
-// The two kinds: without and with calibration (kCalib).  The smaller the code the faster short units are -- it is 54 and 62 KB without calibration, 25 of it
-// the drivers', and was 74: long masks scanned in smaller steps, not at all where there are none, calibration apart, units taken apart by
-// multiplications.  Together: B256 H16 S256 (64..256) 88.7 -> 85.1 us, B32 H12 S512 (256..512) 36.2 -> 35.4, B200 H12 S128 22.1 -> 21.5, B64 H16 S320 53.6 -> 52.5, B8 H32
-// S2048 335 -> 330.  (One copy of the driver per worker, 226 KB: 540.)
+// kShort: for units of up to kShortTiles key tiles.  The maximum of a half tile branches off that of a whole one behind the first loads, or with
+// kShort in front of them.  Behind, the step is faster, and the compiler spills values of the unit (-Xptxas -v: 72 bytes stored, 68 loaded, none in
+// front), which short units pay for.  Behind against in front, per cent of the time: one and two tiles +1 to +2 where lengths differ, -1.5
+// where they do not (B64 H16 S256); three tiles -1.4 to -3; long sequences -3.  (To be measured again when the step changes: what is spilled is
+// the compiler's choice.)
+// kCalib: calibration, apart from the forward pass because short units are the faster the smaller the code is.  It is 54 and 62 KB without
+// calibration, 25 of it the drivers'; with all of it in one instance, long masks scanned in larger steps and units taken apart by divisions it
+// was 74: B256 H16 S256 (64..256) 88.7 -> 85.1 us, B8 H32 S2048 335 -> 330.  (One copy of the driver per worker, 226 KB: 540.)
 constexpr int kShortTiles = 2;
 constexpr int kD = 64;
 constexpr int kWorkers = 4;          // per CTA

@@ -330,10 +330,9 @@ __device__ __forceinline__ void scan_mask_warp(Info* info, const int8_t* mask_ro
   __syncwarp();
 }
 
-// The same for up to kTiles key tiles, less code and shorter: a lane looks at four keys of each.  In the workers it stands between a step's S and its
-// P.V, 2300 cycles in the general form, which P.V of half tiles waits for.  us, with the general form -> with this one, B256 H16 S256 D64 (64..256
-// keys) 85.5 -> 84.3, B64 H16 S64 8.75 -> 8.56, B32 H12 S512 (256..512) 35.1 -> 34.9, B64 H16 S384 (130..384) 48.15 -> 47.7; B64 H32 S256 D128 73.9 -> 73.0, one request 5.49 -> 5.48.
-// (For up to eight tiles, in the workers: 35.5 and 48.7.)
+// The same for up to kTiles key tiles, less code and shorter: a lane looks at four keys of each.  In the workers the scan stands between a step's S
+// and its P.V, 2300 cycles in the general form, which P.V of half tiles waits for: B256 H16 S256 D64 (64..256 keys) 85.5 -> 84.3 us, B64 H16 S64 8.75
+// -> 8.56; in the general kernel B64 H32 S256 D128 73.9 -> 73.0.  (For up to eight tiles, in the workers: B32 H12 S512 (256..512) 34.9 -> 35.5.)
 template <int kTiles, bool kHalves, typename Info>
 __device__ __forceinline__ void scan_few_tiles(Info* info, const int8_t* mask_row, int S) {
   const uint32_t* words = reinterpret_cast<const uint32_t*>(mask_row);

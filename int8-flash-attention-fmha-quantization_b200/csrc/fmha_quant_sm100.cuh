@@ -8,7 +8,7 @@
 //                         ring of bulk copies.  At the end of pass 1 the ring still holds each warp's last tiles, its
 //                         registers the first ones and its part of tensor memory the next (97 MB over the chip); pass 2
 //                         takes those from there and reads the others again, as far as it can from the L2.
-// 255,749 elements take 4.1 us, 67,108,864 take 74 to 78: DRAM, since pass 1 reads all 268 MB from there and pass 2 what neither the SMs
+// 255,749 elements take 4.1 us, 67,108,864 take 74 to 80: DRAM, since pass 1 reads all 268 MB from there and pass 2 what neither the SMs
 // (97 MB) nor the L2 (some 50) kept, 121 MB.  Without tensor memory the latter take 7 % longer, 33,554,432 elements 6 %.
 #pragma once
 #include <cooperative_groups.h>
@@ -130,9 +130,8 @@ constexpr int kQuantWarps = kQuantThreads / 32;
 constexpr int kQuantTile = 1024;               // elements per tile: 8 float4 per lane
 constexpr int kQuantVec = kQuantTile / 128;
 constexpr int kQuantStages = 7;                // ring of 7 x 4 KB per warp: all of shared memory
-// Tiles a warp keeps in registers (32 each): its first.  231 of the 255 that a thread can have are in use then.  4 -> 5 (us): 12,000,000
-// elements 16.1 -> 15.7, 24,000,000 25.3 -> 25.0, 50,000,001 51.6 -> 51.1, 67,108,864 75.0 -> 74.2, 33,554,432 32.7 both; 6: 50.3 and 73.9,
-// but 33,554,432 take 34.8.
+// Tiles a warp keeps in registers (32 each): its first.  231 of the 255 that a thread can have are in use then.  4 -> 5: 12,000,000 elements 16.1
+// -> 15.7 us, 24,000,000 25.3 -> 25.0, 67,108,864 1 % or less (75.0 -> 74.2, on another box 79.3 -> 78.6); 6: 33,554,432 elements 32.7 -> 34.8.
 constexpr int kQuantKeep = 5;
 static_assert(kQuantKeep < kQuantStages, "the first tiles are taken from the slots of their first loads, and the next one from the slot behind");
 constexpr int kQuantTmem = 8;                  // tiles a warp keeps in tensor memory, 32 columns each: the next

@@ -80,15 +80,13 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
     }
   }
 }
-// For kernels that stream through memory and have few waits, where the first probe apart is 0.3 to 0.4 % of the time (the quantiser, 67,108,864 elements
-// 75.8 us, with mbar_wait 76.1; decoding, B16 H32 Sq1 Sk4096 (1025..4096) 57.29, with mbar_wait 57.45).
+// For the kernels that stream through memory and have few waits: the quantiser and decoding are 0.3 to 0.4 % faster with the first probe apart
+// than with the loop below (67,108,864 elements 75.8 and 76.1 us).
 __device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
   return mbar_wait_limited(bar, parity, abort_flag, kWaitLimitCycles, 4096u);
 }
-// The same with kWaitProbes for the limit, in as few instructions as can be: the kernels have some twenty waits each, and how far their code
-// is spread costs them time (with the cycle counter read and a first probe in front of the loop, as above, B64 H32 S256 D128 took 82.9 us instead of
-// 77.8, B256 H16 S256 D64, 64..256 keys, 88.6 instead of 86.0, B8 H32 S2048 D128 424 instead of 419.5; the loop left to the compiler 78.6, 87.1 and 421.7).
-// (kProbes: for tests.)
+// For the forward kernels, in as few instructions as can be: they have some twenty waits each, and how far their code is spread costs them
+// time.  B64 H32 S256 D128: the form above 82.9 us, this loop left to the compiler 78.6, as it is 77.8.  (kProbes: for tests.)
 template <uint32_t kProbes = kWaitProbes>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
   uint32_t ok;
@@ -110,9 +108,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const v
       : "memory");
   return ok != 0u;
 }
-// For a warp whose lanes run together, with one answer for all of them: the vote in the loop makes its branches uniform, and nothing follows it
-// (a vote on the lanes' answers behind the loop above: B256 H16 S256 D64, 64..256 keys, 87.8 us instead of 85.6, B200 H12 S128 22.4 instead of 21.9, B64 H16 S64
-// 8.87 instead of 8.69; the general kernel's waits, of 32 lanes too, measure the same either way).
+// For a warp whose lanes run together, with one answer for all of them: the vote in the loop makes its branches uniform, and none is needed
+// behind it.  The workers: B256 H16 S256 D64 (64..256 keys) 87.8 us with the loop above and a vote behind it, 85.6 with this one; the general
+// kernel is the same with either.
 template <uint32_t kProbes = kWaitProbes>
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
   uint32_t ok;
