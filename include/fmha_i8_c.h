@@ -106,7 +106,7 @@ int fmha_i8_sm100_infer_cross(void* stream, const float amax[5], const int desc5
  *                          every row: amax[4] = s_max, the FMHAParamI8 field the reference fills
  *                          (test_fmha_i8.cpp:152) and never reads (README.md:27; :82-102 of the script)
  * P is unsigned with 127 levels as in the study.  A row's scale is only known when all its keys have been seen: one
- * launch goes over them twice.  row_scratch: caller-owned device memory, 2 floats per query row of the slice
+ * launch goes over them twice (the static scale's with up to 128 keys once).  row_scratch: caller-owned device memory, 2 floats per query row of the slice
  * (8 * bh_count * seq_len_q bytes, 8-byte aligned), for the rows' statistics; its contents after the call are not specified (the
  * present kernel keeps the statistics on the chip and leaves it as it is).  Nothing is allocated.  Other arguments as in
  * fmha_i8_sm100_infer_cross; FMHA_I8_FLAG_UINT8_P is not accepted. */
