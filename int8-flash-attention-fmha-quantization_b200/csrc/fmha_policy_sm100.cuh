@@ -120,7 +120,7 @@ template <int D> constexpr size_t smem_bytes() { return 1024 + kWorkers * Cfg<D>
 // over the keys.  In two phases such units are bound by their chain of dependent steps, and an SM has two units only: with many of them two
 // launches of the forward kernels were faster.  us, those -> two phases -> this, B512 H16 S128 D64 110.5 -> 113.7 -> 84.0, with 64..128 keys 110.6
 // -> 116.8 -> 87.4, 16 query rows 102.9 -> 111.6 -> 82.1, 16384 units of S64 with one row 137.8 -> 147.0 -> 113.1, B512 H16 S128 D128 190 -> 139 -> 109.
-// (The exponentials left in tensor memory meanwhile, which spills nothing instead of 24 bytes: 92.4 for the first.  Both forms in one
+// (The exponentials left in tensor memory meanwhile, which spills nothing instead of some 30 bytes: 92.4 for the first.  Both forms in one
 // instance: the longer units lose 4 to 8 %.)
 // Sixteen scores to their exponentials, in place, and into the sums; a quarter of them on the multiply-add pipe.
 __device__ __forceinline__ void exps_in_place(uint32_t (&r)[16], const RowConsts& k, float2 (&sum)[2]) {
@@ -231,8 +231,8 @@ __device__ __forceinline__ void softmax_role(const FwdParams& p, Ctl* all, const
         pack_shares(r3, share, packed); tmem_st4(tS + 12, packed);
         tmem_wait_st();
         tc_fence_before();
+        mbar_arrive(smem_u32(&ctl->p_brief[chain]));
       }
-      if (chain < n) mbar_arrive(smem_u32(&ctl->p_brief[chain]));
     } else {
       // ---- phase 1: the row's maximum over all keys, as a biased integer (static: and the exp-sum, in terms of that of `ref`)
       int imax = INT_MIN;
@@ -536,7 +536,7 @@ __device__ __forceinline__ void issuer_role(const FwdParams& p, Ctl* all, const 
   const bool lead = elect_one();
   uint32_t fail = 0u, used = 0, groups = 0, uses0 = 0, uses1 = 0;      // places of the ring, and S, so far
   Ring<C::kBufs> s_set, p_set;
-  uint32_t briefs[kChains] = {};                                        // kBrief: units that had such a group
+  uint32_t briefs[kChains] = {};                                        // kBrief: units that had a first, a second group
   auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
     if (warp_wait(bar, parity, abort_flag)) return true;
     fail = code;

@@ -626,7 +626,7 @@ LARGE_SCALES = [0.0031, 0.077, 0.317, 0.931, 2.37, 3.13, 10.7, 49.3, 71.9, 1.3e4
 LARGE_SCALE_CALLS = {  # B, H, Sq, Sk, D -> the kernel that runs it
     (2, 3, 1, 704, 128): "KERNEL_FEW_ROWS", (2, 3, 3, 704, 64): "KERNEL_FEW_ROWS", (1, 3, 200, 1024, 128): "KERNEL_GENERAL",
     (8, 20, 256, 512, 128): "KERNEL_GENERAL", (2, 3, 70, 448, 64): "KERNEL_GENERAL", (40, 12, 256, 320, 64): "KERNEL_WORKERS",
-    (18, 16, 256, 640, 64): "KERNEL_WORKERS"}
+    (18, 16, 256, 640, 64): "KERNEL_WORKERS", (2, 3, 70, 128, 64): "KERNEL_GENERAL", (2, 3, 70, 128, 128): "KERNEL_GENERAL"}
 
 
 @pytest.mark.parametrize("c2", LARGE_SCALES)
